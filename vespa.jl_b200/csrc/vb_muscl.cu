@@ -23,7 +23,7 @@
 #include <cstring>
 
 #include "vb_internal.h"
-#include "vb_tma.cuh"
+#include "vb_physics.cuh"
 
 namespace vb {
 namespace {
@@ -114,7 +114,7 @@ __device__ __forceinline__ void hll5(const double L[5], const double R[5], doubl
 //  - primitives of the resulting U (_cons2prim_k!, muscl_grid.jl:23-34):
 //    prim = (rho, eint, vx, vy, vz), eint floored at small_rho.
 template <bool COPY, bool FILL>
-__global__ void __launch_bounds__(MB) k_muscl_prep(MusclGeom m, MusclFields U, double *U0, double *prim)
+__global__ void __launch_bounds__(MB) k_muscl_prep(MusclGeom m, MusclFields U, double *U0, double *prim, int *nonfinite)
 {
     const int64_t c[3] = {(int64_t)blockIdx.x * 32 + threadIdx.x % 32,
                           (int64_t)blockIdx.y * 8 + threadIdx.x / 32, (int64_t)blockIdx.z};
@@ -144,7 +144,9 @@ __global__ void __launch_bounds__(MB) k_muscl_prep(MusclGeom m, MusclFields U, d
     prim[2 * N + i] = vx;
     prim[3 * N + i] = vy;
     prim[4 * N + i] = vz;
-    prim[N + i] = jmax(u[4] / d - 0.5 * (vx * vx + vy * vy + vz * vz), m.small_rho);
+    const double e = jmax(u[4] / d - 0.5 * (vx * vx + vy * vy + vz * vz), m.small_rho);
+    prim[N + i] = e;
+    if (!isfinite(d + e + vx + vy + vz)) *nonfinite = 1;
 }
 
 // Tile of one CTA: TX x TY cells of one z-plane, one thread per cell column.
@@ -157,17 +159,88 @@ constexpr int FXN = (TX + 1) * TY;       // x faces of one plane tile
 constexpr int FYN = TX * (TY + 1);       // y faces of one plane tile
 constexpr size_t TILE_SMEM = sizeof(double) * (NSLOT * PS + 5 * FXN + 5 * FYN);
 
+// plm_pt of finite values: minmod3 is zero unless the three differences share
+// their sign bit (a zero among them gives zero either way), else the smallest
+// of them, added by predicated multiply-adds (half of it is exact, so the fused
+// form rounds as the product and sum do)
+__device__ __forceinline__ double plm_finite(double vm1, double v, double vp1, double th)
+{
+    const double a = (v - vm1) * th, b = (vp1 - v) * th, c = 0.5 * (vp1 - vm1);
+    const int ha = __double2hiint(a), hb = __double2hiint(b), hc = __double2hiint(c);
+    const bool on = ((ha ^ hb) | (ha ^ hc)) >= 0;
+    const double x = fabs(a) < fabs(b) ? a : b;
+    const bool lo = fabs(c) < fabs(x);
+    double w = v;
+    if (on && lo) w = __fma_rn(0.5, c, w);
+    if (on && !lo) w = __fma_rn(0.5, x, w);
+    return w;
+}
+
+// hll5 with its divisions as quot64 (one reciprocal of ap + am for the five
+// components) and root64; false, F untouched, unless every operand lies where
+// those round as `/` and sqrt do: densities, g p and ap + am positive within
+// 2^+-120, numerators zero or within 2^+-700 (a subnormal one counts as zero:
+// its quotient may be off by 2^-1074).
+__device__ __forceinline__ bool hll5_quot(const double L[5], const double R[5], double g, double gm1,
+                                          double F[5])
+{
+    const double h = 0.5;
+    const double rl = L[0], el = L[1], ul = L[2], vl = L[3], wl = L[4];
+    const double rr = R[0], er = R[1], ur = R[2], vr = R[3], wr = R[4];
+    const double pl = gm1 * rl * el, pr = gm1 * rr * er, gl = g * pl, gr = g * pr;
+    const double csl = root64(quot64(gl, rl, rcp64(rl))), csr = root64(quot64(gr, rr, rcp64(rr)));
+    const double lpl = ul + csl, nml = -(ul - csl), lpr = ur + csr, nmr = -(ur - csr);
+    const double sp = lpl > lpr ? lpl : lpr, sm = nml > nmr ? nml : nmr;
+    const double ap = sp > 0.0 ? sp : 0.0, am = sm > 0.0 ? sm : 0.0;
+    const double d = ap + am, y = rcp64(d), aa = ap * am;
+    const double etl = el + h * (ul * ul + vl * vl + wl * wl);
+    const double etr = er + h * (ur * ur + vr * vr + wr * wr);
+    const double l1 = rl * ul, l2 = rl * vl, l3 = rl * wl, l4 = rl * etl;
+    const double r1 = rr * ur, r2 = rr * vr, r3 = rr * wr, r4 = rr * etr;
+    double N[5];
+    N[0] = ap * l1 + am * r1 - aa * (rr - rl);
+    N[1] = ap * (l1 * ul + pl) + am * (r1 * ur + pr) - aa * (r1 - l1);
+    N[2] = ap * (l2 * ul) + am * (r2 * ur) - aa * (r2 - l2);
+    N[3] = ap * (l3 * ul) + am * (r3 * ur) - aa * (r3 - l3);
+    N[4] = ap * ((l4 + pl) * ul) + am * ((r4 + pr) * ur) - aa * (r4 - l4);
+    auto hw = [](double x) { return (unsigned)__double2hiint(x); };
+    const unsigned lo = __vimin3_u32(__vimin3_u32(hw(rl), hw(rr), hw(gl)), hw(gr), hw(d));
+    const unsigned hi = __vimax3_u32(__vimax3_u32(hw(rl), hw(rr), hw(gl)), hw(gr), hw(d));
+    unsigned nlo = 0xffffffffu, nhi = 0;
+#pragma unroll
+    for (int f = 0; f < 5; ++f) {
+        const unsigned n = hw(N[f]) & 0x7fffffffu;
+        nlo = umin(nlo, n - 1u);
+        nhi = umax(nhi, n);
+    }
+    if (!(lo >= 0x38700000u && hi < 0x47700000u && nlo >= 0x14300000u && nhi < 0x6bb00000u)) return false;
+#pragma unroll
+    for (int f = 0; f < 5; ++f) F[f] = quot64(N[f], d, y);
+    return true;
+}
+
 // HLL flux through one interface from the primitives of its four stencil
 // cells qm1, q0 | q1, q2 (field f of a cell at offset off[f]), in the
 // reference's flux-line form (_muscl_hll_kernel!, muscl.jl:181-215): the left
 // state is q0's right face, the right state is q1's left face taken as the
 // right face of the reversed stencil.  off[] lists (rho, eint, u_normal, t1,
-// t2); F comes back in that frame.
+// t2); F comes back in that frame.  finite: every primitive of the grid is.
 __device__ __forceinline__ void face_flux(const double *qm1, const double *q0, const double *q1,
                                           const double *q2, const int off[5], const MusclGeom &m,
-                                          double F[5])
+                                          bool finite, double F[5])
 {
     double L[5], R[5];
+    if (finite) {
+#pragma unroll
+        for (int f = 0; f < 5; ++f) {
+            const double a = qm1[off[f]], b = q0[off[f]], c = q1[off[f]], d = q2[off[f]];
+            L[f] = plm_finite(a, b, c, m.theta);
+            R[f] = plm_finite(d, c, b, m.theta);
+        }
+        L[0] = L[0] > m.small_rho ? L[0] : m.small_rho;
+        R[0] = R[0] > m.small_rho ? R[0] : m.small_rho;
+        if (hll5_quot(L, R, m.gamma, m.gamma - 1.0, F)) return;
+    }
 #pragma unroll
     for (int f = 0; f < 5; ++f) {
         const double a = qm1[off[f]], b = q0[off[f]], c = q1[off[f]], d = q2[off[f]];
@@ -204,7 +277,7 @@ __device__ __forceinline__ void load_plane(const MusclGeom &m, const double *__r
 template <int STAGE>
 __global__ void __launch_bounds__(NT, 2) k_muscl_tile(MusclGeom m, const double *__restrict__ prim,
                                                       MusclFields U, const double *__restrict__ U0,
-                                                      int kz)
+                                                      int kz, const int *nonfinite)
 {
     extern __shared__ __align__(16) double smem[];
     double *const ring = smem, *const fx = smem + NSLOT * PS, *const fy = fx + 5 * FXN;
@@ -214,6 +287,7 @@ __global__ void __launch_bounds__(NT, 2) k_muscl_tile(MusclGeom m, const double 
     const int64_t k0 = (int64_t)blockIdx.z * kz, k1 = k0 + kz < nz ? k0 + kz : nz;
     const int64_t x = x0 + tx, y = y0 + ty;
     const bool in = x < nx && y < ny;
+    const bool finite = *nonfinite == 0;
     const bool act_x = x >= ng && x < nx - ng, act_y = y >= ng && y < ny - ng;
     // a face between cells c and c + 1 along an axis of n cells is needed iff
     // one of the two is active; its stencil c - 1 .. c + 2 is then in the grid
@@ -229,7 +303,7 @@ __global__ void __launch_bounds__(NT, 2) k_muscl_tile(MusclGeom m, const double 
     double flo[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // z flux through this cell's lower face
     if (in && face_ok(k0 - 1, nz))
         face_flux(slot(k0 - 2) + own, slot(k0 - 1) + own, slot(k0) + own, slot(k0 + 1) + own, zoff,
-                  m, flo);
+                  m, finite, flo);
     __syncthreads();  // slot of plane k0 - 2 is free
     if (k0 + 3 <= k1 + 1) load_plane(m, prim, slot(k0 + 3), x0, y0, k0 + 3);
     cp_async_commit();
@@ -241,7 +315,7 @@ __global__ void __launch_bounds__(NT, 2) k_muscl_tile(MusclGeom m, const double 
         double fhi[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
         if (in && face_ok(k, nz))
             face_flux(slot(k - 1) + own, pk + own, slot(k + 1) + own, slot(k + 2) + own, zoff, m,
-                      fhi);
+                      finite, fhi);
         // the plane's x faces (33 per row) and y faces (9 per column), spread
         // over the CTA
         for (int it = t; it < FXN + FYN; it += NT) {
@@ -270,7 +344,7 @@ __global__ void __launch_bounds__(NT, 2) k_muscl_tile(MusclGeom m, const double 
             }
             if (ok) {
                 double F[5];
-                face_flux(c0 - st, c0, c0 + st, c0 + 2 * st, off, m, F);
+                face_flux(c0 - st, c0, c0 + st, c0 + 2 * st, off, m, finite, F);
 #pragma unroll
                 for (int f = 0; f < 5; ++f) out[f * ostr] = F[f];
             }
@@ -331,6 +405,7 @@ struct vb_muscl {
     double *U = nullptr;     // owned state, 5 x N
     double *U0 = nullptr;    // step-start copy
     double *prim = nullptr;  // primitives of the stage input
+    int *nonfinite = nullptr;  // set by a stage's preparation pass: a primitive is not finite
     int kz = 1;              // z-planes per CTA of the tile pass (fixed by dims)
 };
 
@@ -382,18 +457,19 @@ int queue_step(vb_muscl *mu, const vb::MusclFields &F, const vb_muscl_params *p)
     const dim3 pgrid((unsigned)((m.n[0] + 31) / 32), (unsigned)((m.n[1] + 7) / 8), (unsigned)m.n[2]);
     const int64_t gx = (m.n[0] + vb::TX - 1) / vb::TX, gy = (m.n[1] + vb::TY - 1) / vb::TY;
     const int kz = mu->kz;
+    VB_CUDA(cudaMemsetAsync(mu->nonfinite, 0, sizeof(int), s));
     const dim3 tgrid((unsigned)gx, (unsigned)gy, (unsigned)((m.n[2] + kz - 1) / kz));
     if (p->bc == VB_MUSCL_BC_PERIODIC)
-        vb::k_muscl_prep<true, true><<<pgrid, vb::MB, 0, s>>>(m, F, mu->U0, mu->prim);
+        vb::k_muscl_prep<true, true><<<pgrid, vb::MB, 0, s>>>(m, F, mu->U0, mu->prim, mu->nonfinite);
     else
-        vb::k_muscl_prep<true, false><<<pgrid, vb::MB, 0, s>>>(m, F, mu->U0, mu->prim);
-    vb::k_muscl_tile<1><<<tgrid, vb::NT, vb::TILE_SMEM, s>>>(m, mu->prim, F, mu->U0, kz);
+        vb::k_muscl_prep<true, false><<<pgrid, vb::MB, 0, s>>>(m, F, mu->U0, mu->prim, mu->nonfinite);
+    vb::k_muscl_tile<1><<<tgrid, vb::NT, vb::TILE_SMEM, s>>>(m, mu->prim, F, mu->U0, kz, mu->nonfinite);
     VB_CHECK_LAUNCH(mu->ctx, 2);
     if (p->bc == VB_MUSCL_BC_PERIODIC)
-        vb::k_muscl_prep<false, true><<<pgrid, vb::MB, 0, s>>>(m, F, mu->U0, mu->prim);
+        vb::k_muscl_prep<false, true><<<pgrid, vb::MB, 0, s>>>(m, F, mu->U0, mu->prim, mu->nonfinite);
     else
-        vb::k_muscl_prep<false, false><<<pgrid, vb::MB, 0, s>>>(m, F, mu->U0, mu->prim);
-    vb::k_muscl_tile<2><<<tgrid, vb::NT, vb::TILE_SMEM, s>>>(m, mu->prim, F, mu->U0, kz);
+        vb::k_muscl_prep<false, false><<<pgrid, vb::MB, 0, s>>>(m, F, mu->U0, mu->prim, mu->nonfinite);
+    vb::k_muscl_tile<2><<<tgrid, vb::NT, vb::TILE_SMEM, s>>>(m, mu->prim, F, mu->U0, kz, mu->nonfinite);
     VB_CHECK_LAUNCH(mu->ctx, 2);
     return VB_OK;
 }
@@ -447,12 +523,14 @@ int vb_muscl_create(vb_ctx *ctx, const int64_t dims[3], int32_t ng, vb_muscl **o
     cudaError_t e = cudaMalloc(&mu->U, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&mu->U0, bytes);
     if (e == cudaSuccess) e = cudaMalloc(&mu->prim, bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&mu->nonfinite, sizeof(int));
     if (e == cudaSuccess) e = cudaMemsetAsync(mu->U, 0, bytes, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         cudaFree(mu->U);
         cudaFree(mu->U0);
         cudaFree(mu->prim);
+        cudaFree(mu->nonfinite);
         delete mu;
         return fail(e == cudaErrorMemoryAllocation ? VB_ENOMEM : VB_ECUDA,
                     std::string("muscl allocation: ") + cudaGetErrorString(e));
@@ -469,6 +547,7 @@ int vb_muscl_destroy(vb_muscl *mu)
     cudaFree(mu->U);
     cudaFree(mu->U0);
     cudaFree(mu->prim);
+    cudaFree(mu->nonfinite);
     delete mu;
     return VB_OK;
 }

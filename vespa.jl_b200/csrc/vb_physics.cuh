@@ -69,8 +69,189 @@ __device__ __forceinline__ T total_energy(const T W[5], T g)
     return W[4] / (g - T(1)) + T(0.5) * W[0] * (W[1] * W[1] + W[2] * W[2] + W[3] * W[3]);
 }
 
+// Float64 quotients and square roots without the range branch that the `/` and
+// sqrt operators carry, so that independent ones overlap and share reciprocals.
+// Valid for operands well inside the exponent range, which the caller checks
+// (see hllc_frame); there they round as `/` and sqrt do:
+//   rcp64: Newton-Raphson, y <- y + y (1 - b y), from the hardware's
+//     approximation to within an ulp of 1/b;
+//   quot64: a y corrected by its exact residual (P. Markstein, IBM J. Res. Dev.
+//     34(1), 1990);
+//   root64: R. E. Goldschmidt's coupled iteration for sqrt x and 1 / (2 sqrt x),
+//     and the same kind of residual correction.
+// The corrected value is off the exact one by at most 2^-104 of it before its
+// rounding, so it could go wrong only where the exact one lies that close to a
+// midpoint between two numbers (one operand pair in 2^50); of 10^10 quotients
+// built to lie as close to one as any can, none did.
+__device__ __forceinline__ double rcp64(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    return y;
+}
+__device__ __forceinline__ double quot64(double a, double b, double y)
+{
+    const double q = __dmul_rn(a, y);
+    return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+__device__ __forceinline__ double root64(double x)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = __dmul_rn(x, y), h = __dmul_rn(0.5, y);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const double r = __fma_rn(-g, h, 0.5);
+        g = __fma_rn(g, r, g);
+        h = __fma_rn(h, r, h);
+    }
+    return __fma_rn(__fma_rn(-g, g, x), h, g);
+}
+// a / b in that form where both are positive and within 1e+-30
+__device__ __forceinline__ double div64(double a, double b)
+{
+    return a > 1e-30 && a < 1e30 && b > 1e-30 && b < 1e30 ? quot64(a, b, rcp64(b)) : a / b;
+}
+// 1 / (gamma - 1) for hllc_frame; NaN (every solve then takes the general form)
+// when gamma - 1 is out of quot64's range
+__device__ __forceinline__ double inv_gamma1(double gamma)
+{
+    const double d = gamma - 1.0;
+    return d > 1e-30 && d < 1e30 ? 1.0 / d : __longlong_as_double(0x7ff8000000000000ll);
+}
+
+// hllc_flux (src/riemann.jl:33-66 with euler_flux, 9-20, and _hllc_star, 69-88)
+// in the face-normal frame (rho, u_n, u_t1, u_t2, p) of both states and of F.
+// |v|^2 is summed as the reference does, (vx^2 + vy^2) + vz^2: for an x or y
+// face with t1 the other of the two, that is (n + t1) + t2 (a sum of two
+// commutes); Z, a z face: n last.  Every operation rounds as the reference's.
+// ig1: 1 / (g - 1).  Only the selected side's conserved state and physical flux
+// are needed: SL >= 0 -> FL;  SR <= 0 -> FR;  else the star flux of the side
+// picked by the sign of S*.
+template <bool Z>
+__device__ __forceinline__ void hllc_frame_any(const double L[5], const double R[5], double g,
+                                               double F[5])
+{
+    const double cL = sqrt(g * L[4] / L[0]);
+    const double cR = sqrt(g * R[4] / R[0]);
+    const double SL = fmin(L[1] - cL, R[1] - cR);
+    const double SR = fmax(L[1] + cL, R[1] + cR);
+    bool left, star;
+    double SK, Ss = 0.0;
+    if (SL >= 0.0) {
+        left = true; SK = SL; star = false;
+    } else if (SR <= 0.0) {
+        left = false; SK = SR; star = false;
+    } else {
+        Ss = (R[4] - L[4] + L[0] * L[1] * (SL - L[1]) - R[0] * R[1] * (SR - R[1])) /
+             (L[0] * (SL - L[1]) - R[0] * (SR - R[1]));
+        left = Ss >= 0.0;
+        SK = left ? SL : SR;
+        star = true;
+    }
+    // value selects (not a pointer to one side) keep both states in registers
+    const double rho = left ? L[0] : R[0], un = left ? L[1] : R[1];
+    const double u1 = left ? L[2] : R[2], u2 = left ? L[3] : R[3], p = left ? L[4] : R[4];
+    const double v2 = Z ? u1 * u1 + u2 * u2 + un * un : un * un + u1 * u1 + u2 * u2;
+    const double E = p / (g - 1.0) + 0.5 * rho * v2;
+    const double mn = rho * un, m1 = rho * u1, m2 = rho * u2;
+    // euler_flux; the +0 on tangential momentum is omitted (it only changes
+    // the sign of an exact zero)
+    F[0] = mn;
+    F[1] = mn * un + p;
+    F[2] = m1 * un;
+    F[3] = m2 * un;
+    F[4] = (E + p) * un;
+    if (!star) return;
+    // _hllc_star: F* = F + SK (U* - U)
+    const double factor = rho * (SK - un) / (SK - Ss);
+    const double Es = E / rho + (Ss - un) * (Ss + p / (rho * (SK - un)));
+    F[0] = F[0] + SK * (factor - rho);
+    F[1] = F[1] + SK * (factor * Ss - mn);
+    F[2] = F[2] + SK * (factor * u1 - m1);
+    F[3] = F[3] + SK * (factor * u2 - m2);
+    F[4] = F[4] + SK * (factor * Es - E);
+}
+
+// Whether the operands of an HLLC solve's quotients and roots lie where quot64
+// and root64 round as `/` and sqrt do, by their high words: densities and
+// pressures (positive) and the denominators D, d, q within 2^+-120, E below
+// 2^120 (it is at least p / (g - 1)), N zero or above 2^-700.  A NaN fails.
+__device__ __forceinline__ bool hllc_operands_ok(const double L[5], const double R[5], double D,
+                                                 double d, double q, double E, double N)
+{
+    const unsigned hD = __double2hiint(D) & 0x7fffffff, hd = __double2hiint(d) & 0x7fffffff;
+    const unsigned hq = __double2hiint(q) & 0x7fffffff, hN = __double2hiint(N) & 0x7fffffff;
+    const unsigned h0 = __double2hiint(L[0]), h1 = __double2hiint(R[0]);
+    const unsigned h2 = __double2hiint(L[4]), h3 = __double2hiint(R[4]);
+    const unsigned lo = __vimin3_u32(__vimin3_u32(h0, h1, h2), __vimin3_u32(h3, hD, hd), hq);
+    const unsigned hi = __vimax3_u32(__vimax3_u32(h0, h1, h2), __vimax3_u32(h3, hD, hd),
+                                     umax(hq, (unsigned)__double2hiint(E)));
+    return lo >= 0x38700000u && hi < 0x47700000u && (hN >= 0x14300000u || N == 0.0);
+}
+
+template <bool Z>
+__device__ __forceinline__ void hllc_frame(const double L[5], const double R[5], double g,
+                                           double ig1, double F[5])
+{
+    const double yL = rcp64(L[0]), yR = rcp64(R[0]);
+    const double cL = root64(quot64(g * L[4], L[0], yL));
+    const double cR = root64(quot64(g * R[4], R[0], yR));
+    const double lL = L[1] - cL, lR = R[1] - cR, rL = L[1] + cL, rR = R[1] + cR;
+    const double SL = lL < lR ? lL : lR, SR = rL > rR ? rL : rR;
+    const double dL = SL - L[1], dR = SR - R[1];
+    const double N = R[4] - L[4] + L[0] * L[1] * dL - R[0] * R[1] * dR;
+    const double D = L[0] * dL - R[0] * dR;
+    const double Ss = quot64(N, D, rcp64(D));
+    const bool supL = SL >= 0.0, supR = SR <= 0.0;
+    const bool left = supL || (!supR && Ss >= 0.0);
+    const double SK = left ? SL : SR;
+    const double rho = left ? L[0] : R[0], un = left ? L[1] : R[1], y = left ? yL : yR;
+    const double u1 = left ? L[2] : R[2], u2 = left ? L[3] : R[3], p = left ? L[4] : R[4];
+    const double v2 = Z ? u1 * u1 + u2 * u2 + un * un : un * un + u1 * u1 + u2 * u2;
+    const double E = quot64(p, g - 1.0, ig1) + 0.5 * rho * v2;
+    const double mn = rho * un, m1 = rho * u1, m2 = rho * u2;
+    const double d = SK - Ss, q = rho * (SK - un);
+    if (!hllc_operands_ok(L, R, D, d, q, E, N)) {
+        hllc_frame_any<Z>(L, R, g, F);
+        return;
+    }
+    F[0] = mn;
+    F[1] = mn * un + p;
+    F[2] = m1 * un;
+    F[3] = m2 * un;
+    F[4] = (E + p) * un;
+    if (supL || supR) return;
+    const double factor = quot64(q, d, rcp64(d));
+    const double Es = quot64(E, rho, y) + (Ss - un) * (Ss + quot64(p, q, rcp64(q)));
+    F[0] = F[0] + SK * (factor - rho);
+    F[1] = F[1] + SK * (factor * Ss - mn);
+    F[2] = F[2] + SK * (factor * u1 - m1);
+    F[3] = F[3] + SK * (factor * u2 - m2);
+    F[4] = F[4] + SK * (factor * Es - E);
+}
+
+// The same by components: DIM is the 1-based face-normal axis.
+template <int DIM>
+__device__ __forceinline__ void hllc_flux64(const double WL[5], const double WR[5], double g,
+                                            double ig1, double F[5])
+{
+    constexpr int t1 = DIM == 1 ? 2 : 1, t2 = DIM == 3 ? 2 : 3;
+    const double L[5] = {WL[0], WL[DIM], WL[t1], WL[t2], WL[4]};
+    const double R[5] = {WR[0], WR[DIM], WR[t1], WR[t2], WR[4]};
+    double f[5];
+    hllc_frame<DIM == 3>(L, R, g, ig1, f);
+    F[0] = f[0];
+    F[DIM] = f[1];
+    F[t1] = f[2];
+    F[t2] = f[3];
+    F[4] = f[4];
+}
+
 // hllc_flux, src/riemann.jl:33-66 with euler_flux (9-20) and _hllc_star
-// (69-88).  DIM is the 1-based face-normal axis.
+// (69-88), in the precision T.  DIM is the 1-based face-normal axis.
 template <typename T, int DIM>
 __device__ __forceinline__ void hllc_flux(const T WL[5], const T WR[5], double gamma, T F[5])
 {
@@ -133,12 +314,12 @@ __device__ __forceinline__ void hllc_flux(const T WL[5], const T WR[5], double g
     for (int k = 0; k < 5; ++k) F[k] = Fk[k] + SK * (Us[k] - Uk[k]);
 }
 
-// PLM face value w + h*s (src/driver.jl:227-233).  In float the product-add
-// is an explicit fused multiply-add so every call site rounds identically (a
-// face evaluated from both neighbouring cells must give one value); in the
-// float64 unit (-fmad=false) it is a separately rounded product and sum, as
-// in the reference.
-__device__ __forceinline__ double face_val(double w, double h, double s) { return w + h * s; }
+// PLM face value w + h*s (src/driver.jl:227-233), h = +-0.5.  In float the
+// product-add is an explicit fused multiply-add so every call site rounds
+// identically (a face evaluated from both neighbouring cells must give one
+// value); in float64 the product by a power of two is exact, so the fused form
+// rounds as the reference's separate product and sum do.
+__device__ __forceinline__ double face_val(double w, double h, double s) { return __fma_rn(h, s, w); }
 __device__ __forceinline__ float face_val(float w, float h, float s) { return __fmaf_rn(h, s, w); }
 
 // The same Riemann solve behind one call for every face of the cell-centric
