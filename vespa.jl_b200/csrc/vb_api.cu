@@ -5,11 +5,13 @@
 // the device, and error reporting.  No C++ exception crosses the ABI.
 #include <cudaTypedefs.h>
 
+#include <algorithm>
 #include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <new>
@@ -202,47 +204,88 @@ int encode_maps(vb::TiledMaps *m, const double *base, const vb::Geom &g)
     return rc;
 }
 
-int default_kz(const vb::Geom &g)
-{
-    const int64_t n = vb::march_extent(g);
-    return n >= 64 ? 32 : (int)((n + 1) / 2);
-}
-
 // Column tiles (3D) or row segments (2D) per chunk of the marching axis.
 int64_t tiles_per_chunk(const vb::Geom &g)
 {
-    return g.nd == 2 ? g.n[0] / 256 : (g.n[0] / 16) * (g.n[1] / 16);
+    return g.nd == 2 ? (g.n[0] + 255) / 256 : ((g.n[0] + 15) / 16) * ((g.n[1] + 15) / 16);
 }
 
-// The automatic kernel choice takes a tiled kernel only when it yields enough
-// work items for the persistent grid (two blocks per SM on 148 SMs, with a
-// chunk of at least 8 planes/rows); small grids keep the cell-centric kernel.
-bool tiled_auto(const vb::Geom &g)
+// The automatic kernel choice.  3D: the tiled kernels once the cell-centric one
+// (256 cells a block, one block per SM) needs a second wave on 148 SMs: at 32^3
+// the two are level (mixed 25.5 and 24.5 us a step, float64 30 and 41), at 48^3
+// the tiles win (36 and 30, 75 and 54).  2D mixed: when a chunk of at least 8
+// rows gives every persistent block an item.  2D float64: the marching kernel
+// against the plane kernel runs 93 % at 1024^2, level at 2048^2 and 110 % at
+// 4096^2, so from the size on where 32-row chunks give each block four items.
+bool tiled_auto(const vb::Geom &g, int precision)
 {
-    if (!vb::tiled_supported(g)) return false;
-    const int64_t ext = vb::march_extent(g);
-    return tiles_per_chunk(g) * ((ext + 7) / 8) >= 296;
+    if (!vb::tiled_any(g, precision)) return false;
+    if (g.nd == 3) return g.ncell > 148 * 256;
+    if (precision == VB_FP64) return tiles_per_chunk(g) * ((vb::march_extent(g) + 31) / 32) >= 4 * 296;
+    return tiles_per_chunk(g) * ((vb::march_extent(g) + 7) / 8) >= 296;
 }
 
-// Default chunk of a single grid.  3D: the largest of 48, 40, 32, 24, 16 that
-// gives two work items per persistent block (long chunks amortise the 4-plane
-// prologue of an item), else the largest giving one (measured on B200, 128^3
-// to 384^3: within 2 % of the best chunk); 2D: the largest of 32, 16 giving
-// two.  Otherwise 8.
-int grid_default_kz(const vb::Geom &g)
+QueueSpan::QueueSpan(double p) : prologue(p), slot(SLOTS, 0.0) {}
+void QueueSpan::add(int planes, int64_t count)
 {
-    const int64_t ext = vb::march_extent(g);
-    const int64_t tiles = tiles_per_chunk(g);
-    auto items = [&](int kz) { return tiles * ((ext + kz - 1) / kz); };
-    if (g.nd == 3) {
-        for (int64_t need : {592, 296})
-            for (int kz : {48, 40, 32, 24, 16})
-                if (kz <= ext && items(kz) >= need) return kz;
-    } else {
-        for (int kz : {32, 16})
-            if (kz <= ext && items(kz) >= 592) return kz;
+    for (int64_t i = 0; i < count; ++i) {
+        std::pop_heap(slot.begin(), slot.end(), std::greater<double>());
+        slot.back() += planes + prologue;
+        end = std::max(end, slot.back());
+        std::push_heap(slot.begin(), slot.end(), std::greater<double>());
     }
-    return (int)(ext >= 8 ? 8 : ext);
+}
+double tile_prologue(int precision) { return precision == VB_MIXED ? 4.0 : 1.5; }
+
+// Chunk and queue shape a single grid starts from.  3D, with q planes per
+// resident block (296 of them): up to 12, uniform chunks of one round of items;
+// from 24 and 48 on, tapered chunks of that size; between, the shortest of 8 or
+// 16 uniform and 16 tapered by a count of rounds (an item costs its planes plus
+// a prologue).  Against the best of 2 .. 128 planes, uniform and tapered, this
+// is within 3 % from 48^3 to 256^3 and on 150 x 90 x 75 and 99 x 101 x 103, in
+// both precisions; the largest chunk giving every block two items, used before
+// in float64, lost 20-40 % below 128^3.  2D: the largest of 32, 16 rows giving
+// two items per block, else 8.
+int grid_default_kz(const vb::Geom &g, int precision, bool *taper)
+{
+    const int64_t ext = vb::march_extent(g), tiles = tiles_per_chunk(g);
+    *taper = precision == VB_MIXED;
+    if (g.nd != 3) {
+        for (int kz : {32, 16})
+            if (kz <= ext && tiles * ((ext + kz - 1) / kz) >= 592) return kz;
+        return (int)(ext >= 8 ? 8 : ext);
+    }
+    constexpr int64_t SLOTS = QueueSpan::SLOTS;
+    const double q = (double)tiles * ext / SLOTS;
+    *taper = false;
+    if (q <= 12.0) {
+        const int64_t nch = std::max<int64_t>(1, std::min<int64_t>(ext, SLOTS / tiles));
+        return (int)((ext + nch - 1) / nch);
+    }
+    *taper = true;
+    if (q >= 24.0) return q >= 48.0 && ext >= 48 ? 48 : ext >= 24 ? 24 : (int)ext;
+    const double prologue = tile_prologue(precision);
+    int best_kz = 8;
+    double best = INFINITY;
+    for (int c = 0; c < 3; ++c) {
+        const int kz = c == 0 ? 8 : 16;
+        if (kz > ext) continue;
+        int nchu = 0;
+        const int nch = vb::chunk_count((int)ext, kz, c == 2, &nchu);
+        QueueSpan span(prologue);
+        for (int j = 0; j < nch; ++j) {
+            int k0, k1;
+            vb::chunk_span((int)ext, kz, nchu, j, k0, k1);
+            span.add(k1 - k0, tiles);
+        }
+        const double end = span.end;
+        if (end < best) {
+            best = end;
+            best_kz = kz;
+            *taper = c == 2;
+        }
+    }
+    return best_kz;
 }
 
 // Geometry of a descriptor, validated as Problem is (src/problem.jl:39-46),
@@ -323,11 +366,11 @@ vb::BoxDesc make_box(const vb::TiledMaps &mU, const vb::TiledMaps &mU1, const vb
     b.ctrl = ctrl;
     b.kz = kz;
     if (g.nd == 2) {
-        b.ntx = (int)(g.n[0] / 256);
+        b.ntx = (int)tiles_per_chunk(g);
         b.ntiles = b.ntx;
     } else {
-        b.ntx = (int)(g.n[0] / 16);
-        b.ntiles = (int)((g.n[0] / 16) * (g.n[1] / 16));
+        b.ntx = (int)((g.n[0] + 15) / 16);
+        b.ntiles = (int)tiles_per_chunk(g);
         b.nch = vb::chunk_count((int)g.n[2], kz, taper, &b.nchu);
     }
     b.item0 = item0;
@@ -336,9 +379,9 @@ vb::BoxDesc make_box(const vb::TiledMaps &mU, const vb::TiledMaps &mU1, const vb
 
 int64_t box_items(const vb::Geom &g, int kz, bool taper)
 {
-    if (g.nd == 2) return (g.n[0] / 256) * ((g.n[1] + kz - 1) / kz);
+    if (g.nd == 2) return tiles_per_chunk(g) * ((g.n[1] + kz - 1) / kz);
     int nchu = 0;
-    return (g.n[0] / 16) * (g.n[1] / 16) * vb::chunk_count((int)g.n[2], kz, taper, &nchu);
+    return tiles_per_chunk(g) * vb::chunk_count((int)g.n[2], kz, taper, &nchu);
 }
 
 }  // namespace detail
@@ -350,13 +393,13 @@ using vb::detail::box_items;
 using vb::detail::encode_maps;
 using vb::detail::make_box;
 
-// Whether the grid's 3D work queue uses tapered z chunks (VB_OPT_TILE_TAPER;
-// by default single VB_MIXED grids do).
+// Whether the grid's 3D work queue uses tapered z chunks: VB_OPT_TILE_TAPER,
+// else the autotuner's choice, else what the grid started with.
 bool grid_taper(const vb_grid *gr)
 {
     if (gr->taper >= 0) return gr->taper != 0;
     if (gr->taper_tuned >= 0) return gr->taper_tuned != 0;
-    return gr->precision == VB_MIXED;
+    return gr->taper_start;
 }
 
 // Refresh the grid's box descriptor after kz, the taper (or the maps) changed.
@@ -465,7 +508,7 @@ constexpr int64_t GRAPH_STEPS = 8;
 uint64_t graph_key(const vb_grid *gr)
 {
     return (gr->tiled ? 1u : 0u) | (gr->bflux_on ? 2u : 0u) | (grid_taper(gr) ? 4u : 0u) |
-           (gr->bflux_interior ? 8u : 0u) | ((uint64_t)gr->kz << 4);
+           (gr->bflux_interior ? 8u : 0u) | ((uint64_t)gr->kz << 5);
 }
 
 // Capture GRAPH_STEPS steps into the grid's graph for its current configuration.
@@ -521,12 +564,12 @@ int queue_steps(vb_grid *gr, int64_t count)
     return VB_OK;
 }
 
-// Host-side write of control fields (stream-ordered through a tiny copy).
+// Host-side write of control fields, queued on the stream: whoever writes the
+// pinned mirror next reads the block first (pull_ctrl), which waits for this.
 int push_ctrl(vb_grid *gr)
 {
     VB_CUDA(cudaMemcpyAsync(gr->ctrl, gr->hctrl, sizeof(vb::Ctrl), cudaMemcpyHostToDevice,
                             gr->ctx->stream));
-    VB_CUDA(cudaStreamSynchronize(gr->ctx->stream));
     return VB_OK;
 }
 
@@ -693,8 +736,9 @@ int vb_hllc_faces(vb_ctx *ctx, int64_t nf, const double *WL, const double *WR,
     if (nf < 0) return fail(VB_EINVAL, "nf < 0");
     if (nf == 0) return VB_OK;  // the reference returns F untouched for nf == 0
     if (!WL || !WR || !axis || !F) return fail(VB_EINVAL, "null buffer");
-    for (int64_t f = 0; f < nf; ++f)
-        if (axis[f] < 1 || axis[f] > 3) return fail(VB_EINVAL, "axis entries must be 1, 2 or 3");
+    unsigned bad = 0;  // no early exit: the loop vectorises
+    for (int64_t f = 0; f < nf; ++f) bad |= (unsigned)(axis[f] - 1) > 2u;
+    if (bad) return fail(VB_EINVAL, "axis entries must be 1, 2 or 3");
     const size_t bw = sizeof(double) * 5 * (size_t)nf;
     const size_t ba = sizeof(int32_t) * (size_t)nf;
     const size_t need = 3 * bw + ((ba + 255) & ~(size_t)255);
@@ -756,15 +800,17 @@ int vb_grid_create(vb_ctx *ctx, const vb_problem_desc *d, int precision, vb_grid
         std::string m = g_err;
         return cleanup(rc, m);
     }
-    if (vb::tiled_supported(g)) {
-        rc = encode_maps(&gr->maps_U, gr->U, g);
-        if (!rc) rc = encode_maps(&gr->maps_U1, gr->U1, g);
+    if (vb::tiled_any(g, precision)) {
+        if (vb::tiled_supported(g) || precision == VB_MIXED) {  // the TMA kernels' descriptors
+            rc = encode_maps(&gr->maps_U, gr->U, g);
+            if (!rc) rc = encode_maps(&gr->maps_U1, gr->U1, g);
+        }
         if (rc) {
             std::string m = g_err;
             return cleanup(rc, m);
         }
-        gr->tiled = vb::detail::tiled_auto(g);
-        gr->kz = vb::detail::grid_default_kz(g);
+        gr->tiled = vb::detail::tiled_auto(g, precision);
+        gr->kz = vb::detail::grid_default_kz(g, precision, &gr->taper_start);
         std::lock_guard<std::mutex> lk(g_tune_mu);
         const std::string key = tune_key(ctx->device, g, precision);
         auto it = g_tune_kz.find(key);
@@ -870,19 +916,16 @@ int vb_grid_set_option(vb_grid *gr, int option, int64_t value)
         if (value == VB_KERNEL_CELL) {
             gr->tiled = false;
         } else if (value == VB_KERNEL_AUTO || value == VB_KERNEL_TILED) {
-            if (!vb::tiled_supported(gr->g)) {
-                if (value == VB_KERNEL_TILED)
-                    return fail(VB_ENOTSUP, "tiled kernels need a 3D grid with nx, ny multiples of "
-                                            "16 or a 2D grid with nx a multiple of 256");
-                gr->tiled = false;
-                return VB_OK;
-            }
-            if (!gr->maps_U.in_int.opaque[0] && !gr->maps_U.in_int.opaque[1]) {
+            if (value == VB_KERNEL_TILED && !vb::tiled_supported(gr->g))
+                return fail(VB_ENOTSUP, "tiled kernels need a 3D grid with nx, ny multiples of "
+                                        "16 or a 2D grid with nx a multiple of 256");
+            if (vb::tiled_supported(gr->g) && !gr->maps_U.in_int.opaque[0] &&
+                !gr->maps_U.in_int.opaque[1]) {
                 int rc = encode_maps(&gr->maps_U, gr->U, gr->g);
                 if (!rc) rc = encode_maps(&gr->maps_U1, gr->U1, gr->g);
                 if (rc) return rc;
             }
-            gr->tiled = value == VB_KERNEL_TILED || vb::detail::tiled_auto(gr->g);
+            gr->tiled = value == VB_KERNEL_TILED || vb::detail::tiled_auto(gr->g, gr->precision);
         } else {
             return fail(VB_EINVAL, "unknown kernel selector");
         }
@@ -891,6 +934,7 @@ int vb_grid_set_option(vb_grid *gr, int option, int64_t value)
         if (value < 1 || value > vb::march_extent(gr->g))
             return fail(VB_EINVAL, "the chunk must be in 1..nz (3D) or 1..ny (2D)");
         gr->kz = (int)value;
+        gr->taper_start = gr->precision == VB_MIXED;
         return VB_OK;
     case VB_OPT_TILE_TAPER:
         if (value < -1 || value > 1) return fail(VB_EINVAL, "taper must be -1 (auto), 0 or 1");
@@ -1022,7 +1066,7 @@ int vb_grid_set_zwindow(vb_grid *gr, int64_t zw0, int64_t zw1, int zcls0, double
 {
     if (!gr) return fail(VB_EINVAL, "null grid");
     vb::Geom &g = gr->g;
-    if (g.nd != 3 || !gr->tiled)
+    if (!vb::tiled3d_supported(g) || !gr->tiled)
         return fail(VB_ENOTSUP, "z windows need a 3D grid on the tiled kernel");
     if (!(zw0 >= 0 && zw0 < zw1 && zw1 <= g.n[2])) return fail(VB_EINVAL, "need 0 <= zw0 < zw1 <= nz");
     if (zcls0 < -1 || zcls0 > 2) return fail(VB_EINVAL, "zcls0 must be -1, 0, 1 or 2");
@@ -1172,11 +1216,14 @@ int vb_evolve(vb_grid *gr, double tfinal, int64_t max_steps, double *t, int64_t 
     if (rc) return rc;
     rc = ensure_cfl(gr);
     if (rc) return rc;
-    // chunks of steps between host checks of the control block
+    // chunks of steps between host checks of the control block, none queued
+    // beyond the step budget
     int64_t chunk = 8;
     int status = VB_OK;
     for (;;) {
-        rc = queue_steps(gr, chunk);
+        const long long left = gr->hctrl->step_limit - gr->hctrl->step;
+        if (left <= 0) break;
+        rc = queue_steps(gr, chunk < left ? chunk : left);
         if (rc) return rc;
         rc = pull_ctrl(gr);
         if (rc) return rc;

@@ -3,11 +3,13 @@
 #pragma once
 
 #include <string>
+#include <vector>
 
 #include <nvtx3/nvToolsExt.h>
 
 #include "../../include/vespa_b200.h"
 #include "vb_launch.h"
+
 
 struct vb_ctx {
     int device = 0;
@@ -43,7 +45,9 @@ struct vb_grid {
     vb::BoxDesc box{};                  // the tiled kernels' box descriptor (passed by value)
     int box_kz = 0;                     // kz the descriptor was written with
     int taper = -1;                     // tapered z chunks: -1 auto, 0 off, 1 on
-    int taper_tuned = -1;               // auto: the autotuner's choice (-1: none, VB_MIXED tapers)
+    int taper_tuned = -1;               // auto: the autotuner's choice (-1: none)
+    bool taper_start = false;           // untuned: what goes with the starting chunk; a caller's
+                                        // own chunk tapers on VB_MIXED grids
     int box_taper = -1;                 // taper the descriptor was written with
     // CUDA graph of GRAPH_STEPS steps (finalize + RK2), replayed by the step loop
     cudaGraphExec_t gexec = nullptr;
@@ -69,11 +73,21 @@ int encode_maps(TiledMaps *m, const double *base, const Geom &g);
 BoxDesc make_box(const TiledMaps &mU, const TiledMaps &mU1, const Geom &g, double *U, double *U1,
                  Ctrl *ctrl, int kz, int item0, bool taper = false);
 int64_t box_items(const Geom &g, int kz, bool taper = false);
-// default z-chunk of a tiled box (batches)
-int default_kz(const Geom &g);
+// Length of a tiled 3D launch in planes: work items (their planes plus a
+// prologue, tile_prologue) taken in queue order by the slot (resident block)
+// that is free first.
+struct QueueSpan {
+    static constexpr int SLOTS = 296;
+    double prologue, end = 0.0;
+    std::vector<double> slot;
+    explicit QueueSpan(double prologue);
+    void add(int planes, int64_t count);
+};
+double tile_prologue(int precision);
 // automatic kernel choice and default chunk of a single grid
-bool tiled_auto(const Geom &g);
-int grid_default_kz(const Geom &g);
+bool tiled_auto(const Geom &g, int precision);
+int64_t tiles_per_chunk(const Geom &g);
+int grid_default_kz(const Geom &g, int precision, bool *taper);
 
 // Context-owned device staging buffer of at least `bytes` (grown with
 // cudaMalloc; reused across calls on the context's stream).

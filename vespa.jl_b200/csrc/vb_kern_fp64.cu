@@ -172,7 +172,7 @@ int launch_stage_tiled3d_fp64(const BoxDesc *hbox, const BoxDesc *boxes, const i
                               int nitems, unsigned int *work, int stage, cudaStream_t s, bool grav,
                               bool bf)
 {
-    return launch_tiled3d_f64<2>(hbox, boxes, item_box, nitems, work, stage, s, grav, bf);
+    return launch_tiled3d_f64(hbox, boxes, item_box, nitems, work, stage, s, grav, bf);
 }
 
 namespace {

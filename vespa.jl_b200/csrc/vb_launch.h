@@ -82,6 +82,14 @@ inline bool tiled3d_supported(const Geom &g)
            g.n[0] <= (1 << 30) && g.n[1] <= (1 << 30) && g.n[2] <= (1 << 30);
 }
 
+// Ragged 3D boxes with room for one tile: a side that is no multiple of 16 ends
+// in a shifted tile (float64 kernel, whose loads need no alignment).
+inline bool tiled3d_ragged(const Geom &g, int precision)
+{
+    return g.nd == 3 && g.n[0] >= 16 && g.n[1] >= 16 && g.n[2] >= 2 && g.n[0] <= (1 << 30) &&
+           g.n[1] <= (1 << 30) && g.n[2] <= (1 << 30) && precision == PREC_FP64;
+}
+
 // Tiled 2D path applicability: 256-cell row segments marching y.
 inline bool tiled2d_supported(const Geom &g)
 {
@@ -89,6 +97,11 @@ inline bool tiled2d_supported(const Geom &g)
            g.n[1] <= (1 << 30);
 }
 inline bool tiled_supported(const Geom &g) { return tiled3d_supported(g) || tiled2d_supported(g); }
+// what a single grid may take automatically
+inline bool tiled_any(const Geom &g, int precision)
+{
+    return tiled_supported(g) || tiled3d_ragged(g, precision);
+}
 // cells along the marching axis (z in 3D, y in 2D)
 inline int64_t march_extent(const Geom &g) { return g.nd == 3 ? g.n[2] : g.n[1]; }
 

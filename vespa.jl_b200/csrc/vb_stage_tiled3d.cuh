@@ -56,35 +56,6 @@ __device__ __forceinline__ int halo_idx(int lx, int ly)
 
 }  // namespace t3
 
-// The float64 HLLC of the tiled 3D kernel, one non-inlined body per face
-// orientation.  The kernel solves faces at seven call sites; inlined at each,
-// its code outgrew the instruction cache (no_instruction stalls), and as a
-// call it runs about 5 % faster.  The operations, hence the bits, are the same.
-struct F64x5 {
-    double v[5];
-};
-template <int DIM>
-__device__ __noinline__ F64x5 hllc_f64_call(F64x5 L, F64x5 R, double gamma)
-{
-    F64x5 F;
-    hllc_flux<double, DIM>(L.v, R.v, gamma, F.v);
-    return F;
-}
-template <int DIM>
-__device__ __forceinline__ void tiled_hllc(const double WL[5], const double WR[5], double gamma,
-                                           double F[5])
-{
-    F64x5 L, R;
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        L.v[k] = WL[k];
-        R.v[k] = WR[k];
-    }
-    const F64x5 r = hllc_f64_call<DIM>(L, R, gamma);
-#pragma unroll
-    for (int k = 0; k < 5; ++k) F[k] = r.v[k];
-}
-
 // A stage load's bounded wait gave up (a block-uniform decision, taken after
 // the barrier that follows the wait): the block issues no further load and
 // skips the rest of its work.  Thread 0 waits, each wait bounded again, for
@@ -184,7 +155,7 @@ namespace vb {
 // Resident blocks of a persistent kernel on the current device (all SMs), with
 // its dynamic shared memory opted in once.
 template <typename K>
-int persistent_blocks(K kernel1, K kernel2, size_t smem)
+int persistent_blocks(K kernel1, K kernel2, size_t smem, int threads = t3::NT)
 {
     if (cudaFuncSetAttribute(kernel1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
             cudaSuccess ||
@@ -194,7 +165,7 @@ int persistent_blocks(K kernel1, K kernel2, size_t smem)
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel2, t3::NT, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel2, threads, smem) != cudaSuccess ||
         per_sm < 1)
         return -1;
     return sms * per_sm;

@@ -1,16 +1,27 @@
 // vb_stage_tiled3d_f64.cuh -- VB_FP64 tiled 3D stage kernel.
 //
-// The exact-float64 counterpart of k_stage_tiled3d_mixed (same tiling, TMA
-// pipeline, persistent queue and plane structure; see that file): a ring of
-// three float64 primitive planes with mirror ghosts at walls; each thread
-// rebuilds the states of its own lo x and lo y faces from the four cells
-// across each and solves them with the reference's HLLC (src/riemann.jl) one
-// after the other; warps 6 and 7 add the tile's hi-edge y and x faces; the z
-// face runs down the thread's column, before the first barrier in warps 4..7
-// and after it in warps 0..3; two barriers per plane.  Every operation is the
-// reference's, rounded separately (-fmad=false), in the reference's per-cell
-// accumulation order, so the result is bit-identical to the cell-centric
-// kernel and to the oracle.
+// A block of 12 warps owns a 16 x 16 column tile of any 3D grid with nx, ny >=
+// 16 and marches it along z.  When a side is no multiple of 16 the last tile
+// is shifted back inside the grid; cells it shares with the tile before it
+// are computed and not written.  Warps 0..7 are one thread per column, warps
+// 8..11 one thread per halo cell of the plane (4 strips of 32).
+//
+// Primitives live in a ring of three planes in shared memory; beyond a wall a
+// halo thread fetches the mirror cell.  Raw conserved values arrive in the slot itself (8-byte
+// cp.async, each element fetched by the thread that converts it in place, so
+// no alignment of the rows is needed and no thread waits for another's copy).
+// One barrier per plane separates iterations; iteration k
+//   - solves the x and y faces of plane k+1 into one of two flux buffers: 17
+//     warp tasks (8 of x, 8 of y, one of both hi edges), one on each column
+//     warp and two or three on each halo warp, all through one body with the
+//     states in the face-normal frame;
+//   - converts plane k+2 and solves the z face k+1/2 down the column;
+//   - updates plane k from the fluxes of the last iteration.
+// Iteration k0-1 is the prologue: the same code without the update.
+//
+// Every operation is the reference's, rounded separately (-fmad=false), in the
+// reference's per-cell accumulation order, so the result is bit-identical to
+// the cell-centric kernel and to the oracle.
 #pragma once
 
 #include "vb_stage_tiled3d_mixed.cuh"
@@ -20,7 +31,6 @@ namespace vb {
 namespace t3d {
 
 using t3::NH;
-using t3::NT;
 using t3::TX;
 using t3::TY;
 using t3m::PC;
@@ -28,71 +38,91 @@ using t3m::PSLOT;
 using t3m::wrow;
 using t3m::wxs;
 
-template <int NS>
+constexpr int NC = TX * TY;           // column threads (one per cell of a plane)
+constexpr int NTH = NC + NH;          // and one thread per halo cell
+constexpr int FX = TY * (TX + 1);     // x faces of a plane
+constexpr int FY = (TY + 1) * TX;     // y faces
+
 struct Smem {
-    double u[NS][t3::UPLANE];     // TMA stage buffers (raw conserved state)
-    double w[3][PSLOT];           // primitive ring (t3m layout, float64)
-    double gx[5][TY * (TX + 1)];  // x-face area * flux
-    double gy[5][(TY + 1) * TX];  // y-face area * flux
-    uint64_t bar[NS];
+    double w[3][PSLOT];          // plane ring (t3m layout): raw state, then primitives in place
+    double g[2][5 * (FX + FY)];  // area * flux of a plane: [5][FX] of x, then [5][FY] of y
+    double hz[5][NC];            // hi z face value of the plane in work, per column
+    double fz[5][NC];            // area * flux through its lower z face
 };
 
-// Left / right states of one face along axis AX (0 x, 1 y) from the four cells
-// across it (ring offsets o[0..3]): the hi face value of the cell behind and
-// the lo face value of the cell ahead (_face_value, src/driver.jl:227-233).
-__device__ __forceinline__ void face_states(const double *wk, const int o[4], double L[5],
-                                            double R[5])
+// face_val(w, h, minmod(a, b))
+__device__ __forceinline__ double face_mm(double w, double h, double a, double b)
 {
-#pragma unroll
-    for (int f = 0; f < 5; ++f) {
-        const double *p = wk + f * PC;
-        const double a0 = p[o[0]], a1 = p[o[1]], a2 = p[o[2]], a3 = p[o[3]];
-        L[f] = face_val(a1, 0.5, limited_slope<double>(a0, a1, a2));
-        R[f] = face_val(a2, -0.5, limited_slope<double>(a1, a2, a3));
+    return face_val(w, h, minmod<double>(a, b));
+}
+
+// An upper bound, in float32, of the cell's compute_dt term max_d (|v_d| + c) /
+// w_d (and of the free-fall rate, GRAV).  Relative slack 4e-6 on the pressure
+// (measured against E + kinetic, which its difference cancels) and on the
+// result covers the float32 roundings; anything out of float32 range, and any
+// negative density or pressure, comes out NaN or Inf.
+template <bool GRAV>
+__device__ __forceinline__ float cfl_bound(const double un[5], const Geom &g, float gf, float iw0,
+                                           float iw1, float iw2)
+{
+    const float ir = rcp_approx((float)un[0]), E = (float)un[4];
+    const float vx = (float)un[1] * ir, vy = (float)un[2] * ir, vz = (float)un[3] * ir;
+    const float ke = 0.5f * (float)un[0] * (vx * vx + vy * vy + vz * vz);
+    const float p = (gf - 1.0f) * (E - ke) + 4e-6f * (fabsf(E) + ke);
+    const float c = sqrt_approx(gf * p * ir);
+    float b = fmaxf(fmaxf((fabsf(vx) + c) * iw0, (fabsf(vy) + c) * iw1), (fabsf(vz) + c) * iw2);
+    if (c != c) b = c;  // fmaxf drops a NaN operand
+    if constexpr (GRAV) {
+        const float f = 2.0f * sqrt_approx(12.566371f * (float)g.grav_G * (float)un[0]);
+        if (!(f <= b)) b = f;
     }
+    return b * (1.0f + 4e-6f);
 }
 
 }  // namespace t3d
 
-template <int NS, int STAGE, bool BATCH, bool GRAV = false, bool BF = false>
-__global__ void __launch_bounds__(256, 2)
+template <int STAGE, bool BATCH, bool GRAV = false, bool BF = false>
+__global__ void __launch_bounds__(t3d::NTH, 2)
 k_stage_tiled3d_f64(const __grid_constant__ BoxDesc box0, const BoxDesc *__restrict__ boxes,
                     const int *__restrict__ item_box, int nitems, unsigned int *work)
 {
-    using namespace t3;
     using namespace t3d;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    // check build only: TMA destinations need a 128-byte aligned base (uniform)
-    if (!VB_DCHECK(((uintptr_t)smem_raw & 127) == 0)) return;
-    t3d::Smem<NS> &S = *reinterpret_cast<t3d::Smem<NS> *>(smem_raw);
+    t3d::Smem &S = *reinterpret_cast<t3d::Smem *>(smem_raw);
     __shared__ double red[32];
     __shared__ int item_sh;
-    __shared__ int stall_sh;  // a stage load's bounded wait gave up
+    __shared__ int cfl_sh;  // float bits: a lower bound of the item's CFL maximum so far
 
     const int t = threadIdx.x;
-    const int tx = t & (TX - 1), ty = t >> 4;
-    const int warp = t >> 5, lane = t & 31;
-    const int o_c = wrow(tx, ty);
-    const int ox[4] = {tx >= 2 ? o_c - 2 : wxs(tx - 2, ty), tx >= 1 ? o_c - 1 : wxs(-1, ty), o_c,
-                       tx <= TX - 2 ? o_c + 1 : wxs(TX, ty)};
-    const int oy[4] = {o_c - 32, o_c - 16, o_c, o_c + 16};
-    const int h_u = halo_uoff(t < NH ? t : 0, 0);
-    const int h_w = t < 32   ? wxs(-2 + (t & 1), t >> 1)
-                    : t < 64 ? wxs(TX + (t & 1), (t - 32) >> 1)
-                    : t < 96 ? wrow((t - 64) & 15, -2 + ((t - 64) >> 4))
-                             : wrow((t - 96) & 15, TY + ((t - 96) >> 4));
-    const bool z_early = warp >= 4;
+    const bool col = t < NC;  // column thread, else halo thread
+    const int tx = t & (TX - 1), ty = (t >> 4) & (TY - 1);
+    // ring offset of the element this thread fetches and converts
+    const int h = t - NC;  // halo thread: strip cell
+    const int o_c = col      ? wrow(tx, ty)
+                    : h < 32 ? wxs(-2 + (h & 1), h >> 1)
+                    : h < 64 ? wxs(TX + (h & 1), (h - 32) >> 1)
+                    : h < 96 ? wrow((h - 64) & 15, -2 + ((h - 64) >> 4))
+                             : wrow((h - 96) & 15, TY + ((h - 96) >> 4));
+    // its cell relative to the tile's corner
+    const int dx = col      ? tx
+                   : h < 32 ? -2 + (h & 1)
+                   : h < 64 ? TX + (h & 1)
+                            : (h & 15);
+    const int dy = col      ? ty
+                   : h < 64 ? (h & 31) >> 1
+                   : h < 96 ? -2 + ((h - 64) >> 4)
+                            : TY + ((h - 96) >> 4);
+    // face tasks: column warps the own lo x face; halo warp i the lo y faces of
+    // rows 4 i .. 4 i + 3 (two tasks), the last one also the hi-edge faces
+    const int ntask = col ? 1 : (t < NTH - 32 ? 2 : 3);
+    const int fr = col ? ty : 4 * (h >> 5) + ((h >> 4) & 1);  // row of the first task
+    const int f_c = wrow(tx, fr);
 
-    if (t == 0) {
-        for (int s = 0; s < NS; ++s) mbar_init(&S.bar[s], 1);
-        fence_mbar_init();
-        stall_sh = 0;
-    }
-    __syncthreads();
-
-    int qb = 0;
     for (;;) {
-    if (t == 0) item_sh = (int)atomicAdd(&work[STAGE - 1], 1u);
+    if (t == 0) {
+        item_sh = (int)atomicAdd(&work[STAGE - 1], 1u);
+        cfl_sh = 0;
+    }
     __syncthreads();
     const int item = item_sh;
     if (item >= nitems) break;
@@ -103,387 +133,341 @@ k_stage_tiled3d_f64(const __grid_constant__ BoxDesc box0, const BoxDesc *__restr
         continue;
     }
     const Geom &g = B.g;
-    const CUtensorMap *tm = B.map[STAGE - 1];
-    if (!VB_DCHECK(((uintptr_t)tm & 63) == 0)) return;  // check build only (uniform)
     const double *__restrict__ Uin = STAGE == 1 ? B.U : B.U1;
     const double *U0 = B.U;
     double *Uout = STAGE == 1 ? B.U1 : B.U;
-    const int kz = B.kz, ntx = B.ntx, ntiles = B.ntiles;
     const int nx = (int)g.n[0], ny = (int)g.n[1], nz = (int)g.n[2];
     const bool perx = g.bc_lo[0] == BC_PERIODIC, pery = g.bc_lo[1] == BC_PERIODIC;
     const bool perz = g.bc_lo[2] == BC_PERIODIC;
     const double gamma = g.gamma;
-    const double invV = ctrl->invV;
     const double bscale = BF ? 0.5 * ctrl->dt : 0.0;  // boundary-flux stage weight
-    const double ax = g.area[0], ay = g.area[1], az = g.area[2];
-    const int bx_lo = g.bc_lo[0], bx_hi = g.bc_hi[0], by_lo = g.bc_lo[1], by_hi = g.bc_hi[1];
-    const int bz_lo = g.bc_lo[2], bz_hi = g.bc_hi[2];
-    double invdt = 0.0;
     const int local = item - B.item0;
-    const int tile = local % ntiles;
-    const int x0 = (tile % ntx) * TX, y0 = (tile / ntx) * TY;
+    const int tile = local % B.ntiles;
+    // the last tile of a side that is no multiple of 16 is shifted back; the
+    // cells left of (below) the nominal corner belong to the tile before it
+    const int xn = (tile % B.ntx) * TX, yn = (tile / B.ntx) * TY;
+    const int x0 = min(xn, nx - TX), y0 = min(yn, ny - TY);
     int k0, k1;
-    chunk_span(nz, kz, B.nchu, local / ntiles, k0, k1);
-    const int nplanes = (k1 - k0) + 4;
-    const bool xlo_bnd = !perx && x0 == 0, xhi_bnd = !perx && x0 + TX == nx;
-    const bool ylo_bnd = !pery && y0 == 0, yhi_bnd = !pery && y0 + TY == ny;
-    const bool h_ghost = t < 32 ? xlo_bnd : (t < 64 ? xhi_bnd : (t < 96 ? ylo_bnd : yhi_bnd));
+    chunk_span(nz, B.kz, B.nchu, local / B.ntiles, k0, k1);
+    const int64_t plane = (int64_t)nx * ny;
+    // this thread's element: its column in the state.  Beyond the grid that is
+    // the wrapped cell on a periodic axis, else the mirror cell, whose normal
+    // velocity (field `flip`) a reflecting wall negates (ghost_state)
+    int ex = x0 + dx, ey = y0 + dy, flip = 0;
+    if (!col) {
+        auto mirror = [&](int &c, int n, bool per, int bl, int bh, int nrm) {
+            if (c < 0) {
+                if (!per && bl == BC_REFLECTING) flip = nrm;
+                c = per ? c + n : -1 - c;
+            } else if (c >= n) {
+                if (!per && bh == BC_REFLECTING) flip = nrm;
+                c = per ? c - n : 2 * n - 1 - c;
+            }
+        };
+        mirror(ex, nx, perx, g.bc_lo[0], g.bc_hi[0], 1);
+        mirror(ey, ny, pery, g.bc_lo[1], g.bc_hi[1], 2);
+    }
+    const int64_t ecol = (int64_t)ex + (int64_t)nx * ey;
+    const bool own = col && ex >= xn && ey >= yn;  // this thread updates its column
+    double cflm = 0.0;
 
-    auto issue = [&](int q) {
-        const int p = k0 - 2 + q;
-        // periodic wrap of the planes k0 - 2 .. k1 + 1 (a modulo only when nz < 3)
+    // cp.async of plane p's element into ring slot ws (periodic planes wrap;
+    // planes beyond a wall are left out, the z face formulas do not read them)
+    auto fetch_plane = [&](int p, double *ws) {
         int z = p;
         if (perz) {
             z = p < 0 ? p + nz : (p >= nz ? p - nz : p);
-            if (z < 0 || z >= nz) z = ((p % nz) + nz) % nz;
+            if (z < 0 || z >= nz) z = ((p % nz) + nz) % nz;  // nz < 3 only
         }
-        double *dst = S.u[(qb + q) % NS];
-        uint64_t *bar = &S.bar[(qb + q) % NS];
-        const int xl = (perx && x0 == 0) ? nx - 2 : x0 - 2;
-        const int xh = (perx && x0 + TX == nx) ? 0 : x0 + TX;
-        const int yl = (pery && y0 == 0) ? ny - 2 : y0 - 2;
-        const int yh = (pery && y0 + TY == ny) ? 0 : y0 + TY;
-        mbar_expect_tx(bar, PLANE_BYTES);
-        tma_load_4d(dst, &tm[0], x0, y0, z, 0, bar);
-        tma_load_4d(dst + U_XLO, &tm[1], xl, y0, z, 0, bar);
-        tma_load_4d(dst + U_XHI, &tm[1], xh, y0, z, 0, bar);
-        tma_load_4d(dst + U_YLO, &tm[2], x0, yl, z, 0, bar);
-        tma_load_4d(dst + U_YHI, &tm[2], x0, yh, z, 0, bar);
+        if (z >= 0 && z < nz) {
+            const double *src = Uin + ecol + plane * z;
+            if (VB_DCHECK(ecol >= 0 && ecol < plane))
+#pragma unroll
+                for (int f = 0; f < 5; ++f) cp_async8(ws + o_c + f * PC, src + f * g.ncell);
+        }
     };
-    // the stage loads are issued by one thread of warp 5, whose share of the
-    // plane's second phase is the smallest
-    if (t == TMA_ISSUER) {
-        fence_proxy_async_smem();
-        for (int q = 0; q < NS && q < nplanes; ++q) issue(q);
+    // in-place conversion of this thread's element of a landed plane
+    auto convert = [&](double *ws, double W[5]) {
+        double u[5];
+#pragma unroll
+        for (int f = 0; f < 5; ++f) u[f] = ws[o_c + f * PC];
+        cons2prim(u, gamma, W);
+        if (flip == 1) W[1] = -W[1];
+        if (flip == 2) W[2] = -W[2];
+#pragma unroll
+        for (int f = 0; f < 5; ++f) ws[o_c + f * PC] = W[f];
+    };
+
+    // ring slots of planes k, k+1, k+2 at the loop's start (k = k0 - 1)
+    double *r0 = S.w[0], *r1 = S.w[1], *r2 = S.w[2];
+    // plane k0-2 passes through slot r2 on its way to the column's hi z face
+    // value of plane k0-1
+    const bool gl = !perz && k0 == 0;  // the chunk's lower z face is a wall
+    if (col) {
+        if (!gl) {
+            fetch_plane(k0 - 2, r2);
+            fetch_plane(k0 - 1, r0);
+        }
     }
-    // Halo strips of staged plane q into ring slot q % 3 (threads t < NH).
-    auto halo_c2p = [&](int q) {
-        if (t < NH && !h_ghost) {
-            const double *u = S.u[(qb + q) % NS];
-            double *ws = S.w[q % 3];
-            double uu[5], w[5];
-#pragma unroll
-            for (int f = 0; f < 5; ++f) uu[f] = u[h_u + f * (2 * TY)];
-            cons2prim(uu, gamma, w);
-#pragma unroll
-            for (int f = 0; f < 5; ++f) ws[h_w + f * PC] = w[f];
-        }
-    };
-    // Wait for staged plane q and convert the own cell into Wn.  keep = 0:
-    // registers only; 1: also into ring slot q % 3 with the mirror ghosts and
-    // the halo strips; 2: as 1 without the halo strips (halo_c2p follows).
-    auto consume = [&](int q, double Wn[5], int keep) {
-        const int b = (qb + q) % NS;
-        if (!mbar_wait(&S.bar[b], ((qb + q) / NS) & 1, WAIT_LIMIT_NS)) stall_sh = 1;
-        const double *u = S.u[b];
-        {
-            double uu[5];
-#pragma unroll
-            for (int f = 0; f < 5; ++f) uu[f] = u[f * NT + t];
-            cons2prim(uu, gamma, Wn);
-        }
-        if (!keep) return;
-        double *ws = S.w[q % 3];
-#pragma unroll
-        for (int f = 0; f < 5; ++f) ws[f * PC + o_c] = Wn[f];
-        if (xlo_bnd && tx < 2) {
-            double *d = ws + wxs(-1 - tx, ty);
-#pragma unroll
-            for (int f = 0; f < 5; ++f) d[f * PC] = (bx_lo == BC_REFLECTING && f == 1) ? -Wn[f] : Wn[f];
-        }
-        if (xhi_bnd && tx >= TX - 2) {
-            double *d = ws + wxs(2 * TX - 1 - tx, ty);
-#pragma unroll
-            for (int f = 0; f < 5; ++f) d[f * PC] = (bx_hi == BC_REFLECTING && f == 1) ? -Wn[f] : Wn[f];
-        }
-        if (ylo_bnd && ty < 2) {
-            double *d = ws + wrow(tx, -1 - ty);
-#pragma unroll
-            for (int f = 0; f < 5; ++f) d[f * PC] = (by_lo == BC_REFLECTING && f == 2) ? -Wn[f] : Wn[f];
-        }
-        if (yhi_bnd && ty >= TY - 2) {
-            double *d = ws + wrow(tx, 2 * TY - 1 - ty);
-#pragma unroll
-            for (int f = 0; f < 5; ++f) d[f * PC] = (by_hi == BC_REFLECTING && f == 2) ? -Wn[f] : Wn[f];
-        }
-        if (keep == 1) halo_c2p(q);
-    };
-    auto release = [&](int q) {
-        if (t == TMA_ISSUER && q + NS < nplanes) {
-            fence_proxy_async_smem();
-            issue(q + NS);
-        }
-    };
-    // after the barrier that follows consume(q): uniform across the block
-    auto stalled = [&](int q) -> bool {
-        if (!stall_sh) return false;
-        stage_abandon<NS>(S.bar, qb, q, nplanes, ctrl);
-        return true;
-    };
-
-    double Wa[5], Wb[5], Wc[5], Wd[5];
-    consume(0, Wa, 0);
-    __syncthreads();
-    if (stalled(0)) return;
-    release(0);
-    consume(1, Wb, 0);
-    __syncthreads();
-    if (stalled(1)) return;
-    release(1);
-    consume(2, Wc, 1);
-    __syncthreads();
-    if (stalled(2)) return;
-    release(2);
-    consume(3, Wd, 1);
-    __syncthreads();
-    if (stalled(3)) return;
-    release(3);
-
-    // z state entering plane k0: hi face value of k0 and the flux through k0-1/2
-    double hz[5], Fzlo[5];
+    fetch_plane(k0, r1);
+    cp_async_commit();
+    cp_async_wait_all();
     {
-        const bool gl = !perz && k0 == 0;
-        const bool gh = !perz && k0 + 1 >= nz;
-        double loz[5];
-#pragma unroll
-        for (int f = 0; f < 5; ++f) {
-            const double wl = gl ? ((bz_lo == BC_REFLECTING && f == 3) ? -Wc[f] : Wc[f]) : Wb[f];
-            const double wr = gh ? ((bz_hi == BC_REFLECTING && f == 3) ? -Wc[f] : Wc[f]) : Wd[f];
-            const double s = limited_slope<double>(wl, Wc[f], wr);
-            hz[f] = face_val(Wc[f], 0.5, s);
-            loz[f] = face_val(Wc[f], -0.5, s);
-        }
-        if (gl) {
-            double gst[5];
-            ghost_state<double>(loz, bz_lo, 2, gst);
-            tiled_hllc<3>(gst, loz, gamma, Fzlo);
-            if constexpr (BF)  // z-lo domain face of cell (x, y, 0)
-                bflux_add(g, B.bflux, 2, 0, (int64_t)(x0 + tx) + (int64_t)nx * (y0 + ty), bscale, az, Fzlo);
-        } else {
+        double Wa[5], Wb[5], Wc[5];
+        convert(r1, Wc);
+        if (col && !gl) {
             const bool gll = !perz && k0 - 2 < 0;
-            double hzm[5];
+            if (!gll) {
+                double u[5];
+#pragma unroll
+                for (int f = 0; f < 5; ++f) u[f] = r2[o_c + f * PC];
+                cons2prim(u, gamma, Wa);
+            }
+            {
+                double u[5];
+#pragma unroll
+                for (int f = 0; f < 5; ++f) u[f] = r0[o_c + f * PC];
+                cons2prim(u, gamma, Wb);
+            }
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
-                const double wl = gll ? ((bz_lo == BC_REFLECTING && f == 3) ? -Wb[f] : Wb[f]) : Wa[f];
-                hzm[f] = face_val(Wb[f], 0.5, limited_slope<double>(wl, Wb[f], Wc[f]));
+                r0[o_c + f * PC] = Wb[f];
+                const double wl = gll ? ((g.bc_lo[2] == BC_REFLECTING && f == 3) ? -Wb[f] : Wb[f]) : Wa[f];
+                S.hz[f][t] = face_val(Wb[f], 0.5, limited_slope<double>(wl, Wb[f], Wc[f]));
             }
-            tiled_hllc<3>(hzm, loz, gamma, Fzlo);
         }
     }
+    if (col || k0 + 1 < k1) fetch_plane(k0 + 1, r2);
+    cp_async_commit();
+    __syncthreads();
 
-    // flux through k+1/2 from planes k, k+1 (ring) and k+2 (W2) of the own
-    // column; advances hz
-    auto zsolve = [&](int k, const double *w0, const double *w1, const double W2[5], double Fzhi[5]) {
-        double zr[5], hz1[5];
-        if (perz || k + 1 < nz) {
-            const bool gh = !perz && k + 2 >= nz;
+    const int cx = lo_class(ex, nx, perx), cy = lo_class(ey, ny, pery);
+    const float gf = (float)gamma;
+    const float iw0 = (float)g.invw[0], iw1 = (float)g.invw[1], iw2 = (float)g.invw[2];
+
+    for (int k = k0 - 1; k < k1; ++k) {
+        // warm L1 for the update's own-cell loads (a 16-cell row spans at most
+        // two 128-byte lines)
+        if (STAGE == 2 && col && k >= k0 && (tx == 0 || tx == TX - 1)) {
+            const int64_t l = ecol + plane * k;
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
-                const double c = w1[f * PC];
-                const double r = gh ? ((bz_hi == BC_REFLECTING && f == 3) ? -c : c) : W2[f];
-                const double s = limited_slope<double>(w0[f * PC], c, r);
-                zr[f] = face_val(c, -0.5, s);
-                hz1[f] = face_val(c, 0.5, s);
+                prefetch_l1(Uin + l + f * g.ncell);
             }
+        }
+        // halo elements of plane k are free (its faces are solved): fetch k+3's
+        if (!col) {
+            if (k + 3 < k1) fetch_plane(k + 3, r0);
+            cp_async_commit();
+        }
+        // ---- x and y faces of plane k+1 ----
+        if (k + 1 < k1) {
+            double *gw = S.g[(k + 1) & 1];
+            const double *w1 = r1;
+            const double ax = g.area[0], ay = g.area[1];
+            for (int it = 0; it < ntask; ++it) {
+                // the four cells across the face; x: cells tx-2 .. tx+1, y: rows
+                int o0, o1, o2, o3, out;
+                bool isy;
+                if (it < 2) {
+                    isy = !col;
+                    const int c = f_c + 32 * it;  // the second task is two rows up
+                    if (isy) {
+                        o0 = c - 32; o1 = c - 16; o2 = c; o3 = c + 16;
+                        out = 5 * FX + (fr + 2 * it) * TX + tx;
+                    } else {
+                        o0 = tx >= 2 ? c - 2 : wxs(tx - 2, fr);
+                        o1 = tx >= 1 ? c - 1 : wxs(-1, fr);
+                        o2 = c;
+                        o3 = tx <= TX - 2 ? c + 1 : wxs(TX, fr);
+                        out = fr * (TX + 1) + tx;
+                    }
+                } else {  // hi edges: lanes 0..15 of x (row tx), 16..31 of y (column tx)
+                    isy = (t & 16) != 0;
+                    if (isy) {
+                        o2 = wrow(tx, TY);
+                        o0 = o2 - 32; o1 = o2 - 16; o3 = o2 + 16;
+                        out = 5 * FX + TY * TX + tx;
+                    } else {
+                        o1 = wrow(TX - 1, tx);
+                        o0 = o1 - 1; o2 = wxs(TX, tx); o3 = wxs(TX + 1, tx);
+                        out = tx * (TX + 1) + TX;
+                    }
+                }
+                // normal and first tangential velocity are fields 1, 2 (x) or 2, 1 (y)
+                const int fn = isy ? 2 * PC : PC, ft = isy ? PC : 2 * PC;
+                double L[5], R[5], F[5];
+#pragma unroll
+                for (int f = 0; f < 5; ++f) {
+                    const double *p = w1 + (f == 1 ? fn : f == 2 ? ft : f * PC);
+                    const double a0 = p[o0], a1 = p[o1], a2 = p[o2], a3 = p[o3];
+                    const double d = a2 - a1;
+                    L[f] = face_mm(a1, 0.5, a1 - a0, d);
+                    R[f] = face_mm(a2, -0.5, d, a3 - a2);
+                }
+                hllc_frame_any<false>(L, R, gamma, F);
+                const int os = isy ? FY : FX;
+                const double ar = isy ? ay : ax;
+                double *o = gw + out;
+                o[0] = ar * F[0];
+                o[(isy ? 2 : 1) * os] = ar * F[1];
+                o[(isy ? 1 : 2) * os] = ar * F[2];
+                o[3 * os] = ar * F[3];
+                o[4 * os] = ar * F[4];
+                if constexpr (BF) {  // domain faces of cells this tile updates
+                    const double Fd[5] = {F[0], isy ? F[2] : F[1], isy ? F[1] : F[2], F[3], F[4]};
+                    const int kk = k + 1;
+                    if (!isy) {
+                        const int fy = y0 + (it < 2 ? fr : tx), side = it < 2 ? 0 : 1;
+                        if (fy >= yn && !perx && (side ? x0 + TX == nx : x0 + tx == 0))
+                            bflux_add(g, B.bflux, 0, side, (int64_t)fy + (int64_t)ny * kk, bscale, ax, Fd);
+                    } else {
+                        const int fx = x0 + tx, side = it < 2 ? 0 : 1;
+                        if (fx >= xn && !pery && (side ? y0 + TY == ny : y0 + fr + 2 * it == 0))
+                            bflux_add(g, B.bflux, 1, side, (int64_t)fx + (int64_t)nx * kk, bscale, ay, Fd);
+                    }
+                }
+            }
+        }
+        if (!col) {
+            cp_async_wait_group<1>();  // plane k+2's element (k+3's is in flight)
+            double W[5];
+            if (k + 2 < k1) convert(r2, W);
         } else {
-            ghost_state<double>(hz, bz_hi, 2, zr);
+            // ---- plane k+2 of the column, and the z face k+1/2 ----
+            cp_async_wait_all();
+            const bool below = perz || k >= 0;       // plane k exists
+            const bool above = perz || k + 1 < nz;   // plane k+1 exists
+            const bool top = !perz && k + 2 >= nz;   // plane k+2 does not
+            double zl[5], zr[5], F[5];
+            {
+                double W2[5];
+                if (!top) convert(r2, W2);
 #pragma unroll
-            for (int f = 0; f < 5; ++f) hz1[f] = hz[f];
-        }
-        tiled_hllc<3>(hz, zr, gamma, Fzhi);
-        if constexpr (BF) {
-            if (!perz && k + 1 >= nz)  // z-hi domain face of cell (x, y, nz-1)
-                bflux_add(g, B.bflux, 2, 1, (int64_t)(x0 + tx) + (int64_t)nx * (y0 + ty), bscale, az, Fzhi);
-        }
-#pragma unroll
-        for (int f = 0; f < 5; ++f) hz[f] = hz1[f];
-    };
-    // the own lo x face and lo y face of plane k (ring slot w0)
-    auto xy_faces = [&](const double *w0, int k) {
-        double L[5], R[5], F[5];
-        face_states(w0, ox, L, R);
-        tiled_hllc<1>(L, R, gamma, F);
-#pragma unroll
-        for (int f = 0; f < 5; ++f) S.gx[f][ty * (TX + 1) + tx] = ax * F[f];
-        if constexpr (BF) {
-            if (xlo_bnd && tx == 0)  // x-lo domain face of cell (0, y, k)
-                bflux_add(g, B.bflux, 0, 0, (int64_t)(y0 + ty) + (int64_t)ny * k, bscale, ax, F);
-        }
-        face_states(w0, oy, L, R);
-        tiled_hllc<2>(L, R, gamma, F);
-#pragma unroll
-        for (int f = 0; f < 5; ++f) S.gy[f][ty * TX + tx] = ay * F[f];
-        if constexpr (BF) {
-            if (ylo_bnd && ty == 0)  // y-lo domain face of cell (x, 0, k)
-                bflux_add(g, B.bflux, 1, 0, (int64_t)(x0 + tx) + (int64_t)nx * k, bscale, ay, F);
-        }
-    };
-    // the hi-edge faces: x at fx = TX (warp 7) or y at fy = TY (warp 6), lanes < 16
-    auto edge_face = [&](const double *w0, int k) {
-        const int j = lane;
-        double L[5], R[5], F[5];
-        if (warp == 7) {
-            const int ex[4] = {wrow(TX - 2, j), wrow(TX - 1, j), wxs(TX, j), wxs(TX + 1, j)};
-            face_states(w0, ex, L, R);
-            tiled_hllc<1>(L, R, gamma, F);
-#pragma unroll
-            for (int f = 0; f < 5; ++f) S.gx[f][j * (TX + 1) + TX] = ax * F[f];
-            if constexpr (BF) {
-                if (xhi_bnd)  // x-hi domain face of cell (nx-1, y0+j, k)
-                    bflux_add(g, B.bflux, 0, 1, (int64_t)(y0 + j) + (int64_t)ny * k, bscale, ax, F);
+                for (int f = 0; f < 5; ++f) {
+                    zl[f] = S.hz[f][t];
+                    if (above) {
+                        const double c = r1[o_c + f * PC];
+                        const double lo = below ? r0[o_c + f * PC]
+                                                : ((g.bc_lo[2] == BC_REFLECTING && f == 3) ? -c : c);
+                        const double hi = top ? ((g.bc_hi[2] == BC_REFLECTING && f == 3) ? -c : c) : W2[f];
+                        zr[f] = face_mm(c, -0.5, c - lo, hi - c);
+                        S.hz[f][t] = face_mm(c, 0.5, c - lo, hi - c);
+                    }
+                }
+                if (!above) ghost_state<double>(zl, g.bc_hi[2], 2, zr);
+                if (!below) ghost_state<double>(zr, g.bc_lo[2], 2, zl);
             }
-        } else {
-            const int ey[4] = {wrow(j, TY - 2), wrow(j, TY - 1), wrow(j, TY), wrow(j, TY + 1)};
-            face_states(w0, ey, L, R);
-            tiled_hllc<2>(L, R, gamma, F);
+            // the column's entries of plane k have been read: until plane k+3
+            // lands there they hold the update's input (U^n in stage 2)
+            const bool write = own && k >= k0;
+            const int64_t lin = ecol + plane * k;
+            const bool inb = write && VB_DCHECK(lin >= 0 && lin < g.ncell);  // check build only
+            if (inb)
 #pragma unroll
-            for (int f = 0; f < 5; ++f) S.gy[f][TY * TX + j] = ay * F[f];
-            if constexpr (BF) {
-                if (yhi_bnd)  // y-hi domain face of cell (x0+j, ny-1, k)
-                    bflux_add(g, B.bflux, 1, 1, (int64_t)(x0 + j) + (int64_t)nx * k, bscale, ay, F);
+                for (int f = 0; f < 5; ++f)
+                    cp_async8(r0 + o_c + f * PC, (STAGE == 1 ? Uin : U0) + lin + f * g.ncell);
+            cp_async_commit();
+            {
+                const double L[5] = {zl[0], zl[3], zl[1], zl[2], zl[4]};
+                const double R[5] = {zr[0], zr[3], zr[1], zr[2], zr[4]};
+                hllc_frame_any<true>(L, R, gamma, F);
             }
-        }
-    };
-
-    const int gx = x0 + tx, gy = y0 + ty;
-    const int cx = lo_class(gx, nx, perx), cy = lo_class(gy, ny, pery);
-    // previous plane's new state: its CFL term is folded one plane later (the
-    // initial value is a finite placeholder whose term is discarded)
-    double unp[5] = {1.0, 0.0, 0.0, 0.0, 1.0};
-    const int64_t plane_cells = (int64_t)nx * ny;
-    int64_t lin = (int64_t)gx + (int64_t)nx * ((int64_t)gy + (int64_t)ny * k0);
-
-    for (int k = k0; k < k1; ++k) {
-        const int q = k - k0 + 4;
-        const double *w0 = S.w[(q - 2) % 3], *w1 = S.w[(q - 1) % 3], *w2 = S.w[q % 3];
-        if (tx == 0) {  // one 128-byte row per field: warm L1 for the epilogue's loads
-            const double *pa = Uin + lin, *pb = U0 + lin;
+            const double Fz[5] = {F[0], F[2], F[3], F[1], F[4]};
+            if constexpr (BF) {
+                if (own && (!below || !above))
+                    bflux_add(g, B.bflux, 2, below ? 1 : 0, ecol, bscale, g.area[2], Fz);
+            }
+            // ---- flux divergence in the reference's order, then the update ----
+            const double az = g.area[2];
+            const int cz = (k == g.zw0 && g.zcls0 >= 0) ? g.zcls0 : lo_class(k, nz, perz);
+            const bool interior = cx == LO_BEFORE && cy == LO_BEFORE && cz == LO_BEFORE;
+            const double invV = ctrl->invV;
+            const double *gr = S.g[k & 1] + ty * (TX + 1) + tx;
+            const double *gq = S.g[k & 1] + 5 * FX + ty * TX + tx;
+            double un[5], acc[5];
 #pragma unroll
             for (int f = 0; f < 5; ++f) {
-                prefetch_l1(pa);
-                if constexpr (STAGE == 2) prefetch_l1(pb);
-                pa += g.ncell;
-                pb += g.ncell;
-            }
-        }
-        // ---- phase 1: plane k+2 to primitives; the CFL term of plane k-1; the
-        //      z face (warps 4..7) or the halo strips (warps 0..3) ----
-        double Fzhi[5];
-        {
-            double Wn[5];
-            consume(q, Wn, 2);
-            double cf = 0.0;
-            if constexpr (STAGE == 2) cf = cfl_term_exact<GRAV>(unp, g, invdt);
-            if (z_early) zsolve(k, w0 + o_c, w1 + o_c, Wn, Fzhi);
-            else halo_c2p(q);
-            if constexpr (STAGE == 2)
-                if (k > k0 && k > g.zw0 && k <= g.zw1) invdt = cf;  // plane k-1, if the slab's own
-        }
-        __syncthreads();  // (1) plane k+2 converted
-        if (stalled(q)) return;
-        release(q);
-        // ---- phase 2: the own lo x / lo y faces; the z face (warps 0..3) or
-        //      a hi-edge face (warps 6, 7) ----
-        if (z_early) {
-            xy_faces(w0, k);
-            if (warp >= 6 && lane < 16) edge_face(w0, k);
-        } else {
-            double W2[5];
-#pragma unroll
-            for (int f = 0; f < 5; ++f) W2[f] = w2[o_c + f * PC];
-            zsolve(k, w0 + o_c, w1 + o_c, W2, Fzhi);
-            xy_faces(w0, k);
-        }
-        __syncthreads();  // (2) fluxes ready
-
-        // ---- flux divergence in the reference's order, then the stage update ----
-        const int cz = (k == g.zw0 && g.zcls0 >= 0) ? g.zcls0 : lo_class(k, nz, perz);
-        const bool interior = cx == LO_BEFORE && cy == LO_BEFORE && cz == LO_BEFORE;
-        double un[5];
-        const bool inb = VB_DCHECK(lin >= 0 && lin < g.ncell);  // check build only
-        const double *pin = Uin + lin, *p0 = U0 + lin;
-        double *po = Uout + lin;
-        double acc[5];  // GRAV: the flux sums, completed by the gravity source
-#pragma unroll
-        for (int f = 0; f < 5; ++f) {
-            const double gxl = S.gx[f][ty * (TX + 1) + tx];
-            const double gxh = S.gx[f][ty * (TX + 1) + tx + 1];
-            const double gyl = S.gy[f][ty * TX + tx];
-            const double gyh = S.gy[f][(ty + 1) * TX + tx];
-            const double gzl = az * Fzlo[f], gzh = az * Fzhi[f];
-            double a = 0.0;
-            if (interior) {
-                a = a - gzl - gyl - gxl + gxh + gyh + gzh;
-            } else {
-                if (cz == LO_BEFORE) a -= gzl;
-                if (cy == LO_BEFORE) a -= gyl;
-                if (cx == LO_BEFORE) a -= gxl;
-                a += gxh;
-                if (cx == LO_SELF) a -= gxl;
-                a += gyh;
-                if (cy == LO_SELF) a -= gyl;
-                a += gzh;
-                if (cz == LO_SELF) a -= gzl;
-                if (cx == LO_AFTER) a -= gxl;
-                if (cy == LO_AFTER) a -= gyl;
-                if (cz == LO_AFTER) a -= gzl;
-            }
-            Fzlo[f] = Fzhi[f];
-            if constexpr (GRAV) {
+                const double gzh = az * Fz[f], gzl = S.fz[f][t];
+                S.fz[f][t] = gzh;
+                const double gxl = gr[f * FX], gxh = gr[f * FX + 1];
+                const double gyl = gq[f * FY], gyh = gq[f * FY + TX];
+                double a = 0.0;
+                if (interior) {
+                    a = a - gzl - gyl - gxl + gxh + gyh + gzh;
+                } else {
+                    if (cz == LO_BEFORE) a -= gzl;
+                    if (cy == LO_BEFORE) a -= gyl;
+                    if (cx == LO_BEFORE) a -= gxl;
+                    a += gxh;
+                    if (cx == LO_SELF) a -= gxl;
+                    a += gyh;
+                    if (cy == LO_SELF) a -= gyl;
+                    a += gzh;
+                    if (cz == LO_SELF) a -= gzl;
+                    if (cx == LO_AFTER) a -= gxl;
+                    if (cy == LO_AFTER) a -= gyl;
+                    if (cz == LO_AFTER) a -= gzl;
+                }
                 acc[f] = a;
-                continue;
             }
-            const double uin = inb ? __ldg(pin) : 0.0;
-            if constexpr (STAGE == 1) {
-                un[f] = uin - invV * a;
-            } else {
-                un[f] = 0.5 * (inb ? *p0 : 0.0) + 0.5 * (uin - invV * a);
+            cp_async_wait_all();
+            if (inb) {
+                if constexpr (GRAV) {  // the source from the stage state, after the fluxes
+                    double u[5];
+#pragma unroll
+                    for (int f = 0; f < 5; ++f)
+                        u[f] = STAGE == 1 ? r0[o_c + f * PC] : __ldg(Uin + lin + f * g.ncell);
+                    gravity_source<3>(g, lin, u, acc);
+                }
+#pragma unroll
+                for (int f = 0; f < 5; ++f) {
+                    const double ep = r0[o_c + f * PC];
+                    if constexpr (STAGE == 1) un[f] = ep - invV * acc[f];
+                    else un[f] = 0.5 * ep + 0.5 * (__ldg(Uin + lin + f * g.ncell) - invV * acc[f]);
+                    Uout[lin + f * g.ncell] = un[f];
+                }
+                if constexpr (STAGE == 2) {
+                    // the exact CFL term only of cells whose bound exceeds the
+                    // item's maximum so far (the slab's own planes)
+                    if (k >= g.zw0 && k < g.zw1) {
+                        const float b = cfl_bound<GRAV>(un, g, gf, iw0, iw1, iw2);
+                        if (!(b <= __int_as_float(*(volatile int *)&cfl_sh))) {
+                            cflm = cfl_term_exact<GRAV>(un, g, cflm);
+                            atomicMax(&cfl_sh, __float_as_int(__double2float_rd(cflm)));
+                        }
+                    }
+                }
             }
-            if (inb) *po = un[f];
-            pin += g.ncell;
-            p0 += g.ncell;
-            po += g.ncell;
+            if (k + 3 <= k1 + 1) fetch_plane(k + 3, r0);
+            cp_async_commit();
         }
-        if constexpr (GRAV) {  // the source from the stage state, after the fluxes
-            double u[5];
-#pragma unroll
-            for (int f = 0; f < 5; ++f) u[f] = inb ? __ldg(pin + f * g.ncell) : 0.0;
-            if (inb) gravity_source<3>(g, lin, u, acc);
-#pragma unroll
-            for (int f = 0; f < 5; ++f) {
-                if constexpr (STAGE == 1) un[f] = u[f] - invV * acc[f];
-                else un[f] = 0.5 * (inb ? p0[f * g.ncell] : 0.0) + 0.5 * (u[f] - invV * acc[f]);
-                if (inb) po[f * g.ncell] = un[f];
-            }
-        }
-        lin += plane_cells;
-        if constexpr (STAGE == 2) {
-#pragma unroll
-            for (int f = 0; f < 5; ++f) unp[f] = un[f];
-        }
+        __syncthreads();  // faces of plane k+1 and primitives of plane k+2 are ready
+        double *rt = r0;
+        r0 = r1;
+        r1 = r2;
+        r2 = rt;
     }
-    if constexpr (STAGE == 2)  // the item's last plane, when it is one of the slab's own
-        if (k1 - 1 >= g.zw0 && k1 - 1 < g.zw1) invdt = cfl_term_exact<GRAV>(unp, g, invdt);
-    qb += nplanes;
-    if constexpr (STAGE == 2) block_max_to(&ctrl->invdt_bits, invdt, red);  // this box's CFL max
+    cp_async_wait_all();
+    if constexpr (STAGE == 2) block_max_to(&ctrl->invdt_bits, cflm, red);  // this box's CFL max
     }  // work items
 }
 
-template <int NS>
-int launch_tiled3d_f64(const BoxDesc *hbox, const BoxDesc *boxes, const int *item_box,
-                       int nitems, unsigned int *work, int stage, cudaStream_t s, bool grav,
-                       bool bf)
+// Boxes the kernel takes: 16 x 16 tiles, the last one shifted back.
+inline int launch_tiled3d_f64(const BoxDesc *hbox, const BoxDesc *boxes, const int *item_box,
+                              int nitems, unsigned int *work, int stage, cudaStream_t s, bool grav,
+                              bool bf)
 {
-    const size_t smem = sizeof(t3d::Smem<NS>);
+    const size_t smem = sizeof(t3d::Smem);
     static int res1 = 0, resb = 0, resg = 0, resf = 0;
-    if (!res1) res1 = persistent_blocks(k_stage_tiled3d_f64<NS, 1, false>,
-                                        k_stage_tiled3d_f64<NS, 2, false>, smem);
-    if (!resb) resb = persistent_blocks(k_stage_tiled3d_f64<NS, 1, true>,
-                                        k_stage_tiled3d_f64<NS, 2, true>, smem);
-    if (!resg) resg = persistent_blocks(k_stage_tiled3d_f64<NS, 1, false, true>,
-                                        k_stage_tiled3d_f64<NS, 2, false, true>, smem);
-    if (!resf) resf = persistent_blocks(k_stage_tiled3d_f64<NS, 1, false, false, true>,
-                                        k_stage_tiled3d_f64<NS, 2, false, false, true>, smem);
+    if (!res1) res1 = persistent_blocks(k_stage_tiled3d_f64<1, false>, k_stage_tiled3d_f64<2, false>,
+                                        smem, t3d::NTH);
+    if (!resb) resb = persistent_blocks(k_stage_tiled3d_f64<1, true>, k_stage_tiled3d_f64<2, true>,
+                                        smem, t3d::NTH);
+    if (!resg) resg = persistent_blocks(k_stage_tiled3d_f64<1, false, true>,
+                                        k_stage_tiled3d_f64<2, false, true>, smem, t3d::NTH);
+    if (!resf) resf = persistent_blocks(k_stage_tiled3d_f64<1, false, false, true>,
+                                        k_stage_tiled3d_f64<2, false, false, true>, smem, t3d::NTH);
     if ((grav || bf) && !hbox) return -1;  // gravity, boundary fluxes: single boxes only
     if (grav && bf) return -1;
     if (bf && !hbox->bflux) return -1;
@@ -493,22 +477,15 @@ int launch_tiled3d_f64(const BoxDesc *hbox, const BoxDesc *boxes, const int *ite
     BoxDesc box0;
     if (hbox) box0 = *hbox;
     else std::memset(&box0, 0, sizeof box0);
-    if (grav && stage == 1)
-        k_stage_tiled3d_f64<NS, 1, false, true><<<grid, t3::NT, smem, s>>>(box0, nullptr, nullptr, nitems, work);
-    else if (grav)
-        k_stage_tiled3d_f64<NS, 2, false, true><<<grid, t3::NT, smem, s>>>(box0, nullptr, nullptr, nitems, work);
-    else if (bf && stage == 1)
-        k_stage_tiled3d_f64<NS, 1, false, false, true><<<grid, t3::NT, smem, s>>>(box0, nullptr, nullptr, nitems, work);
+    auto go = [&](auto k1, auto k2, const BoxDesc *tab, const int *ib) {
+        if (stage == 1) k1<<<grid, t3d::NTH, smem, s>>>(box0, tab, ib, nitems, work);
+        else k2<<<grid, t3d::NTH, smem, s>>>(box0, tab, ib, nitems, work);
+    };
+    if (grav) go(k_stage_tiled3d_f64<1, false, true>, k_stage_tiled3d_f64<2, false, true>, nullptr, nullptr);
     else if (bf)
-        k_stage_tiled3d_f64<NS, 2, false, false, true><<<grid, t3::NT, smem, s>>>(box0, nullptr, nullptr, nitems, work);
-    else if (hbox && stage == 1)
-        k_stage_tiled3d_f64<NS, 1, false><<<grid, t3::NT, smem, s>>>(box0, nullptr, nullptr, nitems, work);
-    else if (hbox)
-        k_stage_tiled3d_f64<NS, 2, false><<<grid, t3::NT, smem, s>>>(box0, nullptr, nullptr, nitems, work);
-    else if (stage == 1)
-        k_stage_tiled3d_f64<NS, 1, true><<<grid, t3::NT, smem, s>>>(box0, boxes, item_box, nitems, work);
-    else
-        k_stage_tiled3d_f64<NS, 2, true><<<grid, t3::NT, smem, s>>>(box0, boxes, item_box, nitems, work);
+        go(k_stage_tiled3d_f64<1, false, false, true>, k_stage_tiled3d_f64<2, false, false, true>, nullptr, nullptr);
+    else if (hbox) go(k_stage_tiled3d_f64<1, false>, k_stage_tiled3d_f64<2, false>, nullptr, nullptr);
+    else go(k_stage_tiled3d_f64<1, true>, k_stage_tiled3d_f64<2, true>, boxes, item_box);
     return 1;
 }
 
