@@ -4,7 +4,7 @@
 #include "vb_launch.h"
 #include "vb_stage_generic.cuh"
 #include "vb_stage_tiled3d_mixed.cuh"
-#include "vb_stage_tiled2d.cuh"
+#include "vb_stage_tiled2d_mixed.cuh"
 
 namespace vb {
 
@@ -34,7 +34,7 @@ int launch_stage_tiled3d_mixed(const BoxDesc *hbox, const BoxDesc *boxes, const 
 int launch_stage_tiled2d_mixed(const BoxDesc *hbox, int nitems, unsigned int *work, int stage,
                                cudaStream_t s, bool bf)
 {
-    return launch_tiled2d<true, 2>(hbox, nitems, work, stage, s, bf);
+    return launch_tiled2d_mixed<2>(hbox, nitems, work, stage, s, bf);
 }
 
 int launch_stage_mixed(const Geom &g, int stage, const double *Uin, const double *U0,

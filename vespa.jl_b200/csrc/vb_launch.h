@@ -83,11 +83,21 @@ inline bool tiled3d_supported(const Geom &g)
 }
 
 // Ragged 3D boxes with room for one tile: a side that is no multiple of 16 ends
-// in a shifted tile (float64 kernel, whose loads need no alignment).
+// in a shifted tile.  The float64 kernel's loads need no alignment; the mixed
+// one's TMA copies start at even x and fetch two halo rows at once, so it takes
+// even nx and leaves out the ny whose second-last tile has one halo row inside
+// the grid and one beyond it.
 inline bool tiled3d_ragged(const Geom &g, int precision)
 {
     return g.nd == 3 && g.n[0] >= 16 && g.n[1] >= 16 && g.n[2] >= 2 && g.n[0] <= (1 << 30) &&
-           g.n[1] <= (1 << 30) && g.n[2] <= (1 << 30) && precision == PREC_FP64;
+           g.n[1] <= (1 << 30) && g.n[2] <= (1 << 30) &&
+           (precision == PREC_FP64 || (g.n[0] % 2 == 0 && g.n[1] % 16 != 1));
+}
+// Ragged 2D grids of the mixed kernel: even rows with room for one segment.
+inline bool tiled2d_ragged(const Geom &g, int precision)
+{
+    return precision == PREC_MIXED && g.nd == 2 && g.n[0] >= 256 && g.n[0] % 2 == 0 &&
+           g.n[1] >= 2 && g.n[0] <= (1 << 30) && g.n[1] <= (1 << 30);
 }
 
 // Tiled 2D path applicability: 256-cell row segments marching y.
@@ -100,14 +110,14 @@ inline bool tiled_supported(const Geom &g) { return tiled3d_supported(g) || tile
 // what a single grid may take automatically
 inline bool tiled_any(const Geom &g, int precision)
 {
-    return tiled_supported(g) || tiled3d_ragged(g, precision);
+    return tiled_supported(g) || tiled3d_ragged(g, precision) || tiled2d_ragged(g, precision);
 }
 // cells along the marching axis (z in 3D, y in 2D)
 inline int64_t march_extent(const Geom &g) { return g.nd == 3 ? g.n[2] : g.n[1]; }
 
 // vb_kern_fp64.cu (compiled with -fmad=false)
 // bflux: the outer boundary-flux planes being recorded (or null); bflux_int:
-// the interior face register [axis][5][ncell] (or null).
+// the interior face register [axis][5][ncell] (or null).  
 int launch_stage_fp64(const Geom &g, int stage, const double *Uin, const double *U0,
                       double *Uout, Ctrl *ctrl, double *bflux, cudaStream_t s,
                       double *bflux_int = nullptr);

@@ -12,14 +12,14 @@
 //     rather than exchanged, which saves a barrier per plane) and solves the
 //     pair as one packed float32x2 HLLC (vb_hllc_x2.cuh, faces rotated into
 //     their normal frame); warp 7 adds the tile's hi-edge faces;
-//   - the z face runs in registers down the thread's column, solved before
-//     the plane's first barrier by warps 4..7 and after it by warps 0..3, so
-//     that it balances the halo conversions (warps 0..3) and the edge faces
-//     (warp 7) across the two phases;
-//   - x/y face fluxes are stored once in float32 and multiplied by the face
-//     area in float64 where the divergence reads them;
-//     the flux divergence and the stage update stay in float64.
-// Two barriers per plane: (1) plane k+2 converted, (2) fluxes of plane k ready.
+//   - the z face runs in registers down the thread's column;
+//   - x/y face fluxes are stored once in float32, in one of two buffers: the
+//     faces of plane k+1 are solved while plane k is updated, so one barrier a
+//     plane suffices (two cost 17 % of the warps' time in waits);
+//   - the update takes the difference of a cell's two fluxes per axis in
+//     float64 (exact for float32 values) and scales it once by dt/V * area.
+// The last tile of a side that is no multiple of 16 is shifted back inside the
+// grid; the cells it shares with the tile before it are not written.
 #pragma once
 
 #include "vb_hllc_x2.cuh"
@@ -55,8 +55,8 @@ struct Smem {
     double u[NS][t3::UPLANE];  // TMA stage buffers (raw conserved state)
     double ep[2][5][NT];       // own-cell epilogue inputs (Uin, U0), fetched by cp.async
     float w[3][PSLOT];         // primitive ring
-    float gx[5][TY * (TX + 1)];  // x-face flux (float32; times the area in the epilogue)
-    float gy[5][(TY + 1) * TX];  // y-face flux
+    float gx[2][5][TY * (TX + 1)];  // x-face fluxes of a plane, by the plane's parity
+    float gy[2][5][(TY + 1) * TX];  // y-face fluxes
     uint64_t bar[NS];
 };
 
@@ -209,10 +209,6 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
                     : t < 64 ? wxs(TX + (t & 1), (t - 32) >> 1)
                     : t < 96 ? wrow((t - 64) & 15, -2 + ((t - 64) >> 4))
                              : wrow((t - 96) & 15, TY + ((t - 96) >> 4));
-    // the z face is solved before barrier (1) by warps 4..7 (balancing the
-    // halo conversions of warps 0..3) and after it by warps 0..3 (balancing
-    // the tile's hi-edge faces, solved by warp 7)
-    const bool z_early = warp >= 4;
 
     if (t == 0) {
         for (int s = 0; s < NS; ++s) mbar_init(&S.bar[s], 1);
@@ -248,6 +244,7 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
     const double invV = ctrl->invV;
     const double bscale = BF ? 0.5 * ctrl->dt : 0.0;  // boundary-flux stage weight
     const double ax = g.area[0], ay = g.area[1], az = g.area[2];
+    const double sx = __dmul_rn(invV, ax), sy = __dmul_rn(invV, ay), sz = __dmul_rn(invV, az);
     const int bx_lo = g.bc_lo[0], bx_hi = g.bc_hi[0], by_lo = g.bc_lo[1], by_hi = g.bc_hi[1];
     const int bz_lo = g.bc_lo[2], bz_hi = g.bc_hi[2];
     double invdt = 0.0;
@@ -255,7 +252,9 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
     const float iw0 = (float)g.invw[0], iw1 = (float)g.invw[1], iw2 = (float)g.invw[2];
     const int local = item - B.item0;
     const int tile = local % ntiles;
-    const int x0 = (tile % ntx) * TX, y0 = (tile / ntx) * TY;
+    const int xn = (tile % ntx) * TX, yn = (tile / ntx) * TY;
+    const int x0 = min(xn, nx - TX), y0 = min(yn, ny - TY);  // a shifted last tile
+    const bool own = x0 + tx >= xn && y0 + ty >= yn;         // this thread updates its column
     int k0, k1;
     chunk_span(nz, kz, B.nchu, local / ntiles, k0, k1);
     const int nplanes = (k1 - k0) + 4;
@@ -393,7 +392,7 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
             float gst[5];
             ghost_state<float>(loz, bz_lo, 2, gst);
             hllc_flux_fast_bf<3>(gst, loz, gf, ig1, Fzlo);
-            if constexpr (BF) {  // z-lo domain face of cell (x, y, 0)
+            if (BF && own) {  // z-lo domain face of cell (x, y, 0)
                 const double Fd[5] = {Fzlo[0], Fzlo[1], Fzlo[2], Fzlo[3], Fzlo[4]};
                 bflux_add(g, B.bflux, 2, 0, (int64_t)(x0 + tx) + (int64_t)nx * (y0 + ty), bscale, az, Fd);
             }
@@ -432,7 +431,7 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
         }
         hllc_flux_fast_bf<3>(hz, zr, gf, ig1, Fzhi);
         if constexpr (BF) {
-            if (!perz && k + 1 >= nz) {  // z-hi domain face of cell (x, y, nz-1)
+            if (own && !perz && k + 1 >= nz) {  // z-hi domain face of cell (x, y, nz-1)
                 const double Fd[5] = {Fzhi[0], Fzhi[1], Fzhi[2], Fzhi[3], Fzhi[4]};
                 bflux_add(g, B.bflux, 2, 1, (int64_t)(x0 + tx) + (int64_t)nx * (y0 + ty), bscale, az, Fd);
             }
@@ -446,13 +445,13 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
         face_pair(w0, ox, oy, L, R);
         f2 F[5];
         hllc_x2(L, R, gf, ig1, F);
-        store_pair(S.gx, S.gy, ty * (TX + 1) + tx, ty * TX + tx, F);
+        store_pair(S.gx[k & 1], S.gy[k & 1], ty * (TX + 1) + tx, ty * TX + tx, F);
         if constexpr (BF) {
-            if (xlo_bnd && tx == 0) {  // x-lo domain face of cell (0, y, k)
+            if (own && xlo_bnd && tx == 0) {  // x-lo domain face of cell (0, y, k)
                 const double Fd[5] = {F[0].v.x, F[1].v.x, F[2].v.x, F[3].v.x, F[4].v.x};
                 bflux_add(g, B.bflux, 0, 0, (int64_t)(y0 + ty) + (int64_t)ny * k, bscale, ax, Fd);
             }
-            if (ylo_bnd && ty == 0) {  // y-lo domain face of cell (x, 0, k), un-rotated
+            if (own && ylo_bnd && ty == 0) {  // y-lo domain face of cell (x, 0, k), un-rotated
                 const double Fd[5] = {F[0].v.y, F[2].v.y, F[1].v.y, F[3].v.y, F[4].v.y};
                 bflux_add(g, B.bflux, 1, 0, (int64_t)(x0 + tx) + (int64_t)nx * k, bscale, ay, Fd);
             }
@@ -467,13 +466,13 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
         face_pair(w0, ex, ey, L, R);
         f2 F[5];
         hllc_x2(L, R, gf, ig1, F);
-        store_pair(S.gx, S.gy, j * (TX + 1) + TX, TY * TX + j, F);
+        store_pair(S.gx[k & 1], S.gy[k & 1], j * (TX + 1) + TX, TY * TX + j, F);
         if constexpr (BF) {
-            if (xhi_bnd) {  // x-hi domain face of cell (nx-1, y0+j, k)
+            if (xhi_bnd && y0 + j >= yn) {  // x-hi domain face of cell (nx-1, y0+j, k)
                 const double Fd[5] = {F[0].v.x, F[1].v.x, F[2].v.x, F[3].v.x, F[4].v.x};
                 bflux_add(g, B.bflux, 0, 1, (int64_t)(y0 + j) + (int64_t)ny * k, bscale, ax, Fd);
             }
-            if (yhi_bnd) {  // y-hi domain face of cell (x0+j, ny-1, k)
+            if (yhi_bnd && x0 + j >= xn) {  // y-hi domain face of cell (x0+j, ny-1, k)
                 const double Fd[5] = {F[0].v.y, F[2].v.y, F[1].v.y, F[3].v.y, F[4].v.y};
                 bflux_add(g, B.bflux, 1, 1, (int64_t)(x0 + j) + (int64_t)nx * k, bscale, ay, Fd);
             }
@@ -481,7 +480,6 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
     };
 
     const int gx = x0 + tx, gy = y0 + ty;
-    const int cx = lo_class(gx, nx, perx), cy = lo_class(gy, ny, pery);
     // previous plane's new state: its CFL term is folded one plane later (the
     // initial value is a finite placeholder whose term is discarded)
     double unp[5] = {1.0, 0.0, 0.0, 0.0, 1.0};
@@ -489,10 +487,12 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
     int64_t lin = (int64_t)gx + (int64_t)nx * ((int64_t)gy + (int64_t)ny * k0);
 
     float *r0 = S.w[2], *r1 = S.w[0], *r2 = S.w[1];  // ring slots of planes k, k+1, k+2
+    xy_faces(r0, k0);
+    if (warp == 7 && lane < 16) edge_faces(r0, k0);
+    __syncthreads();
     for (int k = k0; k < k1; ++k) {
         const int q = k - k0 + 4;
-        const float *w0 = r0, *w1 = r1, *w2 = r2;
-        const bool inb = VB_DCHECK(lin >= 0 && lin < g.ncell);  // check build only
+        const bool inb = own && VB_DCHECK(lin >= 0 && lin < g.ncell);  // check build only
         if (inb) {
             const double *pa = Uin + lin, *pb = U0 + lin;
 #pragma unroll
@@ -504,84 +504,44 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
             }
         }
         cp_async_commit();
-        // ---- phase 1: plane k+2 to primitives; the CFL term of plane k-1; the
-        //      z face (warps 4..7) or the halo strips (warps 0..3) ----
+        // ---- the x / y faces of plane k+1 ----
+        if (k + 1 < k1) {
+            xy_faces(r1, k + 1);
+            if (warp == 7 && lane < 16) edge_faces(r1, k + 1);
+        }
+        // ---- plane k+2 to primitives; the CFL term of plane k-1; the z face ----
         float Fzhi[5];
         {
             float Wn[5];
             consume(q, Wn, 2, r2);
-            float cf = 0.f;
-            if constexpr (STAGE == 2) cf = cfl_mixed<GRAV>(unp, g, gf, iw0, iw1, iw2, invdtf);
-            if (z_early) {
-                zsolve(k, w0 + o_c, w1 + o_c, Wn, Fzhi);
-            } else {
-                halo_c2p(q, r2);
+            if (k + 2 < k1) halo_c2p(q, r2);
+            if constexpr (STAGE == 2) {
+                const float cf = cfl_mixed<GRAV>(unp, g, gf, iw0, iw1, iw2, invdtf);
+                if (own && k > k0 && k > g.zw0 && k <= g.zw1) invdtf = cf;  // plane k-1, if the slab's own
             }
-            if constexpr (STAGE == 2)
-                if (k > k0 && k > g.zw0 && k <= g.zw1) invdtf = cf;  // plane k-1, if the slab's own
+            zsolve(k, r0 + o_c, r1 + o_c, Wn, Fzhi);
         }
-        __syncthreads();  // (1) plane k+2 converted
-        if (stalled(q)) return;
-        release(q);
-        // ---- phase 2: the own lo x / lo y face pair; the z face (warps 0..3)
-        //      or the tile's hi-edge faces (warp 7) ----
-        if (z_early) {
-            xy_faces(w0, k);
-            if (warp == 7 && lane < 16) edge_faces(w0, k);
-        } else {
-            float W2[5];
-#pragma unroll
-            for (int f = 0; f < 5; ++f) W2[f] = w2[o_c + f * PC];
-            zsolve(k, w0 + o_c, w1 + o_c, W2, Fzhi);
-            xy_faces(w0, k);
-        }
-        __syncthreads();  // (2) fluxes ready
-
-        // ---- flux divergence (float64, reference order) and the stage update ----
-        const int cz = (k == g.zw0 && g.zcls0 >= 0) ? g.zcls0 : lo_class(k, nz, perz);
-        const bool interior = cx == LO_BEFORE && cy == LO_BEFORE && cz == LO_BEFORE;
+        // ---- the stage update from plane k's fluxes (solved one iteration ago) ----
+        const float (*fx)[TY * (TX + 1)] = S.gx[k & 1];
+        const float (*fy)[(TY + 1) * TX] = S.gy[k & 1];
         double un[5];
         double *po = Uout + lin;
         double acc[5];  // GRAV: the flux sums, completed by the gravity source
         cp_async_wait_all();  // this thread's own epilogue inputs have landed
 #pragma unroll
         for (int f = 0; f < 5; ++f) {
-            const double gxl = __dmul_rn(ax, (double)S.gx[f][ty * (TX + 1) + tx]);
-            const double gxh = __dmul_rn(ax, (double)S.gx[f][ty * (TX + 1) + tx + 1]);
-            const double gyl = __dmul_rn(ay, (double)S.gy[f][ty * TX + tx]);
-            const double gyh = __dmul_rn(ay, (double)S.gy[f][(ty + 1) * TX + tx]);
+            const double dx = (double)fx[f][ty * (TX + 1) + tx + 1] - (double)fx[f][ty * (TX + 1) + tx];
+            const double dy = (double)fy[f][(ty + 1) * TX + tx] - (double)fy[f][ty * TX + tx];
+            const double dz = (double)Fzhi[f] - (double)fzl[f];
+            fzl[f] = Fzhi[f];
             // explicit roundings: the result must not depend on how the compiler
             // contracts this code in each kernel instantiation
-            const double gzh = __dmul_rn(az, (double)Fzhi[f]);
-            const double gz0 = __dmul_rn(az, (double)fzl[f]);
-            double a = 0.0;
-            if (interior) {
-                a = a - gz0 - gyl - gxl + gxh + gyh + gzh;
-            } else {
-                if (cz == LO_BEFORE) a -= gz0;
-                if (cy == LO_BEFORE) a -= gyl;
-                if (cx == LO_BEFORE) a -= gxl;
-                a += gxh;
-                if (cx == LO_SELF) a -= gxl;
-                a += gyh;
-                if (cy == LO_SELF) a -= gyl;
-                a += gzh;
-                if (cz == LO_SELF) a -= gz0;
-                if (cx == LO_AFTER) a -= gxl;
-                if (cy == LO_AFTER) a -= gyl;
-                if (cz == LO_AFTER) a -= gz0;
-            }
-            fzl[f] = Fzhi[f];
             if constexpr (GRAV) {
-                acc[f] = a;
+                acc[f] = __fma_rn(az, dz, __fma_rn(ay, dy, __dmul_rn(ax, dx)));
                 continue;
             }
-            if constexpr (STAGE == 1) {
-                un[f] = __fma_rn(-invV, a, S.ep[0][f][t]);
-            } else {
-                un[f] = __fma_rn(0.5, S.ep[1][f][t],
-                                 __dmul_rn(0.5, __fma_rn(-invV, a, S.ep[0][f][t])));
-            }
+            const double u = __fma_rn(-sz, dz, __fma_rn(-sy, dy, __fma_rn(-sx, dx, S.ep[0][f][t])));
+            un[f] = STAGE == 1 ? u : __dmul_rn(0.5, __dadd_rn(S.ep[1][f][t], u));
             if (inb) *po = un[f];
             po += g.ncell;
         }
@@ -602,13 +562,16 @@ k_stage_tiled3d_mixed(const __grid_constant__ BoxDesc box0, const BoxDesc *__res
 #pragma unroll
             for (int f = 0; f < 5; ++f) unp[f] = un[f];
         }
+        __syncthreads();  // plane k+2 converted, faces of plane k+1 solved, those of k read
+        if (stalled(q)) return;
+        release(q);
         float *rt = r0;
         r0 = r1;
         r1 = r2;
         r2 = rt;
     }
     if constexpr (STAGE == 2)  // the item's last plane
-        invdt = (k1 - 1 >= g.zw0 && k1 - 1 < g.zw1)
+        invdt = (own && k1 - 1 >= g.zw0 && k1 - 1 < g.zw1)
                     ? (double)cfl_mixed<GRAV>(unp, g, gf, iw0, iw1, iw2, invdtf)
                     : (double)invdtf;
     qb += nplanes;
