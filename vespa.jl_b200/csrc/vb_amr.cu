@@ -44,6 +44,7 @@ struct vb_amr {
     // leaf-indexed device buffers (stride cap)
     int64_t cap = 0;
     double *U = nullptr, *U1 = nullptr, *reg = nullptr;
+    double *W = nullptr;                        // primitives of the single-rate loop
     int *lev = nullptr, *cx = nullptr;          // level, [3][cap] coordinates
     double *U2 = nullptr;                       // refinement targets, swapped in
     int *lev2 = nullptr, *cx2 = nullptr;
@@ -91,7 +92,7 @@ void release(vb_amr *a)
     if (a->sg_exec) cudaGraphExecDestroy(a->sg_exec);
     cudaFree(a->sub);
     cudaFree(a->suberr);
-    void *p[] = {a->U, a->U1, a->U2, a->lev2, a->cx2, a->reg, a->lev, a->cx, a->rep, a->faceid, a->kind, a->off,
+    void *p[] = {a->U, a->U1, a->U2, a->lev2, a->cx2, a->reg, a->W, a->lev, a->cx, a->rep, a->faceid, a->kind, a->off,
                  a->fbase, a->cnt, a->fcnt, a->ecnt, a->bsum, a->tag, a->F, a->farea,
                  a->fL, a->fR, a->ent, a->fax, a->hkey, a->hval, a->word, a->ctrl,
                  a->partials, a->totals};
@@ -122,6 +123,7 @@ int alloc_leaf_buffers(vb_amr *a, int64_t c)
     if (!rc) rc = realloc_dev(&a->lev2, c, a->ctx->stream);
     if (!rc) rc = realloc_dev(&a->cx2, 3 * c, a->ctx->stream);
     if (!rc) rc = realloc_dev(&a->reg, 5 * c, a->ctx->stream);
+    if (!rc) rc = realloc_dev(&a->W, 5 * c, a->ctx->stream);
     if (!rc) rc = realloc_dev(&a->rep, 6 * c, a->ctx->stream);
     if (!rc) rc = realloc_dev(&a->faceid, 6 * c, a->ctx->stream);
     if (!rc) rc = realloc_dev(&a->kind, 6 * c, a->ctx->stream);
@@ -246,6 +248,7 @@ int build_tables(vb_amr *a)
     m.off = a->off;
     m.ent = a->ent;
     m.reg = a->reg;
+    m.W = a->W;
     ++a->table_version;  // kernels capture the tables by value: graphs are stale
     return VB_OK;
 }
@@ -884,16 +887,17 @@ int vb_amr_evolve(vb_amr *a, double tfinal, int64_t max_steps, double refine_abo
             // pull below has synchronised the stream
             VB_CUDA(cudaMemcpyAsync(a->ctrl, a->hctrl, sizeof(vb::Ctrl), cudaMemcpyHostToDevice, st));
             VB_CUDA(cudaMemsetAsync(&a->ctrl->invdt_bits, 0, sizeof(unsigned long long), st));
-            VB_CHECK_LAUNCH(a->ctx, vb::launch_amr_cfl(a->dev, a->U, -1, a->ctrl, st));
+            VB_CHECK_LAUNCH(a->ctx, vb::launch_amr_prims(a->dev, a->U, a->ctrl, st));
+            VB_CHECK_LAUNCH(a->ctx, vb::launch_finalize_cfl(gq, a->ctrl, st));
             vb::AmrStageArgs s{};
             s.level = -1;
             s.cfl_all = 1;
             s.dt = -1.0;  // read from the control block
+            s.loop = 1;
+            s.cfl = a->g.cfl;
             for (int64_t k = 0; k < chunk; ++k) {
-                VB_CHECK_LAUNCH(a->ctx, vb::launch_finalize_cfl(gq, a->ctrl, st));
                 VB_CHECK_LAUNCH(a->ctx, vb::launch_amr_stage(a->dev, 1, a->U, a->U, a->U1, a->F, s, a->ctrl, st));
                 VB_CHECK_LAUNCH(a->ctx, vb::launch_amr_stage(a->dev, 2, a->U1, a->U, a->U, a->F, s, a->ctrl, st));
-                VB_CHECK_LAUNCH(a->ctx, vb::launch_advance(a->ctrl, st));
             }
             rc = pull_ctrl(a);
             if (rc) return rc;

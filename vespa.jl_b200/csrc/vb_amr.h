@@ -24,6 +24,7 @@ struct AmrDev {
     const int *off;       // CSR offsets, nleaf+1
     const int *ent;       // CSR entries: face*2 + (1 if the leaf is the face's right side)
     double *reg;          // flux registers, [5][cap]
+    double *W;            // primitives of the stage input, [5][cap] (single-rate loop)
     double vol[AMR_MAX_LEVEL + 1];
     double w[AMR_MAX_LEVEL + 1][3];
 };
@@ -42,6 +43,12 @@ struct AmrStageArgs {
     // the device) and reg_scale holds the register signs (+1 / -1), the scale
     // being sign * (0.5 * dt) as evolve_level! forms it
     const double *dt_dev;
+    // the single-rate loop (level -1, dt in the control block): faces read the
+    // primitives from AmrDev::W, cells leave those of the state they write
+    // there, and stage 2's last block advances the clock and sets the next
+    // step's dt (cfl: the Courant number)
+    int loop;
+    double cfl;
 };
 
 // Device state of one level of a subcycled root step (evolve_level!,
@@ -100,6 +107,9 @@ int launch_amr_csr_fill(const AmrTopo &t, const int8_t *kind, const int *rep, co
 int launch_amr_stage(const AmrDev &m, int stage, const double *Uin, const double *U0,
                      double *Uout, double *F, const AmrStageArgs &a, Ctrl *ctrl, cudaStream_t s);
 int launch_amr_cfl(const AmrDev &m, const double *U, int level, Ctrl *ctrl, cudaStream_t s);
+// Start of the single-rate loop: primitives of every leaf into AmrDev::W and
+// the CFL maximum over them.
+int launch_amr_prims(const AmrDev &m, const double *U, Ctrl *ctrl, cudaStream_t s);
 // The same maximum into the word `bits` (not reset here).
 int launch_amr_cfl_bits(const AmrDev &m, const double *U, int level, unsigned long long *bits,
                         cudaStream_t s);

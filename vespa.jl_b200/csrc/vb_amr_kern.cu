@@ -13,6 +13,14 @@
 // One RK2 stage is two launches: k_amr_faces (one thread per face: PLM face
 // states, HLLC) and k_amr_cells (one thread per leaf: ordered flux
 // divergence, flux-register capture, stage update, CFL maximum).
+//
+// The single-rate loop runs them as k_amr_faces_loop and k_amr_cells_loop.
+// With a few 10^4 leaves a launch is one wave of dependent loads, so these are
+// launched programmatically: a kernel starts while the one before it still
+// runs, reads the mesh tables (which no stage writes), and waits only then.
+// Primitives come from an array the cells keep (not six conversions a face),
+// and the last block of stage 2 advances the clock and sets the next dt in
+// place of two more launches.
 #include "vb_amr.h"
 #include "vb_physics.cuh"
 
@@ -79,6 +87,168 @@ __global__ void __launch_bounds__(256) k_amr_faces(AmrDev m, const double *__res
     case 0: amr_face<1>(m, U, f, F); break;
     case 1: amr_face<2>(m, U, f, F); break;
     default: amr_face<3>(m, U, f, F); break;
+    }
+}
+
+// The same for the single-rate loop: the states in the face-normal frame, from
+// the primitives m.W.
+__global__ void __launch_bounds__(128) k_amr_faces_loop(AmrDev m, double *__restrict__ F, const Ctrl *ctrl)
+{
+    cudaTriggerProgrammaticLaunchCompletion();
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    int L = -1, R = -1, ax = 0, nb[4] = {-1, -1, -1, -1};
+    bool in = f < m.nface;
+    if (in) {
+        L = m.fL[f];
+        R = m.fR[f];
+        ax = m.fax[f];
+        in = VB_DCHECK(L < m.nleaf && R < m.nleaf && (L >= 0 || R >= 0));  // check build only
+        if (in && L >= 0) {
+            nb[0] = m.rep[(2 * ax) * m.cap + L];
+            nb[1] = m.rep[(2 * ax + 1) * m.cap + L];
+        }
+        if (in && R >= 0) {
+            nb[2] = m.rep[(2 * ax) * m.cap + R];
+            nb[3] = m.rep[(2 * ax + 1) * m.cap + R];
+        }
+    }
+    cudaGridDependencySynchronize();
+    if (!in || !ctrl->active) return;
+    const int64_t fo[5] = {0, (1 + ax) * m.cap, (ax == 0 ? 2 : 1) * m.cap, (ax == 2 ? 2 : 3) * m.cap,
+                           4 * m.cap};
+    const double *__restrict__ W = m.W;
+    const bool rlo = m.bc_lo[ax] == BC_REFLECTING, rhi = m.bc_hi[ax] == BC_REFLECTING;
+    // face value of leaf i (representatives jl, jr) on its hi (h = 0.5) or lo side
+    auto value = [&](int i, int jl, int jr, double h, double out[5]) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            const double c = W[fo[k] + i];
+            const double l = jl >= 0 ? W[fo[k] + jl] : (k == 1 && rlo ? -c : c);
+            const double r = jr >= 0 ? W[fo[k] + jr] : (k == 1 && rhi ? -c : c);
+            out[k] = face_val(c, h, limited_slope<double>(l, c, r));
+        }
+    };
+    double WL[5], WR[5], out[5];
+    if (L >= 0) value(L, nb[0], nb[1], 0.5, WL);
+    if (R >= 0) value(R, nb[2], nb[3], -0.5, WR);
+    if (R < 0) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) WR[k] = k == 1 && rhi ? -WL[k] : WL[k];
+    } else if (L < 0) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) WL[k] = k == 1 && rlo ? -WR[k] : WR[k];
+    }
+    const double ig1 = inv_gamma1(m.gamma);
+    if (ax == 2) hllc_frame<true>(WL, WR, m.gamma, ig1, out);
+    else hllc_frame<false>(WL, WR, m.gamma, ig1, out);
+    const int64_t oo[5] = {0, (1 + ax) * m.fcap, (ax == 0 ? 2 : 1) * m.fcap, (ax == 2 ? 2 : 3) * m.fcap,
+                           4 * m.fcap};
+#pragma unroll
+    for (int k = 0; k < 5; ++k) F[oo[k] + f] = out[k];
+}
+
+// One stage of the single-rate loop over every leaf.
+template <int STAGE>
+__global__ void __launch_bounds__(128)
+k_amr_cells_loop(AmrDev m, const double *__restrict__ Uin, const double *U0, double *Uout,
+                 const double *__restrict__ F, double cfl, Ctrl *ctrl)
+{
+    __shared__ double red[32];
+    cudaTriggerProgrammaticLaunchCompletion();
+    constexpr int NE = 4;  // entries whose fluxes are loaded together
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int li = 0, e0 = 0, e1 = 0, code[NE];
+    double ar[NE];
+    auto entries = [&](int e) {  // codes and areas of entries e .. e + NE - 1
+#pragma unroll
+        for (int j = 0; j < NE; ++j) {
+            code[j] = -1;
+            ar[j] = 0.0;
+            if (e + j < e1 && VB_DCHECK(e + j >= 0 && e + j < m.nent)) {
+                const int c = m.ent[e + j];
+                if (VB_DCHECK((c >> 1) >= 0 && (c >> 1) < m.nface)) {
+                    code[j] = c;
+                    ar[j] = m.farea[c >> 1];
+                }
+            }
+        }
+    };
+    if (i < m.nleaf) {
+        li = m.lev[i];
+        e0 = m.off[i];
+        e1 = m.off[i + 1];
+        entries(e0);
+    }
+    cudaGridDependencySynchronize();
+    if (!ctrl->active) return;
+    const double dt = ctrl->dt;
+    double invdt = 0.0;
+    if (i < m.nleaf) {
+        double un[5], acc[5] = {0, 0, 0, 0, 0}, u0[5], ui[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            u0[k] = U0[(int64_t)k * m.cap + i];
+            if constexpr (STAGE == 2) ui[k] = Uin[(int64_t)k * m.cap + i];
+        }
+        for (int e = e0; e < e1; e += NE) {
+            if (e > e0) entries(e);
+            double Fk[NE][5];
+#pragma unroll
+            for (int j = 0; j < NE; ++j)
+#pragma unroll
+                for (int k = 0; k < 5; ++k)
+                    Fk[j][k] = code[j] >= 0 ? F[(int64_t)k * m.fcap + (code[j] >> 1)] : 0.0;
+#pragma unroll
+            for (int j = 0; j < NE; ++j)
+                if (code[j] >= 0) {
+                    const double s = (code[j] & 1) ? -ar[j] : ar[j];
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) acc[k] = acc[k] + s * Fk[j][k];
+                }
+        }
+        const double invV = dt / (m.aexp * m.vol[li]);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            if constexpr (STAGE == 1) un[k] = u0[k] - invV * acc[k];
+            else un[k] = 0.5 * u0[k] + 0.5 * (ui[k] - invV * acc[k]);
+            Uout[(int64_t)k * m.cap + i] = un[k];
+        }
+        double W[5];
+        cons2prim(un, m.gamma, W);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) m.W[(int64_t)k * m.cap + i] = W[k];
+        if constexpr (STAGE == 2) {
+            const double c = sqrt(m.gamma * W[4] / W[0]);
+            for (int d = 0; d < m.nd; ++d)
+                invdt = nan_max(invdt, (fabs(W[1 + d]) + c) / m.w[li][d]);
+        }
+    }
+    if constexpr (STAGE == 2) {
+        block_max_to(&ctrl->invdt_bits, invdt, red);
+        // the last block to get here: the clock (k_advance), then evolve!'s loop
+        // head for the next step (k_finalize_cfl)
+        if (threadIdx.x == 0) {
+            __threadfence();
+            if (atomicAdd(&ctrl->work[0], 1u) == gridDim.x - 1) {
+                const double v = __longlong_as_double((long long)atomicExch(&ctrl->invdt_bits, 0ull));
+                const double t = ctrl->t + dt;
+                const long long step = ctrl->step + 1;
+                ctrl->t = t;
+                ctrl->step = step;
+                ctrl->work[0] = 0u;
+                if (!(t < ctrl->tfinal * (1.0 - 1e-12)) || step >= ctrl->step_limit) {
+                    ctrl->active = 0;
+                } else {
+                    const double h = fmin(v == 0.0 ? (double)INFINITY : cfl / v, ctrl->tfinal - t);
+                    if (v != v || !(h < (double)INFINITY)) {
+                        ctrl->flags |= CTRL_F_NONFINITE;
+                        ctrl->active = 0;
+                    } else {
+                        ctrl->dt = h;
+                    }
+                }
+            }
+        }
     }
 }
 
@@ -185,6 +355,25 @@ __global__ void __launch_bounds__(256) k_amr_cfl(AmrDev m, const double *__restr
     if (i < m.nleaf && (level < 0 || m.lev[i] == level)) {
         double W[5];
         amr_prim(m, U, i, W);
+        const double c = sqrt(m.gamma * W[4] / W[0]);
+        for (int d = 0; d < m.nd; ++d)
+            invdt = nan_max(invdt, (fabs(W[1 + d]) + c) / m.w[m.lev[i]][d]);
+    }
+    block_max_to(&ctrl->invdt_bits, invdt, red);
+}
+
+// start of the single-rate loop: the maximum over every leaf, whose primitives
+// stay in m.W
+__global__ void __launch_bounds__(256) k_amr_prims(AmrDev m, const double *__restrict__ U, Ctrl *ctrl)
+{
+    __shared__ double red[32];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    double invdt = 0.0;
+    if (i < m.nleaf) {
+        double W[5];
+        amr_prim(m, U, i, W);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) m.W[(int64_t)k * m.cap + i] = W[k];
         const double c = sqrt(m.gamma * W[4] / W[0]);
         for (int d = 0; d < m.nd; ++d)
             invdt = nan_max(invdt, (fabs(W[1 + d]) + c) / m.w[m.lev[i]][d]);
@@ -336,9 +525,39 @@ __global__ void __launch_bounds__(256) k_amr_totals_part(AmrDev m, const double 
 
 static unsigned blocks(int64_t n, int bs) { return (unsigned)((n + bs - 1) / bs > 0 ? (n + bs - 1) / bs : 1); }
 
+// launch with programmatic stream serialization: the kernel may start before
+// the one ahead of it ends (it waits in cudaGridDependencySynchronize)
+template <typename... P, typename... A>
+static bool launch_early(void (*k)(P...), unsigned grid, unsigned block, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, P(args)...) == cudaSuccess;
+}
+
+int launch_amr_prims(const AmrDev &m, const double *U, Ctrl *ctrl, cudaStream_t s)
+{
+    k_amr_prims<<<blocks(m.nleaf, 256), 256, 0, s>>>(m, U, ctrl);
+    return 1;
+}
+
 int launch_amr_stage(const AmrDev &m, int stage, const double *Uin, const double *U0,
                      double *Uout, double *F, const AmrStageArgs &a, Ctrl *ctrl, cudaStream_t s)
 {
+    if (a.loop) {
+        bool ok = m.nface == 0 || launch_early(k_amr_faces_loop, blocks(m.nface, 128), 128, s, m, F, ctrl);
+        if (ok)
+            ok = stage == 1 ? launch_early(k_amr_cells_loop<1>, blocks(m.nleaf, 128), 128, s, m, Uin, U0, Uout, F, a.cfl, ctrl)
+                            : launch_early(k_amr_cells_loop<2>, blocks(m.nleaf, 128), 128, s, m, Uin, U0, Uout, F, a.cfl, ctrl);
+        return ok ? (m.nface > 0 ? 2 : 1) : -1;
+    }
     if (m.nface > 0)
         k_amr_faces<<<blocks(m.nface, 256), 256, 0, s>>>(m, Uin, F,
                                                          (a.dt < 0.0 && !a.dt_dev) ? ctrl : nullptr);
