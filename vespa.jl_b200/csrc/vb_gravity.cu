@@ -19,6 +19,7 @@
 // + r.r partials, beta, direction update); groups of iterations replay as one
 // CUDA graph, each launch returning at once after convergence, and the host
 // reads the stop flag between groups.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -36,7 +37,8 @@ constexpr int GRAPH_ITERS = 8;
 struct GravCtrl {
     double rhobar, rsold, pAp, alpha, beta, bnorm, relres, mu, mgmu;
     long long iters, maxiter;
-    int done, pad;
+    int done;
+    unsigned int ticket;  // blocks past a grid_sum; zero between launches
     double tol;
 };
 
@@ -165,11 +167,6 @@ __device__ __forceinline__ double lap_row(const Geom &g, const GravP &P, const d
     return s;
 }
 
-// (A x)[i] on a periodic n^3 grid (the multigrid preconditioner's, and the CG
-// matvec's when the grid is such a cube), in the
-// same CSR row order as lap_row (lo faces of lower cells z, y, x; hi faces
-// x, y, z, a 1-cell axis twice; lo faces wrapped to a higher index x, y, z),
-// with 32-bit indices: the same bits as lap_row<3> on that grid.
 // (x, y, z) of cell i of a periodic n^3 cube, x fastest: masks and shifts
 // when n is a power of two, else two unsigned divisions
 __device__ __forceinline__ void cube_coords(int n, int i, int c[3])
@@ -186,28 +183,6 @@ __device__ __forceinline__ void cube_coords(int n, int i, int c[3])
         c[1] = (int)(q - r * un);
         c[2] = (int)r;
     }
-}
-
-__device__ __forceinline__ double lap_cube(int n, const GravP &P, const double *__restrict__ x, int i)
-{
-    int c[3];
-    cube_coords(n, i, c);
-    const int st[3] = {1, n, n * n};
-    const double xc = x[i];
-    double s = 0.0;
-#pragma unroll
-    for (int d = 2; d >= 0; --d)
-        if (c[d] > 0) s = s + P.coef[d] * (xc - x[i - st[d]]);
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const int nb = c[d] < n - 1 ? i + st[d] : i - (n - 1) * st[d];
-        s = s + P.coef[d] * (xc - x[nb]);
-        if (nb == i) s = s + P.coef[d] * (xc - x[nb]);
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d)
-        if (c[d] == 0 && n > 1) s = s + P.coef[d] * (xc - x[i + (n - 1) * st[d]]);
-    return s;
 }
 
 // Deterministic sum over the block's threads (fixed tree: a shuffle tree in
@@ -337,39 +312,6 @@ __global__ void __launch_bounds__(GB, GP_SM) k_cg_matvec(Geom g, GravP P, const 
     if (threadIdx.x == 0) part[blockIdx.x] = s;
 }
 
-// k_cg_matvec on the periodic cube (lap_cube, the same row sums), one thread
-// per cell; each block's p.Ap partial goes to cpart[block]
-__global__ void __launch_bounds__(GB) k_cg_matvec_cube(int n, GravP P, const double *__restrict__ p,
-                                                      double *__restrict__ Ap, double *cpart,
-                                                      const GravCtrl *gc)
-{
-    __shared__ double sh[GB / 32 + 1];
-    if (gc->done) return;
-    const int i = blockIdx.x * GB + threadIdx.x;
-    double s = 0.0;
-    if (i < n * n * n) {
-        const double a = lap_cube(n, P, p, i);
-        Ap[i] = a;
-        s = p[i] * a;
-    }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) cpart[blockIdx.x] = s;
-}
-
-// fold nb block partials into the GP partials the one-block final sums read:
-// block b sums its fixed contiguous range of cpart (a fixed tree)
-__global__ void __launch_bounds__(GB, GP_SM) k_fold_parts(const double *__restrict__ cpart, int nb,
-                                                         double *part, const GravCtrl *gc)
-{
-    __shared__ double sh[GB / 32 + 1];
-    if (gc->done) return;
-    const int per = (nb + GP - 1) / GP, lo = blockIdx.x * per, hi = min(nb, lo + per);
-    double s = 0.0;
-    for (int j = lo + (int)threadIdx.x; j < hi; j += GB) s = s + cpart[j];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
 // iters = k; stop when p.Ap <= 0, else alpha = rsold / p.Ap
 __global__ void __launch_bounds__(1024) k_cg_alpha(const double *part, GravCtrl *gc)
 {
@@ -465,181 +407,410 @@ __global__ void __launch_bounds__(GB, GP_SM) k_lap(Geom g, GravP P, const double
 }
 
 // ---------------------------------------------------------------------------
-// Multigrid-preconditioned CG (precond = VB_GRAV_PRECOND_MG), after the
-// reference's ext/mg_pcg.jl: the outer CG runs on the exact operator A; the
-// preconditioner z = M^-1 r is one composite-smoothed two-level cycle
+// The solver on a periodic n^3 cube: plain CG (the recurrence above) and CG
+// preconditioned after the reference's ext/mg_pcg.jl (precond =
+// VB_GRAV_PRECOND_MG): z = M^-1 r is one composite-smoothed two-level cycle
 // (_amg_cycle!, mg_pcg.jl:152-174): two damped-Jacobi sweeps on A from z = 0,
 // the residual moved to the base grid (on a uniform mesh the cells
 // themselves), one periodic cell-centred V-cycle of -lap there (_mg_vcycle!,
 // 123-145: damped Jacobi 2 + 2, full-weighting restriction, trilinear
 // prolongation, 30 sweeps on the coarsest level), the correction de-meaned,
 // scaled by 1/V and added, two more Jacobi sweeps on A.
+//
+// Every pass streams arrays of the fine grid, so passes are merged where one's
+// values can be formed from another's inputs:
+//   - the direction p = z + beta p and A p are one pass (p in two buffers);
+//   - a smoother's two sweeps from zero are one pass over its right-hand side
+//     (the first sweep is a multiple of it), on A and on every level;
+//   - residual and restriction are one pass; the correction's (e - mean) / V
+//     is formed where the first post-smoothing sweep reads it;
+//   - diag(A) is one number here (every row lists the same six coefficients);
+//   - each inner product is finished by the last block of the pass that forms
+//     it (fixed-order sums of the block partials: the same bits every run),
+//     which also sets the step's scalars.
+// That is 280 B of fine-grid traffic an iteration against 456 B as separate
+// passes, and about 25 launches against 90.  Levels of 16^3 and below run in
+// one block, in shared memory.  The iterations run as one graph with a WHILE
+// node on the stop flag, so the host reads nothing in between.
+//
+// A thread owns an (x, y) column and marches z over a chunk with the values
+// below and above in registers; the four side neighbours come from L1.
 
 constexpr double MG_OMEGA = 0.8;
+constexpr int MG_BLOCK = 16;  // levels of at most MG_BLOCK^3 cells run in one block
 
-// diag(A): the row's coefficients summed in the row's order; 1 for an empty row
-template <int ND>
-__global__ void __launch_bounds__(GB, GP_SM) k_diag(Geom g, GravP P, double *diag)
+struct CubeP {
+    int n;
+    double c[3];  // the operator's coefficients
+    double w;     // MG_OMEGA / diag(A)
+};
+
+__host__ __device__ inline int cube_kz(int n) { return n >= 512 ? 64 : n >= 128 ? 16 : 4; }
+
+// f(i, v(i), sx, sy, sz) for this thread's cells, s* the sums of v over the two
+// neighbours per axis
+template <class V, class F>
+__device__ __forceinline__ void cube_cells(int n, V &&v, F &&f)
 {
-    for_cells<ND>(g, [&](int64_t i, const int64_t cc[3]) {
-        double s = 0.0;
-#pragma unroll
-        for (int d = ND - 1; d >= 0; --d) {
-            const int64_t nb = gnb(g, P, i, cc[d], d, false);
-            if (nb >= 0 && nb < i) s = s + P.coef[d];
-        }
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            const int64_t nb = gnb(g, P, i, cc[d], d, true);
-            if (nb < 0) continue;
-            s = s + P.coef[d];
-            if (nb == i) s = s + P.coef[d];
-        }
-#pragma unroll
-        for (int d = 0; d < ND; ++d) {
-            const int64_t nb = gnb(g, P, i, cc[d], d, false);
-            if (nb > i) s = s + P.coef[d];
-        }
-        diag[i] = s == 0.0 ? 1.0 : s;
-    });
+    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
+    const int kz = cube_kz(n), z0 = blockIdx.z * kz, z1 = min(n, z0 + kz);
+    if (x >= n || y >= n) return;
+    const int nn = n * n, base = x + n * y;
+    const int xm = x > 0 ? -1 : n - 1, xp = x + 1 < n ? 1 : 1 - n;
+    const int ym = (y > 0 ? -1 : n - 1) * n, yp = (y + 1 < n ? 1 : 1 - n) * n;
+    double lo = v(base + (z0 > 0 ? z0 - 1 : n - 1) * nn), c = v(base + z0 * nn);
+    for (int z = z0; z < z1; ++z) {
+        const int i = base + z * nn;
+        const double hi = v(base + (z + 1 < n ? z + 1 : 0) * nn);
+        f(i, c, v(i + xm) + v(i + xp), v(i + ym) + v(i + yp), lo + hi);
+        lo = c;
+        c = hi;
+    }
 }
 
-// one damped-Jacobi sweep on A (_matvec! then _csr_jacobi!, mg_pcg.jl:148-150):
-// xout = x + omega (rhs - A x) / diag, xin == nullptr standing for x = 0; one
-// thread per cell of the periodic cube
-__global__ void __launch_bounds__(GB) k_ajac_cube(int n, GravP P, const double *__restrict__ xin,
-                                                 const double *__restrict__ rhs,
-                                                 const double *__restrict__ diag,
-                                                 double *__restrict__ xout, const GravCtrl *gc)
+// A v at a cell from cube_cells' sums
+__device__ __forceinline__ double cube_lap(const CubeP &P, double c, double sx, double sy, double sz)
 {
-    if (gc->done) return;
-    const int i = blockIdx.x * GB + threadIdx.x;
-    if (i >= n * n * n) return;
-    const double ax = xin ? lap_cube(n, P, xin, i) : 0.0;
-    const double xv = xin ? xin[i] : 0.0;
-    xout[i] = xv + MG_OMEGA * (rhs[i] - ax) / diag[i];
+    return P.c[0] * (2.0 * c - sx) + P.c[1] * (2.0 * c - sy) + P.c[2] * (2.0 * c - sz);
 }
 
-// mr = rhs - A x, and the base-grid right-hand side (0 + mr: the scatter onto
-// a zeroed base grid, one base cell per cell on a uniform mesh), whose
-// correction e starts at zero; one thread per cell of the periodic cube
-__global__ void __launch_bounds__(GB) k_aresid_cube(int n, GravP P, const double *__restrict__ x,
-                                                   const double *__restrict__ rhs,
-                                                   double *__restrict__ mr, double *__restrict__ tb,
-                                                   double *__restrict__ te, const GravCtrl *gc)
+// The grid's sum of s over its threads: true in thread 0 of the last block to
+// get here, with the total of the block partials summed in block order strides.
+__device__ __forceinline__ bool grid_sum(double s, double *part, unsigned int *ticket, double &total)
+{
+    __shared__ double sh[GB / 32 + 1];
+    __shared__ bool last;
+    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
+    s = block_sum(s, sh);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = s;
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == nb - 1;
+        if (last) *ticket = 0u;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    double r = 0.0;
+    for (unsigned j = threadIdx.x; j < nb; j += GB) r = r + __ldcg(part + j);
+    total = block_sum(r, sh);
+    return threadIdx.x == 0;
+}
+
+// p = z + beta p (beta 0: z) into the other of the two direction buffers,
+// Ap = A p, alpha = rsold / p.Ap; stop when p.Ap <= 0
+__global__ void __launch_bounds__(GB) k_cube_dir(CubeP P, const double *__restrict__ z, double *pa,
+                                                double *pb, double *__restrict__ Ap, double *part,
+                                                GravCtrl *gc)
 {
     if (gc->done) return;
-    const int i = blockIdx.x * GB + threadIdx.x;
-    if (i >= n * n * n) return;
-    const double m = rhs[i] - lap_cube(n, P, x, i);
-    mr[i] = m;
-    tb[i] = 0.0 + m;
-    te[i] = 0.0;
+    const bool odd = gc->iters & 1;
+    const double *__restrict__ po = odd ? pb : pa;
+    double *__restrict__ pn = odd ? pa : pb;
+    const double beta = gc->beta;
+    double s = 0.0;
+    cube_cells(
+        P.n, [&](int i) { return beta != 0.0 ? z[i] + beta * po[i] : z[i]; },
+        [&](int i, double c, double sx, double sy, double sz) {
+            const double a = cube_lap(P, c, sx, sy, sz);
+            pn[i] = c;
+            Ap[i] = a;
+            s = s + c * a;
+        });
+    double pAp;
+    if (grid_sum(s, part, &gc->ticket, pAp)) {
+        gc->iters += 1;
+        gc->pAp = pAp;
+        if (pAp <= 0.0) gc->done = 1;
+        else gc->alpha = gc->rsold / pAp;
+    }
+}
+
+// phi += alpha p; r -= alpha Ap; relres, stop at tol.  CG (no preconditioner):
+// also beta = r.r / rsold and the iteration limit; `more`: the loop's condition.
+__global__ void __launch_bounds__(GB) k_cube_update(int n, double *__restrict__ phi, const double *pa,
+                                                   const double *pb, double *__restrict__ r,
+                                                   const double *__restrict__ Ap, double *part,
+                                                   GravCtrl *gc, int cg, cudaGraphConditionalHandle more)
+{
+    if (gc->done) {
+        if (cg && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(more, 0);
+        return;
+    }
+    const double *__restrict__ p = (gc->iters & 1) ? pb : pa;
+    const double alpha = gc->alpha;
+    const int64_t N = (int64_t)n * n * n;
+    double s = 0.0;
+#pragma unroll 4
+    for (int64_t i = (int64_t)blockIdx.x * GB + threadIdx.x; i < N; i += (int64_t)gridDim.x * GB) {
+        phi[i] = phi[i] + alpha * p[i];
+        const double ri = r[i] - alpha * Ap[i];
+        r[i] = ri;
+        s = s + ri * ri;
+    }
+    double rr;
+    if (grid_sum(s, part, &gc->ticket, rr)) {
+        gc->relres = sqrt(rr) / gc->bnorm;
+        if (gc->relres <= gc->tol) {
+            gc->done = 1;
+        } else if (cg) {
+            gc->beta = rr / gc->rsold;
+            gc->rsold = rr;
+            if (gc->iters >= gc->maxiter) gc->done = 1;
+        }
+        if (cg) cudaGraphSetConditional(more, gc->done ? 0 : 1);
+    }
+}
+
+// two damped-Jacobi sweeps on A from zero: z1 = w r, z = z1 + w (r - A z1)
+__global__ void __launch_bounds__(GB) k_cube_pre(CubeP P, const double *__restrict__ r,
+                                                double *__restrict__ z, const GravCtrl *gc)
+{
+    if (gc->done) return;
+    cube_cells(
+        P.n, [&](int i) { return r[i]; },
+        [&](int i, double c, double sx, double sy, double sz) {
+            z[i] = P.w * c + P.w * (c - P.w * cube_lap(P, c, sx, sy, sz));
+        });
+}
+
+// the base grid's right-hand side: b = r - A z
+__global__ void __launch_bounds__(GB) k_cube_resid(CubeP P, const double *__restrict__ z,
+                                                  const double *__restrict__ r,
+                                                  double *__restrict__ b, const GravCtrl *gc)
+{
+    if (gc->done) return;
+    cube_cells(
+        P.n, [&](int i) { return z[i]; },
+        [&](int i, double c, double sx, double sy, double sz) { b[i] = r[i] - cube_lap(P, c, sx, sy, sz); });
+}
+
+// first post-smoothing sweep on A of z + (e - mean e) / V
+__global__ void __launch_bounds__(GB) k_cube_post1(CubeP P, const double *__restrict__ z,
+                                                  const double *__restrict__ e,
+                                                  const double *__restrict__ r, double iV,
+                                                  double *__restrict__ z2, const GravCtrl *gc)
+{
+    if (gc->done) return;
+    const double mu = gc->mgmu;
+    cube_cells(
+        P.n, [&](int i) { return z[i] + (e[i] - mu) * iV; },
+        [&](int i, double c, double sx, double sy, double sz) {
+            z2[i] = c + P.w * (r[i] - cube_lap(P, c, sx, sy, sz));
+        });
+}
+
+// second one, and r.z: at the solve's start (start) rsold = r.z and beta = 0,
+// then beta = r.z / rsold and the iteration limit; `more`: the loop's condition
+__global__ void __launch_bounds__(GB) k_cube_post2(CubeP P, const double *__restrict__ z2,
+                                                  const double *__restrict__ r,
+                                                  double *__restrict__ z, double *part, GravCtrl *gc,
+                                                  int start, cudaGraphConditionalHandle more)
+{
+    if (gc->done) {
+        if (!start && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
+            cudaGraphSetConditional(more, 0);
+        return;
+    }
+    double s = 0.0;
+    cube_cells(
+        P.n, [&](int i) { return z2[i]; },
+        [&](int i, double c, double sx, double sy, double sz) {
+            const double ri = r[i], v = c + P.w * (ri - cube_lap(P, c, sx, sy, sz));
+            z[i] = v;
+            s = s + ri * v;
+        });
+    double rz;
+    if (grid_sum(s, part, &gc->ticket, rz)) {
+        gc->beta = start ? 0.0 : rz / gc->rsold;
+        gc->rsold = rz;
+        if (!start) {
+            if (gc->iters >= gc->maxiter) gc->done = 1;
+            cudaGraphSetConditional(more, gc->done ? 0 : 1);
+        }
+    }
 }
 
 __device__ __forceinline__ int mg_wrap(int a, int n) { return a < 0 ? n - 1 : (a >= n ? 0 : a); }
 
 // _mgk_jacobi! (mg_pcg.jl:21-31): phi = (1 - w) phiold + w (sum_nb + h^2 b) / 6
-// for cell i of the periodic n^3 level
-__device__ __forceinline__ double mg_jacobi_cell(int n, int i, double h2, const double *phiold,
-                                                 const double *__restrict__ b)
+__device__ __forceinline__ double mg_jacobi(double c, double nb, double h2b)
 {
-    int c[3];
-    cube_coords(n, i, c);
-    const int x = c[0], y = c[1], z = c[2];
-    const int nn = n * n;
-    const double s = phiold[i - x + mg_wrap(x - 1, n)] + phiold[i - x + mg_wrap(x + 1, n)] +
-                     phiold[i - y * n + mg_wrap(y - 1, n) * n] + phiold[i - y * n + mg_wrap(y + 1, n) * n] +
-                     phiold[i - z * nn + mg_wrap(z - 1, n) * nn] + phiold[i - z * nn + mg_wrap(z + 1, n) * nn];
-    return (1.0 - MG_OMEGA) * phiold[i] + MG_OMEGA * (s + h2 * b[i]) / 6.0;
+    return (1.0 - MG_OMEGA) * c + MG_OMEGA * (nb + h2b) / 6.0;
 }
 
-__global__ void __launch_bounds__(GB, GP_SM) k_mg_jacobi(int n, double h2, const double *__restrict__ phiold,
-                                                 const double *__restrict__ b, double *phi,
-                                                 const GravCtrl *gc)
+// a level's two sweeps from zero: e1 = w h^2 b / 6, then one sweep of it
+__global__ void __launch_bounds__(GB) k_mg_first(int n, double h2, const double *__restrict__ b,
+                                                double *__restrict__ e, const GravCtrl *gc)
 {
     if (gc->done) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n * n * n) return;
-    phi[i] = mg_jacobi_cell(n, i, h2, phiold, b);
+    const double k = MG_OMEGA * h2 / 6.0;
+    cube_cells(
+        n, [&](int i) { return b[i]; },
+        [&](int i, double c, double sx, double sy, double sz) {
+            e[i] = mg_jacobi(k * c, k * (sx + sy + sz), h2 * c);
+        });
 }
 
-// `sweeps` (even) Jacobi sweeps of a small level in one block, alternating
-// e -> t -> e, with a block barrier between sweeps: the same values as
-// `sweeps` launches of k_mg_jacobi
-__global__ void __launch_bounds__(GB, GP_SM) k_mg_jacobi_block(int n, double h2, int sweeps, double *e,
-                                                       const double *__restrict__ b, double *t,
-                                                       const GravCtrl *gc)
+// one sweep; mean: also the mean of the result (the base grid's last sweep)
+__global__ void __launch_bounds__(GB) k_mg_sweep(int n, double h2, const double *__restrict__ old,
+                                                const double *__restrict__ b, double *__restrict__ e,
+                                                int mean, double *part, GravCtrl *gc)
 {
     if (gc->done) return;
-    const int nc = n * n * n;
-    for (int k = 0; k < sweeps; ++k) {
-        const double *src = (k & 1) ? t : e;
-        double *dst = (k & 1) ? e : t;
-        for (int i = threadIdx.x; i < nc; i += GB) dst[i] = mg_jacobi_cell(n, i, h2, src, b);
-        __syncthreads();
-    }
+    double s = 0.0;
+    cube_cells(
+        n, [&](int i) { return old[i]; },
+        [&](int i, double c, double sx, double sy, double sz) {
+            const double v = mg_jacobi(c, sx + sy + sz, h2 * b[i]);
+            e[i] = v;
+            s = s + v;
+        });
+    double total;
+    if (mean && grid_sum(s, part, &gc->ticket, total)) gc->mgmu = total / ((double)n * n * n);
 }
 
-// _mgk_residual! (33-43): r = b - (6 phi - sum_nb) / h^2
-__global__ void __launch_bounds__(GB, GP_SM) k_mg_residual(int n, double invh2, const double *__restrict__ phi,
-                                                   const double *__restrict__ b, double *r,
-                                                   const GravCtrl *gc)
+// _mgk_residual! (33-43) and _mgk_restrict! (45-53): the coarse right-hand side
+// is the mean of the 8 children's b - (6 e - sum_nb) / h^2
+__device__ __forceinline__ double mg_coarse_rhs(int n, double invh2, const double *e, const double *b,
+                                                int X, int Y, int Z)
 {
-    if (gc->done) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n * n * n) return;
-    int c[3];
-    cube_coords(n, i, c);
-    const int x = c[0], y = c[1], z = c[2];
-    const int nn = n * n;
-    const double s = phi[i - x + mg_wrap(x - 1, n)] + phi[i - x + mg_wrap(x + 1, n)] +
-                     phi[i - y * n + mg_wrap(y - 1, n) * n] + phi[i - y * n + mg_wrap(y + 1, n) * n] +
-                     phi[i - z * nn + mg_wrap(z - 1, n) * nn] + phi[i - z * nn + mg_wrap(z + 1, n) * nn];
-    r[i] = b[i] - (6.0 * phi[i] - s) * invh2;
+    const int nn = n * n, x[4] = {mg_wrap(2 * X - 1, n), 2 * X, 2 * X + 1, mg_wrap(2 * X + 2, n)};
+    const int y[4] = {mg_wrap(2 * Y - 1, n) * n, 2 * Y * n, (2 * Y + 1) * n, mg_wrap(2 * Y + 2, n) * n};
+    const int z[4] = {mg_wrap(2 * Z - 1, n) * nn, 2 * Z * nn, (2 * Z + 1) * nn, mg_wrap(2 * Z + 2, n) * nn};
+    double sb = 0.0, in = 0.0, out = 0.0;
+#pragma unroll
+    for (int k = 1; k < 3; ++k)
+#pragma unroll
+        for (int j = 1; j < 3; ++j) {
+#pragma unroll
+            for (int i = 1; i < 3; ++i) {
+                sb = sb + b[x[i] + y[j] + z[k]];
+                in = in + e[x[i] + y[j] + z[k]];
+            }
+            out = out + (e[x[0] + y[j] + z[k]] + e[x[3] + y[j] + z[k]]);
+            out = out + (e[x[j] + y[0] + z[k]] + e[x[j] + y[3] + z[k]]);
+            out = out + (e[x[j] + y[k] + z[0]] + e[x[j] + y[k] + z[3]]);
+        }
+    // each child has three of its siblings and three outer cells as neighbours
+    return 0.125 * (sb - (3.0 * in - out) * invh2);
 }
 
-// _mgk_restrict! (45-53): coarse = mean of the 8 fine children; coarse e = 0
-__global__ void __launch_bounds__(GB, GP_SM) k_mg_restrict(int nc, const double *__restrict__ rf, double *bc,
-                                                   double *ec, const GravCtrl *gc)
+__global__ void __launch_bounds__(GB) k_mg_down(int nc, double invh2, const double *__restrict__ e,
+                                               const double *__restrict__ b, double *__restrict__ bc,
+                                               const GravCtrl *gc)
 {
     if (gc->done) return;
-    const int I = blockIdx.x * blockDim.x + threadIdx.x;
+    const int I = blockIdx.x * GB + threadIdx.x;
     if (I >= nc * nc * nc) return;
     int C[3];
     cube_coords(nc, I, C);
-    const int n = 2 * nc, x = 2 * C[0], y = 2 * C[1], z = 2 * C[2];
-    auto f = [&](int a, int b_, int c) { return rf[a + n * (b_ + n * c)]; };
-    bc[I] = 0.125 * (f(x, y, z) + f(x + 1, y, z) + f(x, y + 1, z) + f(x + 1, y + 1, z) + f(x, y, z + 1) +
-                     f(x + 1, y, z + 1) + f(x, y + 1, z + 1) + f(x + 1, y + 1, z + 1));
-    ec[I] = 0.0;
+    bc[I] = mg_coarse_rhs(2 * nc, invh2, e, b, C[0], C[1], C[2]);
 }
 
 // _mgk_prolong_add! (55-66): trilinear cell-centred prolongation (weights 3/4,
-// 1/4, periodic) added into the fine level
-__global__ void __launch_bounds__(GB, GP_SM) k_mg_prolong_add(int nc, const double *__restrict__ phic,
-                                                      double *phif, const GravCtrl *gc)
+// 1/4, periodic) at fine cell (x, y, z)
+__device__ __forceinline__ double mg_prolong(int nc, const double *ec, int x, int y, int z)
+{
+    const int i0 = x >> 1, i1 = mg_wrap(i0 + ((x & 1) ? 1 : -1), nc);
+    const int j0 = (y >> 1) * nc, j1 = mg_wrap((y >> 1) + ((y & 1) ? 1 : -1), nc) * nc;
+    const int k0 = (z >> 1) * nc * nc, k1 = mg_wrap((z >> 1) + ((z & 1) ? 1 : -1), nc) * nc * nc;
+    auto line = [&](int o) { return 0.75 * ec[i0 + o] + 0.25 * ec[i1 + o]; };
+    auto face = [&](int o) { return 0.75 * line(j0 + o) + 0.25 * line(j1 + o); };
+    return 0.75 * face(k0) + 0.25 * face(k1);
+}
+
+__global__ void __launch_bounds__(GB) k_mg_up(int nc, const double *__restrict__ ec,
+                                             double *__restrict__ e, const GravCtrl *gc)
 {
     if (gc->done) return;
-    const int n = 2 * nc;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = 2 * nc, i = blockIdx.x * GB + threadIdx.x;
     if (i >= n * n * n) return;
     int c[3];
     cube_coords(n, i, c);
-    const int x = c[0], y = c[1], z = c[2];
-    const int ic[2] = {x / 2, mg_wrap(x / 2 + ((x & 1) ? 1 : -1), nc)};
-    const int jc[2] = {y / 2, mg_wrap(y / 2 + ((y & 1) ? 1 : -1), nc)};
-    const int kc[2] = {z / 2, mg_wrap(z / 2 + ((z & 1) ? 1 : -1), nc)};
-    const double w[2] = {0.75, 0.25};
-    double v = 0.0;
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int b = 0; b < 2; ++b)
-#pragma unroll
-            for (int c = 0; c < 2; ++c)
-                v = v + w[a] * w[b] * w[c] * phic[ic[a] + nc * (jc[b] + nc * kc[c])];
-    phif[i] = phif[i] + v;
+    e[i] = e[i] + mg_prolong(nc, ec, c[0], c[1], c[2]);
+}
+
+// The V-cycle from a level of n <= MG_BLOCK down, in one block: b in, e out.
+// Shared memory per level: e, t, b.
+__global__ void __launch_bounds__(1024) k_mg_bottom(int n, double h, const double *__restrict__ b,
+                                                   double *__restrict__ e, const GravCtrl *gc)
+{
+    extern __shared__ double sm[];
+    if (gc->done) return;
+    const int t = threadIdx.x;
+    auto sweep = [&](int m, double h2, const double *old, const double *rhs, double *out) {
+        for (int i = t; i < m * m * m; i += blockDim.x) {
+            int c[3];
+            cube_coords(m, i, c);
+            const int mm = m * m;
+            const double s = old[i - c[0] + mg_wrap(c[0] - 1, m)] + old[i - c[0] + mg_wrap(c[0] + 1, m)] +
+                             old[i + (mg_wrap(c[1] - 1, m) - c[1]) * m] + old[i + (mg_wrap(c[1] + 1, m) - c[1]) * m] +
+                             old[i + (mg_wrap(c[2] - 1, m) - c[2]) * mm] + old[i + (mg_wrap(c[2] + 1, m) - c[2]) * mm];
+            out[i] = mg_jacobi(old[i], s, h2 * rhs[i]);
+        }
+        __syncthreads();
+    };
+    for (int i = t; i < n * n * n; i += blockDim.x) sm[2 * n * n * n + i] = b[i];
+    __syncthreads();
+    double *base = sm;
+    int m = n;
+    double hm = h;
+    for (;;) {  // down: two sweeps from zero, then the coarse right-hand side
+        const int mc = m * m * m;
+        double *E = base, *T = base + mc, *B = base + 2 * mc;
+        const double h2 = hm * hm, k = MG_OMEGA * h2 / 6.0;
+        for (int i = t; i < mc; i += blockDim.x) T[i] = k * B[i];
+        __syncthreads();
+        sweep(m, h2, T, B, E);
+        if (!(m > 4 && m % 2 == 0)) {  // coarsest: 30 more sweeps
+            for (int q = 0; q < 30; q += 2) {
+                sweep(m, h2, E, B, T);
+                sweep(m, h2, T, B, E);
+            }
+            break;
+        }
+        double *next = base + 3 * mc;
+        const int c = m / 2, cc = c * c * c;
+        for (int I = t; I < cc; I += blockDim.x) {
+            int C[3];
+            cube_coords(c, I, C);
+            next[2 * cc + I] = mg_coarse_rhs(m, 1.0 / h2, E, B, C[0], C[1], C[2]);
+        }
+        __syncthreads();
+        base = next;
+        m = c;
+        hm = 2.0 * hm;
+    }
+    while (m < n) {  // up: the coarse correction, then two sweeps
+        const double *ec = base;
+        const int f = 2 * m, fc = f * f * f;
+        base -= 3 * fc;
+        hm = 0.5 * hm;
+        double *E = base, *T = base + fc, *B = base + 2 * fc;
+        for (int i = t; i < fc; i += blockDim.x) {
+            int c[3];
+            cube_coords(f, i, c);
+            E[i] = E[i] + mg_prolong(m, ec, c[0], c[1], c[2]);
+        }
+        __syncthreads();
+        sweep(f, hm * hm, E, B, T);
+        sweep(f, hm * hm, T, B, E);
+        m = f;
+    }
+    for (int i = t; i < n * n * n; i += blockDim.x) e[i] = base[i];
+}
+
+// shared memory of k_mg_bottom
+inline size_t mg_bottom_smem(int n)
+{
+    size_t d = 0;
+    for (;;) {
+        d += 3 * (size_t)n * n * n;
+        if (!(n > 4 && n % 2 == 0)) break;
+        n /= 2;
+    }
+    return d * sizeof(double);
 }
 
 // partials of sum(e) over the base grid (the correction's mean)
@@ -662,81 +833,6 @@ __global__ void __launch_bounds__(1024) k_sum_final(const double *part, int64_t 
     if (threadIdx.x == 0) gc->mgmu = s / (double)n;
 }
 
-// z += (e - mean) / Vbase + 0 * mr / diag  (_mgk_gather! with gamma = 0, then x .+= mc)
-__global__ void __launch_bounds__(GB, GP_SM) k_mg_gather_add(int64_t n, const double *__restrict__ e,
-                                                     const double *__restrict__ mr,
-                                                     const double *__restrict__ diag, double Vbase,
-                                                     double *z, const GravCtrl *gc)
-{
-    if (gc->done) return;
-    const double mu = gc->mgmu;
-    for (int64_t i = (int64_t)blockIdx.x * GB + threadIdx.x; i < n; i += (int64_t)GP * GB) {
-        const double mc = (e[i] - mu) / Vbase + 0.0 * mr[i] / diag[i];
-        z[i] = z[i] + mc;
-    }
-}
-
-// PCG start after z = M^-1 r: p = z; partials of r.z
-__global__ void __launch_bounds__(GB, GP_SM) k_pcg_start(Geom g, const double *__restrict__ r,
-                                                 const double *__restrict__ z, double *p, double *part)
-{
-    __shared__ double sh[GB];
-    double s = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * GB + threadIdx.x; i < g.ncell; i += (int64_t)GP * GB) {
-        p[i] = z[i];
-        s = s + r[i] * z[i];
-    }
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-// rz of the start (r.z): held in rsold, as the reference's rz
-__global__ void __launch_bounds__(1024) k_pcg_start_final(const double *part, GravCtrl *gc)
-{
-    __shared__ double sh[1024];
-    const double rz = final_sum(part, sh);
-    if (threadIdx.x == 0) gc->rsold = rz;
-}
-
-// relres from r.r; stop at tol (mg_pcg.jl:202-203)
-__global__ void __launch_bounds__(1024) k_pcg_check(const double *part, GravCtrl *gc)
-{
-    __shared__ double sh[1024];
-    if (gc->done) return;
-    const double rr = final_sum(part, sh);
-    if (threadIdx.x == 0) {
-        gc->relres = sqrt(rr) / gc->bnorm;
-        if (gc->relres <= gc->tol) gc->done = 1;
-    }
-}
-
-// partials of r.z (after the preconditioner)
-__global__ void __launch_bounds__(GB, GP_SM) k_pcg_rz(Geom g, const double *__restrict__ r,
-                                              const double *__restrict__ z, double *part,
-                                              const GravCtrl *gc)
-{
-    __shared__ double sh[GB];
-    if (gc->done) return;
-    double s = 0.0;
-    for (int64_t i = (int64_t)blockIdx.x * GB + threadIdx.x; i < g.ncell; i += (int64_t)GP * GB)
-        s = s + r[i] * z[i];
-    s = block_sum(s, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-
-// beta = rznew / rz; rz = rznew; stop after maxiter
-__global__ void __launch_bounds__(1024) k_pcg_beta(const double *part, GravCtrl *gc)
-{
-    __shared__ double sh[1024];
-    if (gc->done) return;
-    const double rz = final_sum(part, sh);
-    if (threadIdx.x == 0) {
-        gc->beta = rz / gc->rsold;
-        gc->rsold = rz;
-        if (gc->iters >= gc->maxiter) gc->done = 1;
-    }
-}
-
 }  // namespace
 }  // namespace vb
 
@@ -747,25 +843,26 @@ struct vb_gravity {
     vb::GravP P{};
     double *phi = nullptr, *b = nullptr, *r = nullptr, *p = nullptr, *Ap = nullptr;
     double *gacc = nullptr, *part = nullptr;
-    // periodic cube (n^3, n <= 1024, phi periodic on every side): the
-    // one-thread-per-cell matvec and its per-block partials
+    // periodic cube (n^3, n <= 1024, phi periodic on every side): its solver's
+    // second direction buffer and block partials
     int cube_n = 0;
-    double *cpart = nullptr;
+    double *p2 = nullptr, *cpart = nullptr;
     vb::GravCtrl *gc = nullptr;   // device
     vb::GravCtrl *hgc = nullptr;  // pinned host mirror
     cudaGraphExec_t gexec = nullptr;
-    int64_t maxiter = 500;
+    long long maxiter = 500;
     double tol = 1e-8;
+    bool limits_set = false;      // maxiter and tol are in the device block
     // multigrid preconditioner (precond = VB_GRAV_PRECOND_MG)
     int precond = VB_GRAV_PRECOND_NONE;
-    double *z = nullptr, *z2 = nullptr, *mr = nullptr, *diag = nullptr;
+    double *z = nullptr, *z2 = nullptr;
     struct Level {
         int n;
         double h;
-        double *e, *b, *r, *t;
+        double *e, *b, *t;
     };
     std::vector<Level> lev;  // base grid first, then each coarsening
-    double hbase = 0.0, vbase = 0.0;
+    double vbase = 0.0;
     int64_t graph_launches = 0;  // kernels per replay of the iteration graph
 };
 
@@ -780,26 +877,11 @@ namespace {
 // One CG iteration (five launches; each returns at once after convergence).
 inline unsigned mg_blocks(int64_t n) { return (unsigned)((n + vb::GB - 1) / vb::GB); }
 
-// Ap = A p and the GP partials of p.Ap; evaluates to the launch count
-int queue_matvec(vb_grid *gr, vb_gravity *gv)
-{
-    cudaStream_t s = gr->ctx->stream;
-    const vb::Geom &g = gr->g;
-    if (gv->cube_n) {
-        const int n = gv->cube_n;
-        const unsigned nb = mg_blocks((int64_t)n * n * n);
-        vb::k_cg_matvec_cube<<<nb, vb::GB, 0, s>>>(n, gv->P, gv->p, gv->Ap, gv->cpart, gv->gc);
-        vb::k_fold_parts<<<vb::GP, vb::GB, 0, s>>>(gv->cpart, (int)nb, gv->part, gv->gc);
-        return 2;
-    }
-    return ND_DISPATCH(g.nd, vb::k_cg_matvec, g, gv->P, gv->p, gv->Ap, gv->part, gv->gc);
-}
-
 int queue_iteration(vb_grid *gr, vb_gravity *gv)
 {
     cudaStream_t s = gr->ctx->stream;
     const vb::Geom &g = gr->g;
-    VB_CHECK_LAUNCH(gr->ctx, queue_matvec(gr, gv));
+    VB_CHECK_LAUNCH(gr->ctx, ND_DISPATCH(g.nd, vb::k_cg_matvec, g, gv->P, gv->p, gv->Ap, gv->part, gv->gc));
     vb::k_cg_alpha<<<1, 1024, 0, s>>>(gv->part, gv->gc);
     VB_CHECK_LAUNCH(gr->ctx, 1);
     vb::k_cg_update<<<vb::GP, vb::GB, 0, s>>>(g, gv->phi, gv->p, gv->r, gv->Ap, gv->part, gv->gc);
@@ -811,85 +893,131 @@ int queue_iteration(vb_grid *gr, vb_gravity *gv)
     return VB_OK;
 }
 
-// z = M^-1 r (one composite-smoothed two-level cycle)
-int queue_precond(vb_grid *gr, vb_gravity *gv)
+dim3 cube_grid(int n)
+{
+    const int kz = vb::cube_kz(n);
+    return dim3((unsigned)((n + 31) / 32), (unsigned)((n + 7) / 8), (unsigned)((n + kz - 1) / kz));
+}
+constexpr unsigned CUBE_UPDATE_BLOCKS = 1184;  // k_cube_update: 8 per SM
+
+vb::CubeP cube_params(const vb_gravity *gv)
+{
+    vb::CubeP P;
+    P.n = gv->cube_n;
+    double diag = 0.0;
+    for (int d = 2; d >= 0; --d) diag += gv->P.coef[d];
+    for (int d = 0; d < 3; ++d) diag += gv->P.coef[d];
+    for (int d = 0; d < 3; ++d) P.c[d] = gv->P.coef[d];
+    P.w = vb::MG_OMEGA / diag;
+    return P;
+}
+
+// z = M^-1 r (one composite-smoothed two-level cycle), then r.z and its scalars
+int queue_precond(vb_grid *gr, vb_gravity *gv, bool start, cudaGraphConditionalHandle more)
 {
     cudaStream_t s = gr->ctx->stream;
-    const vb::Geom &g = gr->g;
-    const vb::GravP &P = gv->P;
-    // the preconditioner runs on periodic cubes only: one thread per cell
-    const int n = (int)g.n[0];
-    const unsigned nb = mg_blocks((int64_t)n * n * n);
-    auto ajac = [&](const double *xin, double *xout) {
-        vb::k_ajac_cube<<<nb, vb::GB, 0, s>>>(n, P, xin, gv->r, gv->diag, xout, gv->gc);
+    const vb::CubeP P = cube_params(gv);
+    const dim3 grid = cube_grid(P.n);
+    vb::k_cube_pre<<<grid, vb::GB, 0, s>>>(P, gv->r, gv->z, gv->gc);
+    auto &top = gv->lev[0];
+    vb::k_cube_resid<<<grid, vb::GB, 0, s>>>(P, gv->z, gv->r, top.b, gv->gc);
+    VB_CHECK_LAUNCH(gr->ctx, 2);
+    const int L = (int)gv->lev.size();
+    // the first level that k_mg_bottom takes, or the coarsest one
+    int bot = 0;
+    while (bot < L - 1 && gv->lev[bot].n > vb::MG_BLOCK) ++bot;
+    auto sweep = [&](const vb_gravity::Level &l, const double *old, double *out, bool mean) {
+        vb::k_mg_sweep<<<cube_grid(l.n), vb::GB, 0, s>>>(l.n, l.h * l.h, old, l.b, out, mean ? 1 : 0,
+                                                         gv->cpart, gv->gc);
         return 1;
     };
-    VB_CHECK_LAUNCH(gr->ctx, ajac(nullptr, gv->z2));  // pre-smooth from z = 0
-    VB_CHECK_LAUNCH(gr->ctx, ajac(gv->z2, gv->z));
-    auto &top = gv->lev[0];
-    vb::k_aresid_cube<<<nb, vb::GB, 0, s>>>(n, P, gv->z, gv->r, gv->mr, top.b, top.e, gv->gc);
-    VB_CHECK_LAUNCH(gr->ctx, 1);
-    // V-cycle: down the levels, then back up
-    const int L = (int)gv->lev.size();
-    auto jacobi = [&](const vb_gravity::Level &l, int sweeps) {
-        const double h2 = l.h * l.h;
-        const unsigned nb = mg_blocks((int64_t)l.n * l.n * l.n);
-        for (int k = 0; k < sweeps; k += 2) {  // even counts end in e
-            vb::k_mg_jacobi<<<nb, vb::GB, 0, s>>>(l.n, h2, l.e, l.b, l.t, gv->gc);
-            vb::k_mg_jacobi<<<nb, vb::GB, 0, s>>>(l.n, h2, l.t, l.b, l.e, gv->gc);
-        }
-        return sweeps;
-    };
-    for (int k = 0; k + 1 < L; ++k) {
+    for (int k = 0; k < bot; ++k) {
         const auto &l = gv->lev[k], &c = gv->lev[k + 1];
-        VB_CHECK_LAUNCH(gr->ctx, jacobi(l, 2));
-        vb::k_mg_residual<<<mg_blocks((int64_t)l.n * l.n * l.n), vb::GB, 0, s>>>(
-            l.n, 1.0 / (l.h * l.h), l.e, l.b, l.r, gv->gc);
-        vb::k_mg_restrict<<<mg_blocks((int64_t)c.n * c.n * c.n), vb::GB, 0, s>>>(c.n, l.r, c.b, c.e, gv->gc);
+        vb::k_mg_first<<<cube_grid(l.n), vb::GB, 0, s>>>(l.n, l.h * l.h, l.b, l.e, gv->gc);
+        vb::k_mg_down<<<mg_blocks((int64_t)c.n * c.n * c.n), vb::GB, 0, s>>>(
+            c.n, 1.0 / (l.h * l.h), l.e, l.b, c.b, gv->gc);
         VB_CHECK_LAUNCH(gr->ctx, 2);
     }
-    {  // coarsest: 2 pre + 30 sweeps, in one block when the level is small
-        const auto &l = gv->lev[L - 1];
-        if ((int64_t)l.n * l.n * l.n <= 16 * vb::GB) {
-            vb::k_mg_jacobi_block<<<1, vb::GB, 0, s>>>(l.n, l.h * l.h, 32, l.e, l.b, l.t, gv->gc);
+    {
+        const auto &l = gv->lev[bot];
+        if (l.n <= vb::MG_BLOCK) {
+            vb::k_mg_bottom<<<1, 1024, vb::mg_bottom_smem(l.n), s>>>(l.n, l.h, l.b, l.e, gv->gc);
             VB_CHECK_LAUNCH(gr->ctx, 1);
-        } else {
-            VB_CHECK_LAUNCH(gr->ctx, jacobi(l, 32));
+        } else {  // a coarsest level too large for one block (odd side)
+            vb::k_mg_first<<<cube_grid(l.n), vb::GB, 0, s>>>(l.n, l.h * l.h, l.b, l.e, gv->gc);
+            VB_CHECK_LAUNCH(gr->ctx, 1);
+            for (int q = 0; q < 30; q += 2)
+                VB_CHECK_LAUNCH(gr->ctx, sweep(l, l.e, l.t, false) + sweep(l, l.t, l.e, false));
         }
     }
-    for (int k = L - 2; k >= 0; --k) {
+    for (int k = bot - 1; k >= 0; --k) {
         const auto &l = gv->lev[k], &c = gv->lev[k + 1];
-        vb::k_mg_prolong_add<<<mg_blocks((int64_t)l.n * l.n * l.n), vb::GB, 0, s>>>(c.n, c.e, l.e, gv->gc);
+        vb::k_mg_up<<<mg_blocks((int64_t)l.n * l.n * l.n), vb::GB, 0, s>>>(c.n, c.e, l.e, gv->gc);
         VB_CHECK_LAUNCH(gr->ctx, 1);
-        VB_CHECK_LAUNCH(gr->ctx, jacobi(l, 2));
+        VB_CHECK_LAUNCH(gr->ctx, sweep(l, l.e, l.t, false) + sweep(l, l.t, l.e, k == 0));
     }
-    const int64_t nt = (int64_t)top.n * top.n * top.n;
-    vb::k_sumpart<<<vb::GP, vb::GB, 0, s>>>(nt, top.e, gv->part + 2 * vb::GP, gv->gc);
-    vb::k_sum_final<<<1, 1024, 0, s>>>(gv->part + 2 * vb::GP, nt, gv->gc);
-    vb::k_mg_gather_add<<<vb::GP, vb::GB, 0, s>>>(nt, top.e, gv->mr, gv->diag, gv->vbase, gv->z, gv->gc);
-    VB_CHECK_LAUNCH(gr->ctx, 3);
-    VB_CHECK_LAUNCH(gr->ctx, ajac(gv->z, gv->z2));  // post-smooth
-    VB_CHECK_LAUNCH(gr->ctx, ajac(gv->z2, gv->z));
+    if (bot == 0) {  // the base grid itself was the bottom: its correction's mean
+        vb::k_sumpart<<<vb::GP, vb::GB, 0, s>>>((int64_t)P.n * P.n * P.n, top.e, gv->part + 2 * vb::GP, gv->gc);
+        vb::k_sum_final<<<1, 1024, 0, s>>>(gv->part + 2 * vb::GP, (int64_t)P.n * P.n * P.n, gv->gc);
+        VB_CHECK_LAUNCH(gr->ctx, 2);
+    }
+    vb::k_cube_post1<<<grid, vb::GB, 0, s>>>(P, gv->z, top.e, gv->r, 1.0 / gv->vbase, gv->z2, gv->gc);
+    vb::k_cube_post2<<<grid, vb::GB, 0, s>>>(P, gv->z2, gv->r, gv->z, gv->cpart, gv->gc, start ? 1 : 0, more);
+    VB_CHECK_LAUNCH(gr->ctx, 2);
     return VB_OK;
 }
 
-// One preconditioned CG iteration (mg_pcg.jl:194-209).
-int queue_pcg_iteration(vb_grid *gr, vb_gravity *gv)
+// One iteration on the cube (mg_pcg.jl:194-209, or CG).
+int queue_cube_iteration(vb_grid *gr, vb_gravity *gv, cudaGraphConditionalHandle more)
 {
     cudaStream_t s = gr->ctx->stream;
-    const vb::Geom &g = gr->g;
-    VB_CHECK_LAUNCH(gr->ctx, queue_matvec(gr, gv));
-    vb::k_cg_alpha<<<1, 1024, 0, s>>>(gv->part, gv->gc);
-    vb::k_cg_update<<<vb::GP, vb::GB, 0, s>>>(g, gv->phi, gv->p, gv->r, gv->Ap, gv->part, gv->gc);
-    vb::k_pcg_check<<<1, 1024, 0, s>>>(gv->part, gv->gc);
-    VB_CHECK_LAUNCH(gr->ctx, 4);
-    int rc = queue_precond(gr, gv);
-    if (rc) return rc;
-    vb::k_pcg_rz<<<vb::GP, vb::GB, 0, s>>>(g, gv->r, gv->z, gv->part, gv->gc);
-    vb::k_pcg_beta<<<1, 1024, 0, s>>>(gv->part, gv->gc);
-    vb::k_cg_dir<<<vb::GP, vb::GB, 0, s>>>(g, gv->p, gv->z, gv->gc);  // p = z + beta p
-    VB_CHECK_LAUNCH(gr->ctx, 3);
-    return VB_OK;
+    const bool mg = gv->precond == VB_GRAV_PRECOND_MG;
+    const vb::CubeP P = cube_params(gv);
+    vb::k_cube_dir<<<cube_grid(P.n), vb::GB, 0, s>>>(P, mg ? gv->z : gv->r, gv->p, gv->p2, gv->Ap,
+                                                     gv->cpart, gv->gc);
+    vb::k_cube_update<<<CUBE_UPDATE_BLOCKS, vb::GB, 0, s>>>(P.n, gv->phi, gv->p, gv->p2, gv->r, gv->Ap,
+                                                           gv->cpart, gv->gc, mg ? 0 : 1, more);
+    VB_CHECK_LAUNCH(gr->ctx, 2);
+    return mg ? queue_precond(gr, gv, false, more) : VB_OK;
+}
+
+// The cube's iterations as one graph: a WHILE node whose body is one iteration
+// and whose condition the iteration's last reduction sets from the stop flag.
+int capture_cube(vb_grid *gr, vb_gravity *gv)
+{
+    cudaStream_t s = gr->ctx->stream;
+    cudaGraph_t root = nullptr;
+    VB_CUDA(cudaGraphCreate(&root, 0));
+    cudaGraphConditionalHandle h;
+    cudaGraphNodeParams cp = {};
+    cudaGraphNode_t node;
+    cudaError_t e = cudaGraphConditionalHandleCreate(&h, root, 1, cudaGraphCondAssignDefault);
+    if (e == cudaSuccess) {
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = h;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        e = cudaGraphAddNode(&node, root, nullptr, 0, &cp);
+    }
+    if (e == cudaSuccess)
+        e = cudaStreamBeginCaptureToGraph(s, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                          cudaStreamCaptureModeThreadLocal);
+    int rc = VB_OK;
+    if (e == cudaSuccess) {
+        const int64_t before = gr->ctx->launches;
+        rc = queue_cube_iteration(gr, gv, h);
+        cudaGraph_t out = nullptr;
+        e = cudaStreamEndCapture(s, &out);
+        gv->graph_launches = gr->ctx->launches - before;
+        gr->ctx->launches = before;  // counted when the graph runs
+    }
+    if (!rc && e == cudaSuccess) e = cudaGraphInstantiate(&gv->gexec, root, 0);
+    cudaGraphDestroy(root);
+    if (!rc && e != cudaSuccess) {
+        gv->gexec = nullptr;
+        rc = fail(VB_ECUDA, std::string("gravity graph: ") + cudaGetErrorString(e));
+    }
+    return rc;
 }
 
 int capture_iterations(vb_grid *gr, vb_gravity *gv)
@@ -900,7 +1028,7 @@ int capture_iterations(vb_grid *gr, vb_gravity *gv)
     int rc = VB_OK;
     gv->graph_launches = 0;
     for (int k = 0; k < vb::GRAPH_ITERS && !rc; ++k)
-        rc = gv->precond == VB_GRAV_PRECOND_MG ? queue_pcg_iteration(gr, gv) : queue_iteration(gr, gv);
+        rc = queue_iteration(gr, gv);
     cudaGraph_t graph = nullptr;
     cudaError_t e = cudaStreamEndCapture(s, &graph);
     gv->graph_launches = gr->ctx->launches - before;
@@ -943,12 +1071,10 @@ void free_gravity(vb_gravity *gv)
     cudaFreeHost(gv->hgc);
     cudaFree(gv->z);
     cudaFree(gv->z2);
-    cudaFree(gv->mr);
-    cudaFree(gv->diag);
+    cudaFree(gv->p2);
     for (auto &l : gv->lev) {
         cudaFree(l.e);
         cudaFree(l.b);
-        cudaFree(l.r);
         cudaFree(l.t);
     }
     delete gv;
@@ -970,11 +1096,11 @@ int vb::detail::gravity_solve(vb_grid *gr, int64_t *iters, double *relres)
     vb_gravity *gv = gr->grav;
     cudaStream_t s = gr->ctx->stream;
     const Geom &g = gr->g;
-    gv->hgc->maxiter = gv->maxiter;
-    gv->hgc->tol = gv->tol;
-    VB_CUDA(cudaMemcpyAsync(&gv->gc->maxiter, &gv->hgc->maxiter, sizeof(long long),
-                            cudaMemcpyHostToDevice, s));
-    VB_CUDA(cudaMemcpyAsync(&gv->gc->tol, &gv->hgc->tol, sizeof(double), cudaMemcpyHostToDevice, s));
+    if (!gv->limits_set) {  // the stop criteria, once per configuration
+        VB_CUDA(cudaMemcpyAsync(&gv->gc->maxiter, &gv->maxiter, sizeof(long long), cudaMemcpyHostToDevice, s));
+        VB_CUDA(cudaMemcpyAsync(&gv->gc->tol, &gv->tol, sizeof(double), cudaMemcpyHostToDevice, s));
+        gv->limits_set = true;
+    }
     if (gv->P.project_mean) {
         k_meanpart<<<GP, GB, 0, s>>>(g, gr->U, gv->part);
         VB_CHECK_LAUNCH(gr->ctx, 1);
@@ -986,19 +1112,23 @@ int vb::detail::gravity_solve(vb_grid *gr, int64_t *iters, double *relres)
     VB_CHECK_LAUNCH(gr->ctx, ND_DISPATCH(g.nd, k_cg_init, g, gv->P, gv->phi, gv->b, gv->r, gv->p, gv->part));
     k_cg_init_final<<<1, 1024, 0, s>>>(gv->part, gv->gc);
     VB_CHECK_LAUNCH(gr->ctx, 1);
-    if (gv->precond == VB_GRAV_PRECOND_MG) {  // z = M^-1 r, p = z, rz (mg_pcg.jl:188-191)
-        int rc = queue_precond(gr, gv);
-        if (rc) return rc;
-        k_pcg_start<<<GP, GB, 0, s>>>(g, gv->r, gv->z, gv->p, gv->part);
-        k_pcg_start_final<<<1, 1024, 0, s>>>(gv->part, gv->gc);
-        VB_CHECK_LAUNCH(gr->ctx, 2);
-    }
     if (!gv->gexec) {
-        int rc = capture_iterations(gr, gv);
+        int rc = gv->cube_n ? capture_cube(gr, gv) : capture_iterations(gr, gv);
         if (rc) return rc;
+    }
+    if (gv->cube_n) {
+        // beta = 0 starts the direction from z (mg_pcg.jl:188-191) or r
+        VB_CUDA(cudaMemsetAsync(&gv->gc->beta, 0, sizeof(double), s));
+        if (gv->precond == VB_GRAV_PRECOND_MG) {
+            int rc = queue_precond(gr, gv, true, 0);
+            if (rc) return rc;
+        }
+        VB_CUDA(cudaGraphLaunch(gv->gexec, s));
+        gr->ctx->launches += gv->graph_launches;  // of one iteration: the count stays on the device
+        VB_CUDA(cudaMemcpyAsync(gv->hgc, gv->gc, sizeof(GravCtrl), cudaMemcpyDeviceToHost, s));
     }
     // the stop flag is set by convergence, p.Ap <= 0 or maxiter, so this ends
-    for (;;) {
+    while (!gv->cube_n) {
         VB_CUDA(cudaGraphLaunch(gv->gexec, s));
         gr->ctx->launches += gv->graph_launches;
         VB_CUDA(cudaMemcpyAsync(gv->hgc, gv->gc, sizeof(GravCtrl), cudaMemcpyDeviceToHost, s));
@@ -1015,6 +1145,7 @@ int vb::detail::gravity_solve(vb_grid *gr, int64_t *iters, double *relres)
     }
     int rc = refresh_accel(gr, gv);
     if (rc) return rc;
+    if (gv->cube_n && (iters || relres)) VB_CUDA(cudaStreamSynchronize(s));
     if (iters) *iters = gv->hgc->iters;
     if (relres) *relres = gv->hgc->relres;
     return VB_OK;
@@ -1091,7 +1222,13 @@ int vb_gravity_enable(vb_grid *gr, const vb_gravity_desc *d)
         for (int a = 0; a < 3; ++a) cube = cube && P.per_lo[a] && P.per_hi[a];
         gv->cube_n = cube ? (int)g.n[0] : 0;
         if (cube && !gv->cpart) {
-            const cudaError_t e = cudaMalloc(&gv->cpart, sizeof(double) * mg_blocks(g.ncell));
+            const dim3 b = cube_grid((int)g.n[0]);
+            const size_t nb = std::max<size_t>((size_t)b.x * b.y * b.z, CUBE_UPDATE_BLOCKS);
+            cudaError_t e = cudaMalloc(&gv->cpart, sizeof(double) * nb);
+            if (e == cudaSuccess) e = cudaMalloc(&gv->p2, sizeof(double) * (size_t)g.ncell);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(vb::k_mg_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)vb::mg_bottom_smem(vb::MG_BLOCK));
             if (e != cudaSuccess) {
                 gv->cube_n = 0;
                 if (!gr->grav) free_gravity(gv);
@@ -1102,6 +1239,7 @@ int vb_gravity_enable(vb_grid *gr, const vb_gravity_desc *d)
     }
     gv->maxiter = d->maxiter;
     gv->tol = d->tol;
+    gv->limits_set = false;
     gr->grav = gv;
     if (gv->gexec) {  // the iteration graph depends on the preconditioner
         cudaGraphExecDestroy(gv->gexec);
@@ -1112,27 +1250,20 @@ int vb_gravity_enable(vb_grid *gr, const vb_gravity_desc *d)
         // levels: coarsen while even and > 4 (mg_pcg.jl:111-116)
         const size_t n = (size_t)g.ncell * sizeof(double);
         cudaError_t e = cudaSuccess;
-        for (double **buf : {&gv->z, &gv->z2, &gv->mr, &gv->diag})
+        for (double **buf : {&gv->z, &gv->z2})
             if (e == cudaSuccess) e = cudaMalloc(buf, n);
-        gv->hbase = g.w[0];
-        gv->vbase = gv->hbase * gv->hbase * gv->hbase;
         int nl = (int)g.n[0];
-        double h = gv->hbase;
+        double h = g.w[0];
+        gv->vbase = h * h * h;
         for (;;) {
-            vb_gravity::Level l{nl, h, nullptr, nullptr, nullptr, nullptr};
+            vb_gravity::Level l{nl, h, nullptr, nullptr, nullptr};
             const size_t bytes = sizeof(double) * (size_t)nl * nl * nl;
-            for (double **buf : {&l.e, &l.b, &l.r, &l.t})
+            for (double **buf : {&l.e, &l.b, &l.t})
                 if (e == cudaSuccess) e = cudaMalloc(buf, bytes);
             gv->lev.push_back(l);
             if (!(nl > 4 && nl % 2 == 0)) break;
             nl /= 2;
             h *= 2.0;
-        }
-        if (e == cudaSuccess) {
-            cudaStream_t s = gr->ctx->stream;
-            vb::k_diag<3><<<vb::GP, vb::GB, 0, s>>>(g, P, gv->diag);
-            e = cudaGetLastError();
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         }
         if (e != cudaSuccess) {
             gr->grav = nullptr;
