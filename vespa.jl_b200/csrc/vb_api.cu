@@ -225,17 +225,23 @@ bool tiled_auto(const vb::Geom &g, int precision)
     return tiles_per_chunk(g) * ((vb::march_extent(g) + 7) / 8) >= 296;
 }
 
-QueueSpan::QueueSpan(double p) : prologue(p), slot(SLOTS, 0.0) {}
-void QueueSpan::add(int planes, int64_t count)
-{
-    for (int64_t i = 0; i < count; ++i) {
-        std::pop_heap(slot.begin(), slot.end(), std::greater<double>());
-        slot.back() += planes + prologue;
-        end = std::max(end, slot.back());
-        std::push_heap(slot.begin(), slot.end(), std::greater<double>());
+// Length of a tiled 3D launch in planes: work items (their planes plus a
+// prologue) taken in queue order by the resident block that is free first.
+struct QueueSpan {
+    static constexpr int SLOTS = 296;
+    double prologue, end = 0.0;
+    std::vector<double> slot;
+    explicit QueueSpan(double p) : prologue(p), slot(SLOTS, 0.0) {}
+    void add(int planes, int64_t count)
+    {
+        for (int64_t i = 0; i < count; ++i) {
+            std::pop_heap(slot.begin(), slot.end(), std::greater<double>());
+            slot.back() += planes + prologue;
+            end = std::max(end, slot.back());
+            std::push_heap(slot.begin(), slot.end(), std::greater<double>());
+        }
     }
-}
-double tile_prologue(int precision) { return precision == VB_MIXED ? 4.0 : 1.5; }
+};
 
 // Chunk and queue shape a single grid starts from.  3D, with q planes per
 // resident block (296 of them): up to 12, uniform chunks of one round of items;
@@ -264,7 +270,7 @@ int grid_default_kz(const vb::Geom &g, int precision, bool *taper)
     }
     *taper = true;
     if (q >= 24.0) return q >= 48.0 && ext >= 48 ? 48 : ext >= 24 ? 24 : (int)ext;
-    const double prologue = tile_prologue(precision);
+    const double prologue = precision == VB_MIXED ? 4.0 : 1.5;
     int best_kz = 8;
     double best = INFINITY;
     for (int c = 0; c < 3; ++c) {
@@ -449,17 +455,23 @@ int stage(vb_grid *gr, int st, const double *Uin, const double *U0, double *Uout
     }
     int n = gr->precision == VB_MIXED
                 ? vb::launch_stage_mixed(gr->g, st, Uin, U0, Uout, gr->ctrl, bf, gr->ctx->stream, bfi)
-                : vb::launch_stage_fp64(gr->g, st, Uin, U0, Uout, gr->ctrl, bf, gr->ctx->stream, bfi);
+                : vb::launch_stage_fp64(gr->g, st, Uin, U0, Uout, gr->ctrl, bf, gr->ctx->stream, bfi,
+                                      gr->cell_only);
     VB_CHECK_LAUNCH(gr->ctx, n);
     return VB_OK;
+}
+
+// Both stages of a step whose dt is already in the control block.
+int stages(vb_grid *gr)
+{
+    int rc = stage(gr, 1, gr->U, gr->U, gr->U1);
+    return rc ? rc : stage(gr, 2, gr->U1, gr->U, gr->U);
 }
 
 // One RK2 step whose dt is already in the control block.
 int rk2(vb_grid *gr)
 {
-    int rc = stage(gr, 1, gr->U, gr->U, gr->U1);
-    if (rc) return rc;
-    rc = stage(gr, 2, gr->U1, gr->U, gr->U);
+    int rc = stages(gr);
     if (rc) return rc;
     VB_CHECK_LAUNCH(gr->ctx, vb::launch_advance(gr->ctrl, gr->ctx->stream));
     gr->invdt_valid = true;
@@ -488,9 +500,21 @@ int ensure_cfl(vb_grid *gr)
 // so finalising first is the same); that solve synchronises with the host.
 int queue_direct(vb_grid *gr, int64_t count)
 {
+    if (!gr->grav && count > 0) {
+        // a step's clock and the next one's dt in one launch
+        VB_CHECK_LAUNCH(gr->ctx, vb::launch_finalize_cfl(gr->g, gr->ctrl, gr->ctx->stream));
+        for (int64_t i = 0; i < count; ++i) {
+            int rc = stages(gr);
+            if (rc) return rc;
+            VB_CHECK_LAUNCH(gr->ctx, i + 1 < count ? vb::launch_next_step(gr->g, gr->ctrl, gr->ctx->stream)
+                                                   : vb::launch_advance(gr->ctrl, gr->ctx->stream));
+        }
+        gr->invdt_valid = true;
+        return VB_OK;
+    }
     for (int64_t i = 0; i < count; ++i) {
         VB_CHECK_LAUNCH(gr->ctx, vb::launch_finalize_cfl(gr->g, gr->ctrl, gr->ctx->stream));
-        if (gr->grav) {
+        {
             int rc = pull_ctrl(gr);
             if (rc) return rc;
             if (!gr->hctrl->active) return VB_OK;
@@ -505,10 +529,17 @@ int queue_direct(vb_grid *gr, int64_t count)
 
 constexpr int64_t GRAPH_STEPS = 8;
 
+// Whole runs in one launch (vb_march.cu): small float64 1D and 2D grids under
+// the automatic kernel choice, with nothing recorded or added between stages.
+bool marches(const vb_grid *gr)
+{
+    return gr->march && !gr->bflux_on && !gr->grav && !gr->slab;
+}
+
 uint64_t graph_key(const vb_grid *gr)
 {
     return (gr->tiled ? 1u : 0u) | (gr->bflux_on ? 2u : 0u) | (grid_taper(gr) ? 4u : 0u) |
-           (gr->bflux_interior ? 8u : 0u) | ((uint64_t)gr->kz << 5);
+           (gr->bflux_interior ? 8u : 0u) | (gr->cell_only ? 16u : 0u) | ((uint64_t)gr->kz << 5);
 }
 
 // Capture GRAPH_STEPS steps into the grid's graph for its current configuration.
@@ -547,6 +578,11 @@ int capture_steps(vb_grid *gr)
 // launch directly.
 int queue_steps(vb_grid *gr, int64_t count)
 {
+    if (marches(gr)) {
+        VB_CHECK_LAUNCH(gr->ctx, vb::launch_march(gr->g, gr->U, gr->ctrl, count, gr->ctx->stream));
+        gr->invdt_valid = true;
+        return VB_OK;
+    }
     while (gr->warmed && count >= GRAPH_STEPS && !gr->grav) {
         if (!gr->gexec || gr->gkey != graph_key(gr)) {
             int rc = capture_steps(gr);
@@ -736,9 +772,8 @@ int vb_hllc_faces(vb_ctx *ctx, int64_t nf, const double *WL, const double *WR,
     if (nf < 0) return fail(VB_EINVAL, "nf < 0");
     if (nf == 0) return VB_OK;  // the reference returns F untouched for nf == 0
     if (!WL || !WR || !axis || !F) return fail(VB_EINVAL, "null buffer");
-    unsigned bad = 0;  // no early exit: the loop vectorises
-    for (int64_t f = 0; f < nf; ++f) bad |= (unsigned)(axis[f] - 1) > 2u;
-    if (bad) return fail(VB_EINVAL, "axis entries must be 1, 2 or 3");
+    for (int64_t f = 0; f < nf; ++f)
+        if (axis[f] < 1 || axis[f] > 3) return fail(VB_EINVAL, "axis entries must be 1, 2 or 3");
     const size_t bw = sizeof(double) * 5 * (size_t)nf;
     const size_t ba = sizeof(int32_t) * (size_t)nf;
     const size_t need = 3 * bw + ((ba + 255) & ~(size_t)255);
@@ -800,6 +835,7 @@ int vb_grid_create(vb_ctx *ctx, const vb_problem_desc *d, int precision, vb_grid
         std::string m = g_err;
         return cleanup(rc, m);
     }
+    gr->march = precision == VB_FP64 && vb::march_supported(g);
     if (vb::tiled_any(g, precision)) {
         if (vb::tiled_supported(g) || precision == VB_MIXED) {  // the TMA kernels' descriptors
             rc = encode_maps(&gr->maps_U, gr->U, g);
@@ -913,6 +949,8 @@ int vb_grid_set_option(vb_grid *gr, int option, int64_t value)
     if (!gr) return fail(VB_EINVAL, "null grid");
     switch (option) {
     case VB_OPT_KERNEL:
+        gr->march = value == VB_KERNEL_AUTO && gr->precision == VB_FP64 && vb::march_supported(gr->g);
+        gr->cell_only = value == VB_KERNEL_CELL;
         if (value == VB_KERNEL_CELL) {
             gr->tiled = false;
         } else if (value == VB_KERNEL_AUTO || value == VB_KERNEL_TILED) {
@@ -1194,7 +1232,7 @@ int vb_run_steps_async(vb_grid *gr, int64_t nsteps)
     if (nsteps < 0) return fail(VB_EINVAL, "nsteps < 0");
     int rc = use(gr->ctx);
     if (rc) return rc;
-    rc = ensure_cfl(gr);
+    if (!marches(gr)) rc = ensure_cfl(gr);
     if (rc) return rc;
     return queue_steps(gr, nsteps);
 }
@@ -1214,11 +1252,11 @@ int vb_evolve(vb_grid *gr, double tfinal, int64_t max_steps, double *t, int64_t 
     gr->hctrl->active = 1;
     rc = push_ctrl(gr);
     if (rc) return rc;
-    rc = ensure_cfl(gr);
+    if (!marches(gr)) rc = ensure_cfl(gr);  // a march folds it itself
     if (rc) return rc;
     // chunks of steps between host checks of the control block, none queued
     // beyond the step budget
-    int64_t chunk = 8;
+    int64_t chunk = marches(gr) ? 4096 : 8;
     int status = VB_OK;
     for (;;) {
         const long long left = gr->hctrl->step_limit - gr->hctrl->step;

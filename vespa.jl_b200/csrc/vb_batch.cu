@@ -35,7 +35,6 @@ struct vb_batch {
     int *item_box = nullptr;
     int nitems = 0;
     int kz_cap = 0;                          // chunk cap of the item layout (0: default chunks)
-    int kz_default = 0;                      // the default chunks' cap (0: not chosen yet)
     std::vector<vb::TiledMaps> mU, mU1;      // per-box TMA descriptors
     std::vector<int> order;                  // boxes, largest first
     unsigned int *work = nullptr;  // the two stage cursors
@@ -89,37 +88,12 @@ int queue(vb_batch *b, int64_t nsteps)
     return VB_OK;
 }
 
-// The default chunk of a box with nz planes: nz up to the batch's chunk, the one
-// whose items, largest box first, end soonest on the resident blocks by count
-// of planes (QueueSpan).  Long chunks save prologues and leave the last ones on
-// a few blocks: the 12 boxes of 32^3 to 96^3 of a small batch want short ones,
-// the 64 boxes of a large one long ones.
-int layout_kz(vb_batch *b, int nz)
-{
-    if (!b->kz_default) {
-        double best = INFINITY;
-        for (int kz : {96, 64, 48, 32, 24, 16, 12, 8, 4}) {
-            int64_t items = 0;
-            for (int i : b->order) items += vb::detail::box_items(b->geom[i], (int)std::min<int64_t>(kz, b->geom[i].n[2]));
-            if (items > 65536 && b->kz_default) break;  // far more items than blocks: shorter never wins
-            vb::detail::QueueSpan span(vb::detail::tile_prologue(b->precision));
-            for (int i : b->order) {
-                const vb::Geom &g = b->geom[i];
-                const int n = (int)g.n[2], k = kz < n ? kz : n;
-                const int64_t tiles = vb::detail::tiles_per_chunk(g);
-                span.add(k, tiles * (n / k));
-                if (n % k) span.add(n % k, tiles);
-            }
-            if (span.end < best) {
-                best = span.end;
-                b->kz_default = kz;
-            }
-        }
-    }
-    return b->kz_default < nz ? b->kz_default : nz;
-}
+// The default chunk of a box with nz planes.  (Choosing one cap for the whole
+// batch by a count of rounds, as single grids do, was 6 % slower on 12 boxes of
+// 32^3 to 96^3: items of several sizes share an SM at unequal speeds.)
+int default_kz(int nz) { return nz >= 64 ? 32 : (nz + 1) / 2; }
 
-// Work items for chunk cap `cap` (0: the default chunks, see layout_kz): box
+// Work items for chunk cap `cap` (0: each box's default chunk): box
 // descriptors and the item -> box table, uploaded on the stream.  Captured
 // graphs hold the old item count, so they are dropped.
 int set_layout(vb_batch *b, int cap)
@@ -129,7 +103,7 @@ int set_layout(vb_batch *b, int cap)
     for (int i : b->order) {
         const vb::Geom &g = b->geom[i];
         const int nz = (int)g.n[2];
-        const int kz = cap > 0 ? (cap < nz ? cap : nz) : layout_kz(b, nz);
+        const int kz = cap > 0 ? (cap < nz ? cap : nz) : default_kz(nz);
         const int64_t n = vb::detail::box_items(g, kz);
         if ((int64_t)item_box.size() + n > INT_MAX) return fail(VB_ENOTSUP, "too many work items");
         hb[i] = vb::detail::make_box(b->mU[i], b->mU1[i], g, b->U[i], b->U1[i], b->ctrl + i, kz,

@@ -161,11 +161,16 @@ __device__ __forceinline__ unsigned long long order_bits(double x)
     return b;
 }
 
+// Largest of a warp's non-negative doubles, by their bit patterns: the high
+// words, then the low words among those with the largest (two integer
+// reductions instead of five 64-bit shuffles and compares).  A NaN of either
+// sign comes out as a positive one.
 __device__ __forceinline__ double warp_max(double v)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = nan_max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    const unsigned hi = __double2hiint(v) & 0x7fffffffu;
+    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)__double2loint(v) : 0u);
+    return __hiloint2double((int)mh, (int)ml);
 }
 
 __device__ __forceinline__ double warp_sum(double v)

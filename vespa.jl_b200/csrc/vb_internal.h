@@ -3,7 +3,6 @@
 #pragma once
 
 #include <string>
-#include <vector>
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -55,6 +54,8 @@ struct vb_grid {
     int64_t glaunches = 0;              // kernels per replay
     bool warmed = false;                // one direct step ran (launch setup done)
     vb_gravity *grav = nullptr;         // self-gravity (a solve per step; source in the stages)
+    bool cell_only = false;     // VB_KERNEL_CELL: the cell-centric kernel only
+    bool march = false;         // small grid under the automatic choice: runs in one launch (vb_march.cu)
     bool slab = false;                  // a z window is set (vb_grid_set_zwindow): tiled kernels only
 };
 
@@ -73,17 +74,6 @@ int encode_maps(TiledMaps *m, const double *base, const Geom &g);
 BoxDesc make_box(const TiledMaps &mU, const TiledMaps &mU1, const Geom &g, double *U, double *U1,
                  Ctrl *ctrl, int kz, int item0, bool taper = false);
 int64_t box_items(const Geom &g, int kz, bool taper = false);
-// Length of a tiled 3D launch in planes: work items (their planes plus a
-// prologue, tile_prologue) taken in queue order by the slot (resident block)
-// that is free first.
-struct QueueSpan {
-    static constexpr int SLOTS = 296;
-    double prologue, end = 0.0;
-    std::vector<double> slot;
-    explicit QueueSpan(double prologue);
-    void add(int planes, int64_t count);
-};
-double tile_prologue(int precision);
 // automatic kernel choice and default chunk of a single grid
 bool tiled_auto(const Geom &g, int precision);
 int64_t tiles_per_chunk(const Geom &g);

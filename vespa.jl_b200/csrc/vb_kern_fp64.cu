@@ -9,6 +9,7 @@
 #include "vb_launch.h"
 #include "vb_stage_generic.cuh"
 #include "vb_stage_tiled3d.cuh"
+#include "vb_stage_plane_f64.cuh"
 #include "vb_stage_tiled3d_f64.cuh"
 #include "vb_stage_tiled2d.cuh"
 
@@ -50,7 +51,7 @@ __global__ void k_reset_cfl(Ctrl *ctrl) { ctrl->invdt_bits = 0ull; }
 
 // evolve!'s loop head, src/driver.jl:493-499: stop once t >= tfinal*(1-1e-12)
 // (or the step budget is spent); else dt = min(cfl/invdt, tfinal - t).
-__global__ void k_finalize_cfl(Geom g, Ctrl *ctrl)
+__device__ __forceinline__ void finalize_cfl(const Geom &g, Ctrl *ctrl)
 {
     const double t = ctrl->t;
     if (!(t < ctrl->tfinal * (1.0 - 1e-12)) || ctrl->step >= ctrl->step_limit) {
@@ -70,6 +71,24 @@ __global__ void k_finalize_cfl(Geom g, Ctrl *ctrl)
     ctrl->active = 1;
     ctrl->invdt_bits = 0ull;
     ctrl->work[0] = ctrl->work[1] = 0u;
+}
+
+__global__ void k_finalize_cfl(const __grid_constant__ Geom g, Ctrl *ctrl) { finalize_cfl(g, ctrl); }
+
+// step!'s clock advance (src/driver.jl:353-356) after stage 2.
+__device__ __forceinline__ void advance(Ctrl *ctrl)
+{
+    if (ctrl->active) {
+        ctrl->t = ctrl->t + ctrl->dt;
+        ctrl->step = ctrl->step + 1;
+    }
+}
+
+// the end of one step and the head of the next
+__global__ void k_next_step(const __grid_constant__ Geom g, Ctrl *ctrl)
+{
+    advance(ctrl);
+    finalize_cfl(g, ctrl);
 }
 
 // step!(sim, dt) with a caller-chosen dt.
@@ -149,8 +168,11 @@ __global__ void __launch_bounds__(256) k_hllc_faces(int64_t nf, const double *__
 }  // namespace
 
 int launch_stage_fp64(const Geom &g, int stage, const double *Uin, const double *U0,
-                      double *Uout, Ctrl *ctrl, double *bflux, cudaStream_t s, double *bflux_int)
+                      double *Uout, Ctrl *ctrl, double *bflux, cudaStream_t s, double *bflux_int,
+                      bool cell)
 {
+    if (!cell && !bflux && !bflux_int && !g.grav_g && plane_f64_supported(g))
+        return launch_plane_f64(g, stage, Uin, U0, Uout, ctrl, s);
     switch (g.nd * 10 + stage) {
     case 11: return launch_generic<1, 1>(g, Uin, U0, Uout, ctrl, bflux, bflux_int, s);
     case 12: return launch_generic<1, 2>(g, Uin, U0, Uout, ctrl, bflux, bflux_int, s);
@@ -218,13 +240,7 @@ __global__ void k_advance_boxes(const BoxDesc *boxes, int nbox)
     }
 }
 
-__global__ void k_advance(Ctrl *ctrl)
-{
-    if (ctrl->active) {
-        ctrl->t = ctrl->t + ctrl->dt;
-        ctrl->step = ctrl->step + 1;
-    }
-}
+__global__ void k_advance(Ctrl *ctrl) { advance(ctrl); }
 
 // The running CFL maximum of a slab <-> a device word the ranks all-reduce
 // (max over int64: non-negative doubles order like their bit patterns; a NaN
@@ -313,6 +329,12 @@ int launch_cfl(const Geom &g, const double *U, Ctrl *ctrl, cudaStream_t s)
 int launch_finalize_cfl(const Geom &g, Ctrl *ctrl, cudaStream_t s)
 {
     k_finalize_cfl<<<1, 1, 0, s>>>(g, ctrl);
+    return 1;
+}
+
+int launch_next_step(const Geom &g, Ctrl *ctrl, cudaStream_t s)
+{
+    k_next_step<<<1, 1, 0, s>>>(g, ctrl);
     return 1;
 }
 

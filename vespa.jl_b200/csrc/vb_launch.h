@@ -117,10 +117,12 @@ inline int64_t march_extent(const Geom &g) { return g.nd == 3 ? g.n[2] : g.n[1];
 
 // vb_kern_fp64.cu (compiled with -fmad=false)
 // bflux: the outer boundary-flux planes being recorded (or null); bflux_int:
-// the interior face register [axis][5][ncell] (or null).  
+// the interior face register [axis][5][ncell] (or null).  2D grids with room
+// for a 16 x 16 tile take the plane kernel (vb_stage_plane_f64.cuh) unless
+// `cell` asks for the cell-centric one or something is recorded or added.
 int launch_stage_fp64(const Geom &g, int stage, const double *Uin, const double *U0,
                       double *Uout, Ctrl *ctrl, double *bflux, cudaStream_t s,
-                      double *bflux_int = nullptr);
+                      double *bflux_int = nullptr, bool cell = false);
 int launch_cfl(const Geom &g, const double *U, Ctrl *ctrl, cudaStream_t s);
 int launch_finalize_cfl(const Geom &g, Ctrl *ctrl, cudaStream_t s);
 int launch_set_dt(const Geom &g, Ctrl *ctrl, double dt, cudaStream_t s);
@@ -149,6 +151,8 @@ int launch_stage_tiled2d_mixed(const BoxDesc *hbox, int nitems, unsigned int *wo
 // Per-box dt finalisation (evolve!'s loop head) and clock advance for a table.
 int launch_finalize_boxes(const BoxDesc *boxes, int nbox, unsigned int *work, cudaStream_t s);
 int launch_advance_boxes(const BoxDesc *boxes, int nbox, cudaStream_t s);
+// launch_advance, then launch_finalize_cfl of the next step.
+int launch_next_step(const Geom &g, Ctrl *ctrl, cudaStream_t s);
 // Clock advance of a single control block (t += dt, step += 1 while active).
 int launch_advance(Ctrl *ctrl, cudaStream_t s);
 // Copy the running CFL maximum of ctrl out to (put = 0) or in from (put = 1)
@@ -157,6 +161,12 @@ int launch_cfl_bits(Ctrl *ctrl, unsigned long long *dev, int put, cudaStream_t s
 // A bounded mbarrier wait that must run out after limit_ns, then the stage
 // kernels' abandon path (CTRL_F_TIMEOUT in ctrl).
 int launch_wait_selftest(Ctrl *ctrl, uint64_t limit_ns, cudaStream_t s);
+
+// vb_march.cu: nsteps CFL-limited steps (evolve!'s loop, dt and clock included)
+// of a small float64 1D or 2D grid in one launch; the state and the control
+// block end as that many separate steps leave them.
+bool march_supported(const Geom &g);
+int launch_march(const Geom &g, double *U, Ctrl *ctrl, int64_t nsteps, cudaStream_t s);
 
 // vb_kern_mixed.cu
 int launch_stage_tiled3d_mixed(const BoxDesc *hbox, const BoxDesc *boxes, const int *item_box,
