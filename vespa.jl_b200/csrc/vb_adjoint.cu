@@ -150,9 +150,11 @@ int vb_adjoint_create(vb_grid *gr, int64_t max_steps, int64_t checkpoint_every, 
     if (a->every == 1) get((void **)&a->tape1, a->state_bytes * (size_t)max_steps);
     get((void **)&a->lam, a->state_bytes);
     get((void **)&a->lam1, a->state_bytes);
-    get((void **)&a->gL, a->state_bytes * nd);
-    get((void **)&a->gR, a->state_bytes * nd);
-    get((void **)&a->code, sizeof(uint16_t) * nc * nd);
+    if (nd != 2) {  // the 2D stage keeps its face adjoints on chip
+        get((void **)&a->gL, a->state_bytes * nd);
+        get((void **)&a->gR, a->state_bytes * nd);
+        get((void **)&a->code, sizeof(uint16_t) * nc * nd);
+    }
     get((void **)&a->dts, sizeof(double) * (size_t)max_steps);
     get((void **)&a->ctrl, sizeof(vb::Ctrl));
     if (e == cudaSuccess) e = cudaEventCreate(&a->ev[0]);
@@ -276,7 +278,8 @@ int vb_adjoint_backward(vb_adjoint *a, const double *lam_final, double *lam_init
     int rc = use(gr->ctx);
     if (rc) return rc;
     cudaStream_t s = gr->ctx->stream;
-    VB_CUDA(cudaMemcpyAsync(a->lam, lam_final, a->state_bytes, cudaMemcpyHostToDevice, s));
+    rc = vb::detail::host_copy(gr->ctx, a->lam, lam_final, a->state_bytes, true);
+    if (rc) return rc;
     double ms_re = 0.0, ms_adj = 0.0;
     if (a->tape1) {  // every step's two states were kept: no recompute
         VB_CUDA(cudaEventRecord(a->ev[0], s));
@@ -286,8 +289,8 @@ int vb_adjoint_backward(vb_adjoint *a, const double *lam_final, double *lam_init
             if (rc) return rc;
         }
         VB_CUDA(cudaEventRecord(a->ev[1], s));
-        VB_CUDA(cudaMemcpyAsync(lam_init, a->lam, a->state_bytes, cudaMemcpyDeviceToHost, s));
-        VB_CUDA(cudaStreamSynchronize(s));
+        rc = vb::detail::host_copy(gr->ctx, lam_init, a->lam, a->state_bytes, false);
+        if (rc) return rc;
         a->ms[1] = 0.0;
         a->ms[2] = elapsed(a->ev[0], a->ev[1]);
         return VB_OK;
@@ -318,8 +321,8 @@ int vb_adjoint_backward(vb_adjoint *a, const double *lam_final, double *lam_init
         VB_CUDA(cudaEventSynchronize(a->ev[1]));
         ms_adj += elapsed(a->ev[0], a->ev[1]);
     }
-    VB_CUDA(cudaMemcpyAsync(lam_init, a->lam, a->state_bytes, cudaMemcpyDeviceToHost, s));
-    VB_CUDA(cudaStreamSynchronize(s));
+    rc = vb::detail::host_copy(gr->ctx, lam_init, a->lam, a->state_bytes, false);
+    if (rc) return rc;
     a->ms[1] = ms_re;
     a->ms[2] = ms_adj;
     return VB_OK;

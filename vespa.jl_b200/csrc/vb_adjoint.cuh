@@ -207,4 +207,108 @@ __device__ __forceinline__ void hllc_vjp(const double WL[5], const double WR[5],
     WRb[4] += pRb;
 }
 
+// hllc_vjp in the face-normal frame (rho, u_n, u_t1, u_t2, p), Lb and Rb
+// overwritten.  The forward speeds that decide the branches are formed as
+// hllc_frame forms them (the forward's own bits); the derivatives take products
+// with the reciprocals of the seven denominators, formed side by side.  States
+// outside the range hllc_frame takes go to hllc_vjp.
+__device__ __forceinline__ void hllc_vjp_frame(const double L[5], const double R[5], double g,
+                                               double ig1, const double Fb[5], double Lb[5],
+                                               double Rb[5])
+{
+    const double yL = rcp64(L[0]), yR = rcp64(R[0]);
+    const double cL = root64(quot64(g * L[4], L[0], yL));
+    const double cR = root64(quot64(g * R[4], R[0], yR));
+    const double aL = L[1] - cL, aR = R[1] - cR, bL = L[1] + cL, bR = R[1] + cR;
+    const bool SL_from_L = aL <= aR, SR_from_L = bL >= bR;
+    const double SL = SL_from_L ? aL : aR, SR = SR_from_L ? bL : bR;
+    const double dL = SL - L[1], dR = SR - R[1];
+    const double N = R[4] - L[4] + L[0] * L[1] * dL - R[0] * R[1] * dR;
+    const double D = L[0] * dL - R[0] * dR;
+    const double yD = rcp64(D), Ss = quot64(N, D, yD);
+    const bool supL = SL >= 0.0, supR = SR <= 0.0;
+    const bool left = supL || (!supR && Ss >= 0.0);
+    const double SK = left ? SL : SR;
+    const double rho = left ? L[0] : R[0], un = left ? L[1] : R[1], y = left ? yL : yR;
+    const double u1 = left ? L[2] : R[2], u2 = left ? L[3] : R[3], p = left ? L[4] : R[4];
+    const double v2 = un * un + u1 * u1 + u2 * u2;
+    const double E = p * ig1 + 0.5 * rho * v2;
+    const double d = SK - Ss, a = SK - un, q = rho * a;
+    if (!hllc_operands_ok(L, R, D, d, q, E, N)) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) Lb[k] = Rb[k] = 0.0;
+        hllc_vjp<1>(L, R, g, Fb, Lb, Rb);
+        return;
+    }
+    double lr = 0.0, lu = 0.0, lp = 0.0, rr = 0.0, ru = 0.0, rp = 0.0;
+    // physical flux of the selected side
+    const double w = Fb[1] * un + Fb[2] * u1 + Fb[3] * u2;
+    double rb = (Fb[0] + w) * un;
+    double ub = Fb[0] * rho + rho * w + Fb[4] * (E + p);
+    double nb = Fb[1] * rho * un, t1 = Fb[2] * rho * un, t2 = Fb[3] * rho * un;
+    double pb = Fb[1] + Fb[4] * un, Eb = Fb[4] * un;
+    if (!(supL || supR)) {
+        const double yd = rcp64(d), yq = rcp64(q), ycL = rcp64(cL), ycR = rcp64(cR);
+        const double f = q * yd, r = p * yq, A = Ss - un, B = Ss + r, Es = E * y + A * B;
+        // sum of Fb (U* - U)
+        double Sb = Fb[0] * (f - rho) + Fb[1] * (f * Ss - rho * un) + Fb[2] * (f - rho) * u1 +
+                    Fb[3] * (f - rho) * u2 + Fb[4] * (f * Es - E);
+        rb -= SK * (Fb[0] + w);
+        nb -= SK * Fb[1] * rho;
+        t1 += SK * Fb[2] * (f - rho);
+        t2 += SK * Fb[3] * (f - rho);
+        Eb -= SK * Fb[4];
+        const double fb = SK * (Fb[0] + Fb[1] * Ss + Fb[2] * u1 + Fb[3] * u2 + Fb[4] * Es);
+        double sb = SK * Fb[1] * f;
+        const double Esb = SK * Fb[4] * f;
+        Eb += Esb * y;
+        rb -= Esb * E * y * y;
+        const double Bb = Esb * A;
+        sb += Esb * B + Bb;
+        ub -= Esb * B;
+        pb += Bb * yq;
+        const double qb = fb * yd - Bb * r * yq, db = -fb * f * yd;
+        Sb += db;
+        sb -= db;
+        rb += qb * a;
+        Sb += qb * rho;
+        ub -= qb * rho;
+        // S* = N / D
+        const double Nb = sb * yD, Db = -Nb * Ss;
+        rp += Nb;
+        lp -= Nb;
+        lr += (Nb * L[1] + Db) * dL;
+        lu += Nb * L[0] * (SL - 2.0 * L[1]) - Db * L[0];
+        rr -= (Nb * R[1] + Db) * dR;
+        ru += -Nb * R[0] * (SR - 2.0 * R[1]) + Db * R[0];
+        double SLb = Nb * L[0] * L[1] + Db * L[0], SRb = -Nb * R[0] * R[1] - Db * R[0];
+        if (left) SLb += Sb;
+        else SRb += Sb;
+        double cLb = 0.0, cRb = 0.0;
+        if (SL_from_L) { lu += SLb; cLb -= SLb; } else { ru += SLb; cRb -= SLb; }
+        if (SR_from_L) { lu += SRb; cLb += SRb; } else { ru += SRb; cRb += SRb; }
+        // c = sqrt(g p / rho); c > 0 in the range checked above
+        lp += cLb * (0.5 * g) * ycL * yL;
+        lr -= cLb * cL * 0.5 * yL;
+        rp += cRb * (0.5 * g) * ycR * yR;
+        rr -= cRb * cR * 0.5 * yR;
+    }
+    // E = p / (g - 1) + rho |v|^2 / 2 of the selected side
+    pb += Eb * ig1;
+    rb += Eb * 0.5 * v2;
+    nb += Eb * rho * un + ub;
+    t1 += Eb * rho * u1;
+    t2 += Eb * rho * u2;
+    Lb[0] = lr + (left ? rb : 0.0);
+    Lb[1] = lu + (left ? nb : 0.0);
+    Lb[2] = left ? t1 : 0.0;
+    Lb[3] = left ? t2 : 0.0;
+    Lb[4] = lp + (left ? pb : 0.0);
+    Rb[0] = rr + (left ? 0.0 : rb);
+    Rb[1] = ru + (left ? 0.0 : nb);
+    Rb[2] = left ? 0.0 : t1;
+    Rb[3] = left ? 0.0 : t2;
+    Rb[4] = rp + (left ? 0.0 : pb);
+}
+
 }  // namespace vb

@@ -143,6 +143,147 @@ k_adj_cell(Geom g, const double *__restrict__ U, const double *__restrict__ gL,
     }
 }
 
+// Both passes of a 2D stage in one kernel: a block owns a 16 x 16 tile.  The
+// primitives of the tile and of the three cells around it along each axis come
+// into shared memory (each converted once, not four times per face and axis);
+// the 19 faces per row and per column that the tile's cells depend on are
+// solved there (1.19 times the faces, against writing and gathering ten
+// values a face through memory), then each cell gathers its own.
+namespace adj2 {
+
+constexpr int T = 16, H = 3, S = T + 2 * H;  // tile, halo, extended side
+constexpr int NW = T * S;                     // cells of one extended strip
+constexpr int NF = T * (T + 3);               // faces of one axis: 19 per line
+constexpr int NTH = 320;
+
+struct Smem {
+    double w[2][5][NW];   // primitives: x strip [row][22], y strip [column][22]
+    double gl[2][5][NF], gr[2][5][NF];  // face adjoints WLb, WRb, line-major
+    uint16_t code[2][NF]; // minmod codes of the cell behind each face
+};
+
+}  // namespace adj2
+
+__global__ void __launch_bounds__(adj2::NTH, 2)
+k_adj_plane(const __grid_constant__ Geom g, const double *__restrict__ U, const double *lam,
+            const double *M, double invV, double *out, int ntx)
+{
+    using namespace adj2;
+    extern __shared__ __align__(16) unsigned char raw[];
+    adj2::Smem &S_ = *reinterpret_cast<adj2::Smem *>(raw);
+    const int t = threadIdx.x;
+    const int nx = (int)g.n[0], ny = (int)g.n[1];
+    const int x0 = (int)(blockIdx.x % ntx) * T, y0 = (int)(blockIdx.x / ntx) * T;
+    const int64_t nc = g.ncell;
+    const double gamma = g.gamma, ig1 = 1.0 / (gamma - 1.0);
+    auto wrap = [](int c, int n) {
+        c %= n;
+        return c < 0 ? c + n : c;
+    };
+    // strip a's cell (line, pos): along x position pos - 3 of row `line`, along
+    // y of column `line`
+    auto cell = [&](int a, int line, int pos) {
+        const int x = a == 0 ? x0 + pos - H : x0 + line, y = a == 0 ? y0 + line : y0 + pos - H;
+        return (int64_t)wrap(x, nx) + (int64_t)nx * wrap(y, ny);
+    };
+    // the tile's cells go into both strips, the halo cells into their own
+    for (int i = t; i < T * T + 4 * H * T; i += NTH) {
+        int a = 0, line, pos, pos2 = -1, line2 = 0;
+        if (i < T * T) {
+            line = i / T;
+            pos = (i & (T - 1)) + H;
+            line2 = i & (T - 1);
+            pos2 = line + H;
+        } else {
+            const int h = i - T * T;
+            a = h / (2 * H * T);
+            const int r = h - a * 2 * H * T, k = r / T;  // halo position 0 .. 5
+            // along y consecutive threads take consecutive columns
+            line = r - k * T;
+            pos = k < H ? k : k + T;
+        }
+        const int64_t l = cell(a, line, pos);
+        double u[5], W[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) u[k] = __ldg(U + k * nc + l);
+        cons2prim(u, gamma, W);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) S_.w[a][k][line * S + pos] = W[k];
+        if (pos2 >= 0)
+#pragma unroll
+            for (int k = 0; k < 5; ++k) S_.w[1][k][line2 * S + pos2] = W[k];
+    }
+    __syncthreads();
+    const double *mu = M ? M : lam;  // mu = 0.5 lam (stage 2) or M (stage 1)
+    const double ms = M ? 1.0 : 0.5;
+    for (int i = t; i < 2 * NF; i += NTH) {
+        const int a = i >= NF, j = i - a * NF, line = j / (T + 3), f = j - line * (T + 3);
+        // face f lies between cells f + 1 and f + 2 of the strip
+        const int c = line * S + f + 1;
+        const int64_t lo = cell(a, line, f + 1), hi = cell(a, line, f + 2);
+        double L[5], R[5], Fb[5], Lb[5], Rb[5];
+        unsigned cd = 0;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            // component k of the frame is field kf: normal and first tangential
+            // velocity swap on y faces
+            const int kf = a == 1 && (k == 1 || k == 2) ? 3 - k : k;
+            const double *p = S_.w[a][kf] + c;
+            const double m1 = p[-1], q0 = p[0], q1 = p[1], q2 = p[2], b = q1 - q0;
+            cd |= minmod_code(q0 - m1, b) << (2 * kf);
+            L[k] = face_val(q0, 0.5, minmod<double>(q0 - m1, b));
+            R[k] = face_val(q1, -0.5, minmod<double>(b, q2 - q1));
+            Fb[k] = g.area[a] * (ms * __ldg(mu + kf * nc + lo) - ms * __ldg(mu + kf * nc + hi));
+        }
+        hllc_vjp_frame(L, R, gamma, ig1, Fb, Lb, Rb);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            const int kf = a == 1 && (k == 1 || k == 2) ? 3 - k : k;
+            S_.gl[a][kf][j] = Lb[k];
+            S_.gr[a][kf][j] = Rb[k];
+        }
+        S_.code[a][j] = (uint16_t)cd;
+    }
+    __syncthreads();
+    for (int i = t; i < T * T; i += NTH) {
+        const int lx = i & (T - 1), ly = i / T, x = x0 + lx, y = y0 + ly;
+        if (x >= nx || y >= ny) continue;
+        const int64_t lin = (int64_t)x + (int64_t)nx * y;
+        double Wb[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            // the cell's hi face is face pos + 2 of its line: cell pos + 3 of the
+            // strip is behind it
+            const int o = (a == 0 ? ly * (T + 3) + lx : lx * (T + 3) + ly) + 2;
+            const unsigned ck = S_.code[a][o], cp = S_.code[a][o + 1], cm = S_.code[a][o - 1];
+#pragma unroll
+            for (int k = 0; k < 5; ++k) {
+                const double *gl = S_.gl[a][k] + o, *gr = S_.gr[a][k] + o;
+                const double fl = gl[0], fr = gr[-1];
+                double w = fl + fr;
+                const double sb = 0.5 * fl - 0.5 * fr;
+                const unsigned bk = (ck >> (2 * k)) & 3u;
+                if (bk == 1u) w += sb;
+                else if (bk == 2u) w -= sb;
+                if (((cp >> (2 * k)) & 3u) == 1u) w -= 0.5 * gl[1] - 0.5 * gr[0];
+                if (((cm >> (2 * k)) & 3u) == 2u) w += 0.5 * gl[-1] - 0.5 * gr[-2];
+                Wb[k] += w;
+            }
+        }
+        double u[5], Ub[5];
+#pragma unroll
+        for (int k = 0; k < 5; ++k) u[k] = __ldg(U + k * nc + lin);
+        cons2prim_vjp(u, gamma, Wb, Ub);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            const int64_t o = k * nc + lin;
+            double v = 0.5 * lam[o];
+            if (M) v = v + M[o];
+            out[o] = v - invV * Ub[k];
+        }
+    }
+}
+
 __global__ void k_record_dt(const Ctrl *ctrl, double *dts, long long step0, long long cap)
 {
     if (!ctrl->active) return;
@@ -156,6 +297,15 @@ int launch_adj_stage(const Geom &g, const double *U, const double *lam, const do
                      double invV, double *gL, double *gR, uint16_t *code, double *out,
                      cudaStream_t s)
 {
+    if (g.nd == 2 && g.n[0] <= (1 << 24) && g.n[1] <= (1 << 24)) {
+        const int ntx = (int)((g.n[0] + adj2::T - 1) / adj2::T);
+        const int64_t nt = ntx * ((g.n[1] + adj2::T - 1) / adj2::T);
+        static const cudaError_t set = cudaFuncSetAttribute(
+            k_adj_plane, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(adj2::Smem));
+        if (set != cudaSuccess || nt > 0x7fffffffLL) return -1;
+        k_adj_plane<<<(unsigned)nt, adj2::NTH, sizeof(adj2::Smem), s>>>(g, U, lam, M, invV, out, ntx);
+        return 1;
+    }
     const int64_t nb_f = (g.ncell + 127) / 128;
     if (g.ncell <= 0 || nb_f > 0x7fffffffLL) return -1;
     // mu = 0.5*lam (adjoint of stage 2) or M (adjoint of stage 1)

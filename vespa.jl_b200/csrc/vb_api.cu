@@ -680,6 +680,7 @@ int vb_ctx_destroy(vb_ctx *ctx)
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->scratch) cudaFree(ctx->scratch);
+    vb::detail::host_lanes_free(ctx->lanes);
     for (cudaEvent_t &e : ctx->marks)
         if (e) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -772,8 +773,11 @@ int vb_hllc_faces(vb_ctx *ctx, int64_t nf, const double *WL, const double *WR,
     if (nf < 0) return fail(VB_EINVAL, "nf < 0");
     if (nf == 0) return VB_OK;  // the reference returns F untouched for nf == 0
     if (!WL || !WR || !axis || !F) return fail(VB_EINVAL, "null buffer");
-    for (int64_t f = 0; f < nf; ++f)
-        if (axis[f] < 1 || axis[f] > 3) return fail(VB_EINVAL, "axis entries must be 1, 2 or 3");
+    unsigned bad = 0;  // no early exit: the loop vectorises
+    for (int64_t f = 0; f < nf; ++f) bad |= (unsigned)(axis[f] - 1) > 2u;
+    if (bad) return fail(VB_EINVAL, "axis entries must be 1, 2 or 3");
+    if (nf >= vb::detail::HOST_FACES)
+        return vb::detail::host_faces(ctx, nf, WL, WR, axis, gamma, F);
     const size_t bw = sizeof(double) * 5 * (size_t)nf;
     const size_t ba = sizeof(int32_t) * (size_t)nf;
     const size_t need = 3 * bw + ((ba + 255) & ~(size_t)255);
@@ -1028,11 +1032,8 @@ int vb_grid_upload(vb_grid *gr, const double *U)
     if (!gr || !U) return fail(VB_EINVAL, "null argument");
     int rc = use(gr->ctx);
     if (rc) return rc;
-    VB_CUDA(cudaMemcpyAsync(gr->U, U, sizeof(double) * 5 * (size_t)gr->g.ncell,
-                            cudaMemcpyHostToDevice, gr->ctx->stream));
-    VB_CUDA(cudaStreamSynchronize(gr->ctx->stream));
     gr->invdt_valid = false;
-    return VB_OK;
+    return vb::detail::host_copy(gr->ctx, gr->U, U, sizeof(double) * 5 * (size_t)gr->g.ncell, true);
 }
 
 int vb_grid_download(vb_grid *gr, double *U)
@@ -1041,10 +1042,7 @@ int vb_grid_download(vb_grid *gr, double *U)
     if (!gr || !U) return fail(VB_EINVAL, "null argument");
     int rc = use(gr->ctx);
     if (rc) return rc;
-    VB_CUDA(cudaMemcpyAsync(U, gr->U, sizeof(double) * 5 * (size_t)gr->g.ncell,
-                            cudaMemcpyDeviceToHost, gr->ctx->stream));
-    VB_CUDA(cudaStreamSynchronize(gr->ctx->stream));
-    return VB_OK;
+    return vb::detail::host_copy(gr->ctx, U, gr->U, sizeof(double) * 5 * (size_t)gr->g.ncell, false);
 }
 
 int vb_grid_device_state(vb_grid *gr, double **dU)

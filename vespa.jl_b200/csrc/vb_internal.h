@@ -9,6 +9,7 @@
 #include "../../include/vespa_b200.h"
 #include "vb_launch.h"
 
+struct vb_host_lanes;  // staging of large pageable host arrays (vb_host.cu)
 
 struct vb_ctx {
     int device = 0;
@@ -16,6 +17,7 @@ struct vb_ctx {
     int64_t launches = 0;
     void *scratch = nullptr;  // vb_hllc_faces staging (device)
     size_t scratch_bytes = 0;
+    vb_host_lanes *lanes = nullptr;
     cudaEvent_t marks[16] = {};
 };
 
@@ -82,6 +84,16 @@ int grid_default_kz(const Geom &g, int precision, bool *taper);
 // Context-owned device staging buffer of at least `bytes` (grown with
 // cudaMalloc; reused across calls on the context's stream).
 int ctx_scratch(vb_ctx *ctx, size_t bytes, void **out);
+
+// Copy between a host array and device memory, ordered after the context's
+// stream; returns when done.  Large pageable arrays go through the lanes of
+// vb_host.cu.
+int host_copy(vb_ctx *ctx, void *dst, const void *src, size_t bytes, bool to_device);
+// vb_hllc_faces for at least HOST_FACES faces, staged piece by piece.
+constexpr int64_t HOST_FACES = 32768;
+int host_faces(vb_ctx *ctx, int64_t nf, const double *WL, const double *WR, const int32_t *axis,
+               double gamma, double *F);
+void host_lanes_free(vb_host_lanes *hl);
 
 // Grid stepping helpers shared with the adjoint (vb_api.cu).
 int grid_ensure_cfl(vb_grid *gr);   // CFL max of the current state, if stale
