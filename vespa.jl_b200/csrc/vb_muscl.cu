@@ -149,6 +149,11 @@ __global__ void __launch_bounds__(MB) k_muscl_prep(MusclGeom m, MusclFields U, d
     if (!isfinite(d + e + vx + vy + vz)) *nonfinite = 1;
 }
 
+__device__ __forceinline__ void prefetch_l2(const void *p)
+{
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // Tile of one CTA: TX x TY cells of one z-plane, one thread per cell column.
 constexpr int TX = 32, TY = 8, NT = TX * TY;
 constexpr int PW = TX + 4, PH = TY + 4;  // plane window: 2-cell halo in x and y
@@ -159,13 +164,13 @@ constexpr int FXN = (TX + 1) * TY;       // x faces of one plane tile
 constexpr int FYN = TX * (TY + 1);       // y faces of one plane tile
 constexpr size_t TILE_SMEM = sizeof(double) * (NSLOT * PS + 5 * FXN + 5 * FYN);
 
-// plm_pt of finite values: minmod3 is zero unless the three differences share
-// their sign bit (a zero among them gives zero either way), else the smallest
-// of them, added by predicated multiply-adds (half of it is exact, so the fused
-// form rounds as the product and sum do)
-__device__ __forceinline__ double plm_finite(double vm1, double v, double vp1, double th)
+// plm_pt of finite values from the two scaled differences a = (v - vm1) theta,
+// b = (vp1 - v) theta and c = (vp1 - vm1) / 2: minmod3 is zero unless the three
+// share their sign bit (a zero among them gives zero either way), else the
+// smallest of them, added by predicated multiply-adds (half of it is exact, so
+// the fused form rounds as the product and sum do)
+__device__ __forceinline__ double plm_finite(double v, double a, double b, double c)
 {
-    const double a = (v - vm1) * th, b = (vp1 - v) * th, c = 0.5 * (vp1 - vm1);
     const int ha = __double2hiint(a), hb = __double2hiint(b), hc = __double2hiint(c);
     const bool on = ((ha ^ hb) | (ha ^ hc)) >= 0;
     const double x = fabs(a) < fabs(b) ? a : b;
@@ -234,8 +239,9 @@ __device__ __forceinline__ void face_flux(const double *qm1, const double *q0, c
 #pragma unroll
         for (int f = 0; f < 5; ++f) {
             const double a = qm1[off[f]], b = q0[off[f]], c = q1[off[f]], d = q2[off[f]];
-            L[f] = plm_finite(a, b, c, m.theta);
-            R[f] = plm_finite(d, c, b, m.theta);
+            const double e = (c - b) * m.theta;  // both sides' difference across the face
+            L[f] = plm_finite(b, (b - a) * m.theta, e, 0.5 * (c - a));
+            R[f] = plm_finite(c, (c - d) * m.theta, -e, 0.5 * (b - d));
         }
         L[0] = L[0] > m.small_rho ? L[0] : m.small_rho;
         R[0] = R[0] > m.small_rho ? R[0] : m.small_rho;
@@ -311,6 +317,16 @@ __global__ void __launch_bounds__(NT, 2) k_muscl_tile(MusclGeom m, const double 
     for (int64_t k = k0; k < k1; ++k) {
         cp_async_wait_group<1>();  // plane k + 2 has landed (k + 3 may be in flight)
         __syncthreads();
+        // the next plane's step-start state and stage input into L2 (two
+        // 128-byte lines a row) ahead of its update
+        if (in && (tx & 15) == 0 && k + 1 < k1) {
+            const int64_t i = ((k + 1) * ny + y) * nx + x;
+#pragma unroll
+            for (int f = 0; f < 5; ++f) {
+                prefetch_l2(U0 + f * N + i);
+                if constexpr (STAGE == 2) prefetch_l2(U.f[f] + i);
+            }
+        }
         const double *const pk = slot(k);
         double fhi[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
         if (in && face_ok(k, nz))
@@ -557,10 +573,7 @@ int vb_muscl_upload(vb_muscl *mu, const double *U)
     if (!mu || !U) return fail(VB_EINVAL, "null argument");
     int rc = use(mu->ctx);
     if (rc) return rc;
-    VB_CUDA(cudaMemcpyAsync(mu->U, U, sizeof(double) * 5 * mu->m.N, cudaMemcpyHostToDevice,
-                            mu->ctx->stream));
-    VB_CUDA(cudaStreamSynchronize(mu->ctx->stream));
-    return VB_OK;
+    return vb::detail::host_copy(mu->ctx, mu->U, U, sizeof(double) * 5 * mu->m.N, true);
 }
 
 int vb_muscl_download(vb_muscl *mu, double *U)
@@ -568,10 +581,7 @@ int vb_muscl_download(vb_muscl *mu, double *U)
     if (!mu || !U) return fail(VB_EINVAL, "null argument");
     int rc = use(mu->ctx);
     if (rc) return rc;
-    VB_CUDA(cudaMemcpyAsync(U, mu->U, sizeof(double) * 5 * mu->m.N, cudaMemcpyDeviceToHost,
-                            mu->ctx->stream));
-    VB_CUDA(cudaStreamSynchronize(mu->ctx->stream));
-    return VB_OK;
+    return vb::detail::host_copy(mu->ctx, U, mu->U, sizeof(double) * 5 * mu->m.N, false);
 }
 
 int vb_muscl_state(vb_muscl *mu, double **dU)
