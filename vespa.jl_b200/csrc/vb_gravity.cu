@@ -38,7 +38,7 @@ struct GravCtrl {
     double rhobar, rsold, pAp, alpha, beta, bnorm, relres, mu, mgmu;
     long long iters, maxiter;
     int done;
-    unsigned int ticket;  // blocks past a grid_sum; zero between launches
+    unsigned int ticket, ticket2;  // blocks past a grid_sum; zero between launches
     double tol;
 };
 
@@ -495,6 +495,71 @@ __device__ __forceinline__ bool grid_sum(double s, double *part, unsigned int *t
     for (unsigned j = threadIdx.x; j < nb; j += GB) r = r + __ldcg(part + j);
     total = block_sum(r, sh);
     return threadIdx.x == 0;
+}
+
+// CG start on the cube: r = b - A phi with b = -4 pi G (rho - rhobar) V
+// (k_rhs), and the scalars of k_cg_init_final
+__global__ void __launch_bounds__(GB) k_cube_init(CubeP P, GravP Q, double vol, const double *__restrict__ rho,
+                                                 const double *__restrict__ phi,
+                                                 double *__restrict__ r, double *part, GravCtrl *gc)
+{
+    const double rhobar = Q.project_mean ? gc->rhobar : 0.0;
+    double rr = 0.0, bb = 0.0;
+    cube_cells(
+        P.n, [&](int i) { return phi[i]; },
+        [&](int i, double c, double sx, double sy, double sz) {
+            const double b = -VB_FOURPI * Q.G * (rho[i] - rhobar) * vol;
+            const double ri = b - cube_lap(P, c, sx, sy, sz);
+            r[i] = ri;
+            rr = rr + ri * ri;
+            bb = bb + b * b;
+        });
+    // two sums: the first one's total waits in gc for the second's last block
+    double t;
+    if (grid_sum(rr, part, &gc->ticket, t)) gc->rsold = t;
+    const unsigned nb = gridDim.x * gridDim.y * gridDim.z;
+    if (grid_sum(bb, part + nb, &gc->ticket2, t)) {
+        double bnorm = sqrt(t);
+        if (bnorm == 0.0) bnorm = 1.0;
+        gc->bnorm = bnorm;
+    }
+}
+// the scalars that need both sums
+__global__ void k_cube_init_final(GravCtrl *gc)
+{
+    gc->relres = sqrt(gc->rsold) / gc->bnorm;
+    gc->iters = 0;
+    gc->done = gc->maxiter <= 0 ? 1 : 0;
+    gc->beta = 0.0;  // the first direction is z (mg_pcg.jl:188-191) or r
+}
+
+// k_accel on the cube: the same differences and quotients
+__global__ void __launch_bounds__(GB) k_cube_accel(const __grid_constant__ Geom g, int n,
+                                                  const double *__restrict__ phi,
+                                                  double *__restrict__ gacc)
+{
+    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
+    const int kz = cube_kz(n), z0 = blockIdx.z * kz, z1 = min(n, z0 + kz);
+    if (x >= n || y >= n) return;
+    const int nn = n * n, base = x + n * y;
+    const int xm = x > 0 ? -1 : n - 1, xp = x + 1 < n ? 1 : 1 - n;
+    const int ym = (y > 0 ? -1 : n - 1) * n, yp = (y + 1 < n ? 1 : 1 - n) * n;
+    double d[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double fd = 0.5 * (g.w[a] + g.w[a]);
+        d[a] = fd + fd;
+    }
+    double lo = phi[base + (z0 > 0 ? z0 - 1 : n - 1) * nn], c = phi[base + z0 * nn];
+    for (int z = z0; z < z1; ++z) {
+        const int i = base + z * nn;
+        const double hi = phi[base + (z + 1 < n ? z + 1 : 0) * nn];
+        gacc[i] = -(phi[i + xp] - phi[i + xm]) / d[0];
+        gacc[g.ncell + i] = -(phi[i + yp] - phi[i + ym]) / d[1];
+        gacc[2 * g.ncell + i] = -(hi - lo) / d[2];
+        lo = c;
+        c = hi;
+    }
 }
 
 // p = z + beta p (beta 0: z) into the other of the two direction buffers,
@@ -1051,6 +1116,11 @@ int refresh_accel(vb_grid *gr, vb_gravity *gv)
 {
     cudaStream_t s = gr->ctx->stream;
     const vb::Geom &g = gr->g;
+    if (gv->cube_n) {
+        vb::k_cube_accel<<<cube_grid(gv->cube_n), vb::GB, 0, s>>>(g, gv->cube_n, gv->phi, gv->gacc);
+        VB_CHECK_LAUNCH(gr->ctx, 1);
+        return VB_OK;
+    }
     VB_CHECK_LAUNCH(gr->ctx, ND_DISPATCH(g.nd, vb::k_accel, g, gv->P, gv->phi, gv->gacc));
     return VB_OK;
 }
@@ -1107,18 +1177,23 @@ int vb::detail::gravity_solve(vb_grid *gr, int64_t *iters, double *relres)
         k_mean_final<<<1, 1024, 0, s>>>(gv->part, gv->gc, 0);
         VB_CHECK_LAUNCH(gr->ctx, 1);
     }
-    k_rhs<<<GP, GB, 0, s>>>(g, gv->P, gr->U, gv->b, gv->gc);
-    VB_CHECK_LAUNCH(gr->ctx, 1);
-    VB_CHECK_LAUNCH(gr->ctx, ND_DISPATCH(g.nd, k_cg_init, g, gv->P, gv->phi, gv->b, gv->r, gv->p, gv->part));
-    k_cg_init_final<<<1, 1024, 0, s>>>(gv->part, gv->gc);
-    VB_CHECK_LAUNCH(gr->ctx, 1);
+    if (gv->cube_n) {
+        const CubeP P = cube_params(gv);
+        k_cube_init<<<cube_grid(P.n), GB, 0, s>>>(P, gv->P, g.vol, gr->U, gv->phi, gv->r, gv->cpart, gv->gc);
+        k_cube_init_final<<<1, 1, 0, s>>>(gv->gc);
+        VB_CHECK_LAUNCH(gr->ctx, 2);
+    } else {
+        k_rhs<<<GP, GB, 0, s>>>(g, gv->P, gr->U, gv->b, gv->gc);
+        VB_CHECK_LAUNCH(gr->ctx, 1);
+        VB_CHECK_LAUNCH(gr->ctx, ND_DISPATCH(g.nd, k_cg_init, g, gv->P, gv->phi, gv->b, gv->r, gv->p, gv->part));
+        k_cg_init_final<<<1, 1024, 0, s>>>(gv->part, gv->gc);
+        VB_CHECK_LAUNCH(gr->ctx, 1);
+    }
     if (!gv->gexec) {
         int rc = gv->cube_n ? capture_cube(gr, gv) : capture_iterations(gr, gv);
         if (rc) return rc;
     }
     if (gv->cube_n) {
-        // beta = 0 starts the direction from z (mg_pcg.jl:188-191) or r
-        VB_CUDA(cudaMemsetAsync(&gv->gc->beta, 0, sizeof(double), s));
         if (gv->precond == VB_GRAV_PRECOND_MG) {
             int rc = queue_precond(gr, gv, true, 0);
             if (rc) return rc;
@@ -1223,7 +1298,7 @@ int vb_gravity_enable(vb_grid *gr, const vb_gravity_desc *d)
         gv->cube_n = cube ? (int)g.n[0] : 0;
         if (cube && !gv->cpart) {
             const dim3 b = cube_grid((int)g.n[0]);
-            const size_t nb = std::max<size_t>((size_t)b.x * b.y * b.z, CUBE_UPDATE_BLOCKS);
+            const size_t nb = std::max<size_t>(2 * (size_t)b.x * b.y * b.z, CUBE_UPDATE_BLOCKS);
             cudaError_t e = cudaMalloc(&gv->cpart, sizeof(double) * nb);
             if (e == cudaSuccess) e = cudaMalloc(&gv->p2, sizeof(double) * (size_t)g.ncell);
             if (e == cudaSuccess)
