@@ -12,12 +12,13 @@
 // the reference's serial sums, so a solve matches the reference's to the
 // solver tolerance, not bit for bit.
 //
-// Every pass streams the CG vectors from HBM over a fixed grid of GP blocks
-// (the stencil's neighbours come from L1/L2); the stencil passes walk rows of
-// x so that a cell's coordinates cost no division.  One
-// CG iteration is five launches (matvec + p.Ap partials, alpha, vector update
-// + r.r partials, beta, direction update); groups of iterations replay as one
-// CUDA graph, each launch returning at once after convergence, and the host
+// Periodic cubes (n^3, n <= 1024) have their own passes, below, plain or
+// preconditioned.  On other grids every pass streams the CG vectors from HBM
+// over a fixed grid of GP blocks (the stencil's neighbours come from L1/L2); the
+// stencil passes walk rows of x so that a cell's coordinates cost no division.
+// One CG iteration is then five launches (matvec + p.Ap partials, alpha, vector
+// update + r.r partials, beta, direction update); groups of iterations replay as
+// one CUDA graph, each launch returning at once after convergence, and the host
 // reads the stop flag between groups.
 #include <algorithm>
 #include <cmath>
@@ -25,6 +26,7 @@
 #include <vector>
 
 #include "vb_internal.h"
+#include "vb_physics.cuh"
 
 namespace vb {
 namespace {
@@ -428,13 +430,20 @@ __global__ void __launch_bounds__(GB, GP_SM) k_lap(Geom g, GravP P, const double
 //   - each inner product is finished by the last block of the pass that forms
 //     it (fixed-order sums of the block partials: the same bits every run),
 //     which also sets the step's scalars.
-// That is 280 B of fine-grid traffic an iteration against 456 B as separate
+// That is 275 B of fine-grid traffic an iteration against 456 B as separate
 // passes, and about 25 launches against 90.  Levels of 16^3 and below run in
 // one block, in shared memory.  The iterations run as one graph with a WHILE
 // node on the stop flag, so the host reads nothing in between.
 //
-// A thread owns an (x, y) column and marches z over a chunk with the values
-// below and above in registers; the four side neighbours come from L1.
+// A thread owns an (x, y) column of cells, two side by side where n is even, and
+// marches z over a chunk with the values below and above in registers; the y
+// neighbours come from L1, the x neighbours of a pair from the lanes beside it.
+// What bounds the passes is the loads in flight: with one cell a thread they ran
+// at 2.4-3.6 TB/s at 256^3, with pairs (and 5 blocks an SM, which the sweeps have
+// to be held to) at 4.0-5.8 TB/s, 1.48 -> 1.2 ms an iteration.  Tried and slower:
+// two passes chained through shared memory (half the traffic, but the barrier a
+// plane leaves 2.4 TB/s of it), loads a plane further ahead, passes running
+// alternately up and down through the planes.
 
 constexpr double MG_OMEGA = 0.8;
 constexpr int MG_BLOCK = 16;  // levels of at most MG_BLOCK^3 cells run in one block
@@ -445,31 +454,92 @@ struct CubeP {
     double w;     // MG_OMEGA / diag(A)
 };
 
-__host__ __device__ inline int cube_kz(int n) { return n >= 512 ? 64 : n >= 128 ? 16 : 4; }
+// planes of a thread's chunk: long ones re-read fewer planes, short ones keep
+// the chip full (and the chain of dependent planes short) on small levels
+__host__ __device__ inline int cube_kz(int n)
+{
+    return n >= 512 ? 64 : n >= 192 ? 16 : n >= 96 ? 8 : n >= 48 ? 2 : 1;
+}
 
-// f(i, v(i), sx, sy, sz) for this thread's cells, s* the sums of v over the two
-// neighbours per axis
-template <class V, class F>
+// Two neighbouring cells of a row: the passes below run on D2 when n is even
+// (one 16-byte access for both) and on double otherwise, with the same
+// operations per cell.
+struct alignas(16) D2 {
+    double x, y;
+};
+__device__ __forceinline__ D2 operator+(D2 a, D2 b) { return {a.x + b.x, a.y + b.y}; }
+__device__ __forceinline__ D2 operator-(D2 a, D2 b) { return {a.x - b.x, a.y - b.y}; }
+__device__ __forceinline__ D2 operator-(D2 a, double b) { return {a.x - b, a.y - b}; }
+__device__ __forceinline__ D2 operator*(D2 a, D2 b) { return {a.x * b.x, a.y * b.y}; }
+__device__ __forceinline__ D2 operator*(double a, D2 b) { return {a * b.x, a * b.y}; }
+__device__ __forceinline__ double scaled(double a, double b, double c) { return a * b * c; }
+__device__ __forceinline__ D2 scaled(double a, D2 b, double c) { return {a * b.x * c, a * b.y * c}; }
+__device__ __forceinline__ double total(double a) { return a; }
+__device__ __forceinline__ double total(D2 a) { return a.x + a.y; }
+
+// the cells at i: load from and store to an array
+template <class T>
+struct At {
+    int i;
+    __device__ __forceinline__ T operator()(const double *p) const { return *reinterpret_cast<const T *>(p + i); }
+    __device__ __forceinline__ void put(double *p, T v) const { *reinterpret_cast<T *>(p + i) = v; }
+};
+
+// f(at, v, sx, sy, sz) for this thread's cells, s* the sums of v over the two
+// neighbours per axis; v(at) forms the operand.  Blocks of 32 x 8 cells (D2:
+// 32 x 16).
+template <class T, class V, class F>
 __device__ __forceinline__ void cube_cells(int n, V &&v, F &&f)
 {
-    const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
-    const int kz = cube_kz(n), z0 = blockIdx.z * kz, z1 = min(n, z0 + kz);
-    if (x >= n || y >= n) return;
-    const int nn = n * n, base = x + n * y;
-    const int xm = x > 0 ? -1 : n - 1, xp = x + 1 < n ? 1 : 1 - n;
-    const int ym = (y > 0 ? -1 : n - 1) * n, yp = (y + 1 < n ? 1 : 1 - n) * n;
-    double lo = v(base + (z0 > 0 ? z0 - 1 : n - 1) * nn), c = v(base + z0 * nn);
-    for (int z = z0; z < z1; ++z) {
-        const int i = base + z * nn;
-        const double hi = v(base + (z + 1 < n ? z + 1 : 0) * nn);
-        f(i, c, v(i + xm) + v(i + xp), v(i + ym) + v(i + yp), lo + hi);
-        lo = c;
-        c = hi;
+    constexpr bool PAIR = sizeof(T) == 16;
+    const int kz = cube_kz(n), z0 = blockIdx.z * kz, z1 = min(n, z0 + kz), nn = n * n;
+    if constexpr (PAIR) {
+        // x neighbours of a pair come from the lanes beside it (16 lanes a row),
+        // at the ends of the segment from memory; lanes beyond the cube repeat
+        // its last cells and store nothing
+        const int lane = threadIdx.x & 15, xr = blockIdx.x * 32 + 2 * lane, yr = blockIdx.y * 16 + (threadIdx.x >> 4);
+        const int x = min(xr, n - 2), y = min(yr, n - 1);
+        const bool in = xr < n && yr < n;
+        const int base = x + n * y, ym = (y > 0 ? -1 : n - 1) * n, yp = (y + 1 < n ? 1 : 1 - n) * n;
+        const bool first = lane == 0, last = lane == 15 || x + 2 >= n;
+        const int xe = first ? (x > 0 ? -1 : n - 1) : x + 2 < n ? 2 : 2 - n;
+        D2 lo = v(At<D2>{base + (z0 > 0 ? z0 - 1 : n - 1) * nn}), c = v(At<D2>{base + z0 * nn});
+        for (int z = z0; z < z1; ++z) {
+            const int i = base + z * nn;
+            const D2 hi = v(At<D2>{base + (z + 1 < n ? z + 1 : 0) * nn});
+            const D2 sy = v(At<D2>{i + ym}) + v(At<D2>{i + yp});
+            double l = __shfl_up_sync(0xffffffffu, c.y, 1, 16), r = __shfl_down_sync(0xffffffffu, c.x, 1, 16);
+            if (first || last) {
+                const double e = v(At<double>{i + xe});
+                if (first) l = e;
+                else r = e;
+                if (first && last) r = v(At<double>{i + (x + 2 < n ? 2 : 2 - n)});
+            }
+            if (in) f(At<D2>{i}, c, D2{l + c.y, c.x + r}, sy, lo + hi);
+            lo = c;
+            c = hi;
+        }
+    } else {
+        const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
+        if (x >= n || y >= n) return;
+        const int base = x + n * y;
+        const int xm = x > 0 ? -1 : n - 1, xp = x + 1 < n ? 1 : 1 - n;
+        const int ym = (y > 0 ? -1 : n - 1) * n, yp = (y + 1 < n ? 1 : 1 - n) * n;
+        double lo = v(At<double>{base + (z0 > 0 ? z0 - 1 : n - 1) * nn}), c = v(At<double>{base + z0 * nn});
+        for (int z = z0; z < z1; ++z) {
+            const int i = base + z * nn;
+            const double hi = v(At<double>{base + (z + 1 < n ? z + 1 : 0) * nn});
+            f(At<double>{i}, c, v(At<double>{i + xm}) + v(At<double>{i + xp}),
+              v(At<double>{i + ym}) + v(At<double>{i + yp}), lo + hi);
+            lo = c;
+            c = hi;
+        }
     }
 }
 
 // A v at a cell from cube_cells' sums
-__device__ __forceinline__ double cube_lap(const CubeP &P, double c, double sx, double sy, double sz)
+template <class T>
+__device__ __forceinline__ T cube_lap(const CubeP &P, T c, T sx, T sy, T sz)
 {
     return P.c[0] * (2.0 * c - sx) + P.c[1] * (2.0 * c - sy) + P.c[2] * (2.0 * c - sz);
 }
@@ -499,20 +569,21 @@ __device__ __forceinline__ bool grid_sum(double s, double *part, unsigned int *t
 
 // CG start on the cube: r = b - A phi with b = -4 pi G (rho - rhobar) V
 // (k_rhs), and the scalars of k_cg_init_final
+template <class T>
 __global__ void __launch_bounds__(GB) k_cube_init(CubeP P, GravP Q, double vol, const double *__restrict__ rho,
                                                  const double *__restrict__ phi,
                                                  double *__restrict__ r, double *part, GravCtrl *gc)
 {
     const double rhobar = Q.project_mean ? gc->rhobar : 0.0;
     double rr = 0.0, bb = 0.0;
-    cube_cells(
-        P.n, [&](int i) { return phi[i]; },
-        [&](int i, double c, double sx, double sy, double sz) {
-            const double b = -VB_FOURPI * Q.G * (rho[i] - rhobar) * vol;
-            const double ri = b - cube_lap(P, c, sx, sy, sz);
-            r[i] = ri;
-            rr = rr + ri * ri;
-            bb = bb + b * b;
+    cube_cells<T>(
+        P.n, [&](auto at) { return at(phi); },
+        [&](auto at, T c, T sx, T sy, T sz) {
+            const T b = scaled(-VB_FOURPI * Q.G, at(rho) - rhobar, vol);
+            const T ri = b - cube_lap(P, c, sx, sy, sz);
+            at.put(r, ri);
+            rr = rr + total(ri * ri);
+            bb = bb + total(b * b);
         });
     // two sums: the first one's total waits in gc for the second's last block
     double t;
@@ -564,6 +635,7 @@ __global__ void __launch_bounds__(GB) k_cube_accel(const __grid_constant__ Geom 
 
 // p = z + beta p (beta 0: z) into the other of the two direction buffers,
 // Ap = A p, alpha = rsold / p.Ap; stop when p.Ap <= 0
+template <class T>
 __global__ void __launch_bounds__(GB) k_cube_dir(CubeP P, const double *__restrict__ z, double *pa,
                                                 double *pb, double *__restrict__ Ap, double *part,
                                                 GravCtrl *gc)
@@ -574,13 +646,13 @@ __global__ void __launch_bounds__(GB) k_cube_dir(CubeP P, const double *__restri
     double *__restrict__ pn = odd ? pa : pb;
     const double beta = gc->beta;
     double s = 0.0;
-    cube_cells(
-        P.n, [&](int i) { return beta != 0.0 ? z[i] + beta * po[i] : z[i]; },
-        [&](int i, double c, double sx, double sy, double sz) {
-            const double a = cube_lap(P, c, sx, sy, sz);
-            pn[i] = c;
-            Ap[i] = a;
-            s = s + c * a;
+    cube_cells<T>(
+        P.n, [&](auto at) { return beta != 0.0 ? at(z) + beta * at(po) : at(z); },
+        [&](auto at, T c, T sx, T sy, T sz) {
+            const T a = cube_lap(P, c, sx, sy, sz);
+            at.put(pn, c);
+            at.put(Ap, a);
+            s = s + total(c * a);
         });
     double pAp;
     if (grid_sum(s, part, &gc->ticket, pAp)) {
@@ -628,29 +700,32 @@ __global__ void __launch_bounds__(GB) k_cube_update(int n, double *__restrict__ 
 }
 
 // two damped-Jacobi sweeps on A from zero: z1 = w r, z = z1 + w (r - A z1)
+template <class T>
 __global__ void __launch_bounds__(GB) k_cube_pre(CubeP P, const double *__restrict__ r,
                                                 double *__restrict__ z, const GravCtrl *gc)
 {
     if (gc->done) return;
-    cube_cells(
-        P.n, [&](int i) { return r[i]; },
-        [&](int i, double c, double sx, double sy, double sz) {
-            z[i] = P.w * c + P.w * (c - P.w * cube_lap(P, c, sx, sy, sz));
+    cube_cells<T>(
+        P.n, [&](auto at) { return at(r); },
+        [&](auto at, T c, T sx, T sy, T sz) {
+            at.put(z, P.w * c + P.w * (c - P.w * cube_lap(P, c, sx, sy, sz)));
         });
 }
 
 // the base grid's right-hand side: b = r - A z
+template <class T>
 __global__ void __launch_bounds__(GB) k_cube_resid(CubeP P, const double *__restrict__ z,
                                                   const double *__restrict__ r,
                                                   double *__restrict__ b, const GravCtrl *gc)
 {
     if (gc->done) return;
-    cube_cells(
-        P.n, [&](int i) { return z[i]; },
-        [&](int i, double c, double sx, double sy, double sz) { b[i] = r[i] - cube_lap(P, c, sx, sy, sz); });
+    cube_cells<T>(
+        P.n, [&](auto at) { return at(z); },
+        [&](auto at, T c, T sx, T sy, T sz) { at.put(b, at(r) - cube_lap(P, c, sx, sy, sz)); });
 }
 
 // first post-smoothing sweep on A of z + (e - mean e) / V
+template <class T>
 __global__ void __launch_bounds__(GB) k_cube_post1(CubeP P, const double *__restrict__ z,
                                                   const double *__restrict__ e,
                                                   const double *__restrict__ r, double iV,
@@ -658,15 +733,16 @@ __global__ void __launch_bounds__(GB) k_cube_post1(CubeP P, const double *__rest
 {
     if (gc->done) return;
     const double mu = gc->mgmu;
-    cube_cells(
-        P.n, [&](int i) { return z[i] + (e[i] - mu) * iV; },
-        [&](int i, double c, double sx, double sy, double sz) {
-            z2[i] = c + P.w * (r[i] - cube_lap(P, c, sx, sy, sz));
+    cube_cells<T>(
+        P.n, [&](auto at) { return at(z) + iV * (at(e) - mu); },
+        [&](auto at, T c, T sx, T sy, T sz) {
+            at.put(z2, c + P.w * (at(r) - cube_lap(P, c, sx, sy, sz)));
         });
 }
 
 // second one, and r.z: at the solve's start (start) rsold = r.z and beta = 0,
 // then beta = r.z / rsold and the iteration limit; `more`: the loop's condition
+template <class T>
 __global__ void __launch_bounds__(GB) k_cube_post2(CubeP P, const double *__restrict__ z2,
                                                   const double *__restrict__ r,
                                                   double *__restrict__ z, double *part, GravCtrl *gc,
@@ -678,12 +754,12 @@ __global__ void __launch_bounds__(GB) k_cube_post2(CubeP P, const double *__rest
         return;
     }
     double s = 0.0;
-    cube_cells(
-        P.n, [&](int i) { return z2[i]; },
-        [&](int i, double c, double sx, double sy, double sz) {
-            const double ri = r[i], v = c + P.w * (ri - cube_lap(P, c, sx, sy, sz));
-            z[i] = v;
-            s = s + ri * v;
+    cube_cells<T>(
+        P.n, [&](auto at) { return at(z2); },
+        [&](auto at, T c, T sx, T sy, T sz) {
+            const T ri = at(r), v = c + P.w * (ri - cube_lap(P, c, sx, sy, sz));
+            at.put(z, v);
+            s = s + total(ri * v);
         });
     double rz;
     if (grid_sum(s, part, &gc->ticket, rz)) {
@@ -698,41 +774,55 @@ __global__ void __launch_bounds__(GB) k_cube_post2(CubeP P, const double *__rest
 
 __device__ __forceinline__ int mg_wrap(int a, int n) { return a < 0 ? n - 1 : (a >= n ? 0 : a); }
 
+// a / 6: the reciprocal's product corrected by its residual rounds as the
+// division does unless a step of it leaves the normal numbers
+__device__ __forceinline__ double sixth(double a)
+{
+    const unsigned h = (unsigned)__double2hiint(a) & 0x7fffffffu;
+    return h - 0x06000000u < 0x79000000u ? quot64(a, 6.0, 1.0 / 6.0) : a / 6.0;
+}
+
 // _mgk_jacobi! (mg_pcg.jl:21-31): phi = (1 - w) phiold + w (sum_nb + h^2 b) / 6
 __device__ __forceinline__ double mg_jacobi(double c, double nb, double h2b)
 {
-    return (1.0 - MG_OMEGA) * c + MG_OMEGA * (nb + h2b) / 6.0;
+    return (1.0 - MG_OMEGA) * c + sixth(MG_OMEGA * (nb + h2b));
+}
+__device__ __forceinline__ D2 mg_jacobi(D2 c, D2 nb, D2 h2b)
+{
+    return {mg_jacobi(c.x, nb.x, h2b.x), mg_jacobi(c.y, nb.y, h2b.y)};
 }
 
 // a level's two sweeps from zero: e1 = w h^2 b / 6, then one sweep of it
-__global__ void __launch_bounds__(GB) k_mg_first(int n, double h2, const double *__restrict__ b,
+template <class T>
+__global__ void __launch_bounds__(GB, 5) k_mg_first(int n, double h2, const double *__restrict__ b,
                                                 double *__restrict__ e, const GravCtrl *gc)
 {
     if (gc->done) return;
     const double k = MG_OMEGA * h2 / 6.0;
-    cube_cells(
-        n, [&](int i) { return b[i]; },
-        [&](int i, double c, double sx, double sy, double sz) {
-            e[i] = mg_jacobi(k * c, k * (sx + sy + sz), h2 * c);
+    cube_cells<T>(
+        n, [&](auto at) { return at(b); },
+        [&](auto at, T c, T sx, T sy, T sz) {
+            at.put(e, mg_jacobi(k * c, k * (sx + sy + sz), h2 * c));
         });
 }
 
 // one sweep; mean: also the mean of the result (the base grid's last sweep)
-__global__ void __launch_bounds__(GB) k_mg_sweep(int n, double h2, const double *__restrict__ old,
+template <class T>
+__global__ void __launch_bounds__(GB, 5) k_mg_sweep(int n, double h2, const double *__restrict__ old,
                                                 const double *__restrict__ b, double *__restrict__ e,
                                                 int mean, double *part, GravCtrl *gc)
 {
     if (gc->done) return;
     double s = 0.0;
-    cube_cells(
-        n, [&](int i) { return old[i]; },
-        [&](int i, double c, double sx, double sy, double sz) {
-            const double v = mg_jacobi(c, sx + sy + sz, h2 * b[i]);
-            e[i] = v;
-            s = s + v;
+    cube_cells<T>(
+        n, [&](auto at) { return at(old); },
+        [&](auto at, T c, T sx, T sy, T sz) {
+            const T v = mg_jacobi(c, sx + sy + sz, h2 * at(b));
+            at.put(e, v);
+            if (mean) s = s + total(v);
         });
-    double total;
-    if (mean && grid_sum(s, part, &gc->ticket, total)) gc->mgmu = total / ((double)n * n * n);
+    double all;
+    if (mean && grid_sum(s, part, &gc->ticket, all)) gc->mgmu = all / ((double)n * n * n);
 }
 
 // _mgk_residual! (33-43) and _mgk_restrict! (45-53): the coarse right-hand side
@@ -785,15 +875,39 @@ __device__ __forceinline__ double mg_prolong(int nc, const double *ec, int x, in
     return 0.75 * face(k0) + 0.25 * face(k1);
 }
 
+// The same for a whole level, added to e: a thread takes the 8 children of a
+// coarse cell from the 27 coarse values around it, interpolated along x, then
+// y, then z as above.
 __global__ void __launch_bounds__(GB) k_mg_up(int nc, const double *__restrict__ ec,
                                              double *__restrict__ e, const GravCtrl *gc)
 {
     if (gc->done) return;
-    const int n = 2 * nc, i = blockIdx.x * GB + threadIdx.x;
-    if (i >= n * n * n) return;
-    int c[3];
-    cube_coords(n, i, c);
-    e[i] = e[i] + mg_prolong(nc, ec, c[0], c[1], c[2]);
+    const int I = blockIdx.x * GB + threadIdx.x;
+    if (I >= nc * nc * nc) return;
+    int C[3];
+    cube_coords(nc, I, C);
+    const int n = 2 * nc;
+    const int x[3] = {mg_wrap(C[0] - 1, nc), C[0], mg_wrap(C[0] + 1, nc)};
+    D2 f[3][2];  // the children's x pair: by coarse z and child y
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        D2 l[3];
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double *p = ec + (mg_wrap(C[2] + k - 1, nc) * nc + mg_wrap(C[1] + j - 1, nc)) * nc;
+            const double m = 0.75 * p[x[1]];
+            l[j] = {m + 0.25 * p[x[0]], m + 0.25 * p[x[2]]};
+        }
+        f[k][0] = 0.75 * l[1] + 0.25 * l[0];
+        f[k][1] = 0.75 * l[1] + 0.25 * l[2];
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const At<D2> at{((2 * C[2] + k) * n + 2 * C[1] + j) * n + 2 * C[0]};
+            at.put(e, at(e) + (0.75 * f[1][j] + 0.25 * f[2 * k][j]));
+        }
 }
 
 // The V-cycle from a level of n <= MG_BLOCK down, in one block: b in, e out.
@@ -963,6 +1077,17 @@ dim3 cube_grid(int n)
     const int kz = vb::cube_kz(n);
     return dim3((unsigned)((n + 31) / 32), (unsigned)((n + 7) / 8), (unsigned)((n + kz - 1) / kz));
 }
+// launch kern on the cells of an n^3 cube, in pairs where n is even
+#define CUBE_LAUNCH(kern, n, ...)                                                        \
+    do {                                                                                 \
+        dim3 cg_ = cube_grid(n);                                                         \
+        if ((n) % 2 == 0) {                                                              \
+            cg_.y = ((unsigned)(n) + 15) / 16;                                           \
+            vb::kern<vb::D2><<<cg_, vb::GB, 0, s>>>(__VA_ARGS__);                        \
+        } else {                                                                         \
+            vb::kern<double><<<cg_, vb::GB, 0, s>>>(__VA_ARGS__);                        \
+        }                                                                                \
+    } while (0)
 constexpr unsigned CUBE_UPDATE_BLOCKS = 1184;  // k_cube_update: 8 per SM
 
 vb::CubeP cube_params(const vb_gravity *gv)
@@ -982,23 +1107,21 @@ int queue_precond(vb_grid *gr, vb_gravity *gv, bool start, cudaGraphConditionalH
 {
     cudaStream_t s = gr->ctx->stream;
     const vb::CubeP P = cube_params(gv);
-    const dim3 grid = cube_grid(P.n);
-    vb::k_cube_pre<<<grid, vb::GB, 0, s>>>(P, gv->r, gv->z, gv->gc);
+    CUBE_LAUNCH(k_cube_pre, P.n, P, gv->r, gv->z, gv->gc);
     auto &top = gv->lev[0];
-    vb::k_cube_resid<<<grid, vb::GB, 0, s>>>(P, gv->z, gv->r, top.b, gv->gc);
+    CUBE_LAUNCH(k_cube_resid, P.n, P, gv->z, gv->r, top.b, gv->gc);
     VB_CHECK_LAUNCH(gr->ctx, 2);
     const int L = (int)gv->lev.size();
     // the first level that k_mg_bottom takes, or the coarsest one
     int bot = 0;
     while (bot < L - 1 && gv->lev[bot].n > vb::MG_BLOCK) ++bot;
     auto sweep = [&](const vb_gravity::Level &l, const double *old, double *out, bool mean) {
-        vb::k_mg_sweep<<<cube_grid(l.n), vb::GB, 0, s>>>(l.n, l.h * l.h, old, l.b, out, mean ? 1 : 0,
-                                                         gv->cpart, gv->gc);
+        CUBE_LAUNCH(k_mg_sweep, l.n, l.n, l.h * l.h, old, l.b, out, mean ? 1 : 0, gv->cpart, gv->gc);
         return 1;
     };
     for (int k = 0; k < bot; ++k) {
         const auto &l = gv->lev[k], &c = gv->lev[k + 1];
-        vb::k_mg_first<<<cube_grid(l.n), vb::GB, 0, s>>>(l.n, l.h * l.h, l.b, l.e, gv->gc);
+        CUBE_LAUNCH(k_mg_first, l.n, l.n, l.h * l.h, l.b, l.e, gv->gc);
         vb::k_mg_down<<<mg_blocks((int64_t)c.n * c.n * c.n), vb::GB, 0, s>>>(
             c.n, 1.0 / (l.h * l.h), l.e, l.b, c.b, gv->gc);
         VB_CHECK_LAUNCH(gr->ctx, 2);
@@ -1009,7 +1132,7 @@ int queue_precond(vb_grid *gr, vb_gravity *gv, bool start, cudaGraphConditionalH
             vb::k_mg_bottom<<<1, 1024, vb::mg_bottom_smem(l.n), s>>>(l.n, l.h, l.b, l.e, gv->gc);
             VB_CHECK_LAUNCH(gr->ctx, 1);
         } else {  // a coarsest level too large for one block (odd side)
-            vb::k_mg_first<<<cube_grid(l.n), vb::GB, 0, s>>>(l.n, l.h * l.h, l.b, l.e, gv->gc);
+            CUBE_LAUNCH(k_mg_first, l.n, l.n, l.h * l.h, l.b, l.e, gv->gc);
             VB_CHECK_LAUNCH(gr->ctx, 1);
             for (int q = 0; q < 30; q += 2)
                 VB_CHECK_LAUNCH(gr->ctx, sweep(l, l.e, l.t, false) + sweep(l, l.t, l.e, false));
@@ -1017,7 +1140,7 @@ int queue_precond(vb_grid *gr, vb_gravity *gv, bool start, cudaGraphConditionalH
     }
     for (int k = bot - 1; k >= 0; --k) {
         const auto &l = gv->lev[k], &c = gv->lev[k + 1];
-        vb::k_mg_up<<<mg_blocks((int64_t)l.n * l.n * l.n), vb::GB, 0, s>>>(c.n, c.e, l.e, gv->gc);
+        vb::k_mg_up<<<mg_blocks((int64_t)c.n * c.n * c.n), vb::GB, 0, s>>>(c.n, c.e, l.e, gv->gc);
         VB_CHECK_LAUNCH(gr->ctx, 1);
         VB_CHECK_LAUNCH(gr->ctx, sweep(l, l.e, l.t, false) + sweep(l, l.t, l.e, k == 0));
     }
@@ -1026,8 +1149,8 @@ int queue_precond(vb_grid *gr, vb_gravity *gv, bool start, cudaGraphConditionalH
         vb::k_sum_final<<<1, 1024, 0, s>>>(gv->part + 2 * vb::GP, (int64_t)P.n * P.n * P.n, gv->gc);
         VB_CHECK_LAUNCH(gr->ctx, 2);
     }
-    vb::k_cube_post1<<<grid, vb::GB, 0, s>>>(P, gv->z, top.e, gv->r, 1.0 / gv->vbase, gv->z2, gv->gc);
-    vb::k_cube_post2<<<grid, vb::GB, 0, s>>>(P, gv->z2, gv->r, gv->z, gv->cpart, gv->gc, start ? 1 : 0, more);
+    CUBE_LAUNCH(k_cube_post1, P.n, P, gv->z, top.e, gv->r, 1.0 / gv->vbase, gv->z2, gv->gc);
+    CUBE_LAUNCH(k_cube_post2, P.n, P, gv->z2, gv->r, gv->z, gv->cpart, gv->gc, start ? 1 : 0, more);
     VB_CHECK_LAUNCH(gr->ctx, 2);
     return VB_OK;
 }
@@ -1038,8 +1161,7 @@ int queue_cube_iteration(vb_grid *gr, vb_gravity *gv, cudaGraphConditionalHandle
     cudaStream_t s = gr->ctx->stream;
     const bool mg = gv->precond == VB_GRAV_PRECOND_MG;
     const vb::CubeP P = cube_params(gv);
-    vb::k_cube_dir<<<cube_grid(P.n), vb::GB, 0, s>>>(P, mg ? gv->z : gv->r, gv->p, gv->p2, gv->Ap,
-                                                     gv->cpart, gv->gc);
+    CUBE_LAUNCH(k_cube_dir, P.n, P, mg ? gv->z : gv->r, gv->p, gv->p2, gv->Ap, gv->cpart, gv->gc);
     vb::k_cube_update<<<CUBE_UPDATE_BLOCKS, vb::GB, 0, s>>>(P.n, gv->phi, gv->p, gv->p2, gv->r, gv->Ap,
                                                            gv->cpart, gv->gc, mg ? 0 : 1, more);
     VB_CHECK_LAUNCH(gr->ctx, 2);
@@ -1179,7 +1301,7 @@ int vb::detail::gravity_solve(vb_grid *gr, int64_t *iters, double *relres)
     }
     if (gv->cube_n) {
         const CubeP P = cube_params(gv);
-        k_cube_init<<<cube_grid(P.n), GB, 0, s>>>(P, gv->P, g.vol, gr->U, gv->phi, gv->r, gv->cpart, gv->gc);
+        CUBE_LAUNCH(k_cube_init, P.n, P, gv->P, g.vol, gr->U, gv->phi, gv->r, gv->cpart, gv->gc);
         k_cube_init_final<<<1, 1, 0, s>>>(gv->gc);
         VB_CHECK_LAUNCH(gr->ctx, 2);
     } else {
