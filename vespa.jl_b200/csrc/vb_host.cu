@@ -5,8 +5,9 @@
 // threads ("lanes"), each with its own stream, move pieces of about a megabyte
 // through pinned buffers of their own, so that the host copies of different
 // pieces run on different cores and overlap the transfers (and, for face
-// batches, the kernels).  10.5 MB in: 1.0 -> 0.4 ms; 200 k faces (17 MB in, 8 MB
-// out): 1.59 -> 0.86 ms.  Smaller copies, where the threads would cost more than
+// batches, the kernels).  200 k faces (17 MB in, 8 MB out): 1.59 -> 1.17 ms with
+// arrays new to every call, 0.9 ms with the same ones again; the PCIe link alone
+// takes 0.35 ms.  Smaller copies, where the threads would cost more than
 // they give, and copies of pinned arrays stay plain.
 //
 // The lanes belong to their context, which one host thread uses at a time, are

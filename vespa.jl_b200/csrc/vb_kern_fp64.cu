@@ -187,7 +187,7 @@ int launch_stage_fp64(const Geom &g, int stage, const double *Uin, const double 
 int launch_stage_tiled2d_fp64(const BoxDesc *hbox, int nitems, unsigned int *work, int stage,
                               cudaStream_t s, bool bf)
 {
-    return launch_tiled2d<false, 2>(hbox, nitems, work, stage, s, bf);
+    return launch_tiled2d<2>(hbox, nitems, work, stage, s, bf);
 }
 
 int launch_stage_tiled3d_fp64(const BoxDesc *hbox, const BoxDesc *boxes, const int *item_box,

@@ -1,10 +1,12 @@
 // vb_march.cu -- whole runs of small float64 1D and 2D grids in one launch.
 //
 // A step of such a grid is latency: as separate kernels (dt, stage 1, stage 2,
-// clock) it cost 12 us at 128 cells and 20 us at 64 x 64, nearly all of it
-// launches, loads from L2 and the serial chain of one flux.  Here one cluster
-// of up to 16 blocks keeps the state in shared memory and runs the steps in a
-// loop: 1.6 us and 3.4 us a step.  Each block owns a slab of rows (1D: of
+// clock) it cost 17 us at 128 cells and 26 us at 64 x 64 (a whole run over its
+// steps), nearly all of it launches, loads from L2 and the serial chain of one
+// flux.  Here one cluster of up to 16 blocks keeps the state in shared memory
+// and runs the steps in a loop: 3.6 us and 8.7 us a step.  Of 17 k cycles at
+// 64 x 64 the face solves take 7.5 k (the float64 pipes of 16 SMs), the cluster
+// barriers 3.6 k, both updates 3.6 k.  Each block owns a slab of rows (1D: of
 // cells), about 256 cells; two cluster barriers a step separate the stages,
 // the two rows of halo on each side are read from the neighbours' shared
 // memory, and the CFL maximum rides on the first barrier.  One thread solves

@@ -81,8 +81,8 @@ __device__ __forceinline__ T total_energy(const T W[5], T g)
 //     and the same kind of residual correction.
 // The corrected value is off the exact one by at most 2^-104 of it before its
 // rounding, so it could go wrong only where the exact one lies that close to a
-// midpoint between two numbers (one operand pair in 2^50); of 10^10 quotients
-// built to lie as close to one as any can, none did.
+// midpoint between two numbers (one operand pair in 2^50); of 7.5 10^9 operands,
+// a third of them built to lie as close to one as any can, none did.
 __device__ __forceinline__ double rcp64(double b)
 {
     double y;
@@ -231,23 +231,6 @@ __device__ __forceinline__ void hllc_frame(const double L[5], const double R[5],
     F[2] = F[2] + SK * (factor * u1 - m1);
     F[3] = F[3] + SK * (factor * u2 - m2);
     F[4] = F[4] + SK * (factor * Es - E);
-}
-
-// The same by components: DIM is the 1-based face-normal axis.
-template <int DIM>
-__device__ __forceinline__ void hllc_flux64(const double WL[5], const double WR[5], double g,
-                                            double ig1, double F[5])
-{
-    constexpr int t1 = DIM == 1 ? 2 : 1, t2 = DIM == 3 ? 2 : 3;
-    const double L[5] = {WL[0], WL[DIM], WL[t1], WL[t2], WL[4]};
-    const double R[5] = {WR[0], WR[DIM], WR[t1], WR[t2], WR[4]};
-    double f[5];
-    hllc_frame<DIM == 3>(L, R, g, ig1, f);
-    F[0] = f[0];
-    F[DIM] = f[1];
-    F[t1] = f[2];
-    F[t2] = f[3];
-    F[4] = f[4];
 }
 
 // hllc_flux, src/riemann.jl:33-66 with euler_flux (9-20) and _hllc_star

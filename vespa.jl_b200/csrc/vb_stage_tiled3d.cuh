@@ -1,14 +1,13 @@
 // vb_stage_tiled3d.cuh -- shared pieces of the tiled, z-marching fused RK2
 // stage kernels for 3D uniform meshes (the hot path of the 256^3 benchmark):
-// the tile geometry and the TMA stage-buffer layout (a block owns a 16 x 16
-// column tile and marches z, loading each plane's interior and its four 2-cell
-// halo strips NS planes ahead of use), halo indexing, the per-cell LO_* order
-// classes, the CFL terms, the box lookup and the persistent-grid sizing.  The
+// the tile geometry (a block owns a 16 x 16 column tile and marches z), the
+// mixed kernel's TMA stage-buffer layout (each plane's interior and its four
+// 2-cell halo strips, NS planes ahead of use), the per-cell LO_* order classes, the CFL terms, the box lookup and the persistent-grid sizing.  The
 // kernels are k_stage_tiled3d_f64 (VB_FP64, vb_stage_tiled3d_f64.cuh) and
 // k_stage_tiled3d_mixed (VB_MIXED, vb_stage_tiled3d_mixed.cuh).
 //
-// Requirements (checked on the host): nx % 16 == 0, ny % 16 == 0, nz >= 2, and
-// a periodic axis is periodic on both sides.  The BF instantiations record the
+// Requirements (checked on the host): nz >= 2, a periodic axis periodic on both
+// sides, and nx, ny multiples of 16 or as tiled3d_ragged takes them.  The BF instantiations record the
 // domain-boundary faces' fluxes in the boundary-flux register (bflux_add).
 #pragma once
 
@@ -45,15 +44,6 @@ __device__ __forceinline__ int halo_uoff(int h, int f)
     h -= 96;
     return U_YHI + f * (2 * TX) + (h >> 4) * TX + (h & 15);
 }
-// halo index of local cell (lx, ly) outside the interior (star stencil only)
-__device__ __forceinline__ int halo_idx(int lx, int ly)
-{
-    if (lx < 0) return ly * 2 + (lx + 2);
-    if (lx >= TX) return 32 + ly * 2 + (lx - TX);
-    if (ly < 0) return 64 + (ly + 2) * TX + lx;
-    return 96 + (ly - TY) * TX + lx;
-}
-
 }  // namespace t3
 
 // A stage load's bounded wait gave up (a block-uniform decision, taken after
@@ -130,7 +120,7 @@ __device__ __forceinline__ double cfl_term2d_exact(const double un[5], const Geo
     return nan_max(m, (fabs(W[2]) + cs) / g.w[1]);
 }
 
-// Persistent: a grid of (2 x SMs) blocks pulls work items from work[STAGE-1].
+// Persistent: a grid of the resident blocks pulls work items from work[STAGE-1].
 // An item is a column tile and a z chunk of one box (within a box, item =
 // chunk * ntiles + tile, so concurrently processed items are spatial
 // neighbours and share halo planes in L2).

@@ -7,9 +7,10 @@
 // 8..11 one thread per halo cell of the plane (4 strips of 32).
 //
 // Primitives live in a ring of three planes in shared memory; beyond a wall a
-// halo thread fetches the mirror cell.  Raw conserved values arrive in the slot itself (8-byte
-// cp.async, each element fetched by the thread that converts it in place, so
-// no alignment of the rows is needed and no thread waits for another's copy).
+// halo thread fetches the mirror cell.  Raw conserved values arrive in the slot
+// itself (8-byte cp.async, each element fetched by the thread that converts it
+// in place, so no alignment of the rows is needed and no thread waits for
+// another's copy).
 // One barrier per plane separates iterations; iteration k
 //   - solves the x and y faces of plane k+1 into one of two flux buffers: 17
 //     warp tasks (8 of x, 8 of y, one of both hi edges), one on each column
@@ -22,6 +23,13 @@
 // Every operation is the reference's, rounded separately (-fmad=false), in the
 // reference's per-cell accumulation order, so the result is bit-identical to
 // the cell-centric kernel and to the oracle.
+//
+// What bounds it: issue slots and dependency waits of 24 warps per SM (2050
+// instructions a cell and stage, 61 % of the issue slots, the float64 pipe 43 %
+// busy; its floor at 256^3 would be 1.5 ms a step).  256^3: 3.63 -> 3.05 ms a
+// step against 8 warps of 128 registers with two barriers a plane; 150 x 90 x
+// 75, which the cell-centric kernel ran: 0.68 -> 0.28 ms.  Divisions without
+// range branches (hllc_frame) spill at 80 registers: 3.1-3.35 ms.
 #pragma once
 
 #include "vb_stage_tiled3d_mixed.cuh"
