@@ -158,6 +158,7 @@ constexpr int NTH = 320;
 
 struct Smem {
     double w[2][5][NW];   // primitives: x strip [row][22], y strip [column][22]
+    double mu[2][5][NW];  // the adjoint state that the face fluxes meet, the same way
     double gl[2][5][NF], gr[2][5][NF];  // face adjoints WLb, WRb, line-major
     uint16_t code[2][NF]; // minmod codes of the cell behind each face
 };
@@ -186,6 +187,8 @@ k_adj_plane(const __grid_constant__ Geom g, const double *__restrict__ U, const 
         const int x = a == 0 ? x0 + pos - H : x0 + line, y = a == 0 ? y0 + line : y0 + pos - H;
         return (int64_t)wrap(x, nx) + (int64_t)nx * wrap(y, ny);
     };
+    const double *mu = M ? M : lam;  // mu = 0.5 lam (stage 2) or M (stage 1)
+    const double ms = M ? 1.0 : 0.5;
     // the tile's cells go into both strips, the halo cells into their own
     for (int i = t; i < T * T + 4 * H * T; i += NTH) {
         int a = 0, line, pos, pos2 = -1, line2 = 0;
@@ -203,6 +206,11 @@ k_adj_plane(const __grid_constant__ Geom g, const double *__restrict__ U, const 
             pos = k < H ? k : k + T;
         }
         const int64_t l = cell(a, line, pos);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            cp_async8(&S_.mu[a][k][line * S + pos], mu + k * nc + l);
+            if (pos2 >= 0) cp_async8(&S_.mu[1][k][line2 * S + pos2], mu + k * nc + l);
+        }
         double u[5], W[5];
 #pragma unroll
         for (int k = 0; k < 5; ++k) u[k] = __ldg(U + k * nc + l);
@@ -213,14 +221,13 @@ k_adj_plane(const __grid_constant__ Geom g, const double *__restrict__ U, const 
 #pragma unroll
             for (int k = 0; k < 5; ++k) S_.w[1][k][line2 * S + pos2] = W[k];
     }
+    cp_async_commit();
+    cp_async_wait_all();
     __syncthreads();
-    const double *mu = M ? M : lam;  // mu = 0.5 lam (stage 2) or M (stage 1)
-    const double ms = M ? 1.0 : 0.5;
     for (int i = t; i < 2 * NF; i += NTH) {
         const int a = i >= NF, j = i - a * NF, line = j / (T + 3), f = j - line * (T + 3);
         // face f lies between cells f + 1 and f + 2 of the strip
         const int c = line * S + f + 1;
-        const int64_t lo = cell(a, line, f + 1), hi = cell(a, line, f + 2);
         double L[5], R[5], Fb[5], Lb[5], Rb[5];
         unsigned cd = 0;
 #pragma unroll
@@ -233,7 +240,8 @@ k_adj_plane(const __grid_constant__ Geom g, const double *__restrict__ U, const 
             cd |= minmod_code(q0 - m1, b) << (2 * kf);
             L[k] = face_val(q0, 0.5, minmod<double>(q0 - m1, b));
             R[k] = face_val(q1, -0.5, minmod<double>(b, q2 - q1));
-            Fb[k] = g.area[a] * (ms * __ldg(mu + kf * nc + lo) - ms * __ldg(mu + kf * nc + hi));
+            const double *q = S_.mu[a][kf] + c;
+            Fb[k] = g.area[a] * (ms * q[0] - ms * q[1]);
         }
         hllc_vjp_frame(L, R, gamma, ig1, Fb, Lb, Rb);
 #pragma unroll
@@ -244,11 +252,20 @@ k_adj_plane(const __grid_constant__ Geom g, const double *__restrict__ U, const 
         }
         S_.code[a][j] = (uint16_t)cd;
     }
+    // the own cell's inputs of the last part arrive while others solve faces
+    static_assert(T * T <= NTH, "one cell a thread");
+    const int lx = t & (T - 1), ly = t / T, x = x0 + lx, y = y0 + ly;
+    const bool own = t < T * T && x < nx && y < ny;
+    const int64_t lin = (int64_t)x + (int64_t)nx * y;
+    double u[5], v[5];
+    if (own)
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            u[k] = __ldg(U + k * nc + lin);
+            v[k] = lam[k * nc + lin];
+        }
     __syncthreads();
-    for (int i = t; i < T * T; i += NTH) {
-        const int lx = i & (T - 1), ly = i / T, x = x0 + lx, y = y0 + ly;
-        if (x >= nx || y >= ny) continue;
-        const int64_t lin = (int64_t)x + (int64_t)nx * y;
+    if (own) {
         double Wb[5] = {0, 0, 0, 0, 0};
 #pragma unroll
         for (int a = 0; a < 2; ++a) {
@@ -270,16 +287,13 @@ k_adj_plane(const __grid_constant__ Geom g, const double *__restrict__ U, const 
                 Wb[k] += w;
             }
         }
-        double u[5], Ub[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k) u[k] = __ldg(U + k * nc + lin);
+        double Ub[5];
         cons2prim_vjp(u, gamma, Wb, Ub);
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
-            const int64_t o = k * nc + lin;
-            double v = 0.5 * lam[o];
-            if (M) v = v + M[o];
-            out[o] = v - invV * Ub[k];
+            double b = 0.5 * v[k];
+            if (M) b = b + S_.mu[0][k][ly * S + lx + H];
+            out[k * nc + lin] = b - invV * Ub[k];
         }
     }
 }
