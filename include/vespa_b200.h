@@ -136,12 +136,15 @@ int vb_grid_download(vb_grid *grid, double *U);
 /* Device pointer of the state (5*ncell float64), valid until vb_grid_destroy. */
 int vb_grid_device_state(vb_grid *grid, double **dU);
 /* Kernel selection and tuning knobs (no counterpart in the reference, whose
- * per-face loop has no launch shape).  VB_OPT_KERNEL: VB_KERNEL_AUTO picks the
- * tiled 3D kernel when the grid allows it (nx, ny multiples of 16, nz >= 2),
- * VB_KERNEL_CELL forces the cell-centric kernel, VB_KERNEL_TILED requires the
- * tiled one.  VB_OPT_TILE_KZ: z planes per tiled work item.
+ * per-face loop has no launch shape).  VB_OPT_KERNEL: VB_KERNEL_AUTO picks by
+ * size: small float64 1D and 2D grids march whole runs in one launch, 3D grids
+ * with nx, ny >= 16 (VB_MIXED: nx even) take a tiled kernel unless tiny, 2D
+ * grids the plane (float64) or row (VB_MIXED, nx >= 256 and even) kernel, the
+ * rest the cell-centric one.  VB_KERNEL_CELL forces the cell-centric kernel,
+ * VB_KERNEL_TILED requires a tiled one (3D: nx, ny multiples of 16, nz >= 2; 2D:
+ * nx a multiple of 256).  VB_OPT_TILE_KZ: z planes per tiled work item.
  * VB_OPT_TILE_TAPER: -1 (default) lets the autotuner choose whether the 3D
- * work queue's last z chunks taper (untuned: VB_MIXED grids taper), 0 keeps
+ * work queue's last z chunks taper (untuned: by the grid's size), 0 keeps
  * uniform chunks, 1 tapers in either precision.  Results do not depend on
  * any of these knobs. */
 enum { VB_OPT_KERNEL = 1, VB_OPT_TILE_KZ = 2, VB_OPT_TILE_TAPER = 3 };

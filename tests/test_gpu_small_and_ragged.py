@@ -90,7 +90,7 @@ def test_march_stops_resumes_and_reports(vb, oracle):
 
 
 # 2D grids of the plane kernel (beyond the march's size): ragged both ways
-@pytest.mark.parametrize("dims", [(129, 145), (256, 128), (1000, 17), (16, 900)])
+@pytest.mark.parametrize("dims", [(129, 145), (256, 128), (1000, 17), (16, 900), (400, 401), (512, 512)])
 @pytest.mark.parametrize("lo,hi", WALLS)
 def test_plane_grids_bit_identical(vb, oracle, dims, lo, hi):
     run_pair(oracle, dims, lo, hi, 3)

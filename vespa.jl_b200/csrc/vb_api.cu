@@ -214,9 +214,10 @@ int64_t tiles_per_chunk(const vb::Geom &g)
 // (256 cells a block, one block per SM) needs a second wave on 148 SMs: at 32^3
 // the two are level (mixed 25.5 and 24.5 us a step, float64 30 and 41), at 48^3
 // the tiles win (36 and 30, 75 and 54).  2D mixed: when a chunk of at least 8
-// rows gives every persistent block an item.  2D float64: the marching kernel
-// against the plane kernel runs 93 % at 1024^2, level at 2048^2 and 110 % at
-// 4096^2, so from the size on where 32-row chunks give each block four items.
+// rows gives every persistent block an item.  2D float64: the plane kernel steps
+// faster at every size (vb_stage_plane_f64.cuh) and `plane` has it take them; the
+// choice made here is for steps that record boundary fluxes, which it does not:
+// the marching kernel where 32-row chunks give each block four items.
 bool tiled_auto(const vb::Geom &g, int precision)
 {
     if (!vb::tiled_any(g, precision)) return false;
@@ -426,7 +427,8 @@ int stage(vb_grid *gr, int st, const double *Uin, const double *U0, double *Uout
     const bool grav = gr->grav != nullptr;  // self-gravity: 3D tiled kernels carry the source
     // the tiled kernels record outer boundary fluxes themselves; interior
     // faces, and boundary fluxes together with gravity, take the cell kernel
-    const bool use_tiled = gr->tiled && !bfi && !(bf && grav) && (!grav || gr->g.nd == 3);
+    const bool use_tiled = gr->tiled && !bfi && !(bf && grav) && (!grav || gr->g.nd == 3) &&
+                           !(gr->plane && !bf);
     if (gr->slab && !use_tiled)
         return fail(VB_ENOTSUP, "a z-window (slab) grid steps with the tiled 3D kernels only");
     if (use_tiled) {
@@ -539,7 +541,7 @@ bool marches(const vb_grid *gr)
 uint64_t graph_key(const vb_grid *gr)
 {
     return (gr->tiled ? 1u : 0u) | (gr->bflux_on ? 2u : 0u) | (grid_taper(gr) ? 4u : 0u) |
-           (gr->bflux_interior ? 8u : 0u) | (gr->cell_only ? 16u : 0u) | ((uint64_t)gr->kz << 5);
+           (gr->bflux_interior ? 8u : 0u) | (gr->cell_only ? 16u : 0u) | (gr->plane ? 32u : 0u) | ((uint64_t)gr->kz << 6);
 }
 
 // Capture GRAPH_STEPS steps into the grid's graph for its current configuration.
@@ -840,6 +842,7 @@ int vb_grid_create(vb_ctx *ctx, const vb_problem_desc *d, int precision, vb_grid
         return cleanup(rc, m);
     }
     gr->march = precision == VB_FP64 && vb::march_supported(g);
+    gr->plane = precision == VB_FP64 && vb::plane_f64_supported(g);
     if (vb::tiled_any(g, precision)) {
         if (vb::tiled_supported(g) || precision == VB_MIXED) {  // the TMA kernels' descriptors
             rc = encode_maps(&gr->maps_U, gr->U, g);
@@ -954,6 +957,7 @@ int vb_grid_set_option(vb_grid *gr, int option, int64_t value)
     switch (option) {
     case VB_OPT_KERNEL:
         gr->march = value == VB_KERNEL_AUTO && gr->precision == VB_FP64 && vb::march_supported(gr->g);
+        gr->plane = value == VB_KERNEL_AUTO && gr->precision == VB_FP64 && vb::plane_f64_supported(gr->g);
         gr->cell_only = value == VB_KERNEL_CELL;
         if (value == VB_KERNEL_CELL) {
             gr->tiled = false;

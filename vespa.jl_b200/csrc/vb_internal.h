@@ -57,6 +57,7 @@ struct vb_grid {
     bool warmed = false;                // one direct step ran (launch setup done)
     vb_gravity *grav = nullptr;         // self-gravity (a solve per step; source in the stages)
     bool cell_only = false;     // VB_KERNEL_CELL: the cell-centric kernel only
+    bool plane = false;         // 2D float64 under the automatic choice: the plane kernel, tiled or not
     bool march = false;         // small grid under the automatic choice: runs in one launch (vb_march.cu)
     bool slab = false;                  // a z window is set (vb_grid_set_zwindow): tiled kernels only
 };

@@ -106,6 +106,11 @@ inline bool tiled2d_supported(const Geom &g)
     return g.nd == 2 && g.n[0] % 256 == 0 && g.n[1] >= 2 && g.n[0] <= (1 << 30) &&
            g.n[1] <= (1 << 30);
 }
+// 2D float64 grids with room for one 16 x 16 tile of the plane kernel
+inline bool plane_f64_supported(const Geom &g)
+{
+    return g.nd == 2 && g.n[0] >= 16 && g.n[1] >= 16 && g.n[0] <= (1 << 24) && g.n[1] <= (1 << 24);
+}
 inline bool tiled_supported(const Geom &g) { return tiled3d_supported(g) || tiled2d_supported(g); }
 // what a single grid may take automatically
 inline bool tiled_any(const Geom &g, int precision)

@@ -1,14 +1,17 @@
 // vb_stage_plane_f64.cuh -- VB_FP64 stage kernel of 2D grids of any size from
-// 16 x 16: one block of 12 warps per 16 x 16 tile, no marching.
+// 16 x 16: one block of 9 warps per 16 x 16 tile, no marching.
 //
 // The counterpart of k_stage_tiled3d_f64 for a single plane (tile geometry,
 // shifted last tiles, mirrored or wrapped halo cells, face tasks in the
 // face-normal frame: see that file).  Warps 0..7 hold one cell per thread and
-// keep its state in registers for the update, warps 8..11 one halo cell; after
-// the conversion 17 warp tasks (8 of x faces, 8 of y, one of both hi edges) are
-// dealt to the 12 warps in turn.  Against the row-marching kernel a tile loads
-// 1.5 times its cells, but every tile runs at once: it is the better one while
-// the marching kernel's few long items leave the chip idle.
+// keep its state in registers for the update, the halo cells are converted by
+// warp 8 and, as second cells, warps 0..2; after the conversion 17 warp tasks (8
+// of x faces, 8 of y, one of both hi edges) are dealt to the 9 warps in two
+// rounds.  Against the row-marching kernel a tile loads 1.5 times its cells, but
+// every tile runs at once, 27 warps an SM instead of 16, and no thread waits for
+// a row: 136 against 170 ps a cell and step at 1024 x 2048, 134 against 158 at
+// 2048^2, 132 against 143 at 4096^2.  What bounds it: dependency waits and the
+// two barriers (issue slots 47 % used with 24 warps).
 //
 // Same operations, roundings and accumulation order as the cell-centric
 // kernel: bit-identical to it.
@@ -20,6 +23,8 @@ namespace vb {
 
 namespace t3d {
 
+constexpr int NTP = 288;
+
 struct PlaneSmem {
     double w[PSLOT];           // primitives (t3m layout)
     double g[5 * (FX + FY)];   // area * flux: [5][FX] of x, then [5][FY] of y
@@ -27,8 +32,8 @@ struct PlaneSmem {
 
 }  // namespace t3d
 
-template <int STAGE>
-__global__ void __launch_bounds__(t3d::NTH, 2)
+template <int STAGE, int OCC>
+__global__ void __launch_bounds__(t3d::NTP, OCC)
 k_stage_plane_f64(const __grid_constant__ Geom g, const double *__restrict__ Uin, const double *U0,
                   double *Uout, Ctrl *ctrl, int ntx)
 {
@@ -40,24 +45,22 @@ k_stage_plane_f64(const __grid_constant__ Geom g, const double *__restrict__ Uin
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const bool col = t < NC;
     const int tx = t & (TX - 1), ty = (t >> 4) & (TY - 1);
-    const int h = t - NC;
-    const int o_c = col      ? wrow(tx, ty)
-                    : h < 32 ? wxs(-2 + (h & 1), h >> 1)
-                    : h < 64 ? wxs(TX + (h & 1), (h - 32) >> 1)
-                    : h < 96 ? wrow((h - 64) & 15, -2 + ((h - 64) >> 4))
-                             : wrow((h - 96) & 15, TY + ((h - 96) >> 4));
-    const int dx = col ? tx : h < 32 ? -2 + (h & 1) : h < 64 ? TX + (h & 1) : (h & 15);
-    const int dy = col      ? ty
-                   : h < 64 ? (h & 31) >> 1
-                   : h < 96 ? -2 + ((h - 64) >> 4)
-                            : TY + ((h - 96) >> 4);
     const int nx = (int)g.n[0], ny = (int)g.n[1];
     const bool perx = g.bc_lo[0] == BC_PERIODIC, pery = g.bc_lo[1] == BC_PERIODIC;
     const double gamma = g.gamma;
     const int xn = (int)(blockIdx.x % ntx) * TX, yn = (int)(blockIdx.x / ntx) * TY;
     const int x0 = min(xn, nx - TX), y0 = min(yn, ny - TY);
-    int ex = x0 + dx, ey = y0 + dy, flip = 0;
-    if (!col) {
+    // halo cells: 0..31 on the ninth warp, the others as second cells of warps 0..2
+    const int h = col ? t + 32 : t - NC;
+    int64_t hlin = 0;
+    int o_h = 0, flip = 0;
+    if (h < NH) {
+        o_h = h < 32   ? wxs(-2 + (h & 1), h >> 1)
+              : h < 64 ? wxs(TX + (h & 1), (h - 32) >> 1)
+              : h < 96 ? wrow((h - 64) & 15, -2 + ((h - 64) >> 4))
+                       : wrow((h - 96) & 15, TY + ((h - 96) >> 4));
+        int hx = x0 + (h < 32 ? -2 + (h & 1) : h < 64 ? TX + (h & 1) : (h & 15));
+        int hy = y0 + (h < 64 ? (h & 31) >> 1 : h < 96 ? -2 + ((h - 64) >> 4) : TY + ((h - 96) >> 4));
         auto mirror = [&](int &c, int n, bool per, int bl, int bh, int nrm) {
             if (c < 0) {
                 if (!per && bl == BC_REFLECTING) flip = nrm;
@@ -67,31 +70,41 @@ k_stage_plane_f64(const __grid_constant__ Geom g, const double *__restrict__ Uin
                 c = per ? c - n : 2 * n - 1 - c;
             }
         };
-        mirror(ex, nx, perx, g.bc_lo[0], g.bc_hi[0], 1);
-        mirror(ey, ny, pery, g.bc_lo[1], g.bc_hi[1], 2);
+        mirror(hx, nx, perx, g.bc_lo[0], g.bc_hi[0], 1);
+        mirror(hy, ny, pery, g.bc_lo[1], g.bc_hi[1], 2);
+        hlin = hx + (int64_t)nx * hy;
     }
+    const int ex = x0 + tx, ey = y0 + ty;
     const int64_t lin = ex + (int64_t)nx * ey;
     const bool own = col && ex >= xn && ey >= yn && VB_DCHECK(lin >= 0 && lin < g.ncell);
     // the grid's CFL maximum so far: a lower bound of the final one
     float sofar = 0.0f;
     if constexpr (STAGE == 2)
         sofar = __double2float_rd(__longlong_as_double((long long)__ldcg(&ctrl->invdt_bits)));
-    double u[5], v[5];
+    double u[5], v[5], uh[5];
 #pragma unroll
-    for (int f = 0; f < 5; ++f) u[f] = __ldg(Uin + lin + f * g.ncell);
+    for (int f = 0; f < 5; ++f) u[f] = col ? __ldg(Uin + lin + f * g.ncell) : 0.0;
+    if (h < NH)
+#pragma unroll
+        for (int f = 0; f < 5; ++f) uh[f] = __ldg(Uin + hlin + f * g.ncell);
     if constexpr (STAGE == 2)
 #pragma unroll
         for (int f = 0; f < 5; ++f) v[f] = own ? U0[lin + f * g.ncell] : 0.0;
-    {
-        double W[5];
-        cons2prim(u, gamma, W);
+    double W[5];
+    if (h < NH) {
+        cons2prim(uh, gamma, W);
         if (flip == 1) W[1] = -W[1];
         if (flip == 2) W[2] = -W[2];
 #pragma unroll
-        for (int f = 0; f < 5; ++f) S.w[o_c + f * PC] = W[f];
+        for (int f = 0; f < 5; ++f) S.w[o_h + f * PC] = W[f];
+    }
+    if (col) {
+        cons2prim(u, gamma, W);
+#pragma unroll
+        for (int f = 0; f < 5; ++f) S.w[wrow(tx, ty) + f * PC] = W[f];
     }
     __syncthreads();
-    for (int j = warp; j < 17; j += NTH / 32) {
+    for (int j = warp; j < 17; j += NTP / 32) {
         int o0, o1, o2, o3, out;
         bool isy;
         const int lx = lane & 15, ly = lane >> 4;
@@ -175,12 +188,6 @@ k_stage_plane_f64(const __grid_constant__ Geom g, const double *__restrict__ Uin
     if constexpr (STAGE == 2) block_max_to(&ctrl->invdt_bits, m, red);
 }
 
-// 2D grids with room for one tile
-inline bool plane_f64_supported(const Geom &g)
-{
-    return g.nd == 2 && g.n[0] >= 16 && g.n[1] >= 16 && g.n[0] <= (1 << 24) && g.n[1] <= (1 << 24);
-}
-
 inline int launch_plane_f64(const Geom &g, int stage, const double *Uin, const double *U0,
                             double *Uout, Ctrl *ctrl, cudaStream_t s)
 {
@@ -190,8 +197,14 @@ inline int launch_plane_f64(const Geom &g, int stage, const double *Uin, const d
     if (nt > 0x7fffffffLL) return -1;
     const size_t smem = sizeof(t3d::PlaneSmem);
     static_assert(sizeof(t3d::PlaneSmem) <= 48 * 1024, "within the default shared memory");
-    if (stage == 1) k_stage_plane_f64<1><<<(unsigned)nt, t3d::NTH, smem, s>>>(g, Uin, U0, Uout, ctrl, ntx);
-    else k_stage_plane_f64<2><<<(unsigned)nt, t3d::NTH, smem, s>>>(g, Uin, U0, Uout, ctrl, ntx);
+    // two blocks an SM hold everything in registers, three (72 registers) spill a
+    // little: two where the tiles are done in two rounds of 2 x 148 blocks (384^2:
+    // 27.6 us a step against 30.1), three beyond (512^2: 43.4 against 46.4,
+    // 1000 x 999: 143 against 162)
+    const bool three = nt > 4 * 148;
+    auto k = stage == 1 ? three ? k_stage_plane_f64<1, 3> : k_stage_plane_f64<1, 2>
+                        : three ? k_stage_plane_f64<2, 3> : k_stage_plane_f64<2, 2>;
+    k<<<(unsigned)nt, t3d::NTP, smem, s>>>(g, Uin, U0, Uout, ctrl, ntx);
     return 1;
 }
 
