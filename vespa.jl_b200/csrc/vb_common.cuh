@@ -161,6 +161,15 @@ __device__ __forceinline__ unsigned long long order_bits(double x)
     return b;
 }
 
+// (the intrinsic is not declared for the default architecture, for which the
+// host-side checks compile this header)
+__device__ __forceinline__ unsigned warp_max_u32(unsigned v)
+{
+    unsigned r;
+    asm volatile("redux.sync.max.u32 %0, %1, 0xffffffff;" : "=r"(r) : "r"(v));
+    return r;
+}
+
 // Largest of a warp's non-negative doubles, by their bit patterns: the high
 // words, then the low words among those with the largest (two integer
 // reductions instead of five 64-bit shuffles and compares).  A NaN of either
@@ -168,8 +177,8 @@ __device__ __forceinline__ unsigned long long order_bits(double x)
 __device__ __forceinline__ double warp_max(double v)
 {
     const unsigned hi = __double2hiint(v) & 0x7fffffffu;
-    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)__double2loint(v) : 0u);
+    const unsigned mh = warp_max_u32(hi);
+    const unsigned ml = warp_max_u32(hi == mh ? (unsigned)__double2loint(v) : 0u);
     return __hiloint2double((int)mh, (int)ml);
 }
 

@@ -21,7 +21,7 @@
 // The last tile of a side that is no multiple of 16 is shifted back inside the
 // grid; the cells it shares with the tile before it are not written.
 //
-// What bounds it: issue slots of 16 warps per SM (820 and 920 instructions a
+// What bounds it: issue slots of 16 warps per SM (800 and 900 instructions a
 // cell in stages 1 and 2; two blocks of 110 and 128 registers), with dependency
 // waits 1.1-1.4 and the barrier 0.95 stalls an instruction.  256^3: 1.30 -> 1.22
 // ms a step.  A ninth warp for the halo (96 registers) took 1.33 ms.
