@@ -11,7 +11,8 @@
 // they give, and copies of pinned arrays stay plain.
 //
 // The lanes belong to their context, which one host thread uses at a time, are
-// made on its first large copy (16 MB pinned, 8 MB device) and freed with it.
+// made by its first large face batch or once its large copies add up to COPY_TOTAL
+// (16 MB pinned, 16 MB device) and freed with it.
 #include <cstring>
 #include <new>
 #include <thread>
@@ -27,6 +28,9 @@ constexpr int64_t FACES = 8192;             // faces of a piece: 84 B each in, 4
 constexpr size_t FACES_IN = (size_t)FACES * 84;
 constexpr size_t PIECE = (size_t)FACES * 124;
 constexpr size_t COPY_MIN = 4u << 20;
+// copies alone make the lanes once they have moved this much: making them (16 MB
+// to page-lock, 8 streams) takes 10 ms and more, which short runs never earn back
+constexpr size_t COPY_TOTAL = 256u << 20;
 
 struct Lane {
     char *pin = nullptr, *dev = nullptr;  // pinned: two pieces; device: a piece of faces
@@ -122,7 +126,12 @@ int vb::detail::host_copy(vb_ctx *ctx, void *dst, const void *src, size_t bytes,
     const bool pinned = cudaPointerGetAttributes(&at, to_device ? src : dst) != cudaSuccess ||
                         at.type != cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    if (bytes < COPY_MIN || pinned) {
+    bool plain = bytes < COPY_MIN || pinned;
+    if (!plain && !ctx->lanes) {
+        ctx->copied += bytes;
+        plain = ctx->copied < COPY_TOTAL;
+    }
+    if (plain) {
         VB_CUDA(cudaMemcpyAsync(dst, src, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost,
                                 ctx->stream));
         VB_CUDA(cudaStreamSynchronize(ctx->stream));
