@@ -10,8 +10,8 @@
 // rounds.  Against the row-marching kernel a tile loads 1.5 times its cells, but
 // every tile runs at once, 27 warps an SM instead of 16, and no thread waits for
 // a row: 136 against 170 ps a cell and step at 1024 x 2048, 134 against 158 at
-// 2048^2, 132 against 143 at 4096^2.  What bounds it: dependency waits and the
-// two barriers (issue slots 47 % used with 24 warps).
+// 2048^2, 132 against 143 at 4096^2.  What bounds it: dependency waits, the
+// tile's loads and the two barriers (issue slots 59 % used).
 //
 // Same operations, roundings and accumulation order as the cell-centric
 // kernel: bit-identical to it.
