@@ -1,0 +1,48 @@
+"""Calls at the edge of what they do: no step to take, refused options, states
+and coefficients at the end of a fast form's range.  Each against the oracle or
+against the same run without the edge call."""
+import math
+
+import numpy as np
+import pytest
+
+import vespa_b200 as vb
+from vespa_b200 import problem as P
+
+from test_gpu_parity import assert_bit_identical, make_sim, problem_from
+
+pytestmark = pytest.mark.gpu
+
+
+def box(dims, bc=(0, 2, 1), gamma=1.4):
+    nd = len(dims)
+    return problem_from(dims, [(0.0, 1.0), (0.0, 1.3), (0.0, 0.9)][:nd], bc[:nd], bc[:nd], gamma, 0.4)
+
+
+# cell-centric, plane, row-marching and cluster-marched grids
+@pytest.mark.parametrize("dims,kind", [((20, 12, 9), "auto"), ((48, 47, 40), "auto"), ((129, 145), "auto"),
+                                       ((256, 40), "tiled"), ((64, 32), "auto"), ((64, 32), "cell")])
+def test_evolve_without_steps_changes_nothing(vb, oracle, dims, kind):
+    prob = box(dims)
+    g = oracle.grid_from_problem(prob)
+    sim = make_sim(prob, np.ones((5, int(np.prod(dims)))))
+    sim.set_kernel(kind)
+    for seed, scale in ((1, 1.0), (2, 40.0)):  # the second state's dt differs from the first's
+        U0 = P.initial_state(P.smooth_random_problem(dims, seed=seed))
+        U0[4] *= scale
+        sim.upload(U0)
+        sim.set_time(0.0)
+        for tfinal in (math.inf, 0.05):
+            vb.evolve(sim, tfinal=tfinal, max_steps=0)
+            assert (sim.t, sim.step) == (0.0, 0)
+        assert_bit_identical(sim.state(), U0)
+        vb.evolve(sim, tfinal=0.05, max_steps=3)
+        U = U0.copy()
+        t, n = oracle.evolve(g, U, 0.05, max_steps=3, mode=1)
+        assert (sim.t, sim.step) == (t, n)
+        assert_bit_identical(sim.state(), U)
+        vb.evolve(sim, tfinal=0.05, max_steps=0)  # and after steps: the folded maximum stays good
+        vb.evolve(sim, tfinal=0.05, max_steps=2)
+        t2, n2 = oracle.evolve(g, U, 0.05, max_steps=2, t0=t, mode=1)
+        assert (sim.t, sim.step) == (t2, n + n2)
+        assert_bit_identical(sim.state(), U)

@@ -1248,35 +1248,39 @@ int vb_evolve(vb_grid *gr, double tfinal, int64_t max_steps, double *t, int64_t 
     rc = pull_ctrl(gr);
     if (rc) return rc;
     const long long step0 = gr->hctrl->step;
-    gr->hctrl->tfinal = tfinal;
-    gr->hctrl->step_limit = max_steps < 0 ? LLONG_MAX : step0 + max_steps;
     gr->hctrl->flags = 0;
-    gr->hctrl->active = 1;
-    rc = push_ctrl(gr);
-    if (rc) return rc;
-    if (!marches(gr)) rc = ensure_cfl(gr);  // a march folds it itself
-    if (rc) return rc;
-    // chunks of steps between host checks of the control block, none queued
-    // beyond the step budget
-    int64_t chunk = marches(gr) ? 4096 : 8;
     int status = VB_OK;
-    for (;;) {
-        const long long left = gr->hctrl->step_limit - gr->hctrl->step;
-        if (left <= 0) break;
-        rc = queue_steps(gr, chunk < left ? chunk : left);
+    // without a step to take nothing is queued: a CFL maximum folded here would
+    // be overwritten by the last push, which takes the mirror as pulled above
+    if (max_steps != 0) {
+        gr->hctrl->tfinal = tfinal;
+        gr->hctrl->step_limit = max_steps < 0 ? LLONG_MAX : step0 + max_steps;
+        gr->hctrl->active = 1;
+        rc = push_ctrl(gr);
         if (rc) return rc;
-        rc = pull_ctrl(gr);
+        if (!marches(gr)) rc = ensure_cfl(gr);  // a march folds it itself
         if (rc) return rc;
-        if (gr->hctrl->flags & vb::CTRL_F_NONFINITE) {
-            status = fail(VB_ENONFINITE, "non-finite dt: NaN or negative density/pressure");
-            break;
+        // chunks of steps between host checks of the control block, none queued
+        // beyond the step budget
+        int64_t chunk = marches(gr) ? 4096 : 8;
+        for (;;) {
+            const long long left = gr->hctrl->step_limit - gr->hctrl->step;
+            if (left <= 0) break;
+            rc = queue_steps(gr, chunk < left ? chunk : left);
+            if (rc) return rc;
+            rc = pull_ctrl(gr);
+            if (rc) return rc;
+            if (gr->hctrl->flags & vb::CTRL_F_NONFINITE) {
+                status = fail(VB_ENONFINITE, "non-finite dt: NaN or negative density/pressure");
+                break;
+            }
+            if (gr->hctrl->flags & vb::CTRL_F_TIMEOUT) {
+                status = fail(VB_ETIMEOUT, "a bounded device wait (TMA stage load) gave up");
+                break;
+            }
+            if (!gr->hctrl->active) break;
+            if (chunk < 64) chunk *= 2;
         }
-        if (gr->hctrl->flags & vb::CTRL_F_TIMEOUT) {
-            status = fail(VB_ETIMEOUT, "a bounded device wait (TMA stage load) gave up");
-            break;
-        }
-        if (!gr->hctrl->active) break;
-        if (chunk < 64) chunk *= 2;
     }
     if (t) *t = gr->hctrl->t;
     if (nsteps) *nsteps = gr->hctrl->step - step0;
