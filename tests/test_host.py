@@ -142,3 +142,21 @@ def test_bench_reference_arm_prints_the_contract_line():
     assert d["e2e"]["value"] == d["value"] and d["e2e"]["h2d_bytes_per_step"] == 0
     assert d["cpu_baseline"]["kind"] in ("port", "reference") and d["cpu_baseline"]["cores"] >= 1
     assert d["unit"] == "Mcell-updates/s" and d["steps"] == 1
+
+
+def test_kernels_that_overlap_their_inputs_writers_use_plain_pointers():
+    """A kernel that waits for the one before it (programmatic launch) is
+    resident while its inputs are written; __restrict__ on const data would let
+    the compiler read them as unchanging."""
+    csrc = os.path.join(ROOT, "vespa.jl_b200", "csrc")
+    seen = 0
+    for name in os.listdir(csrc):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        src = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, name)).read())
+        for kernel in src.split("__global__")[1:]:
+            body = kernel.partition("\n}")[0]
+            if "cudaGridDependencySynchronize" in body:
+                seen += 1
+                assert "__restrict__" not in body, (name, body[:200])
+    assert seen >= 2

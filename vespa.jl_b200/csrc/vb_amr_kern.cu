@@ -91,8 +91,11 @@ __global__ void __launch_bounds__(256) k_amr_faces(AmrDev m, const double *__res
 }
 
 // The same for the single-rate loop: the states in the face-normal frame, from
-// the primitives m.W.
-__global__ void __launch_bounds__(128) k_amr_faces_loop(AmrDev m, double *__restrict__ F, const Ctrl *ctrl)
+// the primitives m.W.  This kernel and k_amr_cells_loop are resident while the
+// one before them still writes W, F and the states, so they read those through
+// plain pointers: __restrict__ would declare them unchanged for the kernel's
+// whole life (read-only loads, movable above the dependency wait).
+__global__ void __launch_bounds__(128) k_amr_faces_loop(AmrDev m, double *F, const Ctrl *ctrl)
 {
     cudaTriggerProgrammaticLaunchCompletion();
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -116,7 +119,7 @@ __global__ void __launch_bounds__(128) k_amr_faces_loop(AmrDev m, double *__rest
     if (!in || !ctrl->active) return;
     const int64_t fo[5] = {0, (1 + ax) * m.cap, (ax == 0 ? 2 : 1) * m.cap, (ax == 2 ? 2 : 3) * m.cap,
                            4 * m.cap};
-    const double *__restrict__ W = m.W;
+    const double *W = m.W;
     const bool rlo = m.bc_lo[ax] == BC_REFLECTING, rhi = m.bc_hi[ax] == BC_REFLECTING;
     // face value of leaf i (representatives jl, jr) on its hi (h = 0.5) or lo side
     auto value = [&](int i, int jl, int jr, double h, double out[5]) {
@@ -150,8 +153,8 @@ __global__ void __launch_bounds__(128) k_amr_faces_loop(AmrDev m, double *__rest
 // One stage of the single-rate loop over every leaf.
 template <int STAGE>
 __global__ void __launch_bounds__(128)
-k_amr_cells_loop(AmrDev m, const double *__restrict__ Uin, const double *U0, double *Uout,
-                 const double *__restrict__ F, double cfl, Ctrl *ctrl)
+k_amr_cells_loop(AmrDev m, const double *Uin, const double *U0, double *Uout, const double *F,
+                 double cfl, Ctrl *ctrl)
 {
     __shared__ double red[32];
     cudaTriggerProgrammaticLaunchCompletion();
