@@ -251,3 +251,28 @@ def test_kh512_as_specified_plain_differences_every_cell(vb):
     prob = vb.kelvin_helmholtz_problem(n=512)
     errs = _fd_errors(vb, prob, 200, 20, 32, 1e-6)
     assert errs.max() <= 1e-6, errs
+
+
+def test_long_side_matches_its_period(vb):
+    """A side beyond the on-chip stage's 2^24 cells: a state that repeats every
+    64 cells has the adjoint of one period.  The wrapped cells add their faces
+    in another order (a few roundings of the largest term)."""
+    period, copies = 64, 2 ** 18 + 1
+    small, lam_s = None, np.random.default_rng(5).standard_normal((5, 2, period))
+    for reps in (1, copies):
+        n = period * reps
+        prob = vb.smooth_random_problem((period, 2), seed=9)
+        U0 = np.tile(vb.initial_state(prob).reshape(5, 2, period), (1, 1, reps)).reshape(5, -1)
+        prob.dims, prob.domain = (n, 2), ((0.0, float(n)), (0.0, 2.0))
+        sim = vb.Simulation(vb.B200Mesh(prob.dims, prob.domain), prob, initial=U0)
+        adj = vb.Adjoint(sim, 1, 1)
+        got = adj.step(0.2, np.ascontiguousarray(np.tile(lam_s, (1, 1, reps)).reshape(5, -1)))
+        adj.close()
+        sim.close()
+        got = got.reshape(5, 2, n)
+        if small is None:
+            small = got
+    assert n > 2 ** 24
+    scale = np.abs(small).max()
+    for k in (0, 1, reps // 2, reps - 1):
+        assert np.abs(got[:, :, k * period:(k + 1) * period] - small).max() <= 1e-13 * scale

@@ -1,0 +1,83 @@
+"""The library's host code on paths a GPU run cannot be brought to: allocations
+that fail, a second device, clusters that do not fit, options that are refused.
+Its objects are linked with fake_cudart.cpp, a runtime whose device memory is
+host memory and whose kernels do nothing, and driven through the C ABI."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import vespa_b200 as vb
+from vespa_b200 import _lib
+from vespa_b200 import problem as P
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "vespa.jl_b200", "csrc")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    subprocess.run(["make", "-C", CSRC, "all"], check=True, capture_output=True)
+    so = str(tmp_path_factory.mktemp("fake") / "libvespa_fake.so")
+    objs = [os.path.join(CSRC, "_build", f) for f in os.listdir(os.path.join(CSRC, "_build"))
+            if f.endswith(".o")]
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-o", so,
+                    "-I", os.path.join(CUDA, "include"), os.path.join(ROOT, "tests", "fake_cudart.cpp"),
+                    *objs, "-lpthread"], check=True, capture_output=True)
+    L = C.CDLL(so)
+    for name, args in _lib.SIGNATURES.items():
+        getattr(L, name).argtypes = args
+    for f in ("fake_device_live", "fake_pinned_live", "fake_plain_bytes", "fake_refused", "fake_launched"):
+        getattr(L, f).restype = C.c_longlong
+    L.fake_launched.argtypes = [C.c_char_p]
+    L.fake_refused.argtypes = [C.c_char_p, C.c_size_t]
+    L.fake_fail_device_alloc.argtypes = [C.c_longlong]
+    L.fake_host_alloc.restype = C.c_void_p
+    L.fake_host_alloc.argtypes = [C.c_size_t]
+    L.fake_host_free.argtypes = [C.c_void_p]
+    L.vb_last_error.argtypes = [C.c_char_p, C.c_size_t]
+    return L
+
+
+@pytest.fixture
+def ctx(fake):
+    fake.fake_reset()
+    c = C.c_void_p()
+    assert fake.vb_ctx_create(0, C.byref(c)) == 0
+    yield c
+    fake.fake_reset()
+    fake.vb_ctx_destroy(c)
+
+
+def error(L):
+    buf = C.create_string_buffer(512)
+    L.vb_last_error(buf, 512)
+    return buf.value.decode()
+
+
+def make_grid(L, ctx, dims, precision=_lib.FP64, bc=P.Periodic):
+    prob = P.smooth_random_problem(dims, seed=1)
+    prob.bcs = tuple((bc, bc) for _ in dims)
+    g = C.c_void_p()
+    rc = L.vb_grid_create(ctx, C.byref(vb.simulation.problem_desc(prob)), precision, C.byref(g))
+    assert rc == 0, error(L)
+    return g
+
+
+def test_adjoint_scratch_matches_the_kernels_that_use_it(fake, ctx):
+    """Only 2D grids whose stage keeps its face adjoints on chip go without the
+    three scratch arrays; a longer side takes the kernels that write them."""
+    live = []
+    for dims in ((64, 4), (1, 2 ** 24 + 1)):
+        g = make_grid(fake, ctx, dims)
+        before = fake.fake_device_live()
+        a = C.c_void_p()
+        assert fake.vb_adjoint_create(g, 4, 2, C.byref(a)) == 0, error(fake)
+        live.append(fake.fake_device_live() - before)
+        fake.vb_adjoint_destroy(a)
+        assert fake.fake_device_live() == before
+        fake.vb_grid_destroy(g)
+    assert live[1] == live[0] + 3

@@ -150,7 +150,7 @@ int vb_adjoint_create(vb_grid *gr, int64_t max_steps, int64_t checkpoint_every, 
     if (a->every == 1) get((void **)&a->tape1, a->state_bytes * (size_t)max_steps);
     get((void **)&a->lam, a->state_bytes);
     get((void **)&a->lam1, a->state_bytes);
-    if (nd != 2) {  // the 2D stage keeps its face adjoints on chip
+    if (!vb::adj_on_chip(gr->g)) {
         get((void **)&a->gL, a->state_bytes * nd);
         get((void **)&a->gR, a->state_bytes * nd);
         get((void **)&a->code, sizeof(uint16_t) * nc * nd);

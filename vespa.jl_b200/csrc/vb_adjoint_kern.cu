@@ -311,7 +311,7 @@ int launch_adj_stage(const Geom &g, const double *U, const double *lam, const do
                      double invV, double *gL, double *gR, uint16_t *code, double *out,
                      cudaStream_t s)
 {
-    if (g.nd == 2 && g.n[0] <= (1 << 24) && g.n[1] <= (1 << 24)) {
+    if (adj_on_chip(g)) {
         const int ntx = (int)((g.n[0] + adj2::T - 1) / adj2::T);
         const int64_t nt = ntx * ((g.n[1] + adj2::T - 1) / adj2::T);
         static const cudaError_t set = cudaFuncSetAttribute(

@@ -183,7 +183,13 @@ int launch_stage_mixed(const Geom &g, int stage, const double *Uin, const double
 
 // vb_adjoint_kern.cu (periodic meshes, float64): one adjoint RK2 stage,
 //   out = 0.5*lam + (M ? M : 0) - invV * (dD/dU)^T mu,  mu = M ? M : 0.5*lam,
-// at the state U; gL/gR (2*nd*5*ncell doubles) and code (nd*ncell) are scratch.
+// at the state U; gL/gR (2*nd*5*ncell doubles) and code (nd*ncell) are scratch,
+// which 2D grids whose face adjoints stay on chip do not need (adj_on_chip: the
+// one condition for both; such a side's tile coordinates fit its 32-bit ints).
+inline bool adj_on_chip(const Geom &g)
+{
+    return g.nd == 2 && g.n[0] <= (1 << 24) && g.n[1] <= (1 << 24);
+}
 int launch_adj_stage(const Geom &g, const double *U, const double *lam, const double *M,
                      double invV, double *gL, double *gR, uint16_t *code, double *out,
                      cudaStream_t s);
