@@ -81,3 +81,31 @@ def test_adjoint_scratch_matches_the_kernels_that_use_it(fake, ctx):
         assert fake.fake_device_live() == before
         fake.vb_grid_destroy(g)
     assert live[1] == live[0] + 3
+
+
+def faces(nf):
+    r = np.random.default_rng(nf)
+    return r.random((nf, 5)) + 0.5, r.random((nf, 5)) + 0.5, r.integers(1, 4, nf).astype(np.int32), np.zeros((nf, 5))
+
+
+def hllc(L, ctx, WL, WR, axis, F):
+    return L.vb_hllc_faces(ctx, len(axis), _lib.dptr(WL), _lib.dptr(WR), _lib.i32ptr(axis), 1.4, _lib.dptr(F))
+
+
+def test_copies_and_batches_go_plainly_when_no_lanes_can_be_made(fake, ctx):
+    g = make_grid(fake, ctx, (64, 64, 128))
+    U = np.random.default_rng(0).random((5, 64 * 64 * 128))
+    back = np.zeros_like(U)
+    WL, WR, axis, F = faces(40000)
+    pinned = fake.fake_pinned_live()
+    for i in range(32):  # 40 MB of copies and 5 MB of faces a round: beyond every threshold
+        fake.fake_fail_pinned(i < 16)  # first no page-locked memory, then none on the device
+        fake.fake_fail_device(i >= 16)
+        assert fake.vb_grid_upload(g, _lib.dptr(U)) == 0, error(fake)
+        assert fake.vb_grid_download(g, _lib.dptr(back)) == 0, error(fake)
+        assert np.array_equal(U, back)
+        assert hllc(fake, ctx, WL, WR, axis, F) == 0, error(fake)
+        assert fake.fake_pinned_live() == pinned  # nothing half made is kept
+        U += 1.0
+    fake.fake_fail_device(0)
+    fake.vb_grid_destroy(g)

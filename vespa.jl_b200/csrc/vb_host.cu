@@ -62,11 +62,14 @@ void vb::detail::host_lanes_free(vb_host_lanes *hl)
 
 namespace {
 
-int make_lanes(vb_ctx *ctx)
+// Whether the lanes are there, made now if need be.  When they cannot be (no
+// page-locked or device memory left) the caller's arrays go plainly, and copies
+// try again once they add up anew.
+bool make_lanes(vb_ctx *ctx)
 {
-    if (ctx->lanes) return VB_OK;
+    if (ctx->lanes) return true;
     vb_host_lanes *hl = new (std::nothrow) vb_host_lanes;
-    if (!hl) return fail(VB_ENOMEM, "host allocation failed");
+    if (!hl) return false;
     cudaError_t e = cudaEventCreateWithFlags(&hl->start, cudaEventDisableTiming);
     for (Lane &l : hl->lane) {
         if (e == cudaSuccess) e = cudaMallocHost(&l.pin, 2 * PIECE);
@@ -78,11 +81,11 @@ int make_lanes(vb_ctx *ctx)
     if (e != cudaSuccess) {
         vb::detail::host_lanes_free(hl);
         cudaGetLastError();
-        return fail(e == cudaErrorMemoryAllocation ? VB_ENOMEM : VB_ECUDA,
-                    std::string("host staging buffers: ") + cudaGetErrorString(e));
+        ctx->copied = 0;
+        return false;
     }
     ctx->lanes = hl;
-    return VB_OK;
+    return true;
 }
 
 // work(lane, index, count) on min(lanes, pieces) threads, this one among them,
@@ -129,7 +132,7 @@ int vb::detail::host_copy(vb_ctx *ctx, void *dst, const void *src, size_t bytes,
     bool plain = bytes < COPY_MIN || pinned;
     if (!plain && !ctx->lanes) {
         ctx->copied += bytes;
-        plain = ctx->copied < COPY_TOTAL;
+        plain = ctx->copied < COPY_TOTAL || !make_lanes(ctx);
     }
     if (plain) {
         VB_CUDA(cudaMemcpyAsync(dst, src, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost,
@@ -137,8 +140,6 @@ int vb::detail::host_copy(vb_ctx *ctx, void *dst, const void *src, size_t bytes,
         VB_CUDA(cudaStreamSynchronize(ctx->stream));
         return VB_OK;
     }
-    int rc = make_lanes(ctx);
-    if (rc) return rc;
     const int64_t pieces = (int64_t)((bytes + PIECE - 1) / PIECE);
     auto work = [&](Lane &l, int i, int n) {
         cudaError_t e = cudaSuccess;
@@ -171,11 +172,14 @@ int vb::detail::host_copy(vb_ctx *ctx, void *dst, const void *src, size_t bytes,
     return run_lanes(ctx, pieces, work, "host copy");
 }
 
+bool vb::detail::host_faces_staged(vb_ctx *ctx, int64_t nf)
+{
+    return nf >= HOST_FACES && make_lanes(ctx);
+}
+
 int vb::detail::host_faces(vb_ctx *ctx, int64_t nf, const double *WL, const double *WR,
                            const int32_t *axis, double gamma, double *F)
 {
-    int rc = make_lanes(ctx);
-    if (rc) return rc;
     const int64_t pieces = (nf + FACES - 1) / FACES;
     auto work = [&](Lane &l, int i, int n) {
         cudaError_t e = cudaSuccess;
@@ -213,7 +217,7 @@ int vb::detail::host_faces(vb_ctx *ctx, int64_t nf, const double *WL, const doub
         finish(h ^ 1);
         return e;
     };
-    rc = run_lanes(ctx, pieces, work, "face batch");
+    const int rc = run_lanes(ctx, pieces, work, "face batch");
     ctx->launches += pieces;
     return rc;
 }
