@@ -109,3 +109,28 @@ def test_copies_and_batches_go_plainly_when_no_lanes_can_be_made(fake, ctx):
         U += 1.0
     fake.fake_fail_device(0)
     fake.vb_grid_destroy(g)
+
+
+def test_pinned_and_overlapping_face_batches_stay_whole(fake, ctx):
+    """One launch for the batch; the lanes would take one per 8192 faces."""
+    nf = 40000
+
+    def launches(WL, WR, axis, F):
+        before = fake.fake_launched(b"k_hllc_faces")
+        assert hllc(fake, ctx, WL, WR, axis, F) == 0, error(fake)
+        return fake.fake_launched(b"k_hllc_faces") - before
+
+    WL, WR, axis, F = faces(nf)
+    for _ in range(64):  # by then pageable batches are staged
+        staged = launches(WL, WR, axis, F)
+    assert staged == -(-nf // 8192)
+    for which in range(3):
+        arrays = [WL, WR, F]
+        p = fake.fake_host_alloc(8 * 5 * nf)
+        arrays[which] = np.ctypeslib.as_array((C.c_double * (5 * nf)).from_address(p)).reshape(nf, 5)
+        assert launches(arrays[0], arrays[1], axis, arrays[2]) == 1
+        fake.fake_host_free(p)
+    both = np.random.default_rng(1).random((nf + 10, 5))
+    assert launches(both[10:], WR, axis, both[:nf]) == 1
+    assert launches(WL, both[:nf], axis, both[10:]) == 1
+    assert launches(WL, WR, axis, WL) == 1

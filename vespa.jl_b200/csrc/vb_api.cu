@@ -778,7 +778,7 @@ int vb_hllc_faces(vb_ctx *ctx, int64_t nf, const double *WL, const double *WR,
     unsigned bad = 0;  // no early exit: the loop vectorises
     for (int64_t f = 0; f < nf; ++f) bad |= (unsigned)(axis[f] - 1) > 2u;
     if (bad) return fail(VB_EINVAL, "axis entries must be 1, 2 or 3");
-    if (vb::detail::host_faces_staged(ctx, nf))
+    if (vb::detail::host_faces_staged(ctx, nf, WL, WR, F))
         return vb::detail::host_faces(ctx, nf, WL, WR, axis, gamma, F);
     const size_t bw = sizeof(double) * 5 * (size_t)nf;
     const size_t ba = sizeof(int32_t) * (size_t)nf;

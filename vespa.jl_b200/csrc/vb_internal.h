@@ -92,9 +92,9 @@ int ctx_scratch(vb_ctx *ctx, size_t bytes, void **out);
 // vb_host.cu.
 int host_copy(vb_ctx *ctx, void *dst, const void *src, size_t bytes, bool to_device);
 // vb_hllc_faces for at least HOST_FACES faces, staged piece by piece, where
-// host_faces_staged says so (the lanes are there).
+// host_faces_staged says so (pageable arrays apart from one another, the lanes there).
 constexpr int64_t HOST_FACES = 32768;
-bool host_faces_staged(vb_ctx *ctx, int64_t nf);
+bool host_faces_staged(vb_ctx *ctx, int64_t nf, const double *WL, const double *WR, const double *F);
 int host_faces(vb_ctx *ctx, int64_t nf, const double *WL, const double *WR, const int32_t *axis,
                double gamma, double *F);
 void host_lanes_free(vb_host_lanes *hl);
