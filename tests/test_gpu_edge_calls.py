@@ -46,3 +46,29 @@ def test_evolve_without_steps_changes_nothing(vb, oracle, dims, kind):
         t2, n2 = oracle.evolve(g, U, 0.05, max_steps=2, t0=t, mode=1)
         assert (sim.t, sim.step) == (t2, n + n2)
         assert_bit_identical(sim.state(), U)
+
+
+def test_staged_face_batches_bit_identical(vb, oracle):
+    """Batches and copies before and after the staging lanes come in (256 MiB of
+    them), a last piece of one face, fluxes over the left states, pinned arrays."""
+    from tests.golden.make_golden import random_faces
+    torch = pytest.importorskip("torch")
+    ctx = vb.Context(0)
+    backend = vb.B200Flux(ctx)
+    for nf in (32768, 8192 * 9 + 1):
+        WL, WR, axis = random_faces(nf, seed=nf)
+        ref = oracle.compute_face_fluxes(WL, WR, axis, 1.4)
+        for k in range(36 if nf > 32768 else 2):
+            F = np.zeros_like(WL)
+            vb.compute_face_fluxes(backend, 1.4, F, WL, WR, axis)
+            assert_bit_identical(F, ref)
+    pin = [torch.from_numpy(a.copy()).pin_memory().numpy() for a in (WL, WR, F)]
+    vb.compute_face_fluxes(backend, 1.4, pin[2], pin[0], pin[1], axis)
+    assert_bit_identical(pin[2], ref)
+    both = np.vstack([WL, np.zeros((7, 5))])
+    vb.compute_face_fluxes(backend, 1.4, both[7:], both[:-7], WR, axis)
+    assert_bit_identical(both[7:], ref)
+    prob = box((64, 64, 33))
+    U0 = P.initial_state(P.smooth_random_problem((64, 64, 33), seed=2))
+    sim = vb.Simulation(vb.B200Mesh(prob.dims, prob.domain), prob, initial=U0, ctx=ctx)
+    assert_bit_identical(sim.state(), U0)

@@ -134,3 +134,14 @@ def test_pinned_and_overlapping_face_batches_stay_whole(fake, ctx):
     assert launches(both[10:], WR, axis, both[:nf]) == 1
     assert launches(WL, both[:nf], axis, both[10:]) == 1
     assert launches(WL, WR, axis, WL) == 1
+
+
+def test_lanes_are_made_only_once_large_arrays_add_up(fake, ctx):
+    nf = 200000  # 24.8 MB a batch
+    WL, WR, axis, F = faces(nf)
+    pinned = fake.fake_pinned_live()
+    made = []
+    for _ in range(12):
+        assert hllc(fake, ctx, WL, WR, axis, F) == 0, error(fake)
+        made.append(fake.fake_pinned_live() - pinned)
+    assert made[:10] == [0] * 10 and made[11] == 8, made  # 256 MiB after ten batches

@@ -11,8 +11,8 @@
 // they give, and copies of pinned arrays stay plain.
 //
 // The lanes belong to their context, which one host thread uses at a time, are
-// made by its first large face batch or once its large copies add up to COPY_TOTAL
-// (16 MB pinned, 16 MB device) and freed with it.
+// made once its large copies and face batches add up to LANES_FROM (16 MB pinned,
+// 16 MB device) and freed with it.
 #include <cstdint>
 #include <cstring>
 #include <new>
@@ -27,11 +27,13 @@ namespace {
 constexpr int LANES = 8;
 constexpr int64_t FACES = 8192;             // faces of a piece: 84 B each in, 40 B out
 constexpr size_t FACES_IN = (size_t)FACES * 84;
-constexpr size_t PIECE = (size_t)FACES * 124;
+constexpr size_t FACE_BYTES = 124;
+constexpr size_t PIECE = (size_t)FACES * FACE_BYTES;
 constexpr size_t COPY_MIN = 4u << 20;
-// copies alone make the lanes once they have moved this much: making them (16 MB
-// to page-lock, 8 streams) takes 10 ms and more, which short runs never earn back
-constexpr size_t COPY_TOTAL = 256u << 20;
+// the lanes are made once this much has gone plainly: making them (16 MB to
+// page-lock, 8 streams) takes 12 ms, which short runs never earn back.  Face
+// batches gain about 1 ms per 25 MB, so they do after some 300 MB.
+constexpr size_t LANES_FROM = 256u << 20;
 
 struct Lane {
     char *pin = nullptr, *dev = nullptr;  // pinned: two pieces; device: a piece of faces
@@ -63,12 +65,15 @@ void vb::detail::host_lanes_free(vb_host_lanes *hl)
 
 namespace {
 
-// Whether the lanes are there, made now if need be.  When they cannot be (no
-// page-locked or device memory left) the caller's arrays go plainly, and copies
-// try again once they add up anew.
-bool make_lanes(vb_ctx *ctx)
+// Whether `bytes` more of large arrays find the lanes there, made now if they
+// add up to enough.  When they cannot be (no
+// page-locked or device memory left) the caller's arrays go plainly, and the
+// next try comes when they add up anew.
+bool make_lanes(vb_ctx *ctx, size_t bytes)
 {
     if (ctx->lanes) return true;
+    ctx->copied += bytes;
+    if (ctx->copied < LANES_FROM) return false;
     vb_host_lanes *hl = new (std::nothrow) vb_host_lanes;
     if (!hl) return false;
     cudaError_t e = cudaEventCreateWithFlags(&hl->start, cudaEventDisableTiming);
@@ -135,12 +140,7 @@ bool pageable(const void *p)
 
 int vb::detail::host_copy(vb_ctx *ctx, void *dst, const void *src, size_t bytes, bool to_device)
 {
-    bool plain = bytes < COPY_MIN || !pageable(to_device ? src : dst);
-    if (!plain && !ctx->lanes) {
-        ctx->copied += bytes;
-        plain = ctx->copied < COPY_TOTAL || !make_lanes(ctx);
-    }
-    if (plain) {
+    if (bytes < COPY_MIN || !pageable(to_device ? src : dst) || !make_lanes(ctx, bytes)) {
         VB_CUDA(cudaMemcpyAsync(dst, src, bytes, to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost,
                                 ctx->stream));
         VB_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -189,7 +189,7 @@ bool vb::detail::host_faces_staged(vb_ctx *ctx, int64_t nf, const double *WL, co
         return w + n <= f || f + n <= w;
     };
     return nf >= HOST_FACES && apart(WL) && apart(WR) && pageable(WL) && pageable(WR) && pageable(F) &&
-           make_lanes(ctx);
+           make_lanes(ctx, FACE_BYTES * (size_t)nf);
 }
 
 int vb::detail::host_faces(vb_ctx *ctx, int64_t nf, const double *WL, const double *WR,

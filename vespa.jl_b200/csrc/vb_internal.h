@@ -18,7 +18,7 @@ struct vb_ctx {
     void *scratch = nullptr;  // vb_hllc_faces staging (device)
     size_t scratch_bytes = 0;
     vb_host_lanes *lanes = nullptr;
-    size_t copied = 0;          // bytes of large pageable copies so far (vb_host.cu)
+    size_t copied = 0;          // bytes of large pageable arrays that went plainly (vb_host.cu)
     cudaEvent_t marks[16] = {};
 };
 
