@@ -145,3 +145,22 @@ def test_lanes_are_made_only_once_large_arrays_add_up(fake, ctx):
         assert hllc(fake, ctx, WL, WR, axis, F) == 0, error(fake)
         made.append(fake.fake_pinned_live() - pinned)
     assert made[:10] == [0] * 10 and made[11] == 8, made  # 256 MiB after ten batches
+
+
+@pytest.mark.parametrize("dims", [(64, 48), (20, 12, 9)])
+def test_a_refused_option_leaves_the_grid_as_it_was(fake, ctx, dims):
+    g = make_grid(fake, ctx, dims)
+
+    def kernels():
+        fake.fake_reset()
+        assert fake.vb_run_steps_async(g, 1) == 0, error(fake)
+        return [fake.fake_launched(k) for k in (b"k_march", b"k_stage_plane_f64", b"k_stage_generic")]
+
+    for chosen in ("auto", "cell"):
+        assert fake.vb_grid_set_option(g, _lib.OPT_KERNEL, _lib.KERNELS[chosen]) == 0
+        before = kernels()
+        assert sum(before)
+        for bad, code in ((_lib.KERNELS["tiled"], _lib.VB_ENOTSUP), (7, _lib.VB_EINVAL), (-1, _lib.VB_EINVAL)):
+            assert fake.vb_grid_set_option(g, _lib.OPT_KERNEL, bad) == code
+            assert kernels() == before, (chosen, bad)
+    fake.vb_grid_destroy(g)

@@ -955,27 +955,26 @@ int vb_grid_set_option(vb_grid *gr, int option, int64_t value)
 {
     if (!gr) return fail(VB_EINVAL, "null grid");
     switch (option) {
-    case VB_OPT_KERNEL:
-        gr->march = value == VB_KERNEL_AUTO && gr->precision == VB_FP64 && vb::march_supported(gr->g);
-        gr->plane = value == VB_KERNEL_AUTO && gr->precision == VB_FP64 && vb::plane_f64_supported(gr->g);
-        gr->cell_only = value == VB_KERNEL_CELL;
-        if (value == VB_KERNEL_CELL) {
-            gr->tiled = false;
-        } else if (value == VB_KERNEL_AUTO || value == VB_KERNEL_TILED) {
-            if (value == VB_KERNEL_TILED && !vb::tiled_supported(gr->g))
-                return fail(VB_ENOTSUP, "tiled kernels need a 3D grid with nx, ny multiples of "
-                                        "16 or a 2D grid with nx a multiple of 256");
-            if (vb::tiled_supported(gr->g) && !gr->maps_U.in_int.opaque[0] &&
-                !gr->maps_U.in_int.opaque[1]) {
-                int rc = encode_maps(&gr->maps_U, gr->U, gr->g);
-                if (!rc) rc = encode_maps(&gr->maps_U1, gr->U1, gr->g);
-                if (rc) return rc;
-            }
-            gr->tiled = value == VB_KERNEL_TILED || vb::detail::tiled_auto(gr->g, gr->precision);
-        } else {
+    case VB_OPT_KERNEL: {
+        if (value != VB_KERNEL_AUTO && value != VB_KERNEL_CELL && value != VB_KERNEL_TILED)
             return fail(VB_EINVAL, "unknown kernel selector");
+        const bool automatic = value == VB_KERNEL_AUTO, fp64 = gr->precision == VB_FP64;
+        if (value == VB_KERNEL_TILED && !vb::tiled_supported(gr->g))
+            return fail(VB_ENOTSUP, "tiled kernels need a 3D grid with nx, ny multiples of "
+                                    "16 or a 2D grid with nx a multiple of 256");
+        if (value != VB_KERNEL_CELL && vb::tiled_supported(gr->g) && !gr->maps_U.in_int.opaque[0] &&
+            !gr->maps_U.in_int.opaque[1]) {
+            int rc = encode_maps(&gr->maps_U, gr->U, gr->g);
+            if (!rc) rc = encode_maps(&gr->maps_U1, gr->U1, gr->g);
+            if (rc) return rc;
         }
+        // the choice is made: nothing above changes the grid's
+        gr->march = automatic && fp64 && vb::march_supported(gr->g);
+        gr->plane = automatic && fp64 && vb::plane_f64_supported(gr->g);
+        gr->cell_only = value == VB_KERNEL_CELL;
+        gr->tiled = value == VB_KERNEL_TILED || (automatic && vb::detail::tiled_auto(gr->g, gr->precision));
         return VB_OK;
+    }
     case VB_OPT_TILE_KZ:
         if (value < 1 || value > vb::march_extent(gr->g))
             return fail(VB_EINVAL, "the chunk must be in 1..nz (3D) or 1..ny (2D)");
