@@ -164,3 +164,49 @@ def test_a_refused_option_leaves_the_grid_as_it_was(fake, ctx, dims):
             assert fake.vb_grid_set_option(g, _lib.OPT_KERNEL, bad) == code
             assert kernels() == before, (chosen, bad)
     fake.vb_grid_destroy(g)
+
+
+def test_a_second_device_gets_its_own_kernel_opt_ins(fake, ctx):
+    """Shared-memory and cluster-size opt-ins belong to a device: one run on the
+    first must not stand for the second."""
+    fake.fake_devices(2)
+    other = C.c_void_p()
+    assert fake.vb_ctx_create(1, C.byref(other)) == 0
+    grids = [((64, 64), _lib.FP64, "auto"), ((300,), _lib.FP64, "auto"), ((256, 64), _lib.FP64, "tiled"),
+             ((512, 4096), _lib.MIXED, "auto"), ((48, 48, 48), _lib.FP64, "auto"), ((48, 48, 48), _lib.MIXED, "auto"),
+             ((48, 47, 48), _lib.FP64, "auto")]
+    for c in (ctx, other):
+        for dims, prec, kind in grids:
+            g = make_grid(fake, c, dims, prec)
+            assert fake.vb_grid_set_option(g, _lib.OPT_KERNEL, _lib.KERNELS[kind]) == 0, error(fake)
+            for bflux in (0, 1):
+                assert fake.vb_bflux_enable(g, bflux) == 0, error(fake)
+                assert fake.vb_run_steps_async(g, 2) == 0, (dims, error(fake))
+            if prec == _lib.FP64 and len(dims) == 2:
+                a = C.c_void_p()
+                assert fake.vb_adjoint_create(g, 2, 1, C.byref(a)) == 0, error(fake)
+                U = np.ones((5, int(np.prod(dims))))
+                assert fake.vb_adjoint_step(a, 0.1, _lib.dptr(U), _lib.dptr(U)) == 0, error(fake)
+                fake.vb_adjoint_destroy(a)
+            fake.vb_grid_destroy(g)
+        b = C.c_void_p()
+        prob = P.smooth_random_problem((32, 32, 32), seed=1)
+        assert fake.vb_batch_create(c, 1, C.byref(vb.simulation.problem_desc(prob)), _lib.FP64, C.byref(b)) == 0
+        assert fake.vb_batch_run_steps_async(b, 2) == 0, error(fake)
+        fake.vb_batch_destroy(b)
+    why = C.create_string_buffer(256)
+    assert fake.fake_refused(why, 256) == 0, why.value
+    fake.vb_ctx_destroy(other)
+
+
+def test_grids_march_only_where_their_cluster_fits(fake, ctx):
+    for clusters, kernel in ((1, b"k_march"), (0, b"k_stage_plane_f64")):
+        fake.fake_clusters(clusters)
+        g = make_grid(fake, ctx, (64, 64))
+        for _ in range(2):
+            assert fake.vb_run_steps_async(g, 2) == 0, error(fake)
+            assert fake.fake_launched(kernel) > 0
+            assert fake.vb_grid_set_option(g, _lib.OPT_KERNEL, 0) == 0
+        assert fake.fake_refused(None, 0) == 0
+        fake.vb_grid_destroy(g)
+        fake.fake_reset()

@@ -314,9 +314,14 @@ int launch_adj_stage(const Geom &g, const double *U, const double *lam, const do
     if (adj_on_chip(g)) {
         const int ntx = (int)((g.n[0] + adj2::T - 1) / adj2::T);
         const int64_t nt = ntx * ((g.n[1] + adj2::T - 1) / adj2::T);
-        static const cudaError_t set = cudaFuncSetAttribute(
-            k_adj_plane, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(adj2::Smem));
-        if (set != cudaSuccess || nt > 0x7fffffffLL) return -1;
+        static PerDevice opted;
+        const int set = opted.get([] {
+            return cudaFuncSetAttribute(k_adj_plane, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)sizeof(adj2::Smem)) == cudaSuccess
+                       ? 1
+                       : -1;
+        });
+        if (set < 0 || nt > 0x7fffffffLL) return -1;
         k_adj_plane<<<(unsigned)nt, adj2::NTH, sizeof(adj2::Smem), s>>>(g, U, lam, M, invV, out, ntx);
         return 1;
     }

@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "vb_common.cuh"
 
 namespace vb {
@@ -81,6 +83,26 @@ inline bool tiled3d_supported(const Geom &g)
     return g.nd == 3 && g.n[0] % 16 == 0 && g.n[1] % 16 == 0 && g.n[2] >= 2 &&
            g.n[0] <= (1 << 30) && g.n[1] <= (1 << 30) && g.n[2] <= (1 << 30);
 }
+
+// A number worked out once for each device, with that device current: kernel
+// attributes (shared memory and cluster opt-ins) belong to the device they were
+// set on.  f returns a positive number, kept, or a failure, tried again.
+struct PerDevice {
+    std::atomic<int> v[64] = {};
+    template <typename F>
+    int get(F &&f)
+    {
+        int d = 0;
+        if (cudaGetDevice(&d) != cudaSuccess || d < 0) return -1;
+        if (d >= 64) return f();
+        int r = v[d].load(std::memory_order_acquire);
+        if (r <= 0) {
+            r = f();
+            v[d].store(r, std::memory_order_release);
+        }
+        return r;
+    }
+};
 
 // Ragged 3D boxes with room for one tile: a side that is no multiple of 16 ends
 // in a shifted tile.  The float64 kernel's loads need no alignment; the mixed
@@ -169,7 +191,8 @@ int launch_wait_selftest(Ctrl *ctrl, uint64_t limit_ns, cudaStream_t s);
 
 // vb_march.cu: nsteps CFL-limited steps (evolve!'s loop, dt and clock included)
 // of a small float64 1D or 2D grid in one launch; the state and the control
-// block end as that many separate steps leave them.
+// block end as that many separate steps leave them.  march_supported: the grid
+// fits and the current device can place the cluster.
 bool march_supported(const Geom &g);
 int launch_march(const Geom &g, double *U, Ctrl *ctrl, int64_t nsteps, cudaStream_t s);
 

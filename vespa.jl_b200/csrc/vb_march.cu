@@ -346,17 +346,24 @@ k_march(const __grid_constant__ Geom g, double *__restrict__ U, Ctrl *ctrl, long
     if (C > 1) cl.sync();  // no block leaves while another reads its shared memory
 }
 
+// the opt-ins of k_march on the current device
 template <int ND>
-int go(const Geom &g, const MarchPlan &p, double *U, Ctrl *ctrl, int64_t nsteps, cudaStream_t s)
+bool opted()
 {
-    static const cudaError_t set = [] {
+    static PerDevice set;
+    return set.get([] {
         cudaError_t e = cudaFuncSetAttribute(k_march<ND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)MARCH_SMEM);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(k_march<ND>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        return e;
-    }();
-    if (set != cudaSuccess) return -1;
+        return e == cudaSuccess ? 1 : -1;
+    }) > 0;
+}
+
+// f(configuration) of the plan's launch
+template <typename F>
+cudaError_t configured(const MarchPlan &p, cudaStream_t s, F &&f)
+{
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)p.blocks);
     cfg.blockDim = dim3((unsigned)p.threads);
@@ -368,7 +375,27 @@ int go(const Geom &g, const MarchPlan &p, double *U, Ctrl *ctrl, int64_t nsteps,
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_march<ND>, g, U, ctrl, (long long)nsteps, p.rows) == cudaSuccess ? 1 : -1;
+    return f(cfg);
+}
+
+template <int ND>
+bool fits(const MarchPlan &p)
+{
+    int n = 0;
+    const bool ok = opted<ND>() && configured(p, nullptr, [&](const cudaLaunchConfig_t &cfg) {
+                        return cudaOccupancyMaxActiveClusters(&n, k_march<ND>, &cfg);
+                    }) == cudaSuccess;
+    cudaGetLastError();
+    return ok && n > 0;
+}
+
+template <int ND>
+int go(const Geom &g, const MarchPlan &p, double *U, Ctrl *ctrl, int64_t nsteps, cudaStream_t s)
+{
+    if (!opted<ND>()) return -1;
+    return configured(p, s, [&](const cudaLaunchConfig_t &cfg) {
+               return cudaLaunchKernelEx(&cfg, k_march<ND>, g, U, ctrl, (long long)nsteps, p.rows);
+           }) == cudaSuccess ? 1 : -1;
 }
 
 }  // namespace
@@ -376,7 +403,7 @@ int go(const Geom &g, const MarchPlan &p, double *U, Ctrl *ctrl, int64_t nsteps,
 bool march_supported(const Geom &g)
 {
     MarchPlan p;
-    return march_plan(g, &p);
+    return march_plan(g, &p) && (g.nd == 1 ? fits<1>(p) : fits<2>(p));
 }
 
 int launch_march(const Geom &g, double *U, Ctrl *ctrl, int64_t nsteps, cudaStream_t s)

@@ -376,11 +376,11 @@ int launch_tiled2d(const BoxDesc *hbox, int nitems, unsigned int *work, int stag
                    bool bf)
 {
     const size_t smem = sizeof(t2::Smem<NS>);
-    static int res = 0, resf = 0;
-    if (!res) res = persistent_blocks(k_stage_tiled2d<NS, 1>, k_stage_tiled2d<NS, 2>, smem);
-    if (!resf) resf = persistent_blocks(k_stage_tiled2d<NS, 1, true>, k_stage_tiled2d<NS, 2, true>, smem);
+    static PerDevice res, resf;
     if (!hbox || (bf && !hbox->bflux)) return -1;
-    const int resident = bf ? resf : res;
+    const int resident =
+        bf ? resf.get([&] { return persistent_blocks(k_stage_tiled2d<NS, 1, true>, k_stage_tiled2d<NS, 2, true>, smem); })
+           : res.get([&] { return persistent_blocks(k_stage_tiled2d<NS, 1>, k_stage_tiled2d<NS, 2>, smem); });
     if (resident <= 0 || nitems <= 0) return -1;
     const unsigned grid = (unsigned)(nitems < resident ? nitems : resident);
     if (bf && stage == 1)

@@ -336,11 +336,12 @@ int launch_tiled2d_mixed(const BoxDesc *hbox, int nitems, unsigned int *work, in
 {
     if (!hbox || nitems <= 0 || (bf && !hbox->bflux)) return -1;
     const size_t smem = sizeof(t2m::Smem<NS>);
-    static int res = 0, resf = 0;
-    if (!res) res = persistent_blocks(k_stage_tiled2d_mixed<NS, 1>, k_stage_tiled2d_mixed<NS, 2>, smem);
-    if (!resf) resf = persistent_blocks(k_stage_tiled2d_mixed<NS, 1, true>,
-                                        k_stage_tiled2d_mixed<NS, 2, true>, smem);
-    const int resident = bf ? resf : res;
+    static PerDevice res, resf;
+    const int resident =
+        bf ? resf.get([&] {
+            return persistent_blocks(k_stage_tiled2d_mixed<NS, 1, true>, k_stage_tiled2d_mixed<NS, 2, true>, smem);
+        })
+           : res.get([&] { return persistent_blocks(k_stage_tiled2d_mixed<NS, 1>, k_stage_tiled2d_mixed<NS, 2>, smem); });
     if (resident <= 0) return -1;
     const unsigned grid = (unsigned)(nitems < resident ? nitems : resident);
     auto k = bf ? (stage == 1 ? k_stage_tiled2d_mixed<NS, 1, true> : k_stage_tiled2d_mixed<NS, 2, true>)

@@ -143,7 +143,7 @@ __device__ __forceinline__ const BoxDesc &box_of(const BoxDesc &box0, const BoxD
 namespace vb {
 
 // Resident blocks of a persistent kernel on the current device (all SMs), with
-// its dynamic shared memory opted in once.
+// its dynamic shared memory opted in there (PerDevice keeps the number).
 template <typename K>
 int persistent_blocks(K kernel1, K kernel2, size_t smem, int threads = t3::NT)
 {

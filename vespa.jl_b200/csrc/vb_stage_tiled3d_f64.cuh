@@ -467,19 +467,18 @@ inline int launch_tiled3d_f64(const BoxDesc *hbox, const BoxDesc *boxes, const i
                               bool bf)
 {
     const size_t smem = sizeof(t3d::Smem);
-    static int res1 = 0, resb = 0, resg = 0, resf = 0;
-    if (!res1) res1 = persistent_blocks(k_stage_tiled3d_f64<1, false>, k_stage_tiled3d_f64<2, false>,
-                                        smem, t3d::NTH);
-    if (!resb) resb = persistent_blocks(k_stage_tiled3d_f64<1, true>, k_stage_tiled3d_f64<2, true>,
-                                        smem, t3d::NTH);
-    if (!resg) resg = persistent_blocks(k_stage_tiled3d_f64<1, false, true>,
-                                        k_stage_tiled3d_f64<2, false, true>, smem, t3d::NTH);
-    if (!resf) resf = persistent_blocks(k_stage_tiled3d_f64<1, false, false, true>,
-                                        k_stage_tiled3d_f64<2, false, false, true>, smem, t3d::NTH);
+    static PerDevice res1, resb, resg, resf;
     if ((grav || bf) && !hbox) return -1;  // gravity, boundary fluxes: single boxes only
     if (grav && bf) return -1;
     if (bf && !hbox->bflux) return -1;
-    const int resident = grav ? resg : bf ? resf : hbox ? res1 : resb;
+    auto fits = [&](auto k1, auto k2) { return persistent_blocks(k1, k2, smem, t3d::NTH); };
+    const int resident =
+        grav   ? resg.get([&] { return fits(k_stage_tiled3d_f64<1, false, true>, k_stage_tiled3d_f64<2, false, true>); })
+        : bf   ? resf.get([&] {
+              return fits(k_stage_tiled3d_f64<1, false, false, true>, k_stage_tiled3d_f64<2, false, false, true>);
+          })
+        : hbox ? res1.get([&] { return fits(k_stage_tiled3d_f64<1, false>, k_stage_tiled3d_f64<2, false>); })
+               : resb.get([&] { return fits(k_stage_tiled3d_f64<1, true>, k_stage_tiled3d_f64<2, true>); });
     if (resident <= 0 || nitems <= 0) return -1;
     const unsigned grid = (unsigned)(nitems < resident ? nitems : resident);
     BoxDesc box0;
