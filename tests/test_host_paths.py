@@ -210,3 +210,57 @@ def test_grids_march_only_where_their_cluster_fits(fake, ctx):
         assert fake.fake_refused(None, 0) == 0
         fake.vb_grid_destroy(g)
         fake.fake_reset()
+
+
+def gravity_desc(bc, precond=0, maxiter=100):
+    d = _lib.GravityDesc()
+    d.G, d.tol, d.maxiter, d.project_mean, d.precond, d.flags = 1.0, 1e-8, maxiter, 1, precond, 0
+    for a in range(3):
+        d.bc_lo[a] = d.bc_hi[a] = bc
+    return d
+
+
+@pytest.mark.parametrize("start", [None, (_lib.BC_OUTFLOW, 0), (_lib.BC_PERIODIC, 0)])
+def test_gravity_enable_that_fails_leaves_what_was_there(fake, ctx, start):
+    """Each allocation of a (re-)enable made to fail in turn: the error is
+    reported, gravity that was on stays on with its settings, and the next call
+    has every buffer that one without failures has."""
+    wanted = C.byref(gravity_desc(_lib.BC_PERIODIC, precond=1))
+
+    def grid():
+        g = make_grid(fake, ctx, (32, 32, 32))
+        if start:
+            assert fake.vb_gravity_enable(g, C.byref(gravity_desc(*start))) == 0, error(fake)
+        return g
+
+    phi = np.zeros(32 ** 3)
+    base = fake.fake_device_live()
+    g = grid()
+    assert fake.vb_gravity_enable(g, wanted) == 0, error(fake)
+    full = fake.fake_device_live()
+    fake.vb_grid_destroy(g)
+    assert fake.fake_device_live() == base
+    fails = 0
+    while True:
+        g = grid()
+        fake.fake_fail_device_alloc(fails)
+        rc = fake.vb_gravity_enable(g, wanted)
+        fake.fake_fail_device_alloc(-1)
+        if rc == 0:
+            fake.vb_grid_destroy(g)
+            break
+        assert rc == _lib.VB_ENOMEM, error(fake)
+        cube = start and start[0] == _lib.BC_PERIODIC
+        fake.fake_reset()
+        if start:  # still on, still as it was set up
+            assert fake.vb_gravity_phi(g, _lib.dptr(phi)) == 0, error(fake)
+            assert fake.vb_gravity_set_phi(g, _lib.dptr(phi)) == 0, error(fake)
+            assert (fake.fake_launched(b"k_cube_accel") > 0) == bool(cube), fails
+        else:
+            assert fake.vb_gravity_phi(g, _lib.dptr(phi)) == _lib.VB_EINVAL
+        assert fake.vb_gravity_enable(g, wanted) == 0, error(fake)
+        assert fake.fake_device_live() == full, fails
+        fake.vb_grid_destroy(g)
+        assert fake.fake_device_live() == base
+        fails += 1
+    assert fails >= 4

@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <new>
 #include <vector>
 
 #include "vb_internal.h"
@@ -1391,84 +1392,72 @@ int vb_gravity_enable(vb_grid *gr, const vb_gravity_desc *d)
             return fail(VB_ENOTSUP, "the multigrid preconditioner needs a 3D cubic grid (n <= 1024) "
                                     "with periodic phi on every side");
     }
-    vb_gravity *gv = gr->grav;
-    if (!gv) {
-        gv = new vb_gravity;
-        const size_t n = (size_t)g.ncell * sizeof(double);
-        cudaError_t e = cudaSuccess;
-        for (double **buf : {&gv->phi, &gv->b, &gv->r, &gv->p, &gv->Ap})
-            if (e == cudaSuccess) e = cudaMalloc(buf, n);
-        if (e == cudaSuccess) e = cudaMalloc(&gv->gacc, n * g.nd);
-        if (e == cudaSuccess) e = cudaMalloc(&gv->part, sizeof(double) * 3 * vb::GP);
-        if (e == cudaSuccess) e = cudaMalloc(&gv->gc, sizeof(vb::GravCtrl));
-        if (e == cudaSuccess) e = cudaMallocHost(&gv->hgc, sizeof(vb::GravCtrl));
-        if (e == cudaSuccess) e = cudaMemsetAsync(gv->phi, 0, n, gr->ctx->stream);  // phi starts at 0
+    bool cube = g.nd == 3 && g.n[0] == g.n[1] && g.n[1] == g.n[2] && g.n[0] <= 1024;
+    for (int a = 0; a < 3; ++a) cube = cube && P.per_lo[a] && P.per_hi[a];
+    const bool mg = d->precond == VB_GRAV_PRECOND_MG;
+    // Everything that can fail comes first: a grid that has gravity keeps it, with
+    // its settings, when it does.  Each buffer is guarded by its own pointer (a
+    // failed call's are taken up by the next one, or freed with the rest).
+    vb_gravity *gv = gr->grav ? gr->grav : new (std::nothrow) vb_gravity;
+    if (!gv) return fail(VB_ENOMEM, "host allocation failed");
+    cudaError_t e = cudaSuccess;
+    auto need = [&](auto **p, size_t bytes) {
+        if (e == cudaSuccess && !*p) e = cudaMalloc(p, bytes);
+    };
+    const size_t n = (size_t)g.ncell * sizeof(double);
+    for (double **buf : {&gv->phi, &gv->b, &gv->r, &gv->p, &gv->Ap}) need(buf, n);
+    need(&gv->gacc, n * g.nd);
+    need(&gv->part, sizeof(double) * 3 * vb::GP);
+    need(&gv->gc, sizeof(vb::GravCtrl));
+    if (e == cudaSuccess && !gv->hgc) e = cudaMallocHost(&gv->hgc, sizeof(vb::GravCtrl));
+    if (cube) {
+        const dim3 b = cube_grid((int)g.n[0]);
+        need(&gv->cpart, sizeof(double) * std::max<size_t>(2 * (size_t)b.x * b.y * b.z, CUBE_UPDATE_BLOCKS));
+        need(&gv->p2, n);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(vb::k_mg_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)vb::mg_bottom_smem(vb::MG_BLOCK));
+    }
+    if (mg) {
+        for (double **buf : {&gv->z, &gv->z2}) need(buf, n);
+        if (gv->lev.empty()) {  // levels: coarsen while even and > 4 (mg_pcg.jl:111-116)
+            int nl = (int)g.n[0];
+            double h = g.w[0];
+            gv->vbase = h * h * h;
+            for (;;) {
+                gv->lev.push_back({nl, h, nullptr, nullptr, nullptr});
+                if (!(nl > 4 && nl % 2 == 0)) break;
+                nl /= 2;
+                h *= 2.0;
+            }
+        }
+        for (auto &l : gv->lev)
+            for (double **buf : {&l.e, &l.b, &l.t}) need(buf, sizeof(double) * (size_t)l.n * l.n * l.n);
+    }
+    if (e == cudaSuccess && !gr->grav) {
+        std::memset(gv->hgc, 0, sizeof(vb::GravCtrl));
+        e = cudaMemsetAsync(gv->phi, 0, n, gr->ctx->stream);  // phi starts at 0
         if (e == cudaSuccess) e = cudaMemsetAsync(gv->gacc, 0, n * g.nd, gr->ctx->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(gv->gc, 0, sizeof(vb::GravCtrl), gr->ctx->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(gr->ctx->stream);
-        if (e != cudaSuccess) {
-            free_gravity(gv);
-            return fail(e == cudaErrorMemoryAllocation ? VB_ENOMEM : VB_ECUDA,
-                        std::string("gravity allocation: ") + cudaGetErrorString(e));
-        }
-        std::memset(gv->hgc, 0, sizeof(vb::GravCtrl));
+    }
+    if (e != cudaSuccess) {
+        if (!gr->grav) free_gravity(gv);
+        cudaGetLastError();
+        return fail(e == cudaErrorMemoryAllocation ? VB_ENOMEM : VB_ECUDA,
+                    std::string("gravity allocation: ") + cudaGetErrorString(e));
     }
     gv->P = P;
-    {
-        bool cube = g.nd == 3 && g.n[0] == g.n[1] && g.n[1] == g.n[2] && g.n[0] <= 1024;
-        for (int a = 0; a < 3; ++a) cube = cube && P.per_lo[a] && P.per_hi[a];
-        gv->cube_n = cube ? (int)g.n[0] : 0;
-        if (cube && !gv->cpart) {
-            const dim3 b = cube_grid((int)g.n[0]);
-            const size_t nb = std::max<size_t>(2 * (size_t)b.x * b.y * b.z, CUBE_UPDATE_BLOCKS);
-            cudaError_t e = cudaMalloc(&gv->cpart, sizeof(double) * nb);
-            if (e == cudaSuccess) e = cudaMalloc(&gv->p2, sizeof(double) * (size_t)g.ncell);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(vb::k_mg_bottom, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)vb::mg_bottom_smem(vb::MG_BLOCK));
-            if (e != cudaSuccess) {
-                gv->cube_n = 0;
-                if (!gr->grav) free_gravity(gv);
-                return fail(e == cudaErrorMemoryAllocation ? VB_ENOMEM : VB_ECUDA,
-                            std::string("gravity allocation: ") + cudaGetErrorString(e));
-            }
-        }
-    }
+    gv->cube_n = cube ? (int)g.n[0] : 0;
     gv->maxiter = d->maxiter;
     gv->tol = d->tol;
     gv->limits_set = false;
-    gr->grav = gv;
-    if (gv->gexec) {  // the iteration graph depends on the preconditioner
+    gv->precond = d->precond;
+    if (gv->gexec) {  // the iteration graph depends on all of these
         cudaGraphExecDestroy(gv->gexec);
         gv->gexec = nullptr;
     }
-    gv->precond = d->precond;
-    if (gv->precond == VB_GRAV_PRECOND_MG && !gv->z) {
-        // levels: coarsen while even and > 4 (mg_pcg.jl:111-116)
-        const size_t n = (size_t)g.ncell * sizeof(double);
-        cudaError_t e = cudaSuccess;
-        for (double **buf : {&gv->z, &gv->z2})
-            if (e == cudaSuccess) e = cudaMalloc(buf, n);
-        int nl = (int)g.n[0];
-        double h = g.w[0];
-        gv->vbase = h * h * h;
-        for (;;) {
-            vb_gravity::Level l{nl, h, nullptr, nullptr, nullptr};
-            const size_t bytes = sizeof(double) * (size_t)nl * nl * nl;
-            for (double **buf : {&l.e, &l.b, &l.t})
-                if (e == cudaSuccess) e = cudaMalloc(buf, bytes);
-            gv->lev.push_back(l);
-            if (!(nl > 4 && nl % 2 == 0)) break;
-            nl /= 2;
-            h *= 2.0;
-        }
-        if (e != cudaSuccess) {
-            gr->grav = nullptr;
-            free_gravity(gv);
-            return fail(e == cudaErrorMemoryAllocation ? VB_ENOMEM : VB_ECUDA,
-                        std::string("multigrid allocation: ") + cudaGetErrorString(e));
-        }
-    }
+    gr->grav = gv;
     gr->g.grav_g = gv->gacc;
     gr->g.grav_G = d->G;
     gr->box_kz = -1;          // the tiled kernels' box descriptor carries the geometry
