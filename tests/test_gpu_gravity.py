@@ -401,3 +401,26 @@ def test_mg_refuses_unsupported_grids(vb):
     with pytest.raises(vb.VespaB200Error) as e:
         vb.enable_gravity(sim, precond="mg", bcs=P.Outflow)
     assert e.value.status == 6
+
+
+@pytest.mark.parametrize("n", [5, 6, 33, 34, 64])
+@pytest.mark.parametrize("precond", ["none", "mg"])
+def test_cube_operator_takes_differences(vb, n, precond):
+    """The cube's A phi on a potential far from zero: its differences are exact
+    numbers there, so the first residual (no iteration, no right-hand side) is
+    theirs to rounding; sums of neighbours would lose a part in 1e8 of it."""
+    prob = P.smooth_random_problem((n, n, n), seed=n)
+    U0 = P.initial_state(prob)
+    U0[0] = 1.0
+    sim = make_sim(prob, U0)
+    grav = vb.enable_gravity(sim, G=1.0, tol=0.0, maxiter=0, precond=precond)
+    x, y, z = prob.cell_centers()
+    phi = 1e10 + np.sin(2 * np.pi * x) + 0.5 * np.cos(2 * np.pi * (y + z))
+    grav.phi = phi
+    iters, relres = vb.solve_poisson(sim)
+    c = phi.reshape(n, n, n).astype(np.longdouble)
+    lap = sum((c - np.roll(c, 1, a)) + (c - np.roll(c, -1, a)) for a in range(3)) / n  # area / width
+    want = float(np.sqrt(np.sum(lap * lap)))
+    assert iters == 0 and want > 0.1 / n
+    # seven roundings a cell and the norm's sum
+    assert abs(relres - want) <= 1e-13 * want, (relres, want)

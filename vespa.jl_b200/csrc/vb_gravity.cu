@@ -486,10 +486,21 @@ struct At {
     __device__ __forceinline__ void put(double *p, T v) const { *reinterpret_cast<T *>(p + i) = v; }
 };
 
-// f(at, v, sx, sy, sz) for this thread's cells, s* the sums of v over the two
-// neighbours per axis; v(at) forms the operand.  Blocks of 32 x 8 cells (D2:
-// 32 x 16).
-template <class T, class V, class F>
+// what f gets of a cell's two neighbours on an axis: their sum, or (DIFF) the
+// sum of the cell's differences to them.  The operator of CG takes differences:
+// each is exact where v varies slowly, while 2 c - (a + b) is rounded to a part
+// in 2^53 of v itself, n / 2 pi times more on the longest mode and without bound
+// under a constant offset of v.
+template <bool DIFF, class T>
+__device__ __forceinline__ T cube_axis(T c, T a, T b)
+{
+    if constexpr (DIFF) return (c - a) + (c - b);
+    else return a + b;
+}
+
+// f(at, v, sx, sy, sz) for this thread's cells, s* cube_axis per axis; v(at)
+// forms the operand.  Blocks of 32 x 8 cells (D2: 32 x 16).
+template <class T, bool DIFF = false, class V, class F>
 __device__ __forceinline__ void cube_cells(int n, V &&v, F &&f)
 {
     constexpr bool PAIR = sizeof(T) == 16;
@@ -508,7 +519,7 @@ __device__ __forceinline__ void cube_cells(int n, V &&v, F &&f)
         for (int z = z0; z < z1; ++z) {
             const int i = base + z * nn;
             const D2 hi = v(At<D2>{base + (z + 1 < n ? z + 1 : 0) * nn});
-            const D2 sy = v(At<D2>{i + ym}) + v(At<D2>{i + yp});
+            const D2 sy = cube_axis<DIFF>(c, v(At<D2>{i + ym}), v(At<D2>{i + yp}));
             double l = __shfl_up_sync(0xffffffffu, c.y, 1, 16), r = __shfl_down_sync(0xffffffffu, c.x, 1, 16);
             if (first || last) {
                 const double e = v(At<double>{i + xe});
@@ -516,7 +527,7 @@ __device__ __forceinline__ void cube_cells(int n, V &&v, F &&f)
                 else r = e;
                 if (first && last) r = v(At<double>{i + (x + 2 < n ? 2 : 2 - n)});
             }
-            if (in) f(At<D2>{i}, c, D2{l + c.y, c.x + r}, sy, lo + hi);
+            if (in) f(At<D2>{i}, c, cube_axis<DIFF>(c, D2{l, c.x}, D2{c.y, r}), sy, cube_axis<DIFF>(c, lo, hi));
             lo = c;
             c = hi;
         }
@@ -530,19 +541,20 @@ __device__ __forceinline__ void cube_cells(int n, V &&v, F &&f)
         for (int z = z0; z < z1; ++z) {
             const int i = base + z * nn;
             const double hi = v(At<double>{base + (z + 1 < n ? z + 1 : 0) * nn});
-            f(At<double>{i}, c, v(At<double>{i + xm}) + v(At<double>{i + xp}),
-              v(At<double>{i + ym}) + v(At<double>{i + yp}), lo + hi);
+            f(At<double>{i}, c, cube_axis<DIFF>(c, v(At<double>{i + xm}), v(At<double>{i + xp})),
+              cube_axis<DIFF>(c, v(At<double>{i + ym}), v(At<double>{i + yp})), cube_axis<DIFF>(c, lo, hi));
             lo = c;
             c = hi;
         }
     }
 }
 
-// A v at a cell from cube_cells' sums
+// A v at a cell from cube_cells' sums of differences.  The reference's row sums
+// the same six differences face by face (lap_row); the order differs.
 template <class T>
-__device__ __forceinline__ T cube_lap(const CubeP &P, T c, T sx, T sy, T sz)
+__device__ __forceinline__ T cube_lap(const CubeP &P, T dx, T dy, T dz)
 {
-    return P.c[0] * (2.0 * c - sx) + P.c[1] * (2.0 * c - sy) + P.c[2] * (2.0 * c - sz);
+    return P.c[0] * dx + P.c[1] * dy + P.c[2] * dz;
 }
 
 // The grid's sum of s over its threads: true in thread 0 of the last block to
@@ -577,11 +589,11 @@ __global__ void __launch_bounds__(GB) k_cube_init(CubeP P, GravP Q, double vol, 
 {
     const double rhobar = Q.project_mean ? gc->rhobar : 0.0;
     double rr = 0.0, bb = 0.0;
-    cube_cells<T>(
+    cube_cells<T, true>(
         P.n, [&](auto at) { return at(phi); },
-        [&](auto at, T c, T sx, T sy, T sz) {
+        [&](auto at, T c, T dx, T dy, T dz) {
             const T b = scaled(-VB_FOURPI * Q.G, at(rho) - rhobar, vol);
-            const T ri = b - cube_lap(P, c, sx, sy, sz);
+            const T ri = b - cube_lap(P, dx, dy, dz);
             at.put(r, ri);
             rr = rr + total(ri * ri);
             bb = bb + total(b * b);
@@ -647,10 +659,10 @@ __global__ void __launch_bounds__(GB) k_cube_dir(CubeP P, const double *__restri
     double *__restrict__ pn = odd ? pa : pb;
     const double beta = gc->beta;
     double s = 0.0;
-    cube_cells<T>(
+    cube_cells<T, true>(
         P.n, [&](auto at) { return beta != 0.0 ? at(z) + beta * at(po) : at(z); },
-        [&](auto at, T c, T sx, T sy, T sz) {
-            const T a = cube_lap(P, c, sx, sy, sz);
+        [&](auto at, T c, T dx, T dy, T dz) {
+            const T a = cube_lap(P, dx, dy, dz);
             at.put(pn, c);
             at.put(Ap, a);
             s = s + total(c * a);
@@ -706,10 +718,10 @@ __global__ void __launch_bounds__(GB) k_cube_pre(CubeP P, const double *__restri
                                                 double *__restrict__ z, const GravCtrl *gc)
 {
     if (gc->done) return;
-    cube_cells<T>(
+    cube_cells<T, true>(
         P.n, [&](auto at) { return at(r); },
-        [&](auto at, T c, T sx, T sy, T sz) {
-            at.put(z, P.w * c + P.w * (c - P.w * cube_lap(P, c, sx, sy, sz)));
+        [&](auto at, T c, T dx, T dy, T dz) {
+            at.put(z, P.w * c + P.w * (c - P.w * cube_lap(P, dx, dy, dz)));
         });
 }
 
@@ -720,9 +732,9 @@ __global__ void __launch_bounds__(GB) k_cube_resid(CubeP P, const double *__rest
                                                   double *__restrict__ b, const GravCtrl *gc)
 {
     if (gc->done) return;
-    cube_cells<T>(
+    cube_cells<T, true>(
         P.n, [&](auto at) { return at(z); },
-        [&](auto at, T c, T sx, T sy, T sz) { at.put(b, at(r) - cube_lap(P, c, sx, sy, sz)); });
+        [&](auto at, T c, T dx, T dy, T dz) { at.put(b, at(r) - cube_lap(P, dx, dy, dz)); });
 }
 
 // first post-smoothing sweep on A of z + (e - mean e) / V
@@ -734,10 +746,10 @@ __global__ void __launch_bounds__(GB) k_cube_post1(CubeP P, const double *__rest
 {
     if (gc->done) return;
     const double mu = gc->mgmu;
-    cube_cells<T>(
+    cube_cells<T, true>(
         P.n, [&](auto at) { return at(z) + iV * (at(e) - mu); },
-        [&](auto at, T c, T sx, T sy, T sz) {
-            at.put(z2, c + P.w * (at(r) - cube_lap(P, c, sx, sy, sz)));
+        [&](auto at, T c, T dx, T dy, T dz) {
+            at.put(z2, c + P.w * (at(r) - cube_lap(P, dx, dy, dz)));
         });
 }
 
@@ -755,10 +767,10 @@ __global__ void __launch_bounds__(GB) k_cube_post2(CubeP P, const double *__rest
         return;
     }
     double s = 0.0;
-    cube_cells<T>(
+    cube_cells<T, true>(
         P.n, [&](auto at) { return at(z2); },
-        [&](auto at, T c, T sx, T sy, T sz) {
-            const T ri = at(r), v = c + P.w * (ri - cube_lap(P, c, sx, sy, sz));
+        [&](auto at, T c, T dx, T dy, T dz) {
+            const T ri = at(r), v = c + P.w * (ri - cube_lap(P, dx, dy, dz));
             at.put(z, v);
             s = s + total(ri * v);
         });
