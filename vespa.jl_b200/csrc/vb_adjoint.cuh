@@ -209,9 +209,11 @@ __device__ __forceinline__ void hllc_vjp(const double WL[5], const double WR[5],
 
 // hllc_vjp in the face-normal frame (rho, u_n, u_t1, u_t2, p), Lb and Rb
 // overwritten.  The forward speeds that decide the branches are formed as
-// hllc_frame forms them (the forward's own bits); the derivatives take products
-// with the reciprocals of the seven denominators, formed side by side.  States
-// outside the range hllc_frame takes go to hllc_vjp.
+// hllc_frame forms them (the forward's own bits), and the derivatives divide by
+// the seven denominators as quot64, whose reciprocals are formed side by side.
+// (Products with those reciprocals alone, a rounding more each, took the error of
+// a 512^2 run of 40 steps from 1.15e-15 to 1.17e-15.)  States outside the range
+// hllc_frame takes go to hllc_vjp.
 __device__ __forceinline__ void hllc_vjp_frame(const double L[5], const double R[5], double g,
                                                double ig1, const double Fb[5], double Lb[5],
                                                double Rb[5])
@@ -232,7 +234,7 @@ __device__ __forceinline__ void hllc_vjp_frame(const double L[5], const double R
     const double rho = left ? L[0] : R[0], un = left ? L[1] : R[1], y = left ? yL : yR;
     const double u1 = left ? L[2] : R[2], u2 = left ? L[3] : R[3], p = left ? L[4] : R[4];
     const double v2 = un * un + u1 * u1 + u2 * u2;
-    const double E = p * ig1 + 0.5 * rho * v2;
+    const double E = quot64(p, g - 1.0, ig1) + 0.5 * rho * v2;
     const double d = SK - Ss, a = SK - un, q = rho * a;
     if (!hllc_operands_ok(L, R, D, d, q, E, N)) {
 #pragma unroll
@@ -249,7 +251,8 @@ __device__ __forceinline__ void hllc_vjp_frame(const double L[5], const double R
     double pb = Fb[1] + Fb[4] * un, Eb = Fb[4] * un;
     if (!(supL || supR)) {
         const double yd = rcp64(d), yq = rcp64(q), ycL = rcp64(cL), ycR = rcp64(cR);
-        const double f = q * yd, r = p * yq, A = Ss - un, B = Ss + r, Es = E * y + A * B;
+        const double f = quot64(q, d, yd), r = quot64(p, q, yq), Ey = quot64(E, rho, y);
+        const double A = Ss - un, B = Ss + r, Es = Ey + A * B;
         // sum of Fb (U* - U)
         double Sb = Fb[0] * (f - rho) + Fb[1] * (f * Ss - rho * un) + Fb[2] * (f - rho) * u1 +
                     Fb[3] * (f - rho) * u2 + Fb[4] * (f * Es - E);
@@ -261,20 +264,22 @@ __device__ __forceinline__ void hllc_vjp_frame(const double L[5], const double R
         const double fb = SK * (Fb[0] + Fb[1] * Ss + Fb[2] * u1 + Fb[3] * u2 + Fb[4] * Es);
         double sb = SK * Fb[1] * f;
         const double Esb = SK * Fb[4] * f;
-        Eb += Esb * y;
-        rb -= Esb * E * y * y;
+        const double Esy = quot64(Esb, rho, y);
+        Eb += Esy;
+        rb -= Esy * Ey;
         const double Bb = Esb * A;
         sb += Esb * B + Bb;
         ub -= Esb * B;
-        pb += Bb * yq;
-        const double qb = fb * yd - Bb * r * yq, db = -fb * f * yd;
+        const double Bq = quot64(Bb, q, yq);
+        pb += Bq;
+        const double fd = quot64(fb, d, yd), qb = fd - Bq * r, db = -fd * f;
         Sb += db;
         sb -= db;
         rb += qb * a;
         Sb += qb * rho;
         ub -= qb * rho;
         // S* = N / D
-        const double Nb = sb * yD, Db = -Nb * Ss;
+        const double Nb = quot64(sb, D, yD), Db = -Nb * Ss;
         rp += Nb;
         lp -= Nb;
         lr += (Nb * L[1] + Db) * dL;
@@ -288,13 +293,13 @@ __device__ __forceinline__ void hllc_vjp_frame(const double L[5], const double R
         if (SL_from_L) { lu += SLb; cLb -= SLb; } else { ru += SLb; cRb -= SLb; }
         if (SR_from_L) { lu += SRb; cLb += SRb; } else { ru += SRb; cRb += SRb; }
         // c = sqrt(g p / rho); c > 0 in the range checked above
-        lp += cLb * (0.5 * g) * ycL * yL;
-        lr -= cLb * cL * 0.5 * yL;
-        rp += cRb * (0.5 * g) * ycR * yR;
-        rr -= cRb * cR * 0.5 * yR;
+        lp += quot64(quot64(cLb * (0.5 * g), cL, ycL), L[0], yL);
+        lr -= quot64(0.5 * cLb * cL, L[0], yL);
+        rp += quot64(quot64(cRb * (0.5 * g), cR, ycR), R[0], yR);
+        rr -= quot64(0.5 * cRb * cR, R[0], yR);
     }
     // E = p / (g - 1) + rho |v|^2 / 2 of the selected side
-    pb += Eb * ig1;
+    pb += quot64(Eb, g - 1.0, ig1);
     rb += Eb * 0.5 * v2;
     nb += Eb * rho * un + ub;
     t1 += Eb * rho * u1;
