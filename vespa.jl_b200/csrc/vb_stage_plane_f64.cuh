@@ -77,10 +77,12 @@ k_stage_plane_f64(const __grid_constant__ Geom g, const double *__restrict__ Uin
     const int ex = x0 + tx, ey = y0 + ty;
     const int64_t lin = ex + (int64_t)nx * ey;
     const bool own = col && ex >= xn && ey >= yn && VB_DCHECK(lin >= 0 && lin < g.ncell);
-    // the grid's CFL maximum so far: a lower bound of the final one
+    // the grid's CFL maximum so far: a lower bound of the final one (-1: none)
     float sofar = 0.0f;
-    if constexpr (STAGE == 2)
+    if constexpr (STAGE == 2) {
         sofar = __double2float_rd(__longlong_as_double((long long)__ldcg(&ctrl->invdt_bits)));
+        if (!(sofar > CFL_FLOOR) || !cfl_widths(g)) sofar = -1.0f;
+    }
     double u[5], v[5], uh[5];
 #pragma unroll
     for (int f = 0; f < 5; ++f) u[f] = col ? __ldg(Uin + lin + f * g.ncell) : 0.0;

@@ -64,24 +64,36 @@ __device__ __forceinline__ double face_mm(double w, double h, double a, double b
     return face_val(w, h, minmod<double>(a, b));
 }
 
+// cfl_bound keeps its digits above this maximum, with widths whose inverses are
+// normal float32 numbers
+constexpr float CFL_FLOOR = 1e-30f;
+__device__ __forceinline__ bool cfl_widths(const Geom &g)
+{
+    return g.invw[0] > 1.2e-38 && g.invw[1] > 1.2e-38 && (g.nd < 3 || g.invw[2] > 1.2e-38);
+}
+
 // An upper bound, in float32, of the cell's compute_dt term max_d (|v_d| + c) /
 // w_d (and of the free-fall rate, GRAV).  Relative slack 4e-6 on the pressure
-// (measured against E + kinetic, which its difference cancels) and on the
-// result covers the float32 roundings; anything out of float32 range, and any
-// negative density or pressure, comes out NaN or Inf.
+// (measured against E + kinetic, which its difference cancels; with what the
+// squares may lose below the normal numbers) and on the result covers the
+// float32 roundings.  Operands out of float32's normal range, and any negative
+// density or pressure, come out NaN or Inf, which asks for the exact term: above
+// p c = 1e-30 the pressure has all its digits (the reciprocal of a density below
+// the normal range is Inf).
 template <bool GRAV>
 __device__ __forceinline__ float cfl_bound(const double un[5], const Geom &g, float gf, float iw0,
                                            float iw1, float iw2)
 {
-    const float ir = rcp_approx((float)un[0]), E = (float)un[4];
+    const float rho = (float)un[0], ir = rcp_approx(rho), E = (float)un[4];
     const float vx = (float)un[1] * ir, vy = (float)un[2] * ir, vz = (float)un[3] * ir;
-    const float ke = 0.5f * (float)un[0] * (vx * vx + vy * vy + vz * vz);
-    const float p = (gf - 1.0f) * (E - ke) + 4e-6f * (fabsf(E) + ke);
+    const float ke = 0.5f * rho * (vx * vx + vy * vy + vz * vz);
+    const float p = (gf - 1.0f) * (E - ke) + 4e-6f * (fabsf(E) + fmaf(1.2e-38f, rho, ke));
     const float c = sqrt_approx(gf * p * ir);
     float b = fmaxf(fmaxf((fabsf(vx) + c) * iw0, (fabsf(vy) + c) * iw1), (fabsf(vz) + c) * iw2);
-    if (c != c) b = c;  // fmaxf drops a NaN operand
+    if (!(p * c > 1e-30f)) b = __int_as_float(0x7fc00000);  // NaN operands too, which fmaxf drops
     if constexpr (GRAV) {
-        const float f = 2.0f * sqrt_approx(12.566371f * (float)g.grav_G * (float)un[0]);
+        const float q = 12.566371f * (float)g.grav_G * rho;
+        const float f = q > 1e-30f || g.grav_G == 0.0 ? 2.0f * sqrt_approx(q) : __int_as_float(0x7fc00000);
         if (!(f <= b)) b = f;
     }
     return b * (1.0f + 4e-6f);
@@ -99,7 +111,9 @@ k_stage_tiled3d_f64(const __grid_constant__ BoxDesc box0, const BoxDesc *__restr
     t3d::Smem &S = *reinterpret_cast<t3d::Smem *>(smem_raw);
     __shared__ double red[32];
     __shared__ int item_sh;
-    __shared__ int cfl_sh;  // float bits: a lower bound of the item's CFL maximum so far
+    // float bits: a lower bound of the item's CFL maximum so far; -1: none above
+    // CFL_FLOOR, NaN: every cell takes the exact term
+    __shared__ int cfl_sh;
 
     const int t = threadIdx.x;
     const bool col = t < NC;  // column thread, else halo thread
@@ -127,10 +141,7 @@ k_stage_tiled3d_f64(const __grid_constant__ BoxDesc box0, const BoxDesc *__restr
     const int f_c = wrow(tx, fr);
 
     for (;;) {
-    if (t == 0) {
-        item_sh = (int)atomicAdd(&work[STAGE - 1], 1u);
-        cfl_sh = 0;
-    }
+    if (t == 0) item_sh = (int)atomicAdd(&work[STAGE - 1], 1u);
     __syncthreads();
     const int item = item_sh;
     if (item >= nitems) break;
@@ -149,6 +160,7 @@ k_stage_tiled3d_f64(const __grid_constant__ BoxDesc box0, const BoxDesc *__restr
     const bool perz = g.bc_lo[2] == BC_PERIODIC;
     const double gamma = g.gamma;
     const double bscale = BF ? 0.5 * ctrl->dt : 0.0;  // boundary-flux stage weight
+    if (STAGE == 2 && t == 0) cfl_sh = cfl_widths(g) ? __float_as_int(-1.0f) : 0x7fc00000;
     const int local = item - B.item0;
     const int tile = local % B.ntiles;
     // the last tile of a side that is no multiple of 16 is shifted back; the
@@ -442,7 +454,8 @@ k_stage_tiled3d_f64(const __grid_constant__ BoxDesc box0, const BoxDesc *__restr
                         const float b = cfl_bound<GRAV>(un, g, gf, iw0, iw1, iw2);
                         if (!(b <= __int_as_float(*(volatile int *)&cfl_sh))) {
                             cflm = cfl_term_exact<GRAV>(un, g, cflm);
-                            atomicMax(&cfl_sh, __float_as_int(__double2float_rd(cflm)));
+                            const float m = __double2float_rd(cflm);
+                            if (m > CFL_FLOOR) atomicMax(&cfl_sh, __float_as_int(m));
                         }
                     }
                 }
