@@ -600,7 +600,8 @@ def plane_section(ctx, ranks: Ranks, K: int, W: int, n=4096):
         hbm, _ = measured_hbm()
         s2 = 120 * n * n / (prof["ms_stage2"] / 1e3) / 1e9
         out[prec] = {"value": round(n * n * ranks.world * K / (ms / 1e3) / 1e6, 1), "unit": UNIT,
-                     "ms_per_step": round(ms / K, 4), "kernel": sim.kernel, "row_chunk": ky,
+                     "ms_per_step": round(ms / K, 4), "kernel": sim.kernel,
+                     "row_chunk": ky if sim.kernel == "tiled" else None,
                      "stage2_hbm_frac": round(s2 / hbm, 4)}
         sim.close()
     return out

@@ -142,13 +142,16 @@ int vb_grid_device_state(vb_grid *grid, double **dU);
  * grids the plane (float64) or row (VB_MIXED, nx >= 256 and even) kernel, the
  * rest the cell-centric one.  VB_KERNEL_CELL forces the cell-centric kernel,
  * VB_KERNEL_TILED requires a tiled one (3D: nx, ny multiples of 16, nz >= 2; 2D:
- * nx a multiple of 256).  VB_OPT_TILE_KZ: z planes per tiled work item.
+ * nx a multiple of 256).  Read back, it is the kernel that the grid's CFL steps
+ * take as it is set up now (boundary fluxes, gravity): VB_KERNEL_CELL, _TILED,
+ * _PLANE or _MARCH.  VB_OPT_TILE_KZ: z planes per tiled work item.
  * VB_OPT_TILE_TAPER: -1 (default) lets the autotuner choose whether the 3D
  * work queue's last z chunks taper (untuned: by the grid's size), 0 keeps
  * uniform chunks, 1 tapers in either precision.  Results do not depend on
  * any of these knobs. */
 enum { VB_OPT_KERNEL = 1, VB_OPT_TILE_KZ = 2, VB_OPT_TILE_TAPER = 3 };
-enum { VB_KERNEL_AUTO = 0, VB_KERNEL_CELL = 1, VB_KERNEL_TILED = 2 };
+enum { VB_KERNEL_AUTO = 0, VB_KERNEL_CELL = 1, VB_KERNEL_TILED = 2,
+       VB_KERNEL_PLANE = 3, VB_KERNEL_MARCH = 4 /* reported only */ };
 int vb_grid_set_option(vb_grid *grid, int option, int64_t value);
 int vb_grid_get_option(const vb_grid *grid, int option, int64_t *value);
 /* Autotuner (no counterpart in the reference): times the tiled kernel's

@@ -65,6 +65,8 @@ const VB_OPT_TILE_TAPER = Cint(3)
 const VB_KERNEL_AUTO = 0
 const VB_KERNEL_CELL = 1
 const VB_KERNEL_TILED = 2
+const VB_KERNEL_PLANE = 3  # reported only
+const VB_KERNEL_MARCH = 4  # reported only
 # gravity preconditioners
 const VB_GRAV_PRECOND_NONE = Int32(0)
 const VB_GRAV_PRECOND_MG = Int32(1)

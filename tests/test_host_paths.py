@@ -264,3 +264,46 @@ def test_gravity_enable_that_fails_leaves_what_was_there(fake, ctx, start):
         assert fake.fake_device_live() == base
         fails += 1
     assert fails >= 4
+
+
+CELL, TILED, PLANE, MARCH = 1, 2, 3, 4
+
+
+def kernel_of(L, g):
+    v = C.c_int64()
+    assert L.vb_grid_get_option(g, _lib.OPT_KERNEL, C.byref(v)) == 0
+    return v.value
+
+
+def test_the_reported_kernel_is_the_one_that_runs(fake, ctx):
+    """VB_OPT_KERNEL against the launches of a step, as boundary fluxes and
+    gravity come and go."""
+    names = {CELL: b"k_stage_generic", TILED: b"k_stage_tiled", PLANE: b"k_stage_plane", MARCH: b"k_march"}
+
+    def check(g, want):
+        assert kernel_of(fake, g) == want
+        fake.fake_reset()
+        assert fake.vb_run_steps_async(g, 1) == 0, error(fake)
+        ran = {k for k, n in names.items() if fake.fake_launched(n)}
+        assert ran == {want}
+
+    # (dims, precision, selector): plain, with outer fluxes, with interior ones, with gravity
+    for dims, prec, sel, kernels in [
+            ((64, 48), _lib.FP64, 0, (MARCH, CELL, CELL, CELL)),
+            ((64, 48), _lib.FP64, CELL, (CELL, CELL, CELL, CELL)),
+            ((300, 301), _lib.FP64, 0, (PLANE, CELL, CELL, CELL)),
+            ((256, 37888), _lib.FP64, 0, (PLANE, TILED, CELL, CELL)),
+            ((256, 64), _lib.FP64, TILED, (TILED, TILED, CELL, CELL)),
+            ((512, 1200), _lib.MIXED, 0, (TILED, TILED, CELL, CELL)),
+            ((48, 47, 48), _lib.FP64, 0, (TILED, TILED, CELL, TILED)),
+            ((48, 47, 48), _lib.MIXED, 0, (TILED, TILED, CELL, TILED)),
+            ((20, 12, 9), _lib.FP64, 0, (CELL, CELL, CELL, CELL))]:
+        g = make_grid(fake, ctx, dims, prec)
+        assert fake.vb_grid_set_option(g, _lib.OPT_KERNEL, sel) == 0, error(fake)
+        for mode, want in zip((_lib.BFLUX_OFF, _lib.BFLUX_OUTER, _lib.BFLUX_INTERIOR), kernels):
+            assert fake.vb_bflux_enable(g, mode) == 0, error(fake)
+            check(g, want)
+        assert fake.vb_bflux_enable(g, _lib.BFLUX_OFF) == 0
+        assert fake.vb_gravity_enable(g, C.byref(gravity_desc(_lib.BC_OUTFLOW, maxiter=0))) == 0, error(fake)
+        assert kernel_of(fake, g) == kernels[3]
+        fake.vb_grid_destroy(g)

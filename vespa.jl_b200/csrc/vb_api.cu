@@ -420,15 +420,22 @@ int sync_box(vb_grid *gr)
     return VB_OK;
 }
 
+// Whether the grid's stages take a tiled kernel.  3D ones carry self-gravity's
+// source; they record outer boundary fluxes themselves, while interior faces,
+// and boundary fluxes together with gravity, take the cell kernel.
+bool takes_tiled(const vb_grid *gr)
+{
+    const bool bf = gr->bflux_on, grav = gr->grav != nullptr;
+    return gr->tiled && !(bf && gr->bflux_interior) && !(bf && grav) && (!grav || gr->g.nd == 3) &&
+           !(gr->plane && !bf);
+}
+
 int stage(vb_grid *gr, int st, const double *Uin, const double *U0, double *Uout)
 {
     double *bf = gr->bflux_on ? gr->bflux : nullptr;
     double *bfi = bf && gr->bflux_interior ? gr->bflux + gr->bflux_outer_n : nullptr;
-    const bool grav = gr->grav != nullptr;  // self-gravity: 3D tiled kernels carry the source
-    // the tiled kernels record outer boundary fluxes themselves; interior
-    // faces, and boundary fluxes together with gravity, take the cell kernel
-    const bool use_tiled = gr->tiled && !bfi && !(bf && grav) && (!grav || gr->g.nd == 3) &&
-                           !(gr->plane && !bf);
+    const bool grav = gr->grav != nullptr;
+    const bool use_tiled = takes_tiled(gr);
     if (gr->slab && !use_tiled)
         return fail(VB_ENOTSUP, "a z-window (slab) grid steps with the tiled 3D kernels only");
     if (use_tiled) {
@@ -536,6 +543,17 @@ constexpr int64_t GRAPH_STEPS = 8;
 bool marches(const vb_grid *gr)
 {
     return gr->march && !gr->bflux_on && !gr->grav && !gr->slab;
+}
+
+// Which kernel a step queued now takes (VB_OPT_KERNEL's report): the choices of
+// queue_steps, stage and launch_stage_fp64.
+int step_kernel(const vb_grid *gr)
+{
+    if (marches(gr)) return VB_KERNEL_MARCH;
+    if (takes_tiled(gr)) return VB_KERNEL_TILED;
+    const bool plain = !gr->bflux_on && !gr->g.grav_g && !gr->cell_only;
+    return gr->precision == VB_FP64 && plain && vb::plane_f64_supported(gr->g) ? VB_KERNEL_PLANE
+                                                                                : VB_KERNEL_CELL;
 }
 
 uint64_t graph_key(const vb_grid *gr)
@@ -994,7 +1012,7 @@ int vb_grid_get_option(const vb_grid *gr, int option, int64_t *value)
 {
     if (!gr || !value) return fail(VB_EINVAL, "null argument");
     switch (option) {
-    case VB_OPT_KERNEL: *value = gr->tiled ? VB_KERNEL_TILED : VB_KERNEL_CELL; return VB_OK;
+    case VB_OPT_KERNEL: *value = step_kernel(gr); return VB_OK;
     case VB_OPT_TILE_KZ: *value = gr->kz; return VB_OK;
     case VB_OPT_TILE_TAPER: *value = grid_taper(gr) ? 1 : 0; return VB_OK;
     default: return fail(VB_EINVAL, "unknown option");

@@ -232,10 +232,13 @@ class Simulation:
     # -- kernel selection / tuning (results do not depend on these) --
     def set_kernel(self, kind: str = "auto", kz: Optional[int] = None,
                    taper: Optional[bool] = None) -> None:
-        """kind: "auto", "cell" (cell-centric kernel) or "tiled" (tiled 3D kernel).
-        kz: z planes per tiled work item.  taper: tapered (True) or uniform
-        (False) z chunks in the 3D work queue; None restores the default
-        (tapered for VB_MIXED grids)."""
+        """kind: "auto" (by size: small float64 1D and 2D grids march whole runs in
+        one launch, other float64 2D grids take the plane kernel, 3D and mixed 2D
+        grids a tiled kernel, the rest the cell-centric one), "cell" (the
+        cell-centric kernel) or "tiled" (a tiled kernel; sides must be whole
+        tiles).  kz: z planes (2D: rows) per tiled work item.  taper: tapered
+        (True) or uniform (False) z chunks in the 3D work queue; None restores the
+        default (the autotuner's choice, else by the grid's size)."""
         _lib.call("vb_grid_set_option", self.handle, _lib.OPT_KERNEL, _lib.KERNELS[kind])
         if kz is not None:
             _lib.call("vb_grid_set_option", self.handle, _lib.OPT_TILE_KZ, int(kz))
@@ -263,9 +266,11 @@ class Simulation:
 
     @property
     def kernel(self) -> str:
+        """The kernel that CFL steps take as the grid is set up now: "cell",
+        "tiled", "plane" or "march"."""
         v = C.c_int64()
         _lib.call("vb_grid_get_option", self.handle, _lib.OPT_KERNEL, C.byref(v))
-        return {1: "cell", 2: "tiled"}[v.value]
+        return {1: "cell", 2: "tiled", 3: "plane", 4: "march"}[v.value]
 
     def profile_step(self, nsteps: int = 5) -> dict:
         """Mean device milliseconds of each kernel of a CFL step (advances the state)."""
