@@ -160,8 +160,8 @@ int vb_grid_get_option(const vb_grid *grid, int option, int64_t *value);
  * tapered work queues -- keeps the fastest, and restores the state and clock.  The choice is
  * cached for the process per (device, dims, boundaries, precision) and later
  * grids of the same kind start from it.  Allocates one state-sized scratch
- * buffer for the duration of the call.  No-op (returns the current kz) when
- * the grid uses the cell-centric kernel. */
+ * buffer for the duration of the call.  No-op (returns the current kz and a
+ * time of 0) when the grid's steps take no tiled kernel. */
 int vb_grid_autotune(vb_grid *grid, int nsteps, int64_t *best_kz, double *best_ms_per_step);
 /* Simulation clock (sim.t, sim.step). */
 int vb_grid_set_time(vb_grid *grid, double t, int64_t step);

@@ -307,3 +307,25 @@ def test_the_reported_kernel_is_the_one_that_runs(fake, ctx):
         assert fake.vb_gravity_enable(g, C.byref(gravity_desc(_lib.BC_OUTFLOW, maxiter=0))) == 0, error(fake)
         assert kernel_of(fake, g) == kernels[3]
         fake.vb_grid_destroy(g)
+
+
+@pytest.mark.parametrize("dims,kind,prec", [((256, 37888), "auto", _lib.FP64), ((64, 48), "auto", _lib.FP64),
+                                            ((256, 64), "tiled", _lib.FP64), ((48, 47, 48), "auto", _lib.MIXED)])
+def test_autotune_times_only_grids_whose_steps_are_tiled(fake, ctx, dims, kind, prec):
+    g = make_grid(fake, ctx, dims, prec)
+    assert fake.vb_grid_set_option(g, _lib.OPT_KERNEL, _lib.KERNELS[kind]) == 0
+    kz, best, ms = C.c_int64(), C.c_int64(), C.c_double(7.0)
+    assert fake.vb_grid_get_option(g, _lib.OPT_TILE_KZ, C.byref(kz)) == 0
+    tiled = kernel_of(fake, g) == TILED
+    fake.fake_reset()
+    assert fake.vb_grid_autotune(g, 2, C.byref(best), C.byref(ms)) == 0, error(fake)
+    if tiled:
+        assert fake.fake_launched(b"k_stage_tiled") > 0 and ms.value > 0.0
+    else:
+        assert fake.fake_launched(b"k_") == 0 and ms.value == 0.0 and best.value == kz.value
+    fake.vb_grid_destroy(g)
+    g = make_grid(fake, ctx, dims, prec)  # and nothing is kept for later grids of its kind
+    kept = C.c_int64()
+    assert fake.vb_grid_get_option(g, _lib.OPT_TILE_KZ, C.byref(kept)) == 0
+    assert kept.value == best.value
+    fake.vb_grid_destroy(g)

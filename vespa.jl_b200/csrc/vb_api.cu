@@ -895,7 +895,8 @@ int vb_grid_autotune(vb_grid *gr, int nsteps, int64_t *best_kz, double *best_ms)
     if (!gr || nsteps < 1) return fail(VB_EINVAL, "bad argument");
     int rc = use(gr->ctx);
     if (rc) return rc;
-    if (!gr->tiled || gr->bflux_on || gr->grav) {
+    // nothing to tune where plain steps take another kernel than the tiled ones
+    if (!gr->tiled || gr->plane || gr->bflux_on || gr->grav) {
         if (best_kz) *best_kz = gr->kz;
         if (best_ms) *best_ms = 0.0;
         return VB_OK;
