@@ -138,8 +138,8 @@ int vb_grid_device_state(vb_grid *grid, double **dU);
 /* Kernel selection and tuning knobs (no counterpart in the reference, whose
  * per-face loop has no launch shape).  VB_OPT_KERNEL: VB_KERNEL_AUTO picks by
  * size: small float64 1D and 2D grids march whole runs in one launch, 3D grids
- * with nx, ny >= 16 (VB_MIXED: nx even) take a tiled kernel unless tiny, 2D
- * grids the plane (float64) or row (VB_MIXED, nx >= 256 and even) kernel, the
+ * with nx, ny >= 16 (VB_MIXED: nx even) take a tiled kernel unless tiny or thin
+ * across the tiles, 2D grids the plane (float64) or row (VB_MIXED, nx >= 256 and even) kernel, the
  * rest the cell-centric one.  VB_KERNEL_CELL forces the cell-centric kernel,
  * VB_KERNEL_TILED requires a tiled one (3D: nx, ny multiples of 16, nz >= 2; 2D:
  * nx a multiple of 256).  Read back, it is the kernel that the grid's CFL steps

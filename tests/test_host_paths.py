@@ -329,3 +329,14 @@ def test_autotune_times_only_grids_whose_steps_are_tiled(fake, ctx, dims, kind, 
     assert fake.vb_grid_get_option(g, _lib.OPT_TILE_KZ, C.byref(kept)) == 0
     assert kept.value == best.value
     fake.vb_grid_destroy(g)
+
+
+@pytest.mark.parametrize("dims,precision,kernel", [
+    ((17, 17, 512), _lib.FP64, CELL), ((18, 18, 512), _lib.MIXED, CELL),  # tiles would solve 3.5, 3.2 times the cells
+    ((20, 20, 512), _lib.FP64, CELL), ((20, 20, 512), _lib.MIXED, TILED),  # 2.6
+    ((33, 33, 100), _lib.FP64, TILED), ((16, 16, 512), _lib.FP64, TILED), ((16, 17, 512), _lib.FP64, TILED),
+    ((33, 47, 31), _lib.FP64, TILED), ((32, 32, 32), _lib.FP64, CELL)])
+def test_thin_boxes_keep_the_cell_kernel(fake, ctx, dims, precision, kernel):
+    g = make_grid(fake, ctx, dims, precision)
+    assert kernel_of(fake, g) == kernel
+    fake.vb_grid_destroy(g)
