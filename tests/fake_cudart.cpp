@@ -38,7 +38,7 @@ std::map<const void *, std::string> &names()  // the library's objects register 
 }
 std::map<std::string, long long> launched;
 std::string refused;
-long long nrefused = 0, plain_bytes = 0;
+long long nrefused = 0, plain_bytes = 0, graph_left = -1;  // graph launches until they fail; -1: never
 
 struct Config {
     dim3 grid, block;
@@ -97,12 +97,14 @@ void fake_reset(void)
     dev_fail_in = -1;
     pin_fail_always = dev_fail_always = false;
     nrefused = plain_bytes = 0;
+    graph_left = -1;
     refused.clear();
     launched.clear();
 }
 void fake_devices(int n) { devices = n; }
 void fake_clusters(int n) { clusters = n; }
 void fake_fail_device_alloc(long long in) { dev_fail_in = in; }   // 0: the next one
+void fake_fail_graph_launch(long long in) { graph_left = in; }
 void fake_fail_device(int always) { dev_fail_always = always != 0; }
 void fake_fail_pinned(int always) { pin_fail_always = always != 0; }
 long long fake_device_live(void) { return (long long)dev_live.size(); }
@@ -266,7 +268,12 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long 
     return *e = (cudaGraphExec_t)std::malloc(1), cudaSuccess;
 }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t e) { return std::free(e), cudaSuccess; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t)
+{
+    if (graph_left == 0) return err(cudaErrorUnknown);
+    if (graph_left > 0) --graph_left;
+    return cudaSuccess;
+}
 
 cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute a, int v)
 {

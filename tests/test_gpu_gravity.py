@@ -424,3 +424,26 @@ def test_cube_operator_takes_differences(vb, n, precond):
     assert iters == 0 and want > 0.1 / n
     # seven roundings a cell and the norm's sum
     assert abs(relres - want) <= 1e-13 * want, (relres, want)
+
+
+@pytest.mark.parametrize("precond", ["none", "mg"])
+def test_cube_iterations_past_a_pause(vb, precond):
+    """A limit beyond the iterations a cube's loop makes between looks by the
+    host: a state without a solution runs to the limit, and a converging solve
+    has the bits of one with a small limit."""
+    prob = P.smooth_random_problem((20, 20, 20), seed=3)
+    U0 = P.initial_state(prob)
+    phi = []
+    for maxiter in (400, 1500):
+        sim = make_sim(prob, U0)
+        grav = vb.enable_gravity(sim, G=1.0, tol=1e-10, maxiter=maxiter, precond=precond)
+        iters, relres = vb.solve_poisson(sim)
+        assert iters < 400 and relres <= 1e-10
+        phi.append(grav.phi)
+    assert np.array_equal(*phi)
+    U0[0, 7] = np.nan
+    for maxiter in (1, 511, 512, 513, 1500):
+        sim = make_sim(prob, U0)
+        vb.enable_gravity(sim, G=1.0, tol=1e-10, maxiter=maxiter, precond=precond)
+        iters, relres = vb.solve_poisson(sim)
+        assert iters == maxiter and np.isnan(relres)

@@ -34,7 +34,7 @@ def fake(tmp_path_factory):
         getattr(L, f).restype = C.c_longlong
     L.fake_launched.argtypes = [C.c_char_p]
     L.fake_refused.argtypes = [C.c_char_p, C.c_size_t]
-    L.fake_fail_device_alloc.argtypes = [C.c_longlong]
+    L.fake_fail_device_alloc.argtypes = L.fake_fail_graph_launch.argtypes = [C.c_longlong]
     L.fake_host_alloc.restype = C.c_void_p
     L.fake_host_alloc.argtypes = [C.c_size_t]
     L.fake_host_free.argtypes = [C.c_void_p]
@@ -340,3 +340,15 @@ def test_thin_boxes_keep_the_cell_kernel(fake, ctx, dims, precision, kernel):
     g = make_grid(fake, ctx, dims, precision)
     assert kernel_of(fake, g) == kernel
     fake.vb_grid_destroy(g)
+
+
+def test_long_cube_solves_come_back_to_the_host(fake, ctx):
+    """Iterations beyond 512 are queued a run at a time: the third run's failure
+    to start ends the solve (one run for the whole limit would not see it)."""
+    for maxiter, rc in ((512, 0), (10 ** 9, _lib.VB_ECUDA)):
+        g = make_grid(fake, ctx, (32, 32, 32))
+        assert fake.vb_gravity_enable(g, C.byref(gravity_desc(_lib.BC_PERIODIC, 1, maxiter))) == 0, error(fake)
+        fake.fake_fail_graph_launch(2)
+        assert fake.vb_gravity_solve(g, None, None) == rc
+        fake.fake_reset()
+        fake.vb_grid_destroy(g)

@@ -36,10 +36,15 @@ constexpr int GB = 256;  // threads per block
 constexpr int GP = 592;  // blocks (= partial sums) per reduction pass: 4 per SM, fixed
 constexpr int GP_SM = 4;  // the GP blocks fit in one wave only at <= 64 registers a thread
 constexpr int GRAPH_ITERS = 8;
+// Iterations of a cube's loop between looks by the host: a solve of no more (the
+// default limit is 500) needs none, a longer one cannot hold the device for the
+// whole of a large maxiter (a residual of NaN never meets the tolerance).
+constexpr long long CUBE_RUN = 512;
 
 struct GravCtrl {
     double rhobar, rsold, pAp, alpha, beta, bnorm, relres, mu, mgmu;
     long long iters, maxiter;
+    long long pause;  // iterations after which a cube's loop returns to the host
     int done;
     unsigned int ticket, ticket2;  // blocks past a grid_sum; zero between launches
     double tol;
@@ -614,8 +619,14 @@ __global__ void k_cube_init_final(GravCtrl *gc)
     gc->relres = sqrt(gc->rsold) / gc->bnorm;
     gc->iters = 0;
     gc->done = gc->maxiter <= 0 ? 1 : 0;
+    gc->pause = CUBE_RUN;
     gc->beta = 0.0;  // the first direction is z (mg_pcg.jl:188-191) or r
 }
+
+__global__ void k_cube_resume(GravCtrl *gc) { gc->pause = gc->iters + CUBE_RUN; }
+
+// the loop's condition after an iteration
+__device__ __forceinline__ unsigned cube_more(const GravCtrl *gc) { return !gc->done && gc->iters < gc->pause; }
 
 // k_accel on the cube: the same differences and quotients
 __global__ void __launch_bounds__(GB) k_cube_accel(const __grid_constant__ Geom g, int n,
@@ -708,7 +719,7 @@ __global__ void __launch_bounds__(GB) k_cube_update(int n, double *__restrict__ 
             gc->rsold = rr;
             if (gc->iters >= gc->maxiter) gc->done = 1;
         }
-        if (cg) cudaGraphSetConditional(more, gc->done ? 0 : 1);
+        if (cg) cudaGraphSetConditional(more, cube_more(gc));
     }
 }
 
@@ -780,7 +791,7 @@ __global__ void __launch_bounds__(GB) k_cube_post2(CubeP P, const double *__rest
         gc->rsold = rz;
         if (!start) {
             if (gc->iters >= gc->maxiter) gc->done = 1;
-            cudaGraphSetConditional(more, gc->done ? 0 : 1);
+            cudaGraphSetConditional(more, cube_more(gc));
         }
     }
 }
@@ -1333,17 +1344,19 @@ int vb::detail::gravity_solve(vb_grid *gr, int64_t *iters, double *relres)
             int rc = queue_precond(gr, gv, true, 0);
             if (rc) return rc;
         }
-        VB_CUDA(cudaGraphLaunch(gv->gexec, s));
-        gr->ctx->launches += gv->graph_launches;  // of one iteration: the count stays on the device
-        VB_CUDA(cudaMemcpyAsync(gv->hgc, gv->gc, sizeof(GravCtrl), cudaMemcpyDeviceToHost, s));
     }
     // the stop flag is set by convergence, p.Ap <= 0 or maxiter, so this ends
-    while (!gv->cube_n) {
+    for (;;) {
         VB_CUDA(cudaGraphLaunch(gv->gexec, s));
-        gr->ctx->launches += gv->graph_launches;
+        gr->ctx->launches += gv->graph_launches;  // a cube's: of one iteration, the count stays on the device
         VB_CUDA(cudaMemcpyAsync(gv->hgc, gv->gc, sizeof(GravCtrl), cudaMemcpyDeviceToHost, s));
+        if (gv->cube_n && gv->maxiter <= CUBE_RUN) break;
         VB_CUDA(cudaStreamSynchronize(s));
         if (gv->hgc->done) break;
+        if (gv->cube_n) {
+            k_cube_resume<<<1, 1, 0, s>>>(gv->gc);
+            VB_CHECK_LAUNCH(gr->ctx, 1);
+        }
     }
     if (gv->P.project_mean) {
         k_meanpart<<<GP, GB, 0, s>>>(g, gv->phi, gv->part);
