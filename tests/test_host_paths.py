@@ -352,3 +352,17 @@ def test_long_cube_solves_come_back_to_the_host(fake, ctx):
         assert fake.vb_gravity_solve(g, None, None) == rc
         fake.fake_reset()
         fake.vb_grid_destroy(g)
+
+
+def test_gravity_allocates_what_its_passes_use(fake, ctx):
+    """A cube forms its right-hand side on the fly, and levels that one block
+    runs in shared memory have no second array; walls bring the array back."""
+    g = make_grid(fake, ctx, (32, 32, 32))
+    base = fake.fake_device_live()
+    assert fake.vb_gravity_enable(g, C.byref(gravity_desc(_lib.BC_PERIODIC, precond=1))) == 0, error(fake)
+    # phi r p Ap field partials control; block partials, second direction, z z2;
+    # two arrays a level (32, 16, 8, 4), a third on the first
+    assert fake.fake_device_live() - base == 7 + 4 + 2 * 4 + 1
+    assert fake.vb_gravity_enable(g, C.byref(gravity_desc(_lib.BC_OUTFLOW))) == 0, error(fake)
+    assert fake.fake_device_live() - base == 7 + 4 + 2 * 4 + 1 + 1
+    fake.vb_grid_destroy(g)

@@ -1430,7 +1430,8 @@ int vb_gravity_enable(vb_grid *gr, const vb_gravity_desc *d)
         if (e == cudaSuccess && !*p) e = cudaMalloc(p, bytes);
     };
     const size_t n = (size_t)g.ncell * sizeof(double);
-    for (double **buf : {&gv->phi, &gv->b, &gv->r, &gv->p, &gv->Ap}) need(buf, n);
+    for (double **buf : {&gv->phi, &gv->r, &gv->p, &gv->Ap}) need(buf, n);
+    if (!cube) need(&gv->b, n);  // a cube's first pass forms its right-hand side where it reads it
     need(&gv->gacc, n * g.nd);
     need(&gv->part, sizeof(double) * 3 * vb::GP);
     need(&gv->gc, sizeof(vb::GravCtrl));
@@ -1456,8 +1457,12 @@ int vb_gravity_enable(vb_grid *gr, const vb_gravity_desc *d)
                 h *= 2.0;
             }
         }
-        for (auto &l : gv->lev)
-            for (double **buf : {&l.e, &l.b, &l.t}) need(buf, sizeof(double) * (size_t)l.n * l.n * l.n);
+        for (auto &l : gv->lev) {
+            const size_t bytes = sizeof(double) * (size_t)l.n * l.n * l.n;
+            need(&l.e, bytes);
+            need(&l.b, bytes);
+            if (l.n > vb::MG_BLOCK) need(&l.t, bytes);  // k_mg_bottom's levels sweep in shared memory
+        }
     }
     if (e == cudaSuccess && !gr->grav) {
         std::memset(gv->hgc, 0, sizeof(vb::GravCtrl));
