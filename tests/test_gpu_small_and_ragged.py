@@ -34,27 +34,38 @@ def run_pair(oracle, dims, lo, hi, steps, kz=None, tfinal=math.inf, sharp=True):
     return sim
 
 
-# 3D boxes of the float64 tile kernel: one tile, a shifted last tile that leaves
-# 1 or 15 cells of its own, odd rows, 2 planes, chunks shorter than the box
-@pytest.mark.parametrize("dims", [(16, 16, 2), (17, 19, 7), (31, 33, 20), (18, 17, 6), (35, 16, 16)])
+# 3D boxes around the float64 tile kernel's choice.  Below 148 blocks of cells the
+# cell kernel: one tile, 2 planes, odd sides.  Above it the tile kernel: a shifted
+# last tile that leaves 1 or 15 cells of its own along x, along y or both, one
+# tile along y, 2 planes, chunks shorter than the box
+CELL_BOXES = [(16, 16, 2), (17, 19, 7), (31, 33, 20), (18, 17, 6), (35, 16, 16)]
+TILE_BOXES = [(33, 47, 31), (31, 33, 40), (17, 31, 80), (35, 16, 70), (49, 63, 17), (160, 161, 2), (48, 32, 26)]
+
+
+@pytest.mark.parametrize("dims", CELL_BOXES + TILE_BOXES)
 @pytest.mark.parametrize("lo,hi", WALLS)
 @pytest.mark.parametrize("kz", [None, 3])
 def test_ragged_boxes_bit_identical(vb, oracle, dims, lo, hi, kz):
-    run_pair(oracle, dims, lo, hi, 3, kz if kz and kz < dims[2] else None)
+    sim = run_pair(oracle, dims, lo, hi, 3, kz if kz and kz < dims[2] else None)
+    assert sim.kernel == ("tiled" if dims in TILE_BOXES else "cell")
 
 
-def test_ragged_box_records_boundary_fluxes_and_gravity(vb, oracle):
-    prob = problem_from((19, 33, 9), [(0.0, 1.0)] * 3, (0, 2, 0), (2, 0, 2), 1.4, 0.4)
-    U0 = P.initial_state(P.smooth_random_problem((19, 33, 9), seed=3))
+@pytest.mark.parametrize("dims", [(19, 33, 9), (33, 47, 31), (17, 31, 80), (49, 34, 25)])
+@pytest.mark.parametrize("lo,hi", WALLS[1:])
+def test_ragged_box_records_boundary_fluxes_and_gravity(vb, oracle, dims, lo, hi):
+    prob = problem_from(dims, [(0.0, 1.0)] * 3, lo, hi, 1.4, 0.4)
+    U0 = P.initial_state(P.smooth_random_problem(dims, seed=3))
     out = []
     for kind in ("auto", "cell"):
         sim = make_sim(prob, U0)
         sim.set_kernel(kind)
         sim.bflux_enable()
+        assert sim.kernel == ("tiled" if kind == "auto" and dims[2] > 9 else "cell")
         vb.evolve(sim, max_steps=3)
         out.append((sim.state(), sim.bflux_read()))
         sim.bflux_enable(False)
         vb.enable_gravity(sim, G=0.3, bcs=P.Outflow, tol=1e-10, project_mean=True)
+        assert sim.kernel == ("tiled" if kind == "auto" and dims[2] > 9 else "cell")
         vb.evolve(sim, max_steps=2)
         out[-1] += (sim.state(),)
     for a, b in zip(*out):
@@ -62,12 +73,13 @@ def test_ragged_box_records_boundary_fluxes_and_gravity(vb, oracle):
 
 
 # 1D and 2D grids marched by one cluster: 4 cells, one block, the largest
-# cluster, uneven slabs, thin slabs (halo rows from two blocks away)
-@pytest.mark.parametrize("dims", [(4,), (5,), (255,), (257,), (3000,), (4, 4), (17, 33), (100, 31),
-                                  (31, 100), (8, 300), (300, 8), (112, 113)])
+# cluster, uneven slabs, thin slabs (halo rows from two blocks away), slabs that
+# just fit in shared memory; 112 x 113 does not and takes the plane kernel
+@pytest.mark.parametrize("dims", [(4,), (5,), (255,), (257,), (3000,), (18000,), (4, 4), (17, 33), (100, 31),
+                                  (31, 100), (8, 300), (300, 8), (112, 112), (112, 113)])
 @pytest.mark.parametrize("lo,hi", WALLS)
 def test_marched_grids_bit_identical(vb, oracle, dims, lo, hi):
-    run_pair(oracle, dims, lo, hi, 7)
+    assert run_pair(oracle, dims, lo, hi, 7).kernel == ("plane" if dims == (112, 113) else "march")
 
 
 def test_march_stops_resumes_and_reports(vb, oracle):
@@ -89,11 +101,13 @@ def test_march_stops_resumes_and_reports(vb, oracle):
     assert "VB_ENONFINITE" in str(e.value)
 
 
-# 2D grids of the plane kernel (beyond the march's size): ragged both ways
-@pytest.mark.parametrize("dims", [(129, 145), (256, 128), (1000, 17), (16, 900), (400, 401), (512, 512)])
+# 2D grids of the plane kernel (beyond the march's size, all but 16 x 900): ragged
+# both ways, one tile across
+@pytest.mark.parametrize("dims", [(129, 145), (256, 128), (1000, 17), (16, 900), (16, 2500), (2500, 31), (400, 401),
+                                  (512, 512)])
 @pytest.mark.parametrize("lo,hi", WALLS)
 def test_plane_grids_bit_identical(vb, oracle, dims, lo, hi):
-    run_pair(oracle, dims, lo, hi, 3)
+    assert run_pair(oracle, dims, lo, hi, 3).kernel == ("march" if dims == (16, 900) else "plane")
 
 
 # operands outside the range of the divisions' fast form, zeros among them
@@ -137,7 +151,10 @@ def test_muscl_general_forms_bit_identical(vb, oracle, case):
 # the mixed kernels on shifted tiles and segments: near the float64 result, and
 # conserving as on whole tiles (each updated cell takes both fluxes of a face
 # from one solve)
-@pytest.mark.parametrize("dims", [(18, 34, 9), (48, 47, 60), (258, 20), (510, 130), (20, 18, 130)])
+MIXED_TILED = [(48, 47, 60), (34, 18, 80), (18, 31, 80), (50, 62, 17), (258, 1200), (510, 1190), (766, 800)]
+
+
+@pytest.mark.parametrize("dims", [(18, 34, 9), (258, 20), (510, 130), (20, 18, 130)] + MIXED_TILED)
 @pytest.mark.parametrize("per", [True, False])
 def test_ragged_mixed_grids(vb, dims, per):
     nd = len(dims)
@@ -146,6 +163,7 @@ def test_ragged_mixed_grids(vb, dims, per):
     U0 = P.initial_state(P.smooth_random_problem(dims, seed=4))
     a, b = make_sim(prob, U0), make_sim(prob, U0, "mixed")
     t0 = np.array(vb.conserved_totals(b))
+    assert b.kernel == ("tiled" if dims in MIXED_TILED else "cell")
     for s in (a, b):
         vb.evolve(s, max_steps=10)
     l1 = np.sum(np.abs(a.state()[0] - b.state()[0])) / np.sum(np.abs(a.state()[0]))
