@@ -32,6 +32,8 @@ CASES = {
     "smooth3d_8x6x5": lambda vb: vb.smooth_random_problem((8, 6, 5)),
     "smooth1d_40": lambda vb: vb.smooth_random_problem((40,)),
     "smooth2d_3x2": lambda vb: vb.smooth_random_problem((3, 2)),
+    "smooth2d_2x4737": lambda vb: vb.smooth_random_problem((2, 4737)),  # too thin for the tiles
+    "smooth2d_9x4737": lambda vb: vb.smooth_random_problem((9, 4737)),
 }
 
 

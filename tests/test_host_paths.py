@@ -69,18 +69,26 @@ def make_grid(L, ctx, dims, precision=_lib.FP64, bc=P.Periodic):
 
 def test_adjoint_scratch_matches_the_kernels_that_use_it(fake, ctx):
     """Only 2D grids whose stage keeps its face adjoints on chip go without the
-    three scratch arrays; a longer side takes the kernels that write them."""
+    three scratch arrays; longer or thinner ones take the kernels that write
+    them."""
     live = []
-    for dims in ((64, 4), (1, 2 ** 24 + 1)):
+    for dims, on_chip in (((64, 4), True), ((4, 4000), True), ((4, 65536), False), ((65536, 1), False),
+                          ((8, 65536), True), ((1, 2 ** 24 + 1), False)):
         g = make_grid(fake, ctx, dims)
         before = fake.fake_device_live()
         a = C.c_void_p()
         assert fake.vb_adjoint_create(g, 4, 2, C.byref(a)) == 0, error(fake)
         live.append(fake.fake_device_live() - before)
+        assert live[-1] == live[0] + (0 if on_chip else 3), dims
+        if max(dims) < 2 ** 24:
+            U = np.ones((5, int(np.prod(dims))))
+            fake.fake_reset()
+            assert fake.vb_adjoint_step(a, 0.1, _lib.dptr(U), _lib.dptr(U)) == 0, error(fake)
+            assert (fake.fake_launched(b"k_adj_plane") > 0) == on_chip
+            assert (fake.fake_launched(b"k_adj_face") > 0) == (not on_chip)
         fake.vb_adjoint_destroy(a)
         assert fake.fake_device_live() == before
         fake.vb_grid_destroy(g)
-    assert live[1] == live[0] + 3
 
 
 def faces(nf):

@@ -208,10 +208,17 @@ int launch_stage_mixed(const Geom &g, int stage, const double *Uin, const double
 //   out = 0.5*lam + (M ? M : 0) - invV * (dD/dU)^T mu,  mu = M ? M : 0.5*lam,
 // at the state U; gL/gR (2*nd*5*ncell doubles) and code (nd*ncell) are scratch,
 // which 2D grids whose face adjoints stay on chip do not need (adj_on_chip: the
-// one condition for both; such a side's tile coordinates fit its 32-bit ints).
+// one condition for both).  Those are sides that fit the tiles' 32-bit
+// coordinates, where the 16 x 16 tiles run in one round of two blocks an SM (40
+// stages of 4 x 4000 cells, 250 tiles: 0.58 ms, face and cell kernels 0.74) or
+// hold at most twice the grid's cells (17 x 4000, 1.9 times: 0.94 and 1.05; 8 x
+// 65536, 2.0: 5.45 and 5.31; but 4 x 65536, 4.0: 5.35 and 2.59, 1 x 65536: 6.15 and
+// 1.07).
 inline bool adj_on_chip(const Geom &g)
 {
-    return g.nd == 2 && g.n[0] <= (1 << 24) && g.n[1] <= (1 << 24);
+    if (g.nd != 2 || g.n[0] > (1 << 24) || g.n[1] > (1 << 24)) return false;
+    const int64_t tiles = ((g.n[0] + 15) / 16) * ((g.n[1] + 15) / 16);
+    return tiles <= 2 * 148 || 128 * tiles <= g.ncell;
 }
 int launch_adj_stage(const Geom &g, const double *U, const double *lam, const double *M,
                      double invV, double *gL, double *gR, uint16_t *code, double *out,
