@@ -206,6 +206,7 @@ k_adj_plane(const __grid_constant__ Geom g, const double *__restrict__ U, const 
             pos = k < H ? k : k + T;
         }
         const int64_t l = cell(a, line, pos);
+        if (!VB_DCHECK(l >= 0 && l < nc && line * S + pos < NW && line2 * S + pos2 < NW)) continue;  // check build only
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
             cp_async8(&S_.mu[a][k][line * S + pos], mu + k * nc + l);
@@ -255,8 +256,8 @@ k_adj_plane(const __grid_constant__ Geom g, const double *__restrict__ U, const 
     // the own cell's inputs of the last part arrive while others solve faces
     static_assert(T * T <= NTH, "one cell a thread");
     const int lx = t & (T - 1), ly = t / T, x = x0 + lx, y = y0 + ly;
-    const bool own = t < T * T && x < nx && y < ny;
     const int64_t lin = (int64_t)x + (int64_t)nx * y;
+    const bool own = t < T * T && x < nx && y < ny && VB_DCHECK(lin >= 0 && lin < nc);
     double u[5], v[5];
     if (own)
 #pragma unroll

@@ -524,15 +524,18 @@ __device__ __forceinline__ void cube_cells(int n, V &&v, F &&f)
         for (int z = z0; z < z1; ++z) {
             const int i = base + z * nn;
             const D2 hi = v(At<D2>{base + (z + 1 < n ? z + 1 : 0) * nn});
-            const D2 sy = cube_axis<DIFF>(c, v(At<D2>{i + ym}), v(At<D2>{i + yp}));
+            // check build only: every cell read and written lies in the cube
+            const bool ok = VB_DCHECK(i >= 0 && i + 1 < n * nn && i + ym >= 0 && i + ym + 1 < n * nn && i + yp >= 0 &&
+                                      i + yp + 1 < n * nn && i + xe >= 0 && i + xe < n * nn);
+            const D2 sy = ok ? cube_axis<DIFF>(c, v(At<D2>{i + ym}), v(At<D2>{i + yp})) : c;
             double l = __shfl_up_sync(0xffffffffu, c.y, 1, 16), r = __shfl_down_sync(0xffffffffu, c.x, 1, 16);
-            if (first || last) {
+            if ((first || last) && ok) {
                 const double e = v(At<double>{i + xe});
                 if (first) l = e;
                 else r = e;
                 if (first && last) r = v(At<double>{i + (x + 2 < n ? 2 : 2 - n)});
             }
-            if (in) f(At<D2>{i}, c, cube_axis<DIFF>(c, D2{l, c.x}, D2{c.y, r}), sy, cube_axis<DIFF>(c, lo, hi));
+            if (in && ok) f(At<D2>{i}, c, cube_axis<DIFF>(c, D2{l, c.x}, D2{c.y, r}), sy, cube_axis<DIFF>(c, lo, hi));
             lo = c;
             c = hi;
         }
@@ -545,6 +548,8 @@ __device__ __forceinline__ void cube_cells(int n, V &&v, F &&f)
         double lo = v(At<double>{base + (z0 > 0 ? z0 - 1 : n - 1) * nn}), c = v(At<double>{base + z0 * nn});
         for (int z = z0; z < z1; ++z) {
             const int i = base + z * nn;
+            if (!VB_DCHECK(i >= 0 && i < n * nn && i + xm >= 0 && i + xp < n * nn && i + ym >= 0 && i + yp < n * nn))
+                return;  // check build only
             const double hi = v(At<double>{base + (z + 1 < n ? z + 1 : 0) * nn});
             f(At<double>{i}, c, cube_axis<DIFF>(c, v(At<double>{i + xm}), v(At<double>{i + xp})),
               cube_axis<DIFF>(c, v(At<double>{i + ym}), v(At<double>{i + yp})), cube_axis<DIFF>(c, lo, hi));

@@ -155,6 +155,7 @@ k_march(const __grid_constant__ Geom g, double *__restrict__ U, Ctrl *ctrl, long
             int o = ho, is = hsrc, id = hdst;
             bool flip = hflip;
             if (i != t) halo_place(i, o, is, id, flip);
+            if (!VB_DCHECK(o >= 0 && o < C && is >= 0 && is < ws && id >= 0 && id < ws)) continue;  // check build only
             const double *src = (C > 1 ? cl.map_shared_rank(w, o) : w) + is;
             double v[5];
 #pragma unroll
@@ -206,6 +207,9 @@ k_march(const __grid_constant__ Geom g, double *__restrict__ U, Ctrl *ctrl, long
         for (int j = t; j < nf; j += T) {
             const Face f = j == t ? face0 : face_place(j);
             const bool isx = ND == 1 || (f.flags & 16);
+            if (!VB_DCHECK(f.o[0] >= 0 && f.o[1] >= 0 && f.o[2] >= 0 && f.o[3] >= 0 && f.o[0] < ws && f.o[1] < ws &&
+                           f.o[2] < ws && f.o[3] < ws && f.out >= 0 && f.out < (ND == 2 && isx ? xs : ys)))
+                continue;  // check build only
             // normal and first tangential velocity: fields 1, 2 along x, 2, 1 along y
             const int fn = isx ? 1 : 2, ft = isx ? 2 : 1;
             double Lw[5], Rw[5], F[5];
@@ -265,6 +269,7 @@ k_march(const __grid_constant__ Geom g, double *__restrict__ U, Ctrl *ctrl, long
     double m[ND] = {};
     for (int c = t; c < own; c += T) {
         double u[5];
+        if (!VB_DCHECK((int64_t)ra * L + c < g.ncell && c < us)) continue;  // check build only
 #pragma unroll
         for (int f = 0; f < 5; ++f) {
             u[f] = U[f * g.ncell + (int64_t)ra * L + c];
@@ -331,7 +336,7 @@ k_march(const __grid_constant__ Geom g, double *__restrict__ U, Ctrl *ctrl, long
         time = time + dt;
         step = step + 1;
     }
-    for (int c = t; c < own; c += T)
+    for (int c = t; c < own && VB_DCHECK((int64_t)ra * L + c < g.ncell); c += T)
 #pragma unroll
         for (int f = 0; f < 5; ++f) U[f * g.ncell + (int64_t)ra * L + c] = u0[f * us + c];
     if (rank == 0 && t == 0) {
