@@ -461,9 +461,12 @@ struct CubeP {
 };
 
 // planes of a thread's chunk: long ones re-read fewer planes, short ones keep
-// the chip full (and the chain of dependent planes short) on small levels
+// the chip full (and the chain of dependent planes short) on small levels.  Odd
+// cubes, one cell a thread, want longer ones before even ones do (CG, us an
+// iteration with 2, 5 and 8 planes: 71^3 20.4, 16.8, 19.6; 95^3 25.8, 21.3, 21.7).
 __host__ __device__ inline int cube_kz(int n)
 {
+    if ((n & 1) && n >= 64 && n < 96) return 5;
     return n >= 512 ? 64 : n >= 192 ? 16 : n >= 96 ? 8 : n >= 48 ? 2 : 1;
 }
 
@@ -1198,7 +1201,12 @@ int queue_cube_iteration(vb_grid *gr, vb_gravity *gv, cudaGraphConditionalHandle
 }
 
 // The cube's iterations as one graph: a WHILE node whose body is one iteration
-// and whose condition the iteration's last reduction sets from the stop flag.
+// (CG: 8, each of which returns at once after the stop) and whose condition the
+// last reduction of each sets from the stop flag.  Going round the loop takes 4
+// us, which the two launches of a CG iteration on a small cube show: 19.1, 17.0,
+// 15.9, 15.4 and 15.1 us an iteration at 48^3 with 1, 2, 4, 8 and 16 in the body
+// (five plain launches: 16.0), 245 and 242 at 256^3 with 1 and 8.
+constexpr int CG_BODY = 8;
 int capture_cube(vb_grid *gr, vb_gravity *gv)
 {
     cudaStream_t s = gr->ctx->stream;
@@ -1221,7 +1229,8 @@ int capture_cube(vb_grid *gr, vb_gravity *gv)
     int rc = VB_OK;
     if (e == cudaSuccess) {
         const int64_t before = gr->ctx->launches;
-        rc = queue_cube_iteration(gr, gv, h);
+        const int body = gv->precond == VB_GRAV_PRECOND_MG ? 1 : CG_BODY;
+        for (int k = 0; k < body && !rc; ++k) rc = queue_cube_iteration(gr, gv, h);
         cudaGraph_t out = nullptr;
         e = cudaStreamEndCapture(s, &out);
         gv->graph_launches = gr->ctx->launches - before;
