@@ -300,7 +300,8 @@ def test_the_reported_kernel_is_the_one_that_runs(fake, ctx):
             ((64, 48), _lib.FP64, 0, (MARCH, CELL, CELL, CELL)),
             ((64, 48), _lib.FP64, CELL, (CELL, CELL, CELL, CELL)),
             ((300, 301), _lib.FP64, 0, (PLANE, CELL, CELL, CELL)),
-            ((256, 37888), _lib.FP64, 0, (PLANE, TILED, CELL, CELL)),
+            ((512, 1184), _lib.FP64, 0, (PLANE, TILED, CELL, CELL)),
+            ((512, 1176), _lib.FP64, 0, (PLANE, CELL, CELL, CELL)),
             ((256, 64), _lib.FP64, TILED, (TILED, TILED, CELL, CELL)),
             ((512, 1200), _lib.MIXED, 0, (TILED, TILED, CELL, CELL)),
             ((48, 47, 48), _lib.FP64, 0, (TILED, TILED, CELL, TILED)),
@@ -317,7 +318,7 @@ def test_the_reported_kernel_is_the_one_that_runs(fake, ctx):
         fake.vb_grid_destroy(g)
 
 
-@pytest.mark.parametrize("dims,kind,prec", [((256, 37888), "auto", _lib.FP64), ((64, 48), "auto", _lib.FP64),
+@pytest.mark.parametrize("dims,kind,prec", [((512, 1184), "auto", _lib.FP64), ((64, 48), "auto", _lib.FP64),
                                             ((256, 64), "tiled", _lib.FP64), ((48, 47, 48), "auto", _lib.MIXED)])
 def test_autotune_times_only_grids_whose_steps_are_tiled(fake, ctx, dims, kind, prec):
     g = make_grid(fake, ctx, dims, prec)

@@ -218,18 +218,18 @@ int64_t tiles_per_chunk(const vb::Geom &g)
 // and 2.75 mixed.  (17 x 17 x 1730, 3.5 per cell: tiles 401 us a step, cell kernel
 // 315; 20 x 20 x 1250, 2.56: 328 and 308, mixed 135 and 143; 33 x 33 x 459, 2.1:
 // 266 and 318; 18 x 18 x 6173 mixed, 3.2: 529 and 571, but 159 and 145 at a
-// quarter of its length.)  2D mixed: when a chunk of at least 8
-// rows gives every persistent block an item.  2D float64: the plane kernel steps
-// faster at every size (vb_stage_plane_f64.cuh) and `plane` has it take them; the
-// choice made here is for steps that record boundary fluxes, which it does not:
-// the marching kernel where 32-row chunks give each block four items.
+// quarter of its length.)  2D: when a chunk of at least 8 rows gives every
+// persistent block an item.  In float64 the plane kernel steps faster at every
+// size (vb_stage_plane_f64.cuh) and `plane` has it take them; the choice made here
+// is then for steps that record boundary fluxes, which it does not (row kernel
+// and cell kernel: 512 x 1184 104 and 191 us a step, 512 x 2048 198 and 351, but
+// 256 x 512, 64 items, 88 and 52).
 bool tiled_auto(const vb::Geom &g, int precision)
 {
     if (!vb::tiled_any(g, precision)) return false;
     if (g.nd == 3)
         return g.ncell > 148 * 256 &&
                256 * 4 * tiles_per_chunk(g) <= (precision == VB_FP64 ? 9 : 11) * g.n[0] * g.n[1];
-    if (precision == VB_FP64) return tiles_per_chunk(g) * ((vb::march_extent(g) + 31) / 32) >= 4 * 296;
     return tiles_per_chunk(g) * ((vb::march_extent(g) + 7) / 8) >= 296;
 }
 
