@@ -643,8 +643,8 @@ def bflux_section(ctx, ranks: Ranks, K: int, W: int, n=256):
 def gravity_section(ctx, ranks: Ranks, K: int, W: int, n=256, cpu_n=64):
     """Self-gravity (src/gravity.jl) on the 256^3 cube: (a) a cold Poisson solve
     (phi = 0, tol 1e-8) of a white-noise density with plain CG (the reference's
-    default), whose iterations stream 88 B/cell (matvec r p w Ap, update r phi
-    p r Ap w phi r, direction r p w p), and with the multigrid preconditioner
+    default), whose iterations stream 80 B/cell (direction and matvec r r p w p
+    Ap, update r phi p r Ap w phi r), and with the multigrid preconditioner
     (precond = :mg, ext/mg_pcg.jl); (b) K evolve! steps with gravity after W
     warm-up steps (one warm-started solve per step, stages on the tiled
     kernels with the source): both precisions with the preconditioner, float64
@@ -676,10 +676,10 @@ def gravity_section(ctx, ranks: Ranks, K: int, W: int, n=256, cpu_n=64):
         per_it = ms / its
         rec = {"iters": its, "relres": rr, "ms": round(ms, 3), "ms_per_iteration": round(per_it, 4)}
         if pc == "none":
-            bw = 88 * n ** 3 / (per_it / 1e3) / 1e9
+            bw = 80 * n ** 3 / (per_it / 1e3) / 1e9
             rec.update({"Mcell_iterations_per_s": round(n ** 3 / (per_it / 1e3) / 1e6, 1),
                         "achieved_gbs": round(bw, 1), "hbm_frac": round(bw / hbm, 4),
-                        "bytes_per_cell_iteration": 88})
+                        "bytes_per_cell_iteration": 80})
         out[f"cold_solve_{pc}"] = rec
         sim.close()
     for prec, pc in (("fp64", "mg"), ("mixed", "mg"), ("fp64", "none")):

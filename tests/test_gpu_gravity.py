@@ -4,7 +4,8 @@ test/test_gravity_hydro.jl).
 
 What is bit-identical and what is not:
 - the operator A x = -lap(x) V: bit-identical to the oracle (the reference's
-  CSR row order, every operation rounded separately);
+  CSR row order, every operation rounded separately); inside a periodic cube's
+  solve the same differences are summed axis by axis;
 - the field g = -grad phi, the stage source and the free-fall dt: bit-identical
   for a given phi;
 - a Poisson solve: the device's CG inner products are tree sums, the

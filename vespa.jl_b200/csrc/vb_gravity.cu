@@ -7,7 +7,8 @@
 // updates round every product and sum separately, like the reference's Julia
 // loops.  The operator row is summed in the reference's CSR order
 // (_assemble_poisson_struct, src/gravity.jl:514-545), so A x is bit-identical
-// to the reference's _lap_csr_cpu! (325-334).  The CG inner products are
+// to the reference's _lap_csr_cpu! (325-334); the passes of periodic cubes sum the
+// same differences axis by axis.  The CG inner products are
 // deterministic block-tree sums (fixed partial count and order) rather than
 // the reference's serial sums, so a solve matches the reference's to the
 // solver tolerance, not bit for bit.

@@ -7,10 +7,11 @@
 // and runs the steps in a loop: 3.6 us and 8.7 us a step.  Of 17 k cycles at
 // 64 x 64 the face solves take 7.5 k (the float64 pipes of 16 SMs), the cluster
 // barriers 3.6 k, both updates 3.6 k.  Each block owns a slab of rows (1D: of
-// cells), about 256 cells; two cluster barriers a step separate the stages,
-// the two rows of halo on each side are read from the neighbours' shared
-// memory, and the CFL maximum rides on the first barrier.  One thread solves
-// each face once (hllc_frame with its quotients side by side).
+// cells), about 256 cells; two cluster barriers a step (a grid of one block: two
+// block barriers) separate the stages, the two rows of halo on each side are read
+// from the neighbours' shared memory, and the CFL maximum rides on the first
+// barrier.  One thread solves each face once (hllc_frame with its quotients side
+// by side).
 //
 // Same operations and per-cell accumulation order as the cell-centric kernel,
 // compiled with -fmad=false: bit-identical to it and to the oracle.

@@ -82,7 +82,8 @@ __device__ __forceinline__ T total_energy(const T W[5], T g)
 // The corrected value is off the exact one by at most 2^-104 of it before its
 // rounding, so it could go wrong only where the exact one lies that close to a
 // midpoint between two numbers (one operand pair in 2^50); of 7.5 10^9 operands,
-// a third of them built to lie as close to one as any can, none did.
+// a third of them built to lie as close to one as any can, none did
+// (tests/test_gpu_quotients.py builds and compares such operands).
 __device__ __forceinline__ double rcp64(double b)
 {
     double y;
