@@ -375,3 +375,17 @@ def test_gravity_allocates_what_its_passes_use(fake, ctx):
     assert fake.vb_gravity_enable(g, C.byref(gravity_desc(_lib.BC_OUTFLOW))) == 0, error(fake)
     assert fake.fake_device_live() - base == 7 + 4 + 2 * 4 + 1 + 1
     fake.vb_grid_destroy(g)
+
+
+@pytest.mark.parametrize("precision", [_lib.FP64, _lib.MIXED])
+def test_the_starting_chunk_fits_the_grid(fake, ctx, precision):
+    """The chunk that a grid starts with can be set on a grid of its kind."""
+    for dims in [(512, 512, 4), (640, 512, 3), (768, 768, 2), (512, 512, 7), (256, 256, 8), (48, 48, 48), (16, 16, 300),
+                 (2048, 2), (4096, 5), (2048, 300), (512, 9)]:
+        g = make_grid(fake, ctx, dims, precision)
+        kz = C.c_int64()
+        assert fake.vb_grid_get_option(g, _lib.OPT_TILE_KZ, C.byref(kz)) == 0
+        assert kz.value <= dims[-1], (dims, kz.value)
+        if kernel_of(fake, g) == TILED:
+            assert fake.vb_grid_set_option(g, _lib.OPT_TILE_KZ, kz.value) == 0, (dims, error(fake))
+        fake.vb_grid_destroy(g)

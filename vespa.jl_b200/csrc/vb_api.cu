@@ -279,10 +279,10 @@ int grid_default_kz(const vb::Geom &g, int precision, bool *taper)
     *taper = true;
     if (q >= 24.0) return q >= 48.0 && ext >= 48 ? 48 : ext >= 24 ? 24 : (int)ext;
     const double prologue = precision == VB_MIXED ? 4.0 : 1.5;
-    int best_kz = 8;
+    int best_kz = (int)std::min<int64_t>(8, ext);
     double best = INFINITY;
     for (int c = 0; c < 3; ++c) {
-        const int kz = c == 0 ? 8 : 16;
+        const int kz = c == 0 ? best_kz : 16;
         if (kz > ext) continue;
         int nchu = 0;
         const int nch = vb::chunk_count((int)ext, kz, c == 2, &nchu);
