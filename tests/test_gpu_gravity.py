@@ -404,7 +404,7 @@ def test_mg_refuses_unsupported_grids(vb):
     assert e.value.status == 6
 
 
-@pytest.mark.parametrize("n", [5, 6, 33, 34, 64])
+@pytest.mark.parametrize("n", [5, 6, 33, 34, 64, 71])
 @pytest.mark.parametrize("precond", ["none", "mg"])
 def test_cube_operator_takes_differences(vb, n, precond):
     """The cube's A phi on a potential far from zero: its differences are exact
@@ -448,3 +448,19 @@ def test_cube_iterations_past_a_pause(vb, precond):
         vb.enable_gravity(sim, G=1.0, tol=1e-10, maxiter=maxiter, precond=precond)
         iters, relres = vb.solve_poisson(sim)
         assert iters == maxiter and np.isnan(relres)
+
+
+@pytest.mark.parametrize("n,precond", [(67, "none"), (95, "none"), (96, "none"), (190, "mg")])
+def test_cube_solutions_satisfy_the_general_operator(vb, n, precond):
+    """Converged potentials of cubes whose chunks of planes end unevenly, put
+    through the row-order operator: the residual is the solver's, up to what
+    rounding phi itself to 53 bits leaves (some n^2 parts in 2^53)."""
+    prob = P.smooth_random_problem((n, n, n), seed=n)
+    U0 = P.initial_state(prob)
+    sim = make_sim(prob, U0)
+    grav = vb.enable_gravity(sim, G=1.0, tol=1e-9, maxiter=500, precond=precond)
+    iters, relres = vb.solve_poisson(sim)
+    assert 0 < iters < 500 and relres <= 1e-9
+    b = -4 * np.pi * (U0[0] - U0[0].mean()) / n ** 3
+    r = b - vb.apply_laplacian(sim, grav, grav.phi)
+    assert np.linalg.norm(r) <= (2e-9 + n * n * 2.0 ** -52) * np.linalg.norm(b)

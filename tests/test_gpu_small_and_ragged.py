@@ -189,8 +189,10 @@ def test_large_face_batches_bit_identical(vb, oracle):
 
 
 # cubes whose coarsest level is the base grid, odd and too large for one block,
-# or reached through levels in one block; plain CG through the same graph
-@pytest.mark.parametrize("n,precond", [(4, "mg"), (7, "mg"), (16, "mg"), (17, "mg"), (34, "mg"), (20, "mg"),
+# or reached through levels in one block; cubes whose neighbours are the cell
+# itself or one another; plain CG through the same graph
+@pytest.mark.parametrize("n,precond", [(1, "none"), (1, "mg"), (2, "none"), (2, "mg"), (3, "mg"), (6, "none"),
+                                       (4, "mg"), (7, "mg"), (16, "mg"), (17, "mg"), (34, "mg"), (20, "mg"),
                                        (40, "mg"), (5, "none"), (33, "none")])
 def test_cube_solves_reach_the_oracle(vb, oracle, n, precond):
     prob = P.smooth_random_problem((n, n, n), seed=n)

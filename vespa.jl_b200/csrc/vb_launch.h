@@ -44,8 +44,8 @@ struct alignas(64) BoxDesc {
 // down), a smaller one is taken whole.  With kz >= 16 every piece then has 8
 // to kz planes and the last one fewer than 16, so that the work queue ends on
 // short items and the blocks finish together.  Single grids take the form the
-// autotuner timed faster (the tapered one at 256^3 in both precisions; a
-// VB_MIXED grid defaults to it); batches keep the uniform chunks.
+// autotuner timed faster (the tapered one at 256^3 in both precisions), untuned
+// ones by their size; batches keep the uniform chunks.
 __host__ __device__ inline int chunk_tail_piece(int r, int kz)
 {
     const int p = r >= 16 ? r / 2 : r;
